@@ -34,12 +34,14 @@ struct NearArg {
   const long long* near_zoff;
   const Z* near_z;
   const double2* x;
+  const double* xscale;  // device factor applied to x; null: 1
   double2* w;
   int N;
 };
 
-// w = Z_near x: rows t and N + t of the near field, one warp per RWG; the
-// entries and the arithmetic in the storage type Z (complex128 or complex64).
+// w = Z_near (xscale x): rows t and N + t of the near field, one warp per RWG;
+// the entries and the arithmetic in the storage type Z (complex128 or
+// complex64). x is scaled in FP64 as it is read.
 template <class Z>
 __global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
   const int lane = threadIdx.x & 31;
@@ -50,10 +52,11 @@ __global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
   const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
   const int tl = r - a.leaf_ptr[b];
   const Z* Zr = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
+  const double sc = a.xscale ? *a.xscale : 1.0;
   Z nJ = Cx<Z>::zero(), nM = Cx<Z>::zero();
   for (int j = lane; j < ns; j += 32) {
     const int s = a.near_src[s0 + j];
-    const Z xJ = Cx<Z>::from(a.x[s]), xM = Cx<Z>::from(a.x[a.N + s]);
+    const Z xJ = Cx<Z>::from(cscale(a.x[s], sc)), xM = Cx<Z>::from(cscale(a.x[a.N + s], sc));
     const Z z11 = Zr[3 * j], z12 = Zr[3 * j + 1], z22 = Zr[3 * j + 2];
     nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
     nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
@@ -71,110 +74,28 @@ __global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
   }
 }
 
-// Device state of the preconditioner's inner GMRES: its Hessenberg matrix,
-// rotations and right-hand side live on the GPU, so that the inner steps run
-// without a host round trip.
-struct InnerDev {
-  double2* H;   // [(inner + 1) x inner], column-major, ld = inner + 1
-  double2* cs;  // [inner] rotations
-  double2* sn;
-  double2* g;   // [inner + 1] rotated right-hand side
-  double2* y;   // [inner] solution of the triangular system
-  double2* h1;  // [inner + 1] coefficients of the two Gram-Schmidt passes
-  double2* h2;
-  double2* hn2; // [1] ||u||^2 after the projections (real part)
-  double* sc;   // [0] beta, [1] scale of the next basis vector, [2] 1 / beta
-  int* flags;   // [0] breakdown, [1] columns in use
-};
+}  // namespace
 
-// beta = ||v|| from the norm partials; g = (beta, 0, ...); flags cleared
-__global__ void inner_begin(const double2* partial, int nblk, InnerDev d, int inner) {
-  double s = 0.0;
-  for (int b = 0; b < nblk; ++b) s += partial[b].x;
-  const double beta = sqrt(s);
-  d.sc[0] = beta;
-  d.sc[2] = beta > 0.0 ? 1.0 / beta : 0.0;
-  for (int i = 0; i <= inner; ++i) d.g[i] = c2(i == 0 ? beta : 0.0, 0.0);
-  d.flags[0] = 0;
-  d.flags[1] = 0;
-}
+namespace {
 
-// column j of H from the Gram-Schmidt coefficients, its rotations, and the
-// scale of the next basis vector (0 after a breakdown)
-__global__ void inner_step(InnerDev d, int j, int ld) {
-  if (d.flags[0]) {
-    d.sc[1] = 0.0;
-    return;
+void near_apply_scaled(Plan& P, const double2* x, const double* xscale, double2* w, cudaStream_t s, int prec) {
+  if (prec == 1) {
+    if (P.d_near_z32 == nullptr) throw std::invalid_argument("plan holds no complex64 near field");
+    NearArg<float2> a{P.d_leaf_rwg,  P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src, P.d_near_zoff,
+                      P.d_near_z32,  x,               xscale,       w,             P.N};
+    near_apply_kernel<float2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
+  } else {
+    NearArg<double2> a{P.d_leaf_rwg, P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src, P.d_near_zoff,
+                       P.d_near_z,   x,               xscale,       w,             P.N};
+    near_apply_kernel<double2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
   }
-  double2* Hj = d.H + static_cast<long long>(j) * ld;
-  for (int i = 0; i <= j; ++i) Hj[i] = cadd(d.h1[i], d.h2[i]);
-  const double hn = sqrt(d.hn2[0].x);
-  Hj[j + 1] = c2(hn, 0.0);
-  for (int i = 0; i < j; ++i) blas1::dgivens_apply(Hj[i], Hj[i + 1], d.cs[i], d.sn[i]);
-  d.flags[1] = j + 1;
-  if (hn < 1e-14 * d.sc[0]) {
-    d.flags[0] = 1;
-    d.sc[1] = 0.0;
-    return;
-  }
-  d.sc[1] = 1.0 / hn;
-  blas1::dgivens_make(Hj[j], Hj[j + 1], d.cs[j], d.sn[j]);
-  blas1::dgivens_apply(Hj[j], Hj[j + 1], d.cs[j], d.sn[j]);
-  Hj[j + 1] = c2(0.0, 0.0);
-  blas1::dgivens_apply(d.g[j], d.g[j + 1], d.cs[j], d.sn[j]);
-}
-
-// y = R^{-1} g over the columns in use (Code/GMRES.h:165-182); zero beyond
-__global__ void inner_end(InnerDev d, int ld, int inner) {
-  const int m = d.flags[1];
-  const double eps = 1e-16;
-  for (int i = inner - 1; i >= 0; --i) {
-    if (i >= m) {
-      d.y[i] = c2(0.0, 0.0);
-      continue;
-    }
-    double2 yi = d.g[i];
-    for (int j = i + 1; j < m; ++j) yi = csub(yi, cmul(d.H[i + static_cast<long long>(j) * ld], d.y[j]));
-    const double2 hii = d.H[i + static_cast<long long>(i) * ld];
-    d.y[i] = sqrt(hii.x * hii.x + hii.y * hii.y) > eps ? cdiv(yi, hii) : c2(0.0, 0.0);
-  }
-}
-
-// dst = src * s[0]; dst may be src (the inner step scales its vector in place)
-__global__ void scale_by(const double2* src, const double* s, double2* dst, long long n) {
-  const double a = *s;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = cscale(src[i], a);
-}
-
-// Upper-triangular solve of the rotated least-squares system (Code/GMRES.h:165-182).
-void back_substitute(const std::vector<C>& H, int ld, const std::vector<C>& s, int m, std::vector<C>& y) {
-  const double eps = 1e-16;
-  y.assign(m, C(0.0));
-  for (int i = m - 1; i >= 0; --i) {
-    y[i] = s[i];
-    for (int j = i + 1; j < m; ++j) y[i] -= H[i + j * ld] * y[j];
-    if (std::abs(H[i + i * ld]) > eps)
-      y[i] /= H[i + i * ld];
-    else
-      y[i] = C(0.0);
-  }
+  MLFMA_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
 void near_apply(Plan& P, const double2* x, double2* w, cudaStream_t s, int prec) {
-  if (prec == 1) {
-    if (P.d_near_z32 == nullptr) throw std::invalid_argument("plan holds no complex64 near field");
-    NearArg<float2> a{P.d_leaf_rwg,  P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src,
-                      P.d_near_zoff, P.d_near_z32,    x,            w,             P.N};
-    near_apply_kernel<float2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
-  } else {
-    NearArg<double2> a{P.d_leaf_rwg,  P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src,
-                       P.d_near_zoff, P.d_near_z,      x,            w,             P.N};
-    near_apply_kernel<double2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
-  }
-  MLFMA_CUDA(cudaGetLastError());
+  near_apply_scaled(P, x, nullptr, w, s, prec);
 }
 
 namespace {
@@ -183,53 +104,42 @@ namespace {
 // zero, with the complex64 copy of Z_near (the outer flexible GMRES admits
 // any preconditioner; its operator and residuals stay at the solve's
 // precision). The inner Hessenberg matrix, rotations and triangular solve
-// stay on the GPU: the inner steps run without a host round trip. Buffers
-// come from the caller's Work; the reduction scratch is the caller's Ops.
+// stay on the GPU: the inner steps run without a host round trip, as four
+// launches each (near-field product, then the three of the Gram-Schmidt, the
+// last with the step's rotations). Buffers come from the caller's Work; the
+// reduction scratch is the caller's Ops.
 struct NearPrecond {
   Plan& P;
   cudaStream_t s;
   long long n;
-  int inner_its, ldi;
+  int inner_its;
   blas1::Ops ops;
-  double2* Q = nullptr;
-  InnerDev idv{};
+  double2* Q = nullptr;  // [inner_its + 1][n], unscaled basis
+  blas1::Inner in{};
   NearPrecond(Plan& P_, cudaStream_t s_, int inner, blas1::Work& g, const blas1::Ops& o)
-      : P(P_), s(s_), n(2LL * P_.N), inner_its(inner), ldi(inner + 1), ops(o) {
+      : P(P_), s(s_), n(2LL * P_.N), inner_its(inner), ops(o) {
     if (inner_its <= 0) return;
     Q = g.get(static_cast<size_t>(inner_its + 1) * n);
-    idv.H = g.get(static_cast<size_t>(ldi) * inner_its);
-    idv.cs = g.get(inner_its);
-    idv.sn = g.get(inner_its);
-    idv.g = g.get(ldi);
-    idv.y = g.get(inner_its);
-    idv.h1 = g.get(ldi);
-    idv.h2 = g.get(ldi);
-    idv.hn2 = g.get(1);
-    idv.sc = reinterpret_cast<double*>(g.get(2));
-    idv.flags = reinterpret_cast<int*>(g.get(1));
+    in = blas1::Inner::carve(g.get(blas1::Inner::bytes(1, inner_its) / sizeof(double2) + 1), 1, inner_its);
+  }
+  // v into the basis, then the steps, which read and write this object's own
+  // arrays only (one captured graph serves every v and z), then z
+  void begin(const double2* v) { ops.inner_start(1, nullptr, ops.ref(v), ops.ref(Q), in); }
+  void steps() {
+    for (int j = 0; j < inner_its; ++j) {
+      double2* u = Q + static_cast<long long>(j + 1) * n;
+      near_apply_scaled(P, Q + static_cast<long long>(j) * n, in.vs + j, u, s, 1);
+      ops.orthogonalise(1, nullptr, ops.ref(Q), ops.ref(u), j + 1, &in);
+    }
+  }
+  void end(double2* z) {
+    ops.combine(1, nullptr, ops.ref(Q), ops.ref(z), nullptr, inner_its, in.y, 0, false);
+    MLFMA_CUDA(cudaGetLastError());
   }
   void launch(const double2* v, double2* z) {
-    blas1::norm2<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(nullptr, v, nullptr, n, ops.part);
-    inner_begin<<<1, 1, 0, s>>>(ops.part, blas1::kBlocks, idv, inner_its);
-    scale_by<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(v, idv.sc + 2, Q, n);
-    for (int j = 0; j < inner_its; ++j) {
-      const double2* q = Q + static_cast<long long>(j) * n;
-      double2* u = Q + static_cast<long long>(j + 1) * n;
-      near_apply(P, q, u, s, 1);
-      const int nv = j + 1;
-      blas1::dots<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Q, n, nv, u, ops.part, ops.ldp);
-      blas1::reduce<<<(nv + 63) / 64, 64, 0, s>>>(ops.part, blas1::kBlocks, ops.ldp, nv, idv.h1);
-      blas1::project_out<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Q, n, nv, idv.h1, u, 0, ops.part, ops.ldp);
-      blas1::dots<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Q, n, nv, u, ops.part, ops.ldp);
-      blas1::reduce<<<(nv + 63) / 64, 64, 0, s>>>(ops.part, blas1::kBlocks, ops.ldp, nv, idv.h2);
-      blas1::project_out<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Q, n, nv, idv.h2, u, 1, ops.part, ops.ldp);
-      blas1::reduce<<<1, 64, 0, s>>>(ops.part, blas1::kBlocks, ops.ldp, 1, idv.hn2);
-      inner_step<<<1, 1, 0, s>>>(idv, j, ldi);
-      scale_by<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(u, idv.sc + 1, u, n);
-    }
-    inner_end<<<1, 1, 0, s>>>(idv, ldi, inner_its);
-    blas1::combine<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Q, n, inner_its, idv.y, z, 0);
-    MLFMA_CUDA(cudaGetLastError());
+    begin(v);
+    steps();
+    end(z);
   }
 };
 
@@ -239,8 +149,7 @@ void near_precondition(Plan& P, int inner_its, const double2* v, double2* z, cud
   if (inner_its < 1 || inner_its + 1 > blas1::kMaxBasis) throw std::invalid_argument("inner_its must be in 1..63");
   MLFMA_CUDA(cudaSetDevice(P.device));
   blas1::Work g;
-  const int ldp = blas1::kMaxBasis + 2;
-  blas1::Ops ops{s, 2LL * P.N, g.get(static_cast<size_t>(blas1::kBlocks) * ldp), ldp, g.get(2 * ldp + 2)};
+  const blas1::Ops ops = blas1::make_ops(g, s, 2LL * P.N);
   NearPrecond np(P, s, inner_its, g, ops);
   np.launch(v, z);
   MLFMA_CUDA(cudaStreamSynchronize(s));  // the work arrays are freed on return
@@ -262,7 +171,6 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
   blas1::Work g;
-  const int ldp = blas1::kMaxBasis + 2;
   double2* x = g.get(n);
   double2* b = g.get(n);
   double2* r = g.get(n);
@@ -270,7 +178,7 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   double2* V = g.get(static_cast<size_t>(mr + 1) * n);
   double2* Zd = inner_its > 0 ? g.get(static_cast<size_t>(mr) * n) : V;
   double2* y = g.get(blas1::kMaxBasis);
-  blas1::Ops ops{s, n, g.get(static_cast<size_t>(blas1::kBlocks) * ldp), ldp, g.get(2 * ldp + 2)};
+  blas1::Ops ops = blas1::make_ops(g, s, n);
   MLFMA_CUDA(cudaMemcpyAsync(x, xh, n * sizeof(double2), cudaMemcpyHostToDevice, s));
   MLFMA_CUDA(cudaMemcpyAsync(b, rhs, n * sizeof(double2), cudaMemcpyHostToDevice, s));
   st = SolveStats();
@@ -278,9 +186,9 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   std::vector<C> hcol;
 
   auto true_residual = [&]() {
-    op_apply(x, w, s);
+    op_apply(x, r, s);
     st.matvecs++;
-    return ops.residual(b, w, r);
+    return ops.residual(b, r);
   };
   auto finish = [&](bool ok, double err) {
     MLFMA_CUDA(cudaMemcpyAsync(xh, x, n * sizeof(double2), cudaMemcpyDeviceToHost, s));
@@ -290,16 +198,10 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
     return ok;
   };
   NearPrecond np(P, s, inner_its, g, ops);
-  auto precondition_launch = [&](const double2* v, double2* z) {
-    np.launch(v, z);
-    // a learned correction of z, when a network is attached to the plan
-    if (const __nv_bfloat16* wl = lp_attached(P)) lp_forward(P, wl, v, z, z, false, s);
-  };
-  // The preconditioner's ~10 launches per inner step are captured once per
-  // solve as a CUDA graph on solve-owned input / output vectors (v copied in,
-  // z out): the same graph serves every basis vector.
-  double2* pv = inner_its > 0 ? g.get(n) : nullptr;
-  double2* pz = inner_its > 0 ? g.get(n) : nullptr;
+  // The preconditioner's four launches per inner step are captured once per
+  // solve as a CUDA graph on the preconditioner's own arrays: the same graph
+  // serves every basis vector. A learned correction of z, when a network is
+  // attached to the plan, follows it.
   cudaGraphExec_t pgraph = nullptr;
   struct GraphGuard {
     cudaGraphExec_t& e;
@@ -309,26 +211,30 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   } pguard{pgraph};
   auto precondition = [&](const double2* v, double2* z) {
     st.near_products += inner_its;
-    if (!P.tuning.graph) return precondition_launch(v, z);
-    MLFMA_CUDA(cudaMemcpyAsync(pv, v, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
-    if (pgraph == nullptr) {
-      MLFMA_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      try {
-        precondition_launch(pv, pz);
-      } catch (...) {
+    np.begin(v);
+    if (!P.tuning.graph) {
+      np.steps();
+    } else {
+      if (pgraph == nullptr) {
+        MLFMA_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        try {
+          np.steps();
+        } catch (...) {
+          cudaGraph_t gr = nullptr;
+          cudaStreamEndCapture(s, &gr);
+          if (gr) cudaGraphDestroy(gr);
+          throw;
+        }
         cudaGraph_t gr = nullptr;
-        cudaStreamEndCapture(s, &gr);
-        if (gr) cudaGraphDestroy(gr);
-        throw;
+        MLFMA_CUDA(cudaStreamEndCapture(s, &gr));
+        const cudaError_t e = cudaGraphInstantiate(&pgraph, gr, 0);
+        cudaGraphDestroy(gr);
+        MLFMA_CUDA(e);
       }
-      cudaGraph_t gr = nullptr;
-      MLFMA_CUDA(cudaStreamEndCapture(s, &gr));
-      const cudaError_t e = cudaGraphInstantiate(&pgraph, gr, 0);
-      cudaGraphDestroy(gr);
-      MLFMA_CUDA(e);
+      MLFMA_CUDA(cudaGraphLaunch(pgraph, s));
     }
-    MLFMA_CUDA(cudaGraphLaunch(pgraph, s));
-    MLFMA_CUDA(cudaMemcpyAsync(z, pz, n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    np.end(z);
+    if (const __nv_bfloat16* wl = lp_attached(P)) lp_forward(P, wl, v, z, z, false, s);
   };
 
   const double eps = 1e-16;
@@ -351,7 +257,7 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   int total = 0;
   for (int cycle = 1; cycle <= itr_max; ++cycle) {
     st.restarts = cycle;
-    blas1::scale<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(r, 1.0 / rnorm, V, n);
+    ops.scale(r, 1.0 / rnorm, V);
     std::fill(sv.begin(), sv.end(), C(0.0));
     sv[0] = rnorm;
     std::fill(H.begin(), H.end(), C(0.0));
@@ -365,11 +271,11 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
       if (inner_its > 0) precondition(vk, zk);
       op_apply(zk, w, s);
       st.matvecs++;
-      const double h_next = ops.orthogonalise(V, k + 1, w, hcol);
+      const double h_next = ops.orthogonalise_host(V, k + 1, w, hcol);
       for (int j = 0; j <= k; ++j) H[j + static_cast<size_t>(k) * ld] = hcol[j];
       H[k + 1 + static_cast<size_t>(k) * ld] = h_next;
       if (h_next < eps * rnorm) break;
-      blas1::scale<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(w, 1.0 / h_next, V + static_cast<long long>(k + 1) * n, n);
+      ops.scale(w, 1.0 / h_next, V + static_cast<long long>(k + 1) * n);
       for (int j = 0; j < k; ++j) blas1::givens_apply(H[j + k * ld], H[j + 1 + k * ld], cs[j], sn[j]);
       blas1::givens_make(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
       blas1::givens_apply(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
@@ -380,10 +286,10 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
       if (error < tol_rel || error < tol_abs) break;
     }
     const int m = std::min(k_used, mr);
-    back_substitute(H, ld, sv, m, yy);
+    blas1::back_substitute(H, ld, sv, m, yy);
     if (m > 0) {
       MLFMA_CUDA(cudaMemcpyAsync(y, yy.data(), m * sizeof(double2), cudaMemcpyHostToDevice, s));
-      blas1::combine<<<blas1::kBlocks, blas1::kThreads, 0, s>>>(Zd, n, m, y, x, 1);
+      ops.combine(1, nullptr, ops.ref(Zd), ops.ref(x), nullptr, m, y, 0, true);
     }
     rnorm = true_residual();
     error = rnorm / bnorm;

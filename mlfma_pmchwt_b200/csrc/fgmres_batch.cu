@@ -29,162 +29,7 @@ namespace mlfma {
 namespace {
 
 using C = std::complex<double>;
-constexpr int kBT = 256;  // threads per block of the batched vector kernels
-
-// One operand of a batched kernel: the vector of lockstep position a lives at
-// p + (by_sys ? sys[a] : a) * stride + off.
-struct VecRef {
-  double2* p;
-  long long stride, off;
-  int by_sys;
-  __device__ __forceinline__ double2* at(int a, const int* sys) const {
-    return p + (by_sys ? sys[a] : a) * stride + off;
-  }
-};
-
-__device__ __forceinline__ double2 bsum(double2 v, double2* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = lane < (blockDim.x >> 5) ? sh[lane] : c2(0.0, 0.0);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-  }
-  return v;
-}
-
-// part[(a * nblk + blk) * ldp + j] = block partial of conj(V_j) . w, j < nv
-// (V_j = basis vector j of the operand V: stride between basis vectors n)
-__global__ void __launch_bounds__(kBT) dots_b(VecRef V, VecRef w, const int* sys, long long n, int nv,
-                                             double2* part, int ldp) {
-  __shared__ double2 sh[kBT / 32];
-  const int a = blockIdx.y, nblk = gridDim.x;
-  const double2* Vb = V.at(a, sys);
-  const double2* wb = w.at(a, sys);
-  for (int j0 = 0; j0 < nv; j0 += blas1::kTile) {
-    double2 acc[blas1::kTile];
-#pragma unroll
-    for (int q = 0; q < blas1::kTile; ++q) acc[q] = c2(0.0, 0.0);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)nblk * blockDim.x) {
-      const double2 wi = wb[i];
-#pragma unroll
-      for (int q = 0; q < blas1::kTile; ++q)
-        if (j0 + q < nv) {
-          const double2 v = Vb[(long long)(j0 + q) * n + i];
-          acc[q].x = fma(v.x, wi.x, fma(v.y, wi.y, acc[q].x));
-          acc[q].y = fma(v.x, wi.y, fma(-v.y, wi.x, acc[q].y));
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < blas1::kTile; ++q)
-      if (j0 + q < nv) {
-        const double2 s = bsum(acc[q], sh);
-        if (threadIdx.x == 0) part[((long long)a * nblk + blockIdx.x) * ldp + j0 + q] = s;
-      }
-  }
-}
-
-// out[a * ldo + j] = sum over blocks, j < nv; grid.y = positions
-__global__ void reduce_b(const double2* part, int nblk, int ldp, int nv, double2* out, int ldo) {
-  const int a = blockIdx.y;
-  for (int j = threadIdx.x; j < nv; j += blockDim.x) {
-    double2 s = c2(0.0, 0.0);
-    for (int b = 0; b < nblk; ++b) s = cadd(s, part[((long long)a * nblk + b) * ldp + j]);
-    out[(long long)a * ldo + j] = s;
-  }
-}
-
-// w -= sum_j V_j h[a * ldh + j]; with want_norm the block partials of ||w||^2
-// into part[(a * nblk + blk) * ldp]
-__global__ void __launch_bounds__(kBT) project_b(VecRef V, VecRef w, const int* sys, long long n, int nv,
-                                                const double2* h, int ldh, int want_norm, double2* part,
-                                                int ldp) {
-  __shared__ double2 hs[blas1::kMaxBasis];
-  __shared__ double2 sh[kBT / 32];
-  const int a = blockIdx.y, nblk = gridDim.x;
-  const double2* Vb = V.at(a, sys);
-  double2* wb = w.at(a, sys);
-  for (int j = threadIdx.x; j < nv; j += blockDim.x) hs[j] = h[(long long)a * ldh + j];
-  __syncthreads();
-  double2 nrm = c2(0.0, 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)nblk * blockDim.x) {
-    double2 wi = wb[i];
-    for (int j = 0; j < nv; ++j) wi = csub(wi, cmul(hs[j], Vb[(long long)j * n + i]));
-    wb[i] = wi;
-    nrm.x = fma(wi.x, wi.x, fma(wi.y, wi.y, nrm.x));
-  }
-  if (want_norm) {
-    const double2 s = bsum(nrm, sh);
-    if (threadIdx.x == 0) part[((long long)a * nblk + blockIdx.x) * ldp] = s;
-  }
-}
-
-// block partials of ||w||^2, or of ||b - w||^2 with r = b - w written (has_b)
-__global__ void __launch_bounds__(kBT) norm_b(VecRef b, VecRef w, VecRef r, const int* sys, long long n, int has_b,
-                                             double2* part, int ldp) {
-  __shared__ double2 sh[kBT / 32];
-  const int a = blockIdx.y, nblk = gridDim.x;
-  const double2* wb = w.at(a, sys);
-  const double2* bb = has_b ? b.at(a, sys) : nullptr;
-  double2* rb = has_b ? r.at(a, sys) : nullptr;
-  double2 nrm = c2(0.0, 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)nblk * blockDim.x) {
-    double2 v = wb[i];
-    if (has_b) {
-      v = csub(bb[i], v);
-      rb[i] = v;
-    }
-    nrm.x = fma(v.x, v.x, fma(v.y, v.y, nrm.x));
-  }
-  const double2 s = bsum(nrm, sh);
-  if (threadIdx.x == 0) part[((long long)a * nblk + blockIdx.x) * ldp] = s;
-}
-
-// dst = alpha[a] * src
-__global__ void scale_b(VecRef src, VecRef dst, const int* sys, long long n, const double* alpha) {
-  const int a = blockIdx.y;
-  const double2* s = src.at(a, sys);
-  double2* d = dst.at(a, sys);
-  const double al = alpha[a];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    d[i] = cscale(s[i], al);
-}
-
-// x (+)= sum_{j < m[a]} V_j y[a * ldy + j]
-__global__ void combine_b(VecRef V, VecRef x, const int* sys, long long n, const int* m, const double2* y, int ldy,
-                          int accumulate) {
-  __shared__ double2 ys[blas1::kMaxBasis];
-  const int a = blockIdx.y;
-  const int ma = m[a];
-  const double2* Vb = V.at(a, sys);
-  double2* xb = x.at(a, sys);
-  for (int j = threadIdx.x; j < ma; j += blockDim.x) ys[j] = y[(long long)a * ldy + j];
-  __syncthreads();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double2 xi = accumulate ? xb[i] : c2(0.0, 0.0);
-    for (int j = 0; j < ma; ++j) xi = cfma(ys[j], Vb[(long long)j * n + i], xi);
-    xb[i] = xi;
-  }
-}
-
-// dst = src (gather into / scatter out of the contiguous staging block)
-__global__ void copy_b(VecRef src, VecRef dst, const int* sys, long long n) {
-  const int a = blockIdx.y;
-  const double2* s = src.at(a, sys);
-  double2* d = dst.at(a, sys);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    d[i] = s[i];
-}
+using blas1::VecRef;
 
 // w_a = Z_near x_a for every position (warp per RWG, 4 right-hand sides per
 // warp): the near-field rows of the plan, read once per group of four.
@@ -199,6 +44,8 @@ struct NearBatchArg {
   const Z* near_z;
   VecRef x, w;
   const int* sys;
+  const double* xscale;  // factor of position a's x at xscale[a * lds]
+  int lds;
   int N, R;
 };
 
@@ -217,10 +64,12 @@ __global__ void __launch_bounds__(128) near_batch_kernel(NearBatchArg<Z> a) {
   const Z* Zr = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
   Z nJ[kNearRB], nM[kNearRB];
   const double2* xs[kNearRB];
+  double sc[kNearRB];
 #pragma unroll
   for (int j = 0; j < kNearRB; ++j) {
     nJ[j] = nM[j] = Cx<Z>::zero();
     xs[j] = j < pn ? a.x.at(p0 + j, a.sys) : nullptr;
+    sc[j] = j < pn ? a.xscale[static_cast<long long>(p0 + j) * a.lds] : 0.0;
   }
   for (int q = lane; q < ns; q += 32) {
     const int src = a.near_src[s0 + q];
@@ -228,7 +77,7 @@ __global__ void __launch_bounds__(128) near_batch_kernel(NearBatchArg<Z> a) {
 #pragma unroll
     for (int j = 0; j < kNearRB; ++j) {
       if (j < pn) {
-        const Z xJ = Cx<Z>::from(xs[j][src]), xM = Cx<Z>::from(xs[j][a.N + src]);
+        const Z xJ = Cx<Z>::from(cscale(xs[j][src], sc[j])), xM = Cx<Z>::from(cscale(xs[j][a.N + src], sc[j]));
         nJ[j] = cfma(z11, xJ, cfma(z12, xM, nJ[j]));
         nM[j] = cfma(z22, xM, csub(nM[j], cmul(z12, xJ)));
       }
@@ -265,11 +114,15 @@ __global__ void __launch_bounds__(128) near_batch_box_kernel(NearBatchArg<Z> a) 
   extern __shared__ __align__(16) unsigned char near_smem[];
   Z* xsm = reinterpret_cast<Z*>(near_smem);
   __shared__ const double2* xbase[kNearBoxRB];
+  __shared__ double xsc[kNearBoxRB];
   const int b = blockIdx.x;
   const int p0 = blockIdx.y * kNearBoxRB, pn = min(kNearBoxRB, a.R - p0);
   const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
   const int r0 = a.leaf_ptr[b], nb = a.leaf_ptr[b + 1] - r0;
-  if (threadIdx.x < pn) xbase[threadIdx.x] = a.x.at(p0 + threadIdx.x, a.sys);
+  if (threadIdx.x < pn) {
+    xbase[threadIdx.x] = a.x.at(p0 + threadIdx.x, a.sys);
+    xsc[threadIdx.x] = a.xscale[static_cast<long long>(p0 + threadIdx.x) * a.lds];
+  }
   __syncthreads();
   // one source per thread, the values of 4 systems in flight at once
   constexpr int kStage = 4;
@@ -287,8 +140,8 @@ __global__ void __launch_bounds__(128) near_batch_box_kernel(NearBatchArg<Z> a) 
 #pragma unroll
       for (int j = 0; j < kStage; ++j)
         if (j0 + j < pn) {
-          xsm[(2 * (j0 + j)) * ns + q] = Cx<Z>::from(vJ[j]);
-          xsm[(2 * (j0 + j) + 1) * ns + q] = Cx<Z>::from(vM[j]);
+          xsm[(2 * (j0 + j)) * ns + q] = Cx<Z>::from(cscale(vJ[j], xsc[j0 + j]));
+          xsm[(2 * (j0 + j) + 1) * ns + q] = Cx<Z>::from(cscale(vM[j], xsc[j0 + j]));
         }
     }
   }
@@ -349,167 +202,51 @@ __global__ void __launch_bounds__(128) near_batch_box_kernel(NearBatchArg<Z> a) 
   }
 }
 
-// Device state of the preconditioner's inner GMRES for every lockstep
-// position: Hessenberg columns, rotations, rotated right-hand side,
-// breakdown flags. The inner steps update it with one thread per position
-// (the arithmetic of fgmres.cu's single-system inner_step), so they run
-// without a host round trip.
-struct InnerBatch {
-  double2* H;    // [R][ld * inner], column-major per position
-  double2* cs;   // [R][inner]
-  double2* sn;   // [R][inner]
-  double2* g;    // [R][ld]
-  double* beta;  // [R]
-  int* done;     // [R]
-  int ld, inner;
-};
-
-// beta_a = ||v_a|| from the reduced norms (hred[a * ldh]); alpha_a = 1 / beta_a;
-// g_a = (beta_a, 0, ...); columns in use m_a = 0
-__global__ void inner_begin_b(int Ra, const double2* hred, int ldh, InnerBatch S, double* alpha, int* m) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= Ra) return;
-  const double beta = sqrt(hred[static_cast<long long>(a) * ldh].x);
-  S.beta[a] = beta;
-  alpha[a] = beta > 0.0 ? 1.0 / beta : 0.0;
-  for (int i = 0; i < S.ld; ++i) S.g[static_cast<long long>(a) * S.ld + i] = c2(i == 0 ? beta : 0.0, 0.0);
-  S.done[a] = 0;
-  m[a] = 0;
-}
-
-// Column j of H_a from both Gram-Schmidt passes' coefficients (hred[a * ldh
-// + i] + hred[a * ldh + ldp + i]) and ||u_a||^2 (hred[a * ldh + 2 ldp]); its
-// rotations; alpha_a = scale of the next basis vector (0 after a breakdown).
-__global__ void inner_step_b(int Ra, int j, const double2* hred, int ldh, int ldp, InnerBatch S, double* alpha,
-                             int* m) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= Ra) return;
-  if (S.done[a]) {
-    alpha[a] = 0.0;
-    return;
-  }
-  const double2* h = hred + static_cast<long long>(a) * ldh;
-  double2* Hj = S.H + (static_cast<long long>(a) * S.inner + j) * S.ld;
-  double2* cs = S.cs + static_cast<long long>(a) * S.inner;
-  double2* sn = S.sn + static_cast<long long>(a) * S.inner;
-  double2* g = S.g + static_cast<long long>(a) * S.ld;
-  for (int i = 0; i <= j; ++i) Hj[i] = cadd(h[i], h[ldp + i]);
-  const double hn = sqrt(h[2 * ldp].x);
-  Hj[j + 1] = c2(hn, 0.0);
-  for (int i = 0; i < j; ++i) blas1::dgivens_apply(Hj[i], Hj[i + 1], cs[i], sn[i]);
-  m[a] = j + 1;
-  if (hn < 1e-14 * S.beta[a]) {
-    S.done[a] = 1;
-    alpha[a] = 0.0;
-    return;
-  }
-  alpha[a] = 1.0 / hn;
-  blas1::dgivens_make(Hj[j], Hj[j + 1], cs[j], sn[j]);
-  blas1::dgivens_apply(Hj[j], Hj[j + 1], cs[j], sn[j]);
-  Hj[j + 1] = c2(0.0, 0.0);
-  blas1::dgivens_apply(g[j], g[j + 1], cs[j], sn[j]);
-}
-
-// y_a = R_a^{-1} g_a over the m_a columns in use (Code/GMRES.h:165-182)
-__global__ void inner_end_b(int Ra, InnerBatch S, const int* m, double2* y, int ldy) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= Ra) return;
-  const double eps = 1e-16;
-  const int ma = m[a];
-  const double2* H = S.H + static_cast<long long>(a) * S.inner * S.ld;
-  const double2* g = S.g + static_cast<long long>(a) * S.ld;
-  double2* ya = y + static_cast<long long>(a) * ldy;
-  for (int i = ma - 1; i >= 0; --i) {
-    double2 yi = g[i];
-    for (int j = i + 1; j < ma; ++j) yi = csub(yi, cmul(H[i + static_cast<long long>(j) * S.ld], ya[j]));
-    const double2 hii = H[i + static_cast<long long>(i) * S.ld];
-    ya[i] = sqrt(hii.x * hii.x + hii.y * hii.y) > eps ? cdiv(yi, hii) : c2(0.0, 0.0);
-  }
-}
-
-// Upper-triangular solve of the rotated least-squares system (Code/GMRES.h:165-182).
-void back_substitute(const std::vector<C>& H, int ld, const std::vector<C>& s, int m, std::vector<C>& y) {
-  const double eps = 1e-16;
-  y.assign(m, C(0.0));
-  for (int i = m - 1; i >= 0; --i) {
-    y[i] = s[i];
-    for (int j = i + 1; j < m; ++j) y[i] -= H[i + j * ld] * y[j];
-    if (std::abs(H[i + i * ld]) > eps)
-      y[i] /= H[i + i * ld];
-    else
-      y[i] = C(0.0);
-  }
-}
-
-// Host side of the batched vector steps on one stream, for up to R positions.
-struct BatchOps {
-  Plan& P;  // its device status is read at every host sync
-  cudaStream_t s;
-  long long n;
-  int nblk;          // blocks per system
-  int ldp;           // partial row length
-  double2* part;     // [R][nblk][ldp]
-  double2* hdev;     // [R][2 * ldp + 2]
+// The batched vector steps on one stream with their results on the host, for
+// up to R positions.
+struct BatchOps : blas1::Vec {
+  Plan* P;           // its device status is read at every host sync
   double* alpha;     // [R]
   int* mdev;         // [R]
   double2* ydev;     // [R][kMaxBasis]
   std::vector<C> hbuf;
 
-  dim3 grid(int Ra) const { return dim3(nblk, Ra); }
-
-  // squared norms of the operand (or of b - w, writing r) for Ra positions,
-  // left on the device at hdev[a * (2 ldp + 2)]
-  void norms_dev(int Ra, const int* sys, VecRef w, VecRef b = {}, VecRef r = {}, bool has_b = false) {
-    norm_b<<<grid(Ra), kBT, 0, s>>>(b, w, r, sys, n, has_b ? 1 : 0, part, ldp);
-    reduce_b<<<dim3(1, Ra), 32, 0, s>>>(part, nblk, ldp, 1, hdev, 2 * ldp + 2);
-  }
-  // norms of the operand (or of b - w, writing r) for Ra positions
-  std::vector<double> norms(int Ra, const int* sys, VecRef w, VecRef b = {}, VecRef r = {}, bool has_b = false) {
-    norms_dev(Ra, sys, w, b, r, has_b);
-    hbuf.resize(static_cast<size_t>(Ra) * (2 * ldp + 2));
-    MLFMA_CUDA(cudaMemcpyAsync(hbuf.data(), hdev, hbuf.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-    fetch_device_status(P, s);
+  void fetch(int Ra) {
+    hbuf.resize(static_cast<size_t>(Ra) * blas1::kLdh);
+    MLFMA_CUDA(cudaMemcpyAsync(hbuf.data(), h, hbuf.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    fetch_device_status(*P, s);
     MLFMA_CUDA(cudaStreamSynchronize(s));
-    raise_device_status(P);
+    raise_device_status(*P);
+  }
+  // norms of the operand for Ra positions, or of w = b - w
+  std::vector<double> norms_host(int Ra, const int* sys, VecRef w, const VecRef* b = nullptr) {
+    if (b)
+      residuals(Ra, sys, w, *b);
+    else
+      norms(Ra, sys, w);
+    fetch(Ra);
     std::vector<double> out(Ra);
-    for (int a = 0; a < Ra; ++a) out[a] = std::sqrt(hbuf[static_cast<size_t>(a) * (2 * ldp + 2)].real());
+    for (int a = 0; a < Ra; ++a) out[a] = std::sqrt(hbuf[static_cast<size_t>(a) * blas1::kLdh].real());
     return out;
   }
   // CGS2 of w_a against V_a[0..nv): hcol[a][j] and ||w_a|| after projection
-  // CGS2 launches only: per position a, hdev[a * ldh + j] and [a * ldh + ldp
-  // + j] the two passes' coefficients, [a * ldh + 2 ldp] ||w_a||^2 after them
-  void orthogonalise_dev(int Ra, const int* sys, VecRef V, VecRef w, int nv) {
-    const int ldh = 2 * ldp + 2;
-    dots_b<<<grid(Ra), kBT, 0, s>>>(V, w, sys, n, nv, part, ldp);
-    reduce_b<<<dim3(1, Ra), 64, 0, s>>>(part, nblk, ldp, nv, hdev, ldh);
-    project_b<<<grid(Ra), kBT, 0, s>>>(V, w, sys, n, nv, hdev, ldh, 0, part, ldp);
-    dots_b<<<grid(Ra), kBT, 0, s>>>(V, w, sys, n, nv, part, ldp);
-    reduce_b<<<dim3(1, Ra), 64, 0, s>>>(part, nblk, ldp, nv, hdev + ldp, ldh);
-    project_b<<<grid(Ra), kBT, 0, s>>>(V, w, sys, n, nv, hdev + ldp, ldh, 1, part, ldp);
-    reduce_b<<<dim3(1, Ra), 32, 0, s>>>(part, nblk, ldp, 1, hdev + 2 * ldp, ldh);
-  }
-  void orthogonalise(int Ra, const int* sys, VecRef V, VecRef w, int nv, std::vector<std::vector<C>>& hcol,
-                     std::vector<double>& hn) {
-    const int ldh = 2 * ldp + 2;
-    orthogonalise_dev(Ra, sys, V, w, nv);
-    hbuf.resize(static_cast<size_t>(Ra) * ldh);
-    MLFMA_CUDA(cudaMemcpyAsync(hbuf.data(), hdev, hbuf.size() * sizeof(double2), cudaMemcpyDeviceToHost, s));
-    fetch_device_status(P, s);
-    MLFMA_CUDA(cudaStreamSynchronize(s));
-    raise_device_status(P);
+  void orthogonalise_host(int Ra, const int* sys, VecRef V, VecRef w, int nv, std::vector<std::vector<C>>& hcol,
+                          std::vector<double>& hn) {
+    orthogonalise(Ra, sys, V, w, nv);
+    fetch(Ra);
     hcol.assign(Ra, std::vector<C>(nv));
     hn.assign(Ra, 0.0);
     for (int a = 0; a < Ra; ++a) {
-      const C* h = hbuf.data() + static_cast<size_t>(a) * ldh;
-      for (int j = 0; j < nv; ++j) hcol[a][j] = h[j] + h[ldp + j];
-      hn[a] = std::sqrt(h[2 * ldp].real());
+      const C* hp = hbuf.data() + static_cast<size_t>(a) * blas1::kLdh;
+      for (int j = 0; j < nv; ++j) hcol[a][j] = hp[j] + hp[blas1::kMaxBasis + j];
+      hn[a] = std::sqrt(hp[2 * blas1::kMaxBasis].real());
     }
   }
-  void scale(int Ra, const int* sys, VecRef src, VecRef dst, const std::vector<double>& al) {
+  void scale_host(int Ra, const int* sys, VecRef src, VecRef dst, const std::vector<double>& al) {
     MLFMA_CUDA(cudaMemcpyAsync(alpha, al.data(), Ra * sizeof(double), cudaMemcpyHostToDevice, s));
-    scale_b<<<grid(Ra), kBT, 0, s>>>(src, dst, sys, n, alpha);
+    scale(Ra, sys, src, dst, alpha);
   }
-  void combine(int Ra, const int* sys, VecRef V, VecRef x, const std::vector<std::vector<C>>& y, bool acc) {
+  void combine_host(int Ra, const int* sys, VecRef V, VecRef x, const std::vector<std::vector<C>>& y, bool acc) {
     std::vector<int> m(Ra);
     std::vector<C> yy(static_cast<size_t>(Ra) * blas1::kMaxBasis, C(0.0));
     for (int a = 0; a < Ra; ++a) {
@@ -518,9 +255,8 @@ struct BatchOps {
     }
     MLFMA_CUDA(cudaMemcpyAsync(mdev, m.data(), Ra * sizeof(int), cudaMemcpyHostToDevice, s));
     MLFMA_CUDA(cudaMemcpyAsync(ydev, yy.data(), yy.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
-    combine_b<<<grid(Ra), kBT, 0, s>>>(V, x, sys, n, mdev, ydev, blas1::kMaxBasis, acc ? 1 : 0);
+    combine(Ra, sys, V, x, mdev, 0, ydev, blas1::kMaxBasis, acc);
   }
-  void copy(int Ra, const int* sys, VecRef src, VecRef dst) { copy_b<<<grid(Ra), kBT, 0, s>>>(src, dst, sys, n); }
 };
 
 }  // namespace
@@ -537,51 +273,39 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   reserve_batch(P, R, false);
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
-  const int ldp = blas1::kMaxBasis + 2;
   const long long vs = static_cast<long long>(mr + 1) * n;       // per-system basis stride
   const long long zs = static_cast<long long>(mr) * n;
   const long long qs = static_cast<long long>(inner_its + 1) * n;
   const int G = std::min(R, kBatchSlots);  // staging rows: one batched apply at a time
-  const int nblk = std::max(1, blas1::kBlocks / std::min(R, 8));
-  const int ldi = inner_its + 1;
   const size_t Rz = static_cast<size_t>(R);
   // work arrays (counts of complex128 values), in one block of the plan's
   // arena: no allocation when the last call's block is large enough
-  // the preconditioner's input and output rows (by lockstep position) when
-  // its launches are replayed as a CUDA graph
-  const bool pgraph_on = inner_its > 0 && P.tuning.graph == 1 && lp_attached(P) == nullptr;
-  enum { kX, kB, kR, kV, kZ, kQ, kXs, kWs, kPart, kH, kAlpha, kM, kY, kSys, kIH, kICs, kISn, kIG, kIBeta, kIDone,
-         kPv, kPz, kN };
+  enum { kX, kB, kR, kV, kZ, kQ, kXs, kWs, kPart, kCount, kH, kAlpha, kM, kY, kSys, kInner, kN };
   const size_t cnt[kN] = {Rz * n, Rz * n, Rz * n, Rz * vs, inner_its > 0 ? Rz * zs : 0, inner_its > 0 ? Rz * qs : 0,
-                          static_cast<size_t>(G) * n, static_cast<size_t>(G) * n, Rz * nblk * ldp,
-                          Rz * (2 * ldp + 2), Rz, Rz, Rz * blas1::kMaxBasis, Rz,
-                          inner_its > 0 ? Rz * ldi * inner_its : 0, Rz * inner_its, Rz * inner_its, Rz * ldi, Rz, Rz,
-                          pgraph_on ? Rz * n : 0, pgraph_on ? Rz * n : 0};
+                          static_cast<size_t>(G) * n, static_cast<size_t>(G) * n, blas1::part_count(n, R), Rz,
+                          Rz * blas1::kLdh, Rz, Rz, Rz * blas1::kMaxBasis, Rz,
+                          inner_its > 0 ? blas1::Inner::bytes(R, inner_its) / sizeof(double2) + 1 : 0};
   size_t work_bytes = 0;
   for (size_t c : cnt) work_bytes += (c * sizeof(double2) + 255) & ~size_t(255);
   P.arena.reserve(work_bytes);
   double2* wk[kN];
   for (int i = 0; i < kN; ++i) wk[i] = cnt[i] ? static_cast<double2*>(P.arena.get(cnt[i] * sizeof(double2))) : nullptr;
   double2 *x = wk[kX], *b = wk[kB], *r = wk[kR], *V = wk[kV], *Zd = wk[kZ], *Q = wk[kQ], *Xs = wk[kXs], *Ws = wk[kWs];
-  BatchOps ops{P, s, n, nblk, ldp};
+  BatchOps ops{};
+  ops.s = s;
+  ops.n = n;
   ops.part = wk[kPart];
-  ops.hdev = wk[kH];
+  ops.count = reinterpret_cast<unsigned*>(wk[kCount]);
+  ops.h = wk[kH];
+  ops.P = &P;
   ops.alpha = reinterpret_cast<double*>(wk[kAlpha]);
   ops.mdev = reinterpret_cast<int*>(wk[kM]);
   ops.ydev = wk[kY];
   int* sysd = reinterpret_cast<int*>(wk[kSys]);
   // inner GMRES state on the device (one row per lockstep position)
-  InnerBatch ib{};
-  if (inner_its > 0) {
-    ib.ld = ldi;
-    ib.inner = inner_its;
-    ib.H = wk[kIH];
-    ib.cs = wk[kICs];
-    ib.sn = wk[kISn];
-    ib.g = wk[kIG];
-    ib.beta = reinterpret_cast<double*>(wk[kIBeta]);
-    ib.done = reinterpret_cast<int*>(wk[kIDone]);
-  }
+  blas1::Inner ib{};
+  if (inner_its > 0) ib = blas1::Inner::carve(wk[kInner], R, inner_its);
+  MLFMA_CUDA(cudaMemsetAsync(ops.count, 0, Rz * sizeof(double2), s));
   MLFMA_CUDA(cudaMemsetAsync(P.d_status, 0, sizeof(int), s));
   MLFMA_CUDA(cudaMemcpyAsync(x, xh, static_cast<size_t>(R) * n * sizeof(double2), cudaMemcpyHostToDevice, s));
   MLFMA_CUDA(cudaMemcpyAsync(b, rhs, static_cast<size_t>(R) * n * sizeof(double2), cudaMemcpyHostToDevice, s));
@@ -619,7 +343,8 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     set_sys(list);
     const int Ra = static_cast<int>(list.size());
     // r holds A x: r = b - r in place
-    return ops.norms(Ra, sysd, sysref(r, n, 0), sysref(b, n, 0), sysref(r, n, 0), true);
+    const VecRef br = sysref(b, n, 0);
+    return ops.norms_host(Ra, sysd, sysref(r, n, 0), &br);
   };
   // the box-staged near-field kernel's shared memory: the largest source list
   const int nleaf = static_cast<int>(P.h_near_sptr.size()) - 1;
@@ -632,45 +357,32 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   if (inner_its > 0 && box_smem <= kNearBoxSmemMax)
     MLFMA_CUDA(cudaFuncSetAttribute(near_batch_box_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(kNearBoxSmemMax)));
-  const int ldh = 2 * ldp + 2;
   // z_q = (inner_its GMRES steps on Z_near from zero) applied to v_q, q in
-  // list: every step is launches only, the host waits for none of them
-  // the launches of one preconditioner application to the Ra positions'
-  // vectors vin, writing zout
-  auto precondition_launch = [&](int Ra, VecRef vin, VecRef zout) {
-    const int pb = (Ra + 63) / 64;
-    ops.norms_dev(Ra, sysd, vin);
-    inner_begin_b<<<pb, 64, 0, s>>>(Ra, ops.hdev, ldh, ib, ops.alpha, ops.mdev);
-    scale_b<<<ops.grid(Ra), kBT, 0, s>>>(vin, sysref(Q, qs, 0), sysd, n, ops.alpha);
+  // list: every step is four launches, the host waits for none of them
+  auto precondition_steps = [&](int Ra) {
     for (int j = 0; j < inner_its; ++j) {
-      {  // the preconditioner's near field is the complex64 copy at either precision
-        NearBatchArg<float2> na{P.d_leaf_rwg,  P.d_rwg_leafbox,      P.d_leaf_ptr,
-                                P.d_near_sptr, P.d_near_src,         P.d_near_zoff,
-                                P.d_near_z32,  sysref(Q, qs, j * n), sysref(Q, qs, (j + 1) * n),
-                                sysd,          P.N,                  Ra};
-        if (box_smem <= kNearBoxSmemMax) {
-          const dim3 ng(nleaf, (Ra + kNearBoxRB - 1) / kNearBoxRB);
-          near_batch_box_kernel<float2><<<ng, 128, box_smem, s>>>(na);
-        } else {
-          const dim3 ng((P.N + 3) / 4, (Ra + kNearRB - 1) / kNearRB);
-          near_batch_kernel<float2><<<ng, 128, 0, s>>>(na);
-        }
+      // the preconditioner's near field is the complex64 copy at either precision
+      NearBatchArg<float2> na{P.d_leaf_rwg,  P.d_rwg_leafbox,      P.d_leaf_ptr,
+                              P.d_near_sptr, P.d_near_src,         P.d_near_zoff,
+                              P.d_near_z32,  sysref(Q, qs, j * n), sysref(Q, qs, (j + 1) * n),
+                              sysd,          ib.vs + j,            ib.ld,
+                              P.N,           Ra};
+      if (box_smem <= kNearBoxSmemMax) {
+        const dim3 ng(nleaf, (Ra + kNearBoxRB - 1) / kNearBoxRB);
+        near_batch_box_kernel<float2><<<ng, 128, box_smem, s>>>(na);
+      } else {
+        const dim3 ng((P.N + 3) / 4, (Ra + kNearRB - 1) / kNearRB);
+        near_batch_kernel<float2><<<ng, 128, 0, s>>>(na);
       }
-      ops.orthogonalise_dev(Ra, sysd, sysref(Q, qs, 0), sysref(Q, qs, (j + 1) * n), j + 1);
-      inner_step_b<<<pb, 64, 0, s>>>(Ra, j, ops.hdev, ldh, ldp, ib, ops.alpha, ops.mdev);
-      scale_b<<<ops.grid(Ra), kBT, 0, s>>>(sysref(Q, qs, (j + 1) * n), sysref(Q, qs, (j + 1) * n), sysd, n,
-                                           ops.alpha);
+      ops.orthogonalise(Ra, sysd, sysref(Q, qs, 0), sysref(Q, qs, (j + 1) * n), j + 1, &ib);
     }
-    inner_end_b<<<pb, 64, 0, s>>>(Ra, ib, ops.mdev, ops.ydev, blas1::kMaxBasis);
-    combine_b<<<ops.grid(Ra), kBT, 0, s>>>(sysref(Q, qs, 0), zout, sysd, n, ops.mdev, ops.ydev, blas1::kMaxBasis,
-                                           0);
     MLFMA_CUDA(cudaGetLastError());
   };
-  // With apply.graph 1 (and no learned correction) the ~10 launches per inner
-  // step are captured once as a CUDA graph on fixed input / output rows (the
-  // basis vector copied in, z copied out) and replayed at every outer step;
-  // the graph is captured again only when the number of iterating systems
-  // changes (the system list itself is read from the device at replay).
+  // With apply.graph 1 the launches of the inner steps are captured once as a
+  // CUDA graph on the inner basis (v copied into it, z combined out of it) and
+  // replayed at every outer step; the graph is captured again only when the
+  // number of iterating systems changes (the system list itself is read from
+  // the device at replay).
   cudaGraphExec_t pexec = nullptr;
   int pexec_ra = 0;
   struct GraphGuard {
@@ -683,39 +395,37 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     const int Ra = static_cast<int>(list.size());
     set_sys(list);
     for (int q : list) st[q].near_products += inner_its;
-    if (!pgraph_on) {
-      precondition_launch(Ra, sysref(V, vs, voff), sysref(Zd, zs, zoff));
-      // a learned correction of each z, when a network is attached to the plan
-      if (const __nv_bfloat16* wl = lp_attached(P))
-        for (int q : list) lp_forward(P, wl, V + q * vs + voff, Zd + q * zs + zoff, Zd + q * zs + zoff, false, s);
-      return;
-    }
-    double2* Pv = wk[kPv];
-    double2* Pz = wk[kPz];
-    ops.copy(Ra, sysd, sysref(V, vs, voff), posref(Pv));
-    if (pexec != nullptr && pexec_ra != Ra) {
-      MLFMA_CUDA(cudaGraphExecDestroy(pexec));
-      pexec = nullptr;
-    }
-    if (pexec == nullptr) {
-      MLFMA_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      try {
-        precondition_launch(Ra, posref(Pv), posref(Pz));
-      } catch (...) {
-        cudaGraph_t gr = nullptr;
-        cudaStreamEndCapture(s, &gr);
-        if (gr) cudaGraphDestroy(gr);
-        throw;
+    ops.inner_start(Ra, sysd, sysref(V, vs, voff), sysref(Q, qs, 0), ib);
+    if (P.tuning.graph != 1) {
+      precondition_steps(Ra);
+    } else {
+      if (pexec != nullptr && pexec_ra != Ra) {
+        MLFMA_CUDA(cudaGraphExecDestroy(pexec));
+        pexec = nullptr;
       }
-      cudaGraph_t gr = nullptr;
-      MLFMA_CUDA(cudaStreamEndCapture(s, &gr));
-      const cudaError_t e = cudaGraphInstantiate(&pexec, gr, 0);
-      cudaGraphDestroy(gr);
-      MLFMA_CUDA(e);
-      pexec_ra = Ra;
+      if (pexec == nullptr) {
+        MLFMA_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        try {
+          precondition_steps(Ra);
+        } catch (...) {
+          cudaGraph_t gr = nullptr;
+          cudaStreamEndCapture(s, &gr);
+          if (gr) cudaGraphDestroy(gr);
+          throw;
+        }
+        cudaGraph_t gr = nullptr;
+        MLFMA_CUDA(cudaStreamEndCapture(s, &gr));
+        const cudaError_t e = cudaGraphInstantiate(&pexec, gr, 0);
+        cudaGraphDestroy(gr);
+        MLFMA_CUDA(e);
+        pexec_ra = Ra;
+      }
+      MLFMA_CUDA(cudaGraphLaunch(pexec, s));
     }
-    MLFMA_CUDA(cudaGraphLaunch(pexec, s));
-    ops.copy(Ra, sysd, posref(Pz), sysref(Zd, zs, zoff));
+    ops.combine(Ra, sysd, sysref(Q, qs, 0), sysref(Zd, zs, zoff), ib.m, 0, ib.y, ib.ld, false);
+    // a learned correction of each z, when a network is attached to the plan
+    if (const __nv_bfloat16* wl = lp_attached(P))
+      for (int q : list) lp_forward(P, wl, V + q * vs + voff, Zd + q * zs + zoff, Zd + q * zs + zoff, false, s);
   };
 
   const double eps = 1e-16;
@@ -732,8 +442,9 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   }
   if (!from_x.empty()) batched_apply(from_x, sysref(x, n, 0), sysref(r, n, 0));
   set_sys(all);
-  std::vector<double> rnorm = ops.norms(R, sysd, sysref(r, n, 0), sysref(b, n, 0), sysref(r, n, 0), true);
-  std::vector<double> bnorm = ops.norms(R, sysd, sysref(b, n, 0));
+  const VecRef b_all = sysref(b, n, 0);
+  std::vector<double> rnorm = ops.norms_host(R, sysd, sysref(r, n, 0), &b_all);
+  std::vector<double> bnorm = ops.norms_host(R, sysd, b_all);
   std::vector<double> error(R);
   std::vector<char> conv(R, 0);
   std::vector<int> live, total(R, 0);
@@ -755,7 +466,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     {
       std::vector<double> inv(live.size());
       for (size_t a = 0; a < live.size(); ++a) inv[a] = 1.0 / rnorm[live[a]];
-      ops.scale(static_cast<int>(live.size()), sysd, sysref(r, n, 0), sysref(V, vs, 0), inv);
+      ops.scale_host(static_cast<int>(live.size()), sysd, sysref(r, n, 0), sysref(V, vs, 0), inv);
     }
     for (int q : live) {
       st[q].restarts = cycle;
@@ -784,7 +495,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
       const int Ra = static_cast<int>(step.size());
       std::vector<std::vector<C>> hcol;
       std::vector<double> hn;
-      ops.orthogonalise(Ra, sysd, sysref(V, vs, 0), sysref(V, vs, (k + 1) * n), k + 1, hcol, hn);
+      ops.orthogonalise_host(Ra, sysd, sysref(V, vs, 0), sysref(V, vs, (k + 1) * n), k + 1, hcol, hn);
       std::vector<double> sc(Ra, 1.0);
       std::vector<int> next;
       for (int a = 0; a < Ra; ++a) {
@@ -803,7 +514,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
         hist[q].push_back(error[q]);
         if (!(error[q] < tol_rel || error[q] < tol_abs)) next.push_back(q);
       }
-      ops.scale(Ra, sysd, sysref(V, vs, (k + 1) * n), sysref(V, vs, (k + 1) * n), sc);
+      ops.scale_host(Ra, sysd, sysref(V, vs, (k + 1) * n), sysref(V, vs, (k + 1) * n), sc);
       act = next;
     }
     // update x_q with the cycle's least-squares solution, then true residuals
@@ -811,9 +522,9 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     std::vector<std::vector<C>> y(live.size());
     for (size_t a = 0; a < live.size(); ++a) {
       const int q = live[a];
-      back_substitute(H[q], ld, sv[q], std::min(k_used[q], mr), y[a]);
+      blas1::back_substitute(H[q], ld, sv[q], std::min(k_used[q], mr), y[a]);
     }
-    ops.combine(static_cast<int>(live.size()), sysd, inner_its > 0 ? sysref(Zd, zs, 0) : sysref(V, vs, 0),
+    ops.combine_host(static_cast<int>(live.size()), sysd, inner_its > 0 ? sysref(Zd, zs, 0) : sysref(V, vs, 0),
                 sysref(x, n, 0), y, true);
     const std::vector<double> rn = true_residuals(live);
     std::vector<int> keep;

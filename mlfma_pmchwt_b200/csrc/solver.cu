@@ -17,6 +17,7 @@
 #include <mutex>
 #include <string>
 
+#include "blas1.cuh"
 #include "cplx.cuh"
 #include "solver.hpp"
 
@@ -24,173 +25,7 @@ namespace mlfma {
 
 namespace {
 
-constexpr int kRB = 592;   // reduction blocks (4 per SM)
-constexpr int kRT = 256;   // threads per reduction block
-constexpr int kJT = 8;     // basis vectors per pass of dots_kernel
-
-__device__ __forceinline__ double2 block_sum(double2 v, double2* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = lane < (blockDim.x >> 5) ? sh[lane] : c2(0.0, 0.0);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-  }
-  return v;  // valid in thread 0
-}
-
-// partial[blk * ldp + j] = sum over this block's rows of conj(V_j) w, j < nv
-__global__ void __launch_bounds__(kRT) dots_kernel(const double2* __restrict__ V, long long n, int nv,
-                                                   const double2* __restrict__ w, double2* __restrict__ partial,
-                                                   int ldp) {
-  __shared__ double2 sh[kRT / 32];
-  for (int j0 = 0; j0 < nv; j0 += kJT) {
-    double2 acc[kJT];
-#pragma unroll
-    for (int q = 0; q < kJT; ++q) acc[q] = c2(0.0, 0.0);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-      const double2 wi = w[i];
-#pragma unroll
-      for (int q = 0; q < kJT; ++q)
-        if (j0 + q < nv) {
-          const double2 v = V[(long long)(j0 + q) * n + i];
-          // conj(v) * wi
-          acc[q].x = fma(v.x, wi.x, fma(v.y, wi.y, acc[q].x));
-          acc[q].y = fma(v.x, wi.y, fma(-v.y, wi.x, acc[q].y));
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < kJT; ++q)
-      if (j0 + q < nv) {
-        const double2 s = block_sum(acc[q], sh);
-        if (threadIdx.x == 0) partial[(long long)blockIdx.x * ldp + j0 + q] = s;
-      }
-  }
-}
-
-// out[j] = sum over blocks of partial[blk * ldp + j] (+ add[j] if add != null)
-__global__ void reduce_kernel(const double2* __restrict__ partial, int nblk, int ldp, int nv, double2* out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nv) return;
-  double2 s = c2(0.0, 0.0);
-  for (int b = 0; b < nblk; ++b) s = cadd(s, partial[(long long)b * ldp + j]);
-  out[j] = s;
-}
-
-// w -= sum_j V_j h[j]; with norm != 0 also per-block partial ||w||^2 into partial[blk*ldp]
-__global__ void __launch_bounds__(kRT) update_kernel(const double2* __restrict__ V, long long n, int nv,
-                                                     const double2* __restrict__ h, double2* __restrict__ w,
-                                                     int want_norm, double2* __restrict__ partial, int ldp) {
-  __shared__ double2 hs[64];
-  __shared__ double2 sh[kRT / 32];
-  for (int j = threadIdx.x; j < nv; j += blockDim.x) hs[j] = h[j];
-  __syncthreads();
-  double2 nrm = c2(0.0, 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double2 wi = w[i];
-    for (int j = 0; j < nv; ++j) wi = csub(wi, cmul(hs[j], V[(long long)j * n + i]));
-    w[i] = wi;
-    nrm.x = fma(wi.x, wi.x, fma(wi.y, wi.y, nrm.x));
-  }
-  if (want_norm) {
-    const double2 s = block_sum(nrm, sh);
-    if (threadIdx.x == 0) partial[(long long)blockIdx.x * ldp] = s;
-  }
-}
-
-// r = b - w, partial ||r||^2
-__global__ void __launch_bounds__(kRT) residual_kernel(const double2* __restrict__ b, const double2* __restrict__ w,
-                                                       double2* __restrict__ r, long long n,
-                                                       double2* __restrict__ partial) {
-  __shared__ double2 sh[kRT / 32];
-  double2 nrm = c2(0.0, 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double2 v = csub(b[i], w[i]);
-    r[i] = v;
-    nrm.x = fma(v.x, v.x, fma(v.y, v.y, nrm.x));
-  }
-  const double2 s = block_sum(nrm, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
-__global__ void norm_kernel(const double2* __restrict__ v, long long n, double2* __restrict__ partial) {
-  __shared__ double2 sh[kRT / 32];
-  double2 nrm = c2(0.0, 0.0);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double2 a = v[i];
-    nrm.x = fma(a.x, a.x, fma(a.y, a.y, nrm.x));
-  }
-  const double2 s = block_sum(nrm, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
-__global__ void scale_kernel(const double2* __restrict__ src, double inv, double2* __restrict__ dst, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = cscale(src[i], inv);
-}
-
-// x += sum_j V_j y[j]
-__global__ void combine_kernel(const double2* __restrict__ V, long long n, int m, const double2* __restrict__ y,
-                               double2* __restrict__ x) {
-  __shared__ double2 ys[64];
-  for (int j = threadIdx.x; j < m; j += blockDim.x) ys[j] = y[j];
-  __syncthreads();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    double2 xi = x[i];
-    for (int j = 0; j < m; ++j) xi = cfma(ys[j], V[(long long)j * n + i], xi);
-    x[i] = xi;
-  }
-}
-
 using C = std::complex<double>;
-
-// Code/GMRES.h:22-40
-void givens_make(C a, C b, C& c, C& s) {
-  const double eps = 1e-16;
-  const double an = std::abs(a), bn = std::abs(b);
-  if (bn < eps) {
-    c = 1.0;
-    s = 0.0;
-  } else if (an < eps) {
-    c = 0.0;
-    s = 1.0;
-  } else {
-    const double r = std::sqrt(std::real(a * std::conj(a) + b * std::conj(b)));
-    c = a / r;
-    s = b / r;
-  }
-}
-// Code/GMRES.h:43-48
-void givens_apply(C& x, C& y, C c, C s) {
-  const C t = std::conj(c) * x + std::conj(s) * y;
-  y = -s * x + c * y;
-  x = t;
-}
-
-struct GmresWork {
-  double2 *x = nullptr, *b = nullptr, *r = nullptr, *w = nullptr, *V = nullptr, *h = nullptr, *part = nullptr,
-          *y = nullptr;
-  std::vector<void*> owned;
-  ~GmresWork() {
-    for (void* p : owned) cudaFree(p);
-  }
-  double2* get(size_t count) {
-    void* p = nullptr;
-    MLFMA_CUDA(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(double2)));
-    owned.push_back(p);
-    return static_cast<double2*>(p);
-  }
-};
 
 }  // namespace
 
@@ -201,41 +36,26 @@ bool gmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, do
   MLFMA_CUDA(cudaSetDevice(P.device));
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
-  const int ldp = mr + 2;
-  GmresWork g;
-  g.x = g.get(n);
-  g.b = g.get(n);
-  g.r = g.get(n);
-  g.w = g.get(n);
-  g.V = g.get(static_cast<size_t>(mr + 1) * n);
-  g.h = g.get(2 * (mr + 2));
-  g.part = g.get(static_cast<size_t>(kRB) * ldp);
-  g.y = g.get(mr + 1);
-  MLFMA_CUDA(cudaMemcpyAsync(g.x, xh, n * sizeof(double2), cudaMemcpyHostToDevice, s));
-  MLFMA_CUDA(cudaMemcpyAsync(g.b, rhs, n * sizeof(double2), cudaMemcpyHostToDevice, s));
+  blas1::Work g;
+  double2* x = g.get(n);
+  double2* b = g.get(n);
+  double2* r = g.get(n);
+  double2* w = g.get(n);
+  double2* V = g.get(static_cast<size_t>(mr + 1) * n);
+  double2* yd = g.get(mr + 1);
+  blas1::Ops ops = blas1::make_ops(g, s, n);
+  MLFMA_CUDA(cudaMemcpyAsync(x, xh, n * sizeof(double2), cudaMemcpyHostToDevice, s));
+  MLFMA_CUDA(cudaMemcpyAsync(b, rhs, n * sizeof(double2), cudaMemcpyHostToDevice, s));
   st = SolveStats();
   history.clear();
 
-  auto norm_of = [&](const double2* v) {
-    norm_kernel<<<kRB, kRT, 0, s>>>(v, n, g.part);
-    reduce_kernel<<<1, 64, 0, s>>>(g.part, kRB, 1, 1, g.h);
-    C out;
-    MLFMA_CUDA(cudaMemcpyAsync(&out, g.h, sizeof(double2), cudaMemcpyDeviceToHost, s));
-    MLFMA_CUDA(cudaStreamSynchronize(s));
-    return std::sqrt(out.real());
-  };
   auto true_residual = [&]() {
-    apply_device(P, g.x, g.w, s);
+    apply_device(P, x, r, s);
     st.matvecs++;
-    residual_kernel<<<kRB, kRT, 0, s>>>(g.b, g.w, g.r, n, g.part);
-    reduce_kernel<<<1, 64, 0, s>>>(g.part, kRB, 1, 1, g.h);
-    C out;
-    MLFMA_CUDA(cudaMemcpyAsync(&out, g.h, sizeof(double2), cudaMemcpyDeviceToHost, s));
-    MLFMA_CUDA(cudaStreamSynchronize(s));
-    return std::sqrt(out.real());
+    return ops.residual(b, r);
   };
   auto finish = [&](bool ok, double err) {
-    MLFMA_CUDA(cudaMemcpyAsync(xh, g.x, n * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    MLFMA_CUDA(cudaMemcpyAsync(xh, x, n * sizeof(double2), cudaMemcpyDeviceToHost, s));
     MLFMA_CUDA(cudaStreamSynchronize(s));
     st.rel_residual = err;
     st.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -244,18 +64,17 @@ bool gmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, do
 
   const double eps = 1e-16;
   double rnorm = true_residual();
-  double bnorm = norm_of(g.b);
+  double bnorm = ops.norm(b);
   if (bnorm < eps) bnorm = 1.0;
   double error = rnorm / bnorm;
   if (error < tol_rel || error < tol_abs) return finish(true, error);
 
   const int ld = mr + 1;
-  std::vector<C> H(static_cast<size_t>(ld) * mr), cs(mr), sn(mr), sv(mr + 1), y(mr);
-  std::vector<C> h1, h2;
+  std::vector<C> H(static_cast<size_t>(ld) * mr), cs(mr), sn(mr), sv(mr + 1), y, hcol;
   int total = 0;
   for (int cycle = 1; cycle <= itr_max; ++cycle) {
     st.restarts = cycle;
-    scale_kernel<<<kRB, kRT, 0, s>>>(g.r, 1.0 / rnorm, g.V, n);
+    ops.scale(r, 1.0 / rnorm, V);
     std::fill(sv.begin(), sv.end(), C(0.0));
     sv[0] = rnorm;
     std::fill(H.begin(), H.end(), C(0.0));
@@ -266,51 +85,27 @@ bool gmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, do
       if (total >= itr_max) break;
       ++total;
       k_used = k + 1;
-      apply_device(P, g.V + static_cast<long long>(k) * n, g.w, s);
+      apply_device(P, V + static_cast<long long>(k) * n, w, s);
       st.matvecs++;
-      const int nv = k + 1;
-      // first projection
-      dots_kernel<<<kRB, kRT, 0, s>>>(g.V, n, nv, g.w, g.part, ldp);
-      reduce_kernel<<<(nv + 63) / 64, 64, 0, s>>>(g.part, kRB, ldp, nv, g.h);
-      update_kernel<<<kRB, kRT, 0, s>>>(g.V, n, nv, g.h, g.w, 0, g.part, ldp);
-      h1.resize(nv);
-      MLFMA_CUDA(cudaMemcpyAsync(h1.data(), g.h, nv * sizeof(double2), cudaMemcpyDeviceToHost, s));
-      // re-projection
-      dots_kernel<<<kRB, kRT, 0, s>>>(g.V, n, nv, g.w, g.part, ldp);
-      reduce_kernel<<<(nv + 63) / 64, 64, 0, s>>>(g.part, kRB, ldp, nv, g.h + ldp);
-      update_kernel<<<kRB, kRT, 0, s>>>(g.V, n, nv, g.h + ldp, g.w, 1, g.part, ldp);
-      reduce_kernel<<<1, 64, 0, s>>>(g.part, kRB, ldp, 1, g.h + 2 * ldp - 1);
-      h2.resize(nv + 1);
-      MLFMA_CUDA(cudaMemcpyAsync(h2.data(), g.h + ldp, nv * sizeof(double2), cudaMemcpyDeviceToHost, s));
-      MLFMA_CUDA(cudaMemcpyAsync(&h2[nv], g.h + 2 * ldp - 1, sizeof(double2), cudaMemcpyDeviceToHost, s));
-      MLFMA_CUDA(cudaStreamSynchronize(s));
-      for (int j = 0; j <= k; ++j) H[j + static_cast<size_t>(k) * ld] = h1[j] + h2[j];
-      const double h_next = std::sqrt(h2[nv].real());
+      const double h_next = ops.orthogonalise_host(V, k + 1, w, hcol);
+      for (int j = 0; j <= k; ++j) H[j + static_cast<size_t>(k) * ld] = hcol[j];
       H[k + 1 + static_cast<size_t>(k) * ld] = h_next;
       if (h_next < eps * rnorm) break;  // Krylov space exhausted (Code/GMRES.h:136-139)
-      scale_kernel<<<kRB, kRT, 0, s>>>(g.w, 1.0 / h_next, g.V + static_cast<long long>(k + 1) * n, n);
-      for (int j = 0; j < k; ++j) givens_apply(H[j + k * ld], H[j + 1 + k * ld], cs[j], sn[j]);
-      givens_make(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
-      givens_apply(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
+      ops.scale(w, 1.0 / h_next, V + static_cast<long long>(k + 1) * n);
+      for (int j = 0; j < k; ++j) blas1::givens_apply(H[j + k * ld], H[j + 1 + k * ld], cs[j], sn[j]);
+      blas1::givens_make(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
+      blas1::givens_apply(H[k + k * ld], H[k + 1 + k * ld], cs[k], sn[k]);
       H[k + 1 + k * ld] = C(0.0);
-      givens_apply(sv[k], sv[k + 1], cs[k], sn[k]);
+      blas1::givens_apply(sv[k], sv[k + 1], cs[k], sn[k]);
       error = std::abs(sv[k + 1]) / bnorm;
       history.push_back(error);
       if (error < tol_rel || error < tol_abs) break;
     }
-    // upper-triangular solve (Code/GMRES.h:165-182)
     const int m = std::min(k_used, mr);
-    for (int i = m - 1; i >= 0; --i) {
-      y[i] = sv[i];
-      for (int j = i + 1; j < m; ++j) y[i] -= H[i + j * ld] * y[j];
-      if (std::abs(H[i + i * ld]) > eps)
-        y[i] /= H[i + i * ld];
-      else
-        y[i] = C(0.0);
-    }
+    blas1::back_substitute(H, ld, sv, m, y);
     if (m > 0) {
-      MLFMA_CUDA(cudaMemcpyAsync(g.y, y.data(), m * sizeof(double2), cudaMemcpyHostToDevice, s));
-      combine_kernel<<<kRB, kRT, 0, s>>>(g.V, n, m, g.y, g.x);
+      MLFMA_CUDA(cudaMemcpyAsync(yd, y.data(), m * sizeof(double2), cudaMemcpyHostToDevice, s));
+      ops.combine(1, nullptr, ops.ref(V), ops.ref(x), nullptr, m, yd, 0, true);
     }
     rnorm = true_residual();
     error = rnorm / bnorm;
@@ -427,7 +222,7 @@ __global__ void __launch_bounds__(256) rcs_kernel(RcsArg a, const double* __rest
     }
   }
   for (int c = 0; c < 3; ++c) {
-    const double2 v = block_sum(acc[c], sh);
+    const double2 v = blas1::block_sum(acc[c], sh);
     if (threadIdx.x == 0) out[3 * blockIdx.x + c] = v;
   }
 }
@@ -633,7 +428,7 @@ __global__ void __launch_bounds__(256) rcs_angles_kernel(RcsArg a, const double*
     }
   }
   for (int c = 0; c < 3; ++c) {
-    const double2 v = block_sum(acc[c], sh);
+    const double2 v = blas1::block_sum(acc[c], sh);
     if (threadIdx.x == 0) out[3 * blockIdx.x + c] = v;
   }
 }
