@@ -24,6 +24,7 @@
 
 #include "cplx.cuh"
 #include "plan.hpp"
+#include "reduce.cuh"
 
 namespace mlfma {
 namespace blas1 {
@@ -153,26 +154,6 @@ enum Finish {
   kFinishStep,   // inner GMRES: column j of H, its rotations, the scale of the next vector;
                  // after the last step the solution of the triangular system
 };
-
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
-
-// Sum over the block, valid in thread 0 (sh: one value per warp).
-__device__ __forceinline__ double2 block_sum(double2 v, double2* sh) {
-  v = warp_sum2(v);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  if (w == 0) v = warp_sum2(lane < (blockDim.x >> 5) ? sh[lane] : c2(0.0, 0.0));
-  return v;
-}
 
 // Sums 8 values over the warp; value q ends up in the lanes with (lane >> 2)
 // & 7 == q (bit-reversed halves: 9 shuffles of a complex value instead of 40).

@@ -11,10 +11,13 @@
 // allocate nothing and accept pageable or pinned host tables alike.
 // Quadrature points are formed once per (RWG, point) and reused for every
 // incidence of a chunk.
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <stdexcept>
 
 #include "cplx.cuh"
+#include "reduce.cuh"
 #include "solver.hpp"
 
 namespace mlfma {
@@ -22,8 +25,12 @@ namespace {
 
 constexpr int kRhsChunk = 128;   // incidences per excitation launch (9 KB of parameters)
 constexpr int kRhsTile = 8;      // incidences per thread (grid.y tiles)
-constexpr int kFarChunk = 256;   // angles per bistatic launch (6 KB of parameters)
-constexpr int kFarTile = 4;      // solutions per block of the bistatic far field
+constexpr int kFarChunk = 512;   // angles per far-field launch (12 KB of parameters)
+constexpr int kFarAngles = 4;    // angles and
+constexpr int kFarSols = 32;     // solutions per cluster of the bistatic far field
+constexpr int kFarRwgs = 256;    // RWGs whose moments a block stages at a time
+constexpr int kFarSlices = 8;    // blocks of a cluster, each with a slice of the RWGs
+constexpr int kFarThreads = 512;
 
 struct Geo {
   const double* xyz;
@@ -59,6 +66,12 @@ Geo geo(const Plan& P) {
   return g;
 }
 
+__device__ __forceinline__ void load3(const double* p, double* o) {
+  o[0] = p[0];
+  o[1] = p[1];
+  o[2] = p[2];
+}
+
 // Quadrature point i of side `side` (0: T+, 1: T-) of RWG m: position p and
 // the RWG vector rho (p - free vertex on T+, free vertex - p on T-).
 __device__ __forceinline__ void rwg_point(const Geo& g, int m, int side, int i, double p[3], double rho[3]) {
@@ -72,27 +85,6 @@ __device__ __forceinline__ void rwg_point(const Geo& g, int m, int side, int i, 
     p[c] = g.l1[i] * A[c] + g.l2[i] * B[c] + g.l3[i] * Cc[c];
     rho[c] = side ? fv[c] - p[c] : p[c] - fv[c];
   }
-}
-
-__device__ __forceinline__ double2 block_sum(double2 v, double2* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = lane < (blockDim.x >> 5) ? sh[lane] : c2(0.0, 0.0);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-  }
-  return v;  // valid in thread 0
 }
 
 struct RhsBatchArg {
@@ -140,28 +132,101 @@ __global__ void __launch_bounds__(128) rhs_batch_kernel(const __grid_constant__ 
     }
 }
 
-// The far-field factors of RWG m in direction r: F_J = sum l w (I - r r) rho
-// e^{+j k1 r.p} and F_M = sum l w (r x rho) e^{+j k1 r.p} (Code/RCS.h:140-170).
-__device__ __forceinline__ void far_factors(const Geo& g, int m, const double r[3], double2 FJ[3], double2 FM[3]) {
+// sin and cos of |x| <= 1 by their Taylor series (the first terms left out
+// are below 1e-17 and 5e-19)
+__device__ __forceinline__ void sincos_series(double x, double* sn, double* cs) {
+  const double z = x * x;
+  double s = 1.0 / 355687428096000.0, c = -1.0 / 6402373705728000.0;
+  s = fma(s, z, -1.0 / 1307674368000.0);
+  c = fma(c, z, 1.0 / 20922789888000.0);
+  s = fma(s, z, 1.0 / 6227020800.0);
+  c = fma(c, z, -1.0 / 87178291200.0);
+  s = fma(s, z, -1.0 / 39916800.0);
+  c = fma(c, z, 1.0 / 479001600.0);
+  s = fma(s, z, 1.0 / 362880.0);
+  c = fma(c, z, -1.0 / 3628800.0);
+  s = fma(s, z, -1.0 / 5040.0);
+  c = fma(c, z, 1.0 / 40320.0);
+  s = fma(s, z, 1.0 / 120.0);
+  c = fma(c, z, -1.0 / 720.0);
+  s = fma(s, z, -1.0 / 6.0);
+  c = fma(c, z, 1.0 / 24.0);
+  c = fma(c, z, -0.5);
+  *sn = fma(s * z, x, x);
+  *cs = fma(c, z, 1.0);
+}
+
+// An orthonormal basis u, v of the plane across the unit vector r, u x v = r
+__device__ __forceinline__ void transverse(const double r[3], double u[3], double v[3]) {
+  const bool z = fabs(r[2]) < 0.9;
+  u[0] = z ? -r[1] : 0.0;
+  u[1] = z ? r[0] : -r[2];
+  u[2] = z ? 0.0 : r[1];
+  const double q = 1.0 / sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  for (int c = 0; c < 3; ++c) u[c] *= q;
+  v[0] = r[1] * u[2] - r[2] * u[1];
+  v[1] = r[2] * u[0] - r[0] * u[2];
+  v[2] = r[0] * u[1] - r[1] * u[0];
+}
+
+// The far-field moment A = sum l w rho e^{+j k1 r.p} of RWG m along u and v.
+// The reference's factors (Code/RCS.h:140-170) follow from it: sum l w (I - r r)
+// rho e = Au u + Av v and sum l w (r x rho) e = Au v - Av u.
+// Per triangle, with the phase of its centroid taken out: the moments of the
+// three barycentric coordinates, M_j = sum_q w l_j e^{j k1 r.(p - centroid)},
+// then rho = sum_j l_j (v_j - v_free). Phases up to 1 rad from the centroid
+// (vertices within 0.16 wavelengths) and a real k1 take the series instead
+// of a sine, a cosine and an exponential per point: 7 points cost a third.
+__device__ __forceinline__ void far_moment(const Geo& g, int m, const double r[3], const double u[3],
+                                           const double v[3], double2& Au, double2& Av) {
+  Au = Av = c2(0.0, 0.0);
   const double ln = g.len[m];
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const int f = side ? g.fneg[m] : g.fpos[m];
+    const double* fv = &g.xyz[3 * (side ? g.vneg[m] : g.vpos[m])];
+    double X[3][3], d[3], tc = 0.0;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) FJ[c] = FM[c] = c2(0.0, 0.0);
-  for (int i = 0; i < g.nq; ++i) {
-    for (int side = 0; side < 2; ++side) {
-      double p[3], rho[3];
-      rwg_point(g, m, side, i, p, rho);
-      const double t = p[0] * r[0] + p[1] * r[1] + p[2] * r[2];
-      const double2 e = cexp(make_double2(-g.k1.y * t, g.k1.x * t));
-      const double rr = r[0] * rho[0] + r[1] * rho[1] + r[2] * rho[2];
-      const double Ft[3] = {rho[0] - r[0] * rr, rho[1] - r[1] * rr, rho[2] - r[2] * rr};
-      const double Fm[3] = {r[1] * rho[2] - r[2] * rho[1], r[2] * rho[0] - r[0] * rho[2],
-                            r[0] * rho[1] - r[1] * rho[0]};
-      const double wf = ln * g.w[i];
+    for (int j = 0; j < 3; ++j) load3(&g.xyz[3 * g.face_v[3 * f + j]], X[j]);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        FJ[c] = cadd(FJ[c], cscale(e, wf * Ft[c]));
-        FM[c] = cadd(FM[c], cscale(e, wf * Fm[c]));
+    for (int c = 0; c < 3; ++c) {
+      const double ctr = (X[0][c] + X[1][c] + X[2][c]) * (1.0 / 3.0);
+      tc = fma(r[c], ctr, tc);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) d[j] = fma(r[c], X[j][c] - ctr, c == 0 ? 0.0 : d[j]);
+    }
+    const double2 e0 = cexp(make_double2(-g.k1.y * tc, g.k1.x * tc));
+    double2 M[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) M[j] = c2(0.0, 0.0);
+    if (g.k1.y == 0.0 && fabs(g.k1.x) * fmax(fabs(d[0]), fmax(fabs(d[1]), fabs(d[2]))) <= 1.0) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) d[j] *= g.k1.x;
+      for (int i = 0; i < g.nq; ++i) {
+        double sn, cs;
+        sincos_series(g.l1[i] * d[0] + g.l2[i] * d[1] + g.l3[i] * d[2], &sn, &cs);
+        sn *= g.w[i];
+        cs *= g.w[i];
+        M[0] = cadd(M[0], c2(cs * g.l1[i], sn * g.l1[i]));
+        M[1] = cadd(M[1], c2(cs * g.l2[i], sn * g.l2[i]));
+        M[2] = cadd(M[2], c2(cs * g.l3[i], sn * g.l3[i]));
       }
+    } else {
+      for (int i = 0; i < g.nq; ++i) {
+        const double t = g.l1[i] * d[0] + g.l2[i] * d[1] + g.l3[i] * d[2];
+        const double2 e = cscale(cexp(make_double2(-g.k1.y * t, g.k1.x * t)), g.w[i]);
+        M[0] = cadd(M[0], cscale(e, g.l1[i]));
+        M[1] = cadd(M[1], cscale(e, g.l2[i]));
+        M[2] = cadd(M[2], cscale(e, g.l3[i]));
+      }
+    }
+    const double2 e = cscale(e0, side ? -ln : ln);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double q[3] = {X[j][0] - fv[0], X[j][1] - fv[1], X[j][2] - fv[2]};
+      const double2 t = cmul(e, M[j]);
+      Au = cfmas(q[0] * u[0] + q[1] * u[1] + q[2] * u[2], t, Au);
+      Av = cfmas(q[0] * v[0] + q[1] * v[1] + q[2] * v[2], t, Av);
     }
   }
 }
@@ -174,41 +239,114 @@ struct FarBatchArg {
   double2* out;      // [R][n_total_angles][3]
 };
 
-// block per (angle, tile of kFarTile solutions): E = -j k1 (F_J . I_J - F_M . I_M)
-__global__ void __launch_bounds__(256) far_batch_kernel(const __grid_constant__ FarBatchArg a) {
-  __shared__ double2 sh[8];
+// E = -j k1 (F_M . I_M - F_J . I_J), bistatic: cluster of kFarSlices blocks per
+// (kFarAngles angles, kFarSols solutions), each block over a slice of the RWGs.
+// A block forms the moments of kFarRwgs RWGs at its angles once, in shared
+// memory, for all its solutions; a warp then sums 2 solutions x 4 angles
+// over 32 RWGs at a time (with fewer than 16 pairs of solutions the warps
+// share the RWGs). The blocks' sums meet in distributed shared memory, in
+// rank order.
+// FP64-bound: 361 angles x 32 solutions x 30,720 RWGs are ~0.35 ms of moments
+// and 0.31 ms of sums at the FP64 rate. With a block per (angle, 4
+// solutions), which formed the factors once per 4 solutions from 14 sincos
+// and exp each, that call took 12.3 ms; now 1.5 ms.
+__global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads, 1)
+    far_batch_kernel(const __grid_constant__ FarBatchArg a) {
+  __shared__ double2 A[kFarAngles][2][kFarRwgs];
+  __shared__ double2 sums[kFarSols * kFarAngles * 2];
   const Geo& g = a.g;
-  const int ang = blockIdx.x;
-  const int r0 = blockIdx.y * kFarTile;
-  const int nr = min(kFarTile, a.R - r0);
-  const double r[3] = {a.dir[ang][0], a.dir[ang][1], a.dir[ang][2]};
+  const int ang0 = blockIdx.x * kFarAngles, na = min(kFarAngles, a.n_angles - ang0);
+  const int r0 = blockIdx.y * kFarSols, nr = min(kFarSols, a.R - r0);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  constexpr int kW = kFarThreads / 32;
+  const int npair = (nr + 1) / 2, nsub = kW / npair;
+  const int pair = wp % npair, sub = wp / npair;
+  const bool working = sub < nsub;
+  const bool two = 2 * pair + 1 < nr;
   const size_t n = 2 * static_cast<size_t>(g.N);
-  double2 acc[kFarTile][3];
+  const double2* I0 = a.I + (r0 + 2 * pair) * n;
+  const double2* I1 = two ? I0 + n : I0;
+  double2 acc[2][kFarAngles][2];
 #pragma unroll
-  for (int q = 0; q < kFarTile; ++q)
+  for (int q = 0; q < 2; ++q)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[q][c] = c2(0.0, 0.0);
-  for (int m = threadIdx.x; m < g.N; m += blockDim.x) {
-    double2 FJ[3], FM[3];
-    far_factors(g, m, r, FJ, FM);
+    for (int t = 0; t < kFarAngles; ++t) acc[q][t][0] = acc[q][t][1] = c2(0.0, 0.0);
+  const int tiles = (g.N + kFarRwgs - 1) / kFarRwgs;
+  for (int tile = blockIdx.z; tile < tiles; tile += kFarSlices) {
+    const int m0 = tile * kFarRwgs;
+    __syncthreads();
+    {
+      const int q = threadIdx.x & (kFarRwgs - 1), m = m0 + q;
+#pragma unroll 1
+      for (int t = threadIdx.x / kFarRwgs; t < kFarAngles; t += kFarThreads / kFarRwgs) {
+        double2 Au = c2(0.0, 0.0), Av = c2(0.0, 0.0);
+        if (m < g.N && t < na) {
+          double u[3], v[3];
+          transverse(a.dir[ang0 + t], u, v);
+          far_moment(g, m, a.dir[ang0 + t], u, v, Au, Av);
+        }
+        A[t][0][q] = Au;
+        A[t][1][q] = Av;
+      }
+    }
+    __syncthreads();
+    if (working) {
+#pragma unroll 2
+      for (int c = sub; c < kFarRwgs / 32; c += nsub) {
+        const int q = 32 * c + lane, m = min(m0 + q, g.N - 1);  // moments beyond N are zero
+        const double2 J0 = __ldg(I0 + m), M0 = __ldg(I0 + g.N + m);
+        const double2 J1 = __ldg(I1 + m), M1 = __ldg(I1 + g.N + m);
 #pragma unroll
-    for (int q = 0; q < kFarTile; ++q) {
-      if (q < nr) {
-        const double2 IJ = a.I[(r0 + q) * n + m], IM = a.I[(r0 + q) * n + g.N + m];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc[q][c] = cadd(acc[q][c], csub(cmul(FM[c], IM), cmul(FJ[c], IJ)));
+        for (int t = 0; t < kFarAngles; ++t) {
+          const double2 u = A[t][0][q], v = A[t][1][q], mu = cneg(u), mv = cneg(v);
+          acc[0][t][0] = cfma(mv, M0, cfma(mu, J0, acc[0][t][0]));
+          acc[0][t][1] = cfma(u, M0, cfma(mv, J0, acc[0][t][1]));
+          acc[1][t][0] = cfma(mv, M1, cfma(mu, J1, acc[1][t][0]));
+          acc[1][t][1] = cfma(u, M1, cfma(mv, J1, acc[1][t][1]));
+        }
       }
     }
   }
-  const double2 coeff = c2(g.k1.y, -g.k1.x);  // -j k1 ... applied as -j k1 (-F_J I_J + F_M I_M)
+  __syncthreads();
+  double2* red = &A[0][0][0];  // [kW][2 x kFarAngles x 2]
+  constexpr int kPer = 2 * kFarAngles * 2;
 #pragma unroll
-  for (int q = 0; q < kFarTile; ++q)
+  for (int q = 0; q < 2; ++q)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double2 v = block_sum(acc[q][c], sh);
-      if (threadIdx.x == 0 && q < nr)
-        a.out[((r0 + q) * static_cast<size_t>(a.n_total_angles) + a.angle0 + ang) * 3 + c] = cmul(coeff, v);
+    for (int t = 0; t < kFarAngles; ++t)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const double2 v = blas1::warp_sum2(acc[q][t][c]);
+        if (lane == 0) red[wp * kPer + (q * kFarAngles + t) * 2 + c] = v;
+      }
+  __syncthreads();
+  for (int i = threadIdx.x; i < npair * kPer; i += kFarThreads) {
+    const int p = i / kPer, e = i - p * kPer;
+    double2 v = c2(0.0, 0.0);
+    for (int q = 0; q < nsub; ++q) v = cadd(v, red[(q * npair + p) * kPer + e]);
+    sums[i] = v;
+  }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (cl.block_rank() == 0) {
+    const double2 coeff = c2(g.k1.y, -g.k1.x);  // -j k1
+    for (int i = threadIdx.x; i < nr * na; i += kFarThreads) {
+      const int rr = i / na, t = i - rr * na;
+      double2 su = c2(0.0, 0.0), sv = c2(0.0, 0.0);
+      for (int q = 0; q < kFarSlices; ++q) {
+        const double2* o = cl.map_shared_rank(&sums[0], q) + (rr / 2) * kPer + ((rr & 1) * kFarAngles + t) * 2;
+        su = cadd(su, o[0]);
+        sv = cadd(sv, o[1]);
+      }
+      double u[3], v[3];
+      transverse(a.dir[ang0 + t], u, v);
+      double2* out = a.out + ((r0 + rr) * static_cast<size_t>(a.n_total_angles) + a.angle0 + ang0 + t) * 3;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out[c] = cmul(coeff, cadd(cscale(su, u[c]), cscale(sv, v[c])));
     }
+  }
+  cl.sync();  // the other blocks' sums stay until rank 0 has read them
 }
 
 struct FarMonoArg {
@@ -225,21 +363,24 @@ __global__ void __launch_bounds__(256) far_mono_kernel(const __grid_constant__ F
   const Geo& g = a.g;
   const int q = blockIdx.x;
   const double r[3] = {a.dir[q][0], a.dir[q][1], a.dir[q][2]};
+  double u[3], v[3];
+  transverse(r, u, v);
   const double2* I = a.I + (a.r0 + q) * 2 * static_cast<size_t>(g.N);
-  double2 acc[3] = {c2(0.0, 0.0), c2(0.0, 0.0), c2(0.0, 0.0)};
+  double2 su = c2(0.0, 0.0), sv = c2(0.0, 0.0);
   for (int m = threadIdx.x; m < g.N; m += blockDim.x) {
-    double2 FJ[3], FM[3];
-    far_factors(g, m, r, FJ, FM);
+    double2 Au, Av;
+    far_moment(g, m, r, u, v, Au, Av);
     const double2 IJ = I[m], IM = I[g.N + m];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = cadd(acc[c], csub(cmul(FM[c], IM), cmul(FJ[c], IJ)));
+    su = csub(csub(su, cmul(Av, IM)), cmul(Au, IJ));
+    sv = csub(cadd(sv, cmul(Au, IM)), cmul(Av, IJ));
   }
   const double2 coeff = c2(g.k1.y, -g.k1.x);
+  su = blas1::block_sum(su, sh);
+  sv = blas1::block_sum(sv, sh);
+  if (threadIdx.x == 0)
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const double2 v = block_sum(acc[c], sh);
-    if (threadIdx.x == 0) a.out[(a.r0 + q) * 3 + c] = cmul(coeff, v);
-  }
+    for (int c = 0; c < 3; ++c)
+      a.out[(a.r0 + q) * 3 + c] = cmul(coeff, cadd(cscale(su, u[c]), cscale(sv, v[c])));
 }
 
 // Code/RCS.h:120-123: observation direction of (theta, phi) in degrees
@@ -287,8 +428,8 @@ void rcs_pmchwt_batch(Plan& P, int R, const double2* I_dev, int n_angles, const 
     a.n_angles = std::min(kFarChunk, n_angles - c0);
     a.angle0 = c0;
     for (int q = 0; q < a.n_angles; ++q) direction(theta_deg[c0 + q], phi_deg[c0 + q], a.dir[q]);
-    const dim3 grid(a.n_angles, (R + kFarTile - 1) / kFarTile);
-    far_batch_kernel<<<grid, 256, 0, s>>>(a);
+    const dim3 grid((a.n_angles + kFarAngles - 1) / kFarAngles, (R + kFarSols - 1) / kFarSols, kFarSlices);
+    far_batch_kernel<<<grid, kFarThreads, 0, s>>>(a);
     MLFMA_CUDA(cudaGetLastError());
   }
 }
