@@ -279,6 +279,14 @@ __device__ __forceinline__ void inner_step(const Inner& I, int a, int j, const d
   for (int i = m + lane; i < I.inner; i += 32) y[i] = c2(0.0, 0.0);
 }
 
+// A complex64 copy of the vector worked on, for the lockstep near-field
+// product: the positions in groups of sys, and per RWG the (J, M) pairs of a
+// group side by side, [group][RWG][position][J, M]. Null: none.
+struct Pack {
+  float2* p;
+  int sys;
+};
+
 struct GsArg {
   VecRef V, w;           // basis (vector j at V + j * n) and the vector worked on
   VecRef b;              // Norm: subtracted from, r = b - w written to w (has_b)
@@ -296,7 +304,14 @@ struct GsArg {
   unsigned* count;       // [a] blocks done
   Inner inner;
   int step;
+  Pack pack;
 };
+
+// The packed copy's slot of row i of position a
+__device__ __forceinline__ void pack_row(const Pack& p, long long n, int a, long long i, double2 v) {
+  const long long half = n / 2, id = i < half ? i : i - half;
+  p.p[(((a / p.sys) * half + id) * p.sys + a % p.sys) * 2 + (i >= half)] = Cx<float2>::from(v);
+}
 
 // E rows of each operand per thread and chunk. kProject: w -= sum_j hin_j V_j.
 // kDots: the dot products conj(V_j) . w of the (updated) w; else its squared
@@ -378,6 +393,7 @@ static __global__ void __launch_bounds__(kThreads) gs_kernel(const __grid_consta
             w[at[e]] = wi[e];
           }
           if (cp) cp[at[e]] = wi[e];
+          if (kFin != kFinishNone && g.pack.p) pack_row(g.pack, n, a, at[e], wi[e]);
           nrm.x = fma(wi[e].x, wi[e].x, fma(wi[e].y, wi[e].y, nrm.x));
         }
     }
@@ -512,6 +528,21 @@ struct Work {
   }
 };
 
+// The work arrays of one solve from the plan's arena (at most `values` complex
+// values, pieces rounded up to 256 bytes included): a driver allocation costs
+// milliseconds, and a solve at 34,560 unknowns made 20 of them, 4.5 of its 38
+// ms. The block stays with the plan for its next solve, up to the arena's
+// bound.
+struct ArenaWork {
+  Plan& P;
+  ArenaWork(Plan& P_, size_t values) : P(P_) { P.arena.reserve(values * sizeof(double2)); }
+  ~ArenaWork() {
+    if (P.arena.cap > Plan::SolveArena::kKeepBytes) P.arena.release();
+  }
+  ArenaWork(const ArenaWork&) = delete;
+  double2* get(size_t count) { return static_cast<double2*>(P.arena.get((count ? count : 1) * sizeof(double2))); }
+};
+
 // Launches of the vector steps on one stream for up to R positions.
 struct Vec {
   cudaStream_t s;
@@ -550,7 +581,8 @@ struct Vec {
   // h[a * kLdh + j] and h[a * kLdh + kMaxBasis + j] the passes' coefficients,
   // h[a * kLdh + 2 kMaxBasis] = ||w||^2 after them. With an inner GMRES, the
   // basis is scaled by inner->vs and its step nv - 1 follows the norm.
-  void orthogonalise(int Ra, const int* sys, VecRef V, VecRef w, int nv, const Inner* inner = nullptr) {
+  void orthogonalise(int Ra, const int* sys, VecRef V, VecRef w, int nv, const Inner* inner = nullptr,
+                     Pack pack = {}) {
     GsArg g = base(sys);
     g.V = V;
     g.w = w;
@@ -568,18 +600,20 @@ struct Vec {
     launch_gs<true, true, kFinishNone>(g, Ra, s);
     g.hin = h + kMaxBasis;
     g.hout = h + 2 * kMaxBasis;
+    g.pack = pack;
     if (inner)
       launch_gs<true, false, kFinishStep>(g, Ra, s);
     else
       launch_gs<true, false, kFinishNone>(g, Ra, s);
   }
   // Start of the inner GMRES: v copied into basis vector 0, its norm and scale
-  void inner_start(int Ra, const int* sys, VecRef v, VecRef q0, const Inner& inner) {
+  void inner_start(int Ra, const int* sys, VecRef v, VecRef q0, const Inner& inner, Pack pack = {}) {
     GsArg g = base(sys);
     g.w = v;
     g.copy = q0;
     g.has_copy = 1;
     g.inner = inner;
+    g.pack = pack;
     launch_gs<false, false, kFinishBegin>(g, Ra, s);
   }
   void scale(int Ra, const int* sys, VecRef src, VecRef dst, const double* alpha) {
@@ -627,7 +661,8 @@ struct Ops : Vec {
     return std::sqrt(buf[2 * kMaxBasis].real());
   }
 };
-inline Ops make_ops(Work& g, cudaStream_t s, long long n) {
+template <class W>
+inline Ops make_ops(W& g, cudaStream_t s, long long n) {
   Ops o{};
   o.s = s;
   o.n = n;

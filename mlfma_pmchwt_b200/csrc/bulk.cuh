@@ -111,6 +111,18 @@ __device__ __forceinline__ void cp_async_ca(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(kBytes) : "memory");
 }
 
+// The same for 16 bytes, zeros where !take, and the groups of such copies of a
+// thread (wait: until at most kLeft of its groups are in flight).
+__device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool take) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(take ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }

@@ -938,15 +938,22 @@ long long mlfma_get_near(mlfma_plan* plan, int* target, int* source, double* z11
   int st = guarded([&] {
     MLFMA_CUDA(cudaSetDevice(P.device));
     MLFMA_CUDA(cudaStreamSynchronize(P.stream));
-    std::vector<double2> buf(3 * static_cast<size_t>(P.near_pairs));
+    std::vector<double2> buf(static_cast<size_t>(P.h_near_zoff[B]));
     MLFMA_CUDA(cudaMemcpy(buf.data(), P.d_near_z, buf.size() * sizeof(double2), cudaMemcpyDeviceToHost));
-    for (long long e = 0; e < P.near_pairs; ++e) {
-      double* outs[3] = {z11, z12, z22};
-      for (int q = 0; q < 3; ++q)
-        if (outs[q]) {
-          outs[q][2 * e] = buf[3 * e + q].x;
-          outs[q][2 * e + 1] = buf[3 * e + q].y;
+    long long e = 0;
+    for (int b = 0; b < B; ++b) {
+      const int ns = P.h_near_sptr[b + 1] - P.h_near_sptr[b], pitch = mlfma::near_pitch(ns);
+      for (int t = 0; t < T.leaf_ptr[b + 1] - T.leaf_ptr[b]; ++t) {
+        const double2* row = buf.data() + P.h_near_zoff[b] + 3LL * t * pitch;
+        for (int j = 0; j < ns; ++j, ++e) {
+          double* outs[3] = {z11, z12, z22};
+          for (int q = 0; q < 3; ++q)
+            if (outs[q]) {
+              outs[q][2 * e] = row[q * pitch + j].x;
+              outs[q][2 * e + 1] = row[q * pitch + j].y;
+            }
         }
+      }
     }
     return 0;
   });

@@ -51,13 +51,14 @@ __global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
   const int b = a.rwg_box[id];
   const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
   const int tl = r - a.leaf_ptr[b];
-  const Z* Zr = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
+  const int pitch = near_pitch(ns);
+  const Z* Zr = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
   const double sc = a.xscale ? *a.xscale : 1.0;
   Z nJ = Cx<Z>::zero(), nM = Cx<Z>::zero();
   for (int j = lane; j < ns; j += 32) {
     const int s = a.near_src[s0 + j];
     const Z xJ = Cx<Z>::from(cscale(a.x[s], sc)), xM = Cx<Z>::from(cscale(a.x[a.N + s], sc));
-    const Z z11 = Zr[3 * j], z12 = Zr[3 * j + 1], z22 = Zr[3 * j + 2];
+    const Z z11 = Zr[j], z12 = Zr[pitch + j], z22 = Zr[2 * pitch + j];
     nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
     nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
   }
@@ -74,6 +75,122 @@ __global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
   }
 }
 
+// The same product with a CTA per (leaf box, 8 rows): the box's source values
+// are gathered once into shared memory (in the storage type, a row of J and a
+// row of M), where the CTA's rows read them; the entries load 16 bytes per
+// lane, one source in complex128 and two in complex64, for the two rows of a
+// warp, always one step ahead of the arithmetic (the first before the
+// sources are gathered).
+// HBM- or L2-bound (each entry is read once): 4.35 M pairs in complex64 are
+// 104 MB, 16 us; measured 26 us. A warp per row that gathered its sources
+// from the vectors, with the three values of a pair side by side, took 31 us
+// there; a CTA for all rows of a box 34 us, waiting for the fullest boxes.
+constexpr int kNearThreads = 128;
+constexpr int kNearRows = 2;
+constexpr int kNearCtaRows = kNearRows * kNearThreads / 32;
+constexpr size_t kNearStageMax = 160 * 1024;
+
+template <class Z>
+struct alignas(16) NearVec {
+  static constexpr int kPer = 16 / sizeof(Z);
+  Z v[kPer];
+};
+
+template <class Z>
+__global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
+  using Vec = NearVec<Z>;
+  extern __shared__ __align__(16) unsigned char near_stage[];
+  const int b = blockIdx.x;
+  const int r0 = a.leaf_ptr[b], nb = a.leaf_ptr[b + 1] - r0;
+  if (static_cast<int>(blockIdx.y) * kNearCtaRows >= nb) return;
+  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0, pitch = near_pitch(ns);
+  const int lane = threadIdx.x & 31;
+  const int t0 = blockIdx.y * kNearCtaRows + (threadIdx.x >> 5) * kNearRows;
+  const int nrow = min(kNearRows, nb - t0);  // of this warp
+  const Z* rows = a.near_z + a.near_zoff[b] + 3LL * t0 * pitch;
+  Vec z[2][kNearRows][3];
+  auto fetch = [&](int q, Vec(&f)[kNearRows][3]) {
+#pragma unroll
+    for (int u = 0; u < kNearRows; ++u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (u < nrow && q < pitch) v = __ldg(reinterpret_cast<const uint4*>(rows + (3LL * u + c) * pitch + q));
+        *reinterpret_cast<uint4*>(&f[u][c]) = v;
+      }
+  };
+  int q = lane * Vec::kPer;
+  fetch(q, z[0]);
+  Z* xJ = reinterpret_cast<Z*>(near_stage);
+  Z* xM = xJ + pitch;
+  const double sc = a.xscale ? *a.xscale : 1.0;
+#pragma unroll 2
+  for (int i = threadIdx.x; i < pitch; i += kNearThreads) {
+    double2 J = c2(0.0, 0.0), M = c2(0.0, 0.0);
+    if (i < ns) {
+      const int s = a.near_src[s0 + i];
+      J = a.x[s];
+      M = a.x[a.N + s];
+    }
+    xJ[i] = Cx<Z>::from(cscale(J, sc));
+    xM[i] = Cx<Z>::from(cscale(M, sc));
+  }
+  __syncthreads();
+  Z nJ[kNearRows], nM[kNearRows];
+#pragma unroll
+  for (int u = 0; u < kNearRows; ++u) nJ[u] = nM[u] = Cx<Z>::zero();
+  auto add = [&](int at, const Vec(&f)[kNearRows][3]) {
+    if (at >= pitch) return;
+    const Vec J = *reinterpret_cast<const Vec*>(xJ + at), M = *reinterpret_cast<const Vec*>(xM + at);
+#pragma unroll
+    for (int u = 0; u < kNearRows; ++u)
+#pragma unroll
+      for (int i = 0; i < Vec::kPer; ++i) {
+        nJ[u] = cfma(f[u][0].v[i], J.v[i], cfma(f[u][1].v[i], M.v[i], nJ[u]));
+        nM[u] = cfma(f[u][2].v[i], M.v[i], csub(nM[u], cmul(f[u][1].v[i], J.v[i])));
+      }
+  };
+  constexpr int kStep = 32 * Vec::kPer;
+  for (int base = 0; base < pitch; base += 2 * kStep, q += 2 * kStep) {
+    fetch(q + kStep, z[1]);
+    add(q, z[0]);
+    fetch(q + 2 * kStep, z[0]);
+    add(q + kStep, z[1]);
+  }
+#pragma unroll
+  for (int u = 0; u < kNearRows; ++u) {
+    if (u >= nrow) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      nJ[u].x += __shfl_xor_sync(0xffffffffu, nJ[u].x, o);
+      nJ[u].y += __shfl_xor_sync(0xffffffffu, nJ[u].y, o);
+      nM[u].x += __shfl_xor_sync(0xffffffffu, nM[u].x, o);
+      nM[u].y += __shfl_xor_sync(0xffffffffu, nM[u].y, o);
+    }
+    if (lane == 0) {
+      const int id = a.leaf_rwg[r0 + t0 + u];
+      a.w[id] = Cx<Z>::to64(nJ[u]);
+      a.w[a.N + id] = Cx<Z>::to64(nM[u]);
+    }
+  }
+}
+
+// A box whose staged sources fit shared memory takes the box kernel; a plan
+// with a larger source list anywhere keeps the row kernel.
+template <class Z>
+void launch_near(const Plan& P, const NearArg<Z>& a, cudaStream_t s) {
+  const size_t smem = 2 * sizeof(Z) * static_cast<size_t>(near_pitch(P.max_near_sources));
+  if (smem > kNearStageMax) {
+    near_apply_kernel<Z><<<(P.N + 3) / 4, 128, 0, s>>>(a);
+    return;
+  }
+  if (smem > 48 * 1024)  // the same largest value on every call: safe beside other plans' launches
+    MLFMA_CUDA(cudaFuncSetAttribute(near_box_kernel<Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(kNearStageMax)));
+  const dim3 grid(static_cast<int>(P.h_near_sptr.size()) - 1, (P.max_leaf_rwgs + kNearCtaRows - 1) / kNearCtaRows);
+  near_box_kernel<Z><<<grid, kNearThreads, smem, s>>>(a);
+}
+
 }  // namespace
 
 namespace {
@@ -83,11 +200,11 @@ void near_apply_scaled(Plan& P, const double2* x, const double* xscale, double2*
     if (P.d_near_z32 == nullptr) throw std::invalid_argument("plan holds no complex64 near field");
     NearArg<float2> a{P.d_leaf_rwg,  P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src, P.d_near_zoff,
                       P.d_near_z32,  x,               xscale,       w,             P.N};
-    near_apply_kernel<float2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
+    launch_near(P, a, s);
   } else {
     NearArg<double2> a{P.d_leaf_rwg, P.d_rwg_leafbox, P.d_leaf_ptr, P.d_near_sptr, P.d_near_src, P.d_near_zoff,
                        P.d_near_z,   x,               xscale,       w,             P.N};
-    near_apply_kernel<double2><<<(P.N + 3) / 4, 128, 0, s>>>(a);
+    launch_near(P, a, s);
   }
   MLFMA_CUDA(cudaGetLastError());
 }
@@ -116,7 +233,8 @@ struct NearPrecond {
   blas1::Ops ops;
   double2* Q = nullptr;  // [inner_its + 1][n], unscaled basis
   blas1::Inner in{};
-  NearPrecond(Plan& P_, cudaStream_t s_, int inner, blas1::Work& g, const blas1::Ops& o)
+  template <class W>
+  NearPrecond(Plan& P_, cudaStream_t s_, int inner, W& g, const blas1::Ops& o)
       : P(P_), s(s_), n(2LL * P_.N), inner_its(inner), ops(o) {
     if (inner_its <= 0) return;
     Q = g.get(static_cast<size_t>(inner_its + 1) * n);
@@ -170,7 +288,9 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
   MLFMA_CUDA(cudaSetDevice(P.device));
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
-  blas1::Work g;
+  blas1::ArenaWork g(P, (4 + (mr + 1) + (inner_its > 0 ? mr + inner_its + 1 : 0)) * static_cast<size_t>(n) +
+                            blas1::part_count(n, 1) + blas1::kMaxBasis + blas1::kLdh +
+                            blas1::Inner::bytes(1, inner_its) / sizeof(double2) + 1024);
   double2* x = g.get(n);
   double2* b = g.get(n);
   double2* r = g.get(n);

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "blas1.cuh"
+#include "bulk.cuh"
 #include "cplx.cuh"
 #include "plan.hpp"
 #include "learned.hpp"
@@ -31,176 +32,158 @@ namespace {
 using C = std::complex<double>;
 using blas1::VecRef;
 
-// w_a = Z_near x_a for every position (warp per RWG, 4 right-hand sides per
-// warp): the near-field rows of the plan, read once per group of four.
-template <class Z>
+// w_a = Z_near x_a for every position, in complex64.
 struct NearBatchArg {
   const int* leaf_rwg;
-  const int* rwg_box;
   const int* leaf_ptr;
   const int* near_sptr;
   const int* near_src;
   const long long* near_zoff;
-  const Z* near_z;
-  VecRef x, w;
+  const float2* near_z;
+  VecRef w;
   const int* sys;
   const double* xscale;  // factor of position a's x at xscale[a * lds]
   int lds;
   int N, R;
 };
 
-constexpr int kNearRB = 4;
+// One CTA per (leaf box, 32 / G rows, 2G systems), a small dense product: a
+// lane holds one row and two systems (J and M: 4 sums), a warp all of the
+// CTA's rows and systems over a quarter of the box's sources, so no value is
+// reduced across lanes. The entries (128 (row, source) pairs at a time) and
+// the sources' values, which the Gram-Schmidt kernels leave packed per RWG in
+// complex64 (blas1::Pack), stream through a ring of three stages per warp
+// (cp.async): two chunks are in flight while one is multiplied, and no warp
+// waits for another but for the sum of the quarters at the end.
+// FP32-bound at 8 systems (2.2 M pairs: 7.5 us at the FP32 rate, 52 MB of
+// entries 8 us); measured 33 us. With a lane per source and the sources
+// staged for the whole CTA first (10 warps per SM, each waiting for its
+// loads, 320 shuffles per pair of rows) the product took 92 us there; with a
+// CTA for all rows of a box 56 us, waiting for the fullest boxes.
+constexpr int kNearWarps = 4;
+constexpr int kNearStages = 3;
 
-template <class Z>
-__global__ void __launch_bounds__(128) near_batch_kernel(NearBatchArg<Z> a) {
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (r >= a.N) return;
-  const int p0 = blockIdx.y * kNearRB, pn = min(kNearRB, a.R - p0);
-  const int id = a.leaf_rwg[r];
-  const int b = a.rwg_box[id];
-  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
-  const int tl = r - a.leaf_ptr[b];
-  const Z* Zr = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
-  Z nJ[kNearRB], nM[kNearRB];
-  const double2* xs[kNearRB];
-  double sc[kNearRB];
-#pragma unroll
-  for (int j = 0; j < kNearRB; ++j) {
-    nJ[j] = nM[j] = Cx<Z>::zero();
-    xs[j] = j < pn ? a.x.at(p0 + j, a.sys) : nullptr;
-    sc[j] = j < pn ? a.xscale[static_cast<long long>(p0 + j) * a.lds] : 0.0;
-  }
-  for (int q = lane; q < ns; q += 32) {
-    const int src = a.near_src[s0 + q];
-    const Z z11 = Zr[3 * q], z12 = Zr[3 * q + 1], z22 = Zr[3 * q + 2];
-#pragma unroll
-    for (int j = 0; j < kNearRB; ++j) {
-      if (j < pn) {
-        const Z xJ = Cx<Z>::from(cscale(xs[j][src], sc[j])), xM = Cx<Z>::from(cscale(xs[j][a.N + src], sc[j]));
-        nJ[j] = cfma(z11, xJ, cfma(z12, xM, nJ[j]));
-        nM[j] = cfma(z22, xM, csub(nM[j], cmul(z12, xJ)));
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < kNearRB; ++j) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      nJ[j].x += __shfl_xor_sync(0xffffffffu, nJ[j].x, o);
-      nJ[j].y += __shfl_xor_sync(0xffffffffu, nJ[j].y, o);
-      nM[j].x += __shfl_xor_sync(0xffffffffu, nM[j].x, o);
-      nM[j].y += __shfl_xor_sync(0xffffffffu, nM[j].y, o);
-    }
-    if (lane == 0 && j < pn) {
-      double2* w = a.w.at(p0 + j, a.sys);
-      w[id] = Cx<Z>::to64(nJ[j]);
-      w[a.N + id] = Cx<Z>::to64(nM[j]);
-    }
-  }
-}
+template <int G>
+struct NearTile {
+  static constexpr int kSys = 2 * G, kRows = 32 / G, kSrc = 128 / kRows;
+  static constexpr int kZs = 3 * kSrc + 2;  // row pitch of a stage: 16-byte rows in different banks
+  static constexpr int kOut = kRows * kSys;
+  struct __align__(16) Stage {
+    float2 z[kRows * kZs];
+    float4 x[kSrc * kSys];  // (J, M) per (source, system)
+  };
+  Stage ring[kNearWarps][kNearStages];
+  float4 red[kNearWarps][kOut];
+};
 
-// The same products with one CTA per (leaf box, group of kNearBoxRB systems):
-// the box's source values are staged once in shared memory ([system][J, M]
-// [source]) and read there by every target row of the box, instead of each
-// row gathering them again from the vectors. Each row's sums are formed in
-// near_batch_kernel's order (lane-strided sources, then the warp shuffle),
-// so the results are identical.
-constexpr int kNearBoxRB = 8;
-constexpr size_t kNearBoxSmemMax = 160 * 1024;
-
-template <class Z>
-__global__ void __launch_bounds__(128) near_batch_box_kernel(NearBatchArg<Z> a) {
+template <int G>
+__global__ void __launch_bounds__(32 * kNearWarps) near_batch_tile_kernel(NearBatchArg a,
+                                                                          const float4* __restrict__ packed) {
+  using T = NearTile<G>;
+  constexpr int kSys = T::kSys, kRows = T::kRows, kSrc = T::kSrc, kZs = T::kZs, kOut = T::kOut;
   extern __shared__ __align__(16) unsigned char near_smem[];
-  Z* xsm = reinterpret_cast<Z*>(near_smem);
-  __shared__ const double2* xbase[kNearBoxRB];
-  __shared__ double xsc[kNearBoxRB];
+  T& sm = *reinterpret_cast<T*>(near_smem);
   const int b = blockIdx.x;
-  const int p0 = blockIdx.y * kNearBoxRB, pn = min(kNearBoxRB, a.R - p0);
-  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
+  const int t0 = blockIdx.z * kRows;  // first row of this CTA
   const int r0 = a.leaf_ptr[b], nb = a.leaf_ptr[b + 1] - r0;
-  if (threadIdx.x < pn) {
-    xbase[threadIdx.x] = a.x.at(p0 + threadIdx.x, a.sys);
-    xsc[threadIdx.x] = a.xscale[static_cast<long long>(p0 + threadIdx.x) * a.lds];
+  if (t0 >= nb) return;
+  const int p0 = blockIdx.y * kSys, pn = min(kSys, a.R - p0);
+  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0, pitch = near_pitch(ns);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  typename T::Stage* ring = sm.ring[wp];
+  const float2* Z = a.near_z + a.near_zoff[b];
+  const float4* X = packed + static_cast<long long>(blockIdx.y) * a.N * kSys;
+  const int nchunk = (ns + kSrc - 1) / kSrc;
+  const int nc = nchunk > wp ? (nchunk - wp + kNearWarps - 1) / kNearWarps : 0;  // this warp's chunks
+  auto source = [&](int it) {  // lane q's source of the warp's chunk it
+    const int c = wp + it * kNearWarps;
+    return it < nc ? __ldg(a.near_src + s0 + min(c * kSrc + (lane % kSrc), ns - 1)) : 0;
+  };
+  int ids = source(0);
+  auto stage = [&](int it) {
+    if (it < nc) {
+      const int c = wp + it * kNearWarps;
+      typename T::Stage& st = ring[it % kNearStages];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {  // pairs of sources of one plane of one row
+        constexpr int kPairs = kSrc / 2;
+        const int e = 32 * i + lane, row = e / (3 * kPairs), plane = e / kPairs - 3 * row, pr = e % kPairs;
+        const int gr = t0 + row, src = c * kSrc + 2 * pr;
+        const bool take = gr < nb && src < pitch;
+        cp_async16_or_zero(&st.z[row * kZs + plane * kSrc + 2 * pr],
+                           Z + (take ? (3LL * gr + plane) * pitch + src : 0), take);
+      }
+#pragma unroll
+      for (int i = 0; i < (kSrc * kSys + 31) / 32; ++i) {
+        const int e = 32 * i + lane;
+        const int id = __shfl_sync(0xffffffffu, ids, (e / kSys) % kSrc);
+        if (e < kSrc * kSys) cp_async_ca<16>(&st.x[e], X + static_cast<long long>(id) * kSys + e % kSys);
+      }
+    }
+    cp_async_commit();
+    ids = source(it + 1);
+  };
+#pragma unroll
+  for (int i = 0; i + 1 < kNearStages; ++i) stage(i);
+  const int row = lane / G, g = lane - row * G;
+  float2 aJ[2], aM[2];
+  aJ[0] = aJ[1] = aM[0] = aM[1] = make_float2(0.f, 0.f);
+  for (int it = 0; it < nc; ++it) {
+    stage(it + kNearStages - 1);
+    cp_async_wait<kNearStages - 1>();
+    __syncwarp();
+    const float2* z = ring[it % kNearStages].z + row * kZs;
+    const float4* x = ring[it % kNearStages].x + 2 * g;
+    auto add = [&](int q, float2 z11, float2 z12, float2 z22) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float4 v = x[q * kSys + j];
+        const float2 J = make_float2(v.x, v.y), M = make_float2(v.z, v.w), nJ = make_float2(-v.x, -v.y);
+        aJ[j] = cfma(z11, J, cfma(z12, M, aJ[j]));
+        aM[j] = cfma(z22, M, cfma(z12, nJ, aM[j]));
+      }
+    };
+    const int kn = min(kSrc, ns - (wp + it * kNearWarps) * kSrc);
+    if (kn == kSrc) {
+#pragma unroll
+      for (int q = 0; q < kSrc; q += 2) {
+        const float4 z11 = *reinterpret_cast<const float4*>(z + q);
+        const float4 z12 = *reinterpret_cast<const float4*>(z + kSrc + q);
+        const float4 z22 = *reinterpret_cast<const float4*>(z + 2 * kSrc + q);
+        add(q, make_float2(z11.x, z11.y), make_float2(z12.x, z12.y), make_float2(z22.x, z22.y));
+        add(q + 1, make_float2(z11.z, z11.w), make_float2(z12.z, z12.w), make_float2(z22.z, z22.w));
+      }
+    } else {
+      for (int q = 0; q < kn; ++q) add(q, z[q], z[kSrc + q], z[2 * kSrc + q]);
+    }
+    __syncwarp();
   }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    sm.red[wp][row * kSys + 2 * g + j] = make_float4(aJ[j].x, aJ[j].y, aM[j].x, aM[j].y);
   __syncthreads();
-  // one source per thread, the values of 4 systems in flight at once
-  constexpr int kStage = 4;
-  for (int q = threadIdx.x; q < ns; q += blockDim.x) {
-    const int src = a.near_src[s0 + q];
+  for (int o = threadIdx.x; o < kOut; o += 32 * kNearWarps) {
+    const int rr = t0 + o / kSys, j = o % kSys;
+    if (rr < nb && j < pn) {
+      float4 v = sm.red[0][o];
 #pragma unroll
-    for (int j0 = 0; j0 < kNearBoxRB; j0 += kStage) {
-      double2 vJ[kStage], vM[kStage];
-#pragma unroll
-      for (int j = 0; j < kStage; ++j)
-        if (j0 + j < pn) {
-          vJ[j] = xbase[j0 + j][src];
-          vM[j] = xbase[j0 + j][a.N + src];
-        }
-#pragma unroll
-      for (int j = 0; j < kStage; ++j)
-        if (j0 + j < pn) {
-          xsm[(2 * (j0 + j)) * ns + q] = Cx<Z>::from(cscale(vJ[j], xsc[j0 + j]));
-          xsm[(2 * (j0 + j) + 1) * ns + q] = Cx<Z>::from(cscale(vM[j], xsc[j0 + j]));
-        }
+      for (int q = 1; q < kNearWarps; ++q) {
+        const float4 u = sm.red[q][o];
+        v = make_float4(v.x + u.x, v.y + u.y, v.z + u.z, v.w + u.w);
+      }
+      const double sc = a.xscale[static_cast<long long>(p0 + j) * a.lds];
+      double2* w = a.w.at(p0 + j, a.sys);
+      const int id = a.leaf_rwg[r0 + rr];
+      w[id] = c2(sc * v.x, sc * v.y);
+      w[a.N + id] = c2(sc * v.z, sc * v.w);
     }
   }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int nw = blockDim.x / 32;
-  // each warp takes two target rows at a time (tl and tl + nw): every
-  // staged source value read from shared memory serves both rows, and the
-  // two rows' near-field loads are in flight together. Each row's sums are
-  // formed in the same order as with one row per pass.
-  for (int tl = threadIdx.x >> 5; tl < nb; tl += 2 * nw) {
-    const int tl2 = tl + nw;
-    const bool two = tl2 < nb;
-    const Z* Zr = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
-    const Z* Zr2 = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(two ? tl2 : tl) * ns);
-    Z nJ[kNearBoxRB], nM[kNearBoxRB], nJ2[kNearBoxRB], nM2[kNearBoxRB];
-#pragma unroll
-    for (int j = 0; j < kNearBoxRB; ++j) nJ[j] = nM[j] = nJ2[j] = nM2[j] = Cx<Z>::zero();
-    for (int q = lane; q < ns; q += 32) {
-      const Z z11 = Zr[3 * q], z12 = Zr[3 * q + 1], z22 = Zr[3 * q + 2];
-      const Z y11 = Zr2[3 * q], y12 = Zr2[3 * q + 1], y22 = Zr2[3 * q + 2];
-#pragma unroll
-      for (int j = 0; j < kNearBoxRB; ++j) {
-        if (j < pn) {
-          const Z xJ = xsm[(2 * j) * ns + q], xM = xsm[(2 * j + 1) * ns + q];
-          nJ[j] = cfma(z11, xJ, cfma(z12, xM, nJ[j]));
-          nM[j] = cfma(z22, xM, csub(nM[j], cmul(z12, xJ)));
-          nJ2[j] = cfma(y11, xJ, cfma(y12, xM, nJ2[j]));
-          nM2[j] = cfma(y22, xM, csub(nM2[j], cmul(y12, xJ)));
-        }
-      }
-    }
-    const int id = a.leaf_rwg[r0 + tl];
-    const int id2 = a.leaf_rwg[r0 + (two ? tl2 : tl)];
-#pragma unroll
-    for (int j = 0; j < kNearBoxRB; ++j) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        nJ[j].x += __shfl_xor_sync(0xffffffffu, nJ[j].x, o);
-        nJ[j].y += __shfl_xor_sync(0xffffffffu, nJ[j].y, o);
-        nM[j].x += __shfl_xor_sync(0xffffffffu, nM[j].x, o);
-        nM[j].y += __shfl_xor_sync(0xffffffffu, nM[j].y, o);
-        nJ2[j].x += __shfl_xor_sync(0xffffffffu, nJ2[j].x, o);
-        nJ2[j].y += __shfl_xor_sync(0xffffffffu, nJ2[j].y, o);
-        nM2[j].x += __shfl_xor_sync(0xffffffffu, nM2[j].x, o);
-        nM2[j].y += __shfl_xor_sync(0xffffffffu, nM2[j].y, o);
-      }
-      if (lane == 0 && j < pn) {
-        double2* w = a.w.at(p0 + j, a.sys);
-        w[id] = Cx<Z>::to64(nJ[j]);
-        w[a.N + id] = Cx<Z>::to64(nM[j]);
-        if (two) {
-          w[id2] = Cx<Z>::to64(nJ2[j]);
-          w[a.N + id2] = Cx<Z>::to64(nM2[j]);
-        }
-      }
-    }
-  }
+  cp_async_wait<0>();
 }
+
+// Systems per CTA: 8 from 5 systems on, 4 for 3 or 4, else 2 (lanes without
+// a system would multiply zeros).
+inline int near_tile_groups(int Ra) { return Ra > 4 ? 4 : Ra > 2 ? 2 : 1; }
 
 // The batched vector steps on one stream with their results on the host, for
 // up to R positions.
@@ -280,11 +263,13 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   const size_t Rz = static_cast<size_t>(R);
   // work arrays (counts of complex128 values), in one block of the plan's
   // arena: no allocation when the last call's block is large enough
-  enum { kX, kB, kR, kV, kZ, kQ, kXs, kWs, kPart, kCount, kH, kAlpha, kM, kY, kSys, kInner, kN };
+  enum { kX, kB, kR, kV, kZ, kQ, kXs, kWs, kPart, kCount, kH, kAlpha, kM, kY, kSys, kInner, kPack, kN };
   const size_t cnt[kN] = {Rz * n, Rz * n, Rz * n, Rz * vs, inner_its > 0 ? Rz * zs : 0, inner_its > 0 ? Rz * qs : 0,
                           static_cast<size_t>(G) * n, static_cast<size_t>(G) * n, blas1::part_count(n, R), Rz,
                           Rz * blas1::kLdh, Rz, Rz, Rz * blas1::kMaxBasis, Rz,
-                          inner_its > 0 ? blas1::Inner::bytes(R, inner_its) / sizeof(double2) + 1 : 0};
+                          inner_its > 0 ? blas1::Inner::bytes(R, inner_its) / sizeof(double2) + 1 : 0,
+                          // complex64 values of 2N unknowns for whole groups of positions
+                          inner_its > 0 ? (Rz + 7) / 8 * 8 * n / 2 : 0};
   size_t work_bytes = 0;
   for (size_t c : cnt) work_bytes += (c * sizeof(double2) + 255) & ~size_t(255);
   P.arena.reserve(work_bytes);
@@ -346,35 +331,36 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     const VecRef br = sysref(b, n, 0);
     return ops.norms_host(Ra, sysd, sysref(r, n, 0), &br);
   };
-  // the box-staged near-field kernel's shared memory: the largest source list
+  // shared memory of the near-field kernel (constants: set to the same value
+  // by every solve of every thread)
   const int nleaf = static_cast<int>(P.h_near_sptr.size()) - 1;
-  int ns_max = 0;
-  for (int bx = 0; bx < nleaf; ++bx) ns_max = std::max(ns_max, P.h_near_sptr[bx + 1] - P.h_near_sptr[bx]);
-  const size_t box_smem = static_cast<size_t>(2 * kNearBoxRB) * ns_max * sizeof(float2);
-  // The shared-memory limit is set to the same largest value on every call:
-  // solves of several plans from several host threads then never lower it
-  // under another's launch.
-  if (inner_its > 0 && box_smem <= kNearBoxSmemMax)
-    MLFMA_CUDA(cudaFuncSetAttribute(near_batch_box_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kNearBoxSmemMax)));
+  if (inner_its > 0) {
+    auto allow = [](auto* f, size_t bytes) {
+      MLFMA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    };
+    allow(near_batch_tile_kernel<1>, sizeof(NearTile<1>));
+    allow(near_batch_tile_kernel<2>, sizeof(NearTile<2>));
+    allow(near_batch_tile_kernel<4>, sizeof(NearTile<4>));
+  }
+  auto packed = [&](int Ra) { return blas1::Pack{reinterpret_cast<float2*>(wk[kPack]), 2 * near_tile_groups(Ra)}; };
   // z_q = (inner_its GMRES steps on Z_near from zero) applied to v_q, q in
   // list: every step is four launches, the host waits for none of them
   auto precondition_steps = [&](int Ra) {
     for (int j = 0; j < inner_its; ++j) {
       // the preconditioner's near field is the complex64 copy at either precision
-      NearBatchArg<float2> na{P.d_leaf_rwg,  P.d_rwg_leafbox,      P.d_leaf_ptr,
-                              P.d_near_sptr, P.d_near_src,         P.d_near_zoff,
-                              P.d_near_z32,  sysref(Q, qs, j * n), sysref(Q, qs, (j + 1) * n),
-                              sysd,          ib.vs + j,            ib.ld,
-                              P.N,           Ra};
-      if (box_smem <= kNearBoxSmemMax) {
-        const dim3 ng(nleaf, (Ra + kNearBoxRB - 1) / kNearBoxRB);
-        near_batch_box_kernel<float2><<<ng, 128, box_smem, s>>>(na);
-      } else {
-        const dim3 ng((P.N + 3) / 4, (Ra + kNearRB - 1) / kNearRB);
-        near_batch_kernel<float2><<<ng, 128, 0, s>>>(na);
-      }
-      ops.orthogonalise(Ra, sysd, sysref(Q, qs, 0), sysref(Q, qs, (j + 1) * n), j + 1, &ib);
+      NearBatchArg na{P.d_leaf_rwg,  P.d_leaf_ptr,              P.d_near_sptr, P.d_near_src, P.d_near_zoff,
+                      P.d_near_z32,  sysref(Q, qs, (j + 1) * n), sysd,          ib.vs + j,    ib.ld,
+                      P.N,           Ra};
+      const int G = near_tile_groups(Ra);
+      const dim3 ng(nleaf, (Ra + 2 * G - 1) / (2 * G), (P.max_leaf_rwgs * G + 31) / 32);
+      const float4* px = reinterpret_cast<const float4*>(wk[kPack]);
+      if (G == 4)
+        near_batch_tile_kernel<4><<<ng, 32 * kNearWarps, sizeof(NearTile<4>), s>>>(na, px);
+      else if (G == 2)
+        near_batch_tile_kernel<2><<<ng, 32 * kNearWarps, sizeof(NearTile<2>), s>>>(na, px);
+      else
+        near_batch_tile_kernel<1><<<ng, 32 * kNearWarps, sizeof(NearTile<1>), s>>>(na, px);
+      ops.orthogonalise(Ra, sysd, sysref(Q, qs, 0), sysref(Q, qs, (j + 1) * n), j + 1, &ib, packed(Ra));
     }
     MLFMA_CUDA(cudaGetLastError());
   };
@@ -395,7 +381,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     const int Ra = static_cast<int>(list.size());
     set_sys(list);
     for (int q : list) st[q].near_products += inner_its;
-    ops.inner_start(Ra, sysd, sysref(V, vs, voff), sysref(Q, qs, 0), ib);
+    ops.inner_start(Ra, sysd, sysref(V, vs, voff), sysref(Q, qs, 0), ib, packed(Ra));
     if (P.tuning.graph != 1) {
       precondition_steps(Ra);
     } else {

@@ -115,4 +115,8 @@ struct Quad {
 };
 bool quad_rule(int n, Quad& q);
 
+// Values of one near-field row of ns sources: even, so that every row starts
+// on a 16-byte boundary in complex64 too and two sources load at once.
+constexpr int near_pitch(int ns) { return (ns + 1) & ~1; }
+
 }  // namespace mlfma

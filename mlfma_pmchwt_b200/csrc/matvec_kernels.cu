@@ -1266,12 +1266,13 @@ __global__ void __launch_bounds__(kThreads) leaf_out_kernel(LeafArg<C> a) {
   if constexpr (kNear) {
     const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
     const int tl = r - a.leaf_ptr[b];
-    const C* Z = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
+    const int pitch = near_pitch(ns);
+    const C* Z = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
 #pragma unroll 2
     for (int j = lane; j < ns; j += 32) {
       const int s = a.near_src[s0 + j];
       const C xJ = Cx<C>::from(a.x[s]), xM = Cx<C>::from(a.x[a.N + s]);
-      const C z11 = Z[3 * j], z12 = Z[3 * j + 1], z22 = Z[3 * j + 2];
+      const C z11 = Z[j], z12 = Z[pitch + j], z22 = Z[2 * pitch + j];
       nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
       nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
     }
@@ -1430,13 +1431,14 @@ __global__ void __launch_bounds__(kThreads) leaf_out_batch_kernel(LeafBatchArg<C
   }
   const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
   const int tl = r - a.leaf_ptr[b];
-  const C* Z = a.near_z + 3 * (a.near_zoff[b] + static_cast<long long>(tl) * ns);
+  const int pitch = near_pitch(ns);
+  const C* Z = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
   C nJ[RB], nM[RB];
 #pragma unroll
   for (int j = 0; j < RB; ++j) nJ[j] = nM[j] = Cx<C>::zero();
   for (int q = lane; q < ns; q += 32) {
     const int src = a.near_src[s0 + q];
-    const C z11 = Z[3 * q], z12 = Z[3 * q + 1], z22 = Z[3 * q + 2];
+    const C z11 = Z[q], z12 = Z[pitch + q], z22 = Z[2 * pitch + q];
 #pragma unroll
     for (int j = 0; j < RB; ++j) {
       if (j < jn) {

@@ -269,7 +269,8 @@ void same_triangle_pairs(const Rwg& r, const Tree& t, const std::vector<int>& ne
       for (int si = 0; si < ns; ++si) {
         const int sr = near_src[near_sptr[b] + si];
         if (!share_a_face(r, tr, sr)) continue;
-        pos.push_back(near_zoff[b] + static_cast<long long>(ti - t.leaf_ptr[b]) * ns + si);
+        const long long pitch = near_pitch(ns);
+        pos.push_back(near_zoff[b] + (3 * static_cast<long long>(ti - t.leaf_ptr[b]) + 1) * pitch + si);
         tgt.push_back(tr);
         src.push_back(sr);
       }

@@ -227,9 +227,10 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
       P->h_near_sptr[b + 1] = static_cast<int>(P->h_near_src.size());
       const long long nt = T.leaf_ptr[b + 1] - T.leaf_ptr[b];
       const long long ns = P->h_near_sptr[b + 1] - P->h_near_sptr[b];
-      P->h_near_zoff[b + 1] = P->h_near_zoff[b] + nt * ns;
+      P->max_near_sources = std::max(P->max_near_sources, static_cast<int>(ns));
+      P->h_near_zoff[b + 1] = P->h_near_zoff[b] + nt * 3 * near_pitch(static_cast<int>(ns));
+      P->near_pairs += nt * ns;
     }
-    P->near_pairs = P->h_near_zoff[B];
   }
   if (prm.device < 0) {  // host-only plan: tables for inspection, no device work
     P->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -568,7 +569,7 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
     P->d_near_sptr = P->upload(P->h_near_sptr);
     P->d_near_src = P->upload(P->h_near_src);
     P->d_near_zoff = P->upload(P->h_near_zoff);
-    P->d_near_z = P->alloc<double2>(3 * static_cast<size_t>(std::max<long long>(P->near_pairs, 1)));
+    P->d_near_z = P->alloc<double2>(static_cast<size_t>(P->h_near_zoff.back()));
     launch_near(*P, s);
     if (P->same_triangle_k == 1) {
       // the K entries of RWG pairs sharing a triangle, with the reference's
@@ -620,7 +621,7 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
   // complex64 copy of the near field: the flexible GMRES preconditioner's
   // products (any plan) and the mixed operator's near rows
   {
-    const size_t nz = 3 * static_cast<size_t>(std::max<long long>(P->near_pairs, 1));
+    const size_t nz = static_cast<size_t>(P->h_near_zoff.back());
     P->d_near_z32 = P->alloc<float2>(nz);
     to_c64(P->d_near_z, P->d_near_z32, nz, s);
   }

@@ -4,8 +4,9 @@
 //                   boxes in Morton order; K directions theta-major.
 //   radiation / receive leaf patterns: [rwg in leaf order][3][K_m,leaf].
 //   transfer factors: [vec][K] complex128 with the quadrature weight folded in.
-//   near field: per leaf box b, a dense block [n_b targets][sources of the
-//               27-neighbourhood][3] complex128 (z11, z12, z22; z21 = -z12).
+//   near field: per leaf box b, a dense block [n_b targets][3][sources of the
+//               27-neighbourhood, padded to an even count] complex128 (a row
+//               of z11, one of z12, one of z22; z21 = -z12; the padding is 0).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -206,13 +207,14 @@ struct Plan {
   float2* d_Vs32[2] = {nullptr, nullptr};  // complex64 copies (precision = mixed)
   float2* d_Vf32[2] = {nullptr, nullptr};
   // ---- near field
-  std::vector<long long> h_near_zoff;      // per leaf box, offset of its block (pairs)
+  std::vector<long long> h_near_zoff;      // per leaf box, offset of its block (values)
   std::vector<int> h_near_sptr;            // per leaf box, offset into source list
   std::vector<int> h_near_src;             // concatenated source RWG ids per leaf box
+  int max_near_sources = 0;                // longest of those lists
   int* d_near_sptr = nullptr;       // [Bleaf+1]
   int* d_near_src = nullptr;        // concatenated source RWG ids per box
   long long* d_near_zoff = nullptr; // [Bleaf+1]
-  double2* d_near_z = nullptr;      // [pairs][3]
+  double2* d_near_z = nullptr;      // per leaf box [targets][3][near_pitch(sources)]
   float2* d_near_z32 = nullptr;     // complex64 copy: preconditioner products, mixed operator
   long long near_pairs = 0;
   // ---- vectors
@@ -377,7 +379,7 @@ void launch_transfer(Plan& P, int medium, int level, const std::vector<double>& 
                      const std::vector<double2>& h2, bool weighted, double2* out, cudaStream_t s,
                      bool in_heap = false);
 void launch_near(Plan& P, cudaStream_t s);
-// Z[3 pos[i] + 1] = z12[i] for n entries of the near field (device arrays).
+// Z[pos[i]] = z12[i] for n entries of the near field (device arrays).
 void launch_near_z12_scatter(double2* Z, const long long* pos, const double2* z12, long long n, cudaStream_t s);
 void apply_device(Plan& P, const double2* x, double2* w, cudaStream_t s);
 void clear_graphs(Plan& P);  // after any change that alters what an apply launches

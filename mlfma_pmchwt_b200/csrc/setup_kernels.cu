@@ -412,10 +412,11 @@ __global__ void near_kernel(GeomArg g, QuadArg q, const int* __restrict__ leaf_p
     const double2 z11 = cadd(op[0], cmul(etai, op[1]));
     const double2 z12 = cneg(cadd(op[2], op[3]));
     const double2 z22 = cadd(op[0], cmul(ietai, op[1]));
-    double2* zp = Z + 3 * (base + e);
+    const int pitch = near_pitch(ns);
+    double2* zp = Z + base + 3LL * (e / ns) * pitch + e % ns;
     zp[0] = z11;
-    zp[1] = z12;
-    zp[2] = z22;
+    zp[pitch] = z12;
+    zp[2 * pitch] = z22;
   }
 }
 
@@ -497,7 +498,7 @@ void launch_transfer(Plan& P, int medium, int level, const std::vector<double>& 
 __global__ void near_z12_scatter_kernel(double2* __restrict__ Z, const long long* __restrict__ pos,
                                         const double2* __restrict__ z12, long long n) {
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i < n) Z[3 * pos[i] + 1] = z12[i];
+  if (i < n) Z[pos[i]] = z12[i];
 }
 
 void launch_near_z12_scatter(double2* Z, const long long* pos, const double2* z12, long long n, cudaStream_t s) {
@@ -508,6 +509,8 @@ void launch_near_z12_scatter(double2* Z, const long long* pos, const double2* z1
 
 void launch_near(Plan& P, cudaStream_t s) {
   const int B = P.lv[P.maxL].B;
+  // the rows' padding stays zero
+  MLFMA_CUDA(cudaMemsetAsync(P.d_near_z, 0, static_cast<size_t>(P.h_near_zoff.back()) * sizeof(double2), s));
   near_kernel<<<B, 128, 0, s>>>(geom_arg(P), quad_arg(P.quad), P.d_leaf_ptr, P.d_leaf_rwg, P.d_near_sptr,
                                 P.d_near_src, P.d_near_zoff, c2(P.k1.real(), P.k1.imag()),
                                 c2(P.k2.real(), P.k2.imag()), c2(P.etai.real(), P.etai.imag()),

@@ -36,7 +36,7 @@ bool gmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, do
   MLFMA_CUDA(cudaSetDevice(P.device));
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
-  blas1::Work g;
+  blas1::ArenaWork g(P, (5 + static_cast<size_t>(mr)) * n + blas1::part_count(n, 1) + mr + 1 + blas1::kLdh + 1024);
   double2* x = g.get(n);
   double2* b = g.get(n);
   double2* r = g.get(n);
