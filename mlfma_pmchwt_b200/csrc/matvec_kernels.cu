@@ -739,11 +739,24 @@ struct M2lPairArg {
 };
 
 // kSlots: the slot offsets of the batched tree (grid.y = slot); the single
-// apply instantiates without them (two registers fewer: 96 rather than 98 in
-// FP64, which keeps five CTAs per SM).
+// apply instantiates without them.
 // kW: box pairs (warps) per CTA.
-template <class C, bool kSlots = false, int kW = kPairWarps>
-__global__ void __launch_bounds__(32 * kW) m2l_pair_kernel(const __grid_constant__ M2lPairArg<C> a) {
+// Off: the type of byte offsets into a level's arrays; with 32 bits (arrays
+// below 4 GB) the 6 components share one offset and their base pointers are
+// uniform, which takes a quarter of the instructions off the loop.
+// FP64 is bound by latency and L1 (96 registers, five CTAs per SM), complex64
+// by instruction issue (74 % active before, half of it multiply-adds). One B200,
+// translation of all levels and both media: FP64 at 245,760 unknowns 2.27 ->
+// 2.05 ms, 16 slots of complex64 at 61,440 5.38 -> 4.24 ms. Two directions per
+// lane (16-byte loads) in complex64: 4.45 ms, too few warps.
+template <class C, class Off>
+__device__ __forceinline__ C load_at(const C* base, Off byte) {
+  return __ldg(reinterpret_cast<const C*>(reinterpret_cast<const char*>(base) + byte));
+}
+
+template <class C, bool kSlots, int kW, class Off>
+__global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 * kW))
+    m2l_pair_kernel(const __grid_constant__ M2lPairArg<C> a) {
   int si = 0;
   while (si + 1 < a.nseg && static_cast<int>(blockIdx.x) >= a.seg[si + 1].cta_begin) ++si;
   const M2lPairSeg<C>& g = a.seg[si];
@@ -758,23 +771,34 @@ __global__ void __launch_bounds__(32 * kW) m2l_pair_kernel(const __grid_constant
   C a0[6], a1[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) a0[c] = a1[c] = Cx<C>::zero();
+  // The next entry's source and factor rows are read one entry ahead, and an
+  // entry's 6 pattern and up to 2 factor values are requested together: one
+  // memory latency per entry instead of three (indices, then the patterns and
+  // the first box's factor, then the second's behind its branch).
   const int e1 = g.pair_ptr[pg + 1];
-  for (int e = g.pair_ptr[pg]; e < e1; ++e) {
-    const int src = __ldg(g.pair_src + e);
-    const int2 v = __ldg(g.pair_vec + e);
-    const C* p = Sl + static_cast<size_t>(src) * 6 * K + k;
-    C sv[6];
+  int e = g.pair_ptr[pg];
+  int src = e < e1 ? __ldg(g.pair_src + e) : 0;
+  int2 v = e < e1 ? __ldg(g.pair_vec + e) : make_int2(-1, -1);
+  const Off row = static_cast<Off>(K) * static_cast<Off>(sizeof(C)), at = static_cast<Off>(k) * static_cast<Off>(sizeof(C));
+  while (e < e1) {
+    const Off o = static_cast<Off>(src) * (6 * row) + at;
+    C sv[6], t0, t1;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sv[c] = __ldg(p + static_cast<size_t>(c) * K);
-    if (v.x >= 0) {
-      const C t = __ldg(g.tfw + static_cast<size_t>(v.x) * K + k);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) a0[c] = cfma(t, sv[c], a0[c]);
+    for (int c = 0; c < 6; ++c) sv[c] = load_at(Sl + static_cast<size_t>(c) * K, o);
+    const bool in0 = v.x >= 0, in1 = v.y >= 0;
+    if (in0) t0 = load_at(g.tfw, static_cast<Off>(v.x) * row + at);
+    if (in1) t1 = load_at(g.tfw, static_cast<Off>(v.y) * row + at);
+    if (++e < e1) {
+      src = __ldg(g.pair_src + e);
+      v = __ldg(g.pair_vec + e);
     }
-    if (v.y >= 0) {
-      const C t = __ldg(g.tfw + static_cast<size_t>(v.y) * K + k);
+    if (in0) {
 #pragma unroll
-      for (int c = 0; c < 6; ++c) a1[c] = cfma(t, sv[c], a1[c]);
+      for (int c = 0; c < 6; ++c) a0[c] = cfma(t0, sv[c], a0[c]);
+    }
+    if (in1) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) a1[c] = cfma(t1, sv[c], a1[c]);
     }
   }
   C* out0 = Bl + static_cast<size_t>(2 * pg) * 6 * K + k;
@@ -839,14 +863,27 @@ __global__ void __launch_bounds__(64 * kPairWarps) m2l_pairh_kernel(const __grid
 inline int pair_warps(const Plan& P) { return 2 << P.tuning.m2l_pair_warps; }
 inline int up_threads(const Plan& P) { return 64 << P.tuning.up_threads; }
 
+template <class C, bool kSlots, class Off>
+void launch_m2l_pair_as(int w, dim3 grid, const M2lPairArg<C>& a, cudaStream_t st) {
+  if (w == 2)
+    m2l_pair_kernel<C, kSlots, 2, Off><<<grid, 64, 0, st>>>(a);
+  else if (w == 8)
+    m2l_pair_kernel<C, kSlots, 8, Off><<<grid, 256, 0, st>>>(a);
+  else
+    m2l_pair_kernel<C, kSlots, 4, Off><<<grid, 128, 0, st>>>(a);
+}
+
 template <class C, bool kSlots>
 void launch_m2l_pair(int w, dim3 grid, const M2lPairArg<C>& a, cudaStream_t st) {
-  if (w == 2)
-    m2l_pair_kernel<C, kSlots, 2><<<grid, 64, 0, st>>>(a);
-  else if (w == 8)
-    m2l_pair_kernel<C, kSlots, 8><<<grid, 256, 0, st>>>(a);
+  bool small = true;  // every level's patterns and factors within 32-bit byte offsets
+  for (int i = 0; i < a.nseg; ++i) {
+    const size_t row = sizeof(C) * static_cast<size_t>(a.seg[i].K);
+    small = small && row * 6 * static_cast<size_t>(a.seg[i].B) < (1ull << 32) && row * 343 < (1ull << 32);
+  }
+  if (small)
+    launch_m2l_pair_as<C, kSlots, uint32_t>(w, grid, a, st);
   else
-    m2l_pair_kernel<C, kSlots, 4><<<grid, 128, 0, st>>>(a);
+    launch_m2l_pair_as<C, kSlots, size_t>(w, grid, a, st);
 }
 
 // Translation with staged sources: a CTA takes a group of 8 Morton-
