@@ -182,10 +182,102 @@ __global__ void __launch_bounds__(kT) up_kernel(UpArg<C> a) {
   (kSlots ? a.Sp + slot * a.slot_p : a.Sp)[(static_cast<size_t>(b) * 6 + c) * a.Kp + kk] = acc;
 }
 
-// grid: (parent boxes, direction tiles of t, zdim = 6 components x slots)
+template <class C>
+struct Up2Arg {
+  const C* Sc;   // child level patterns [Bc][6][Kc]
+  C* Sp;         // parent level patterns [Bp][6][Kp]
+  const int* child_begin;
+  const int* octant;  // of child boxes
+  const int4* row;    // per pair of parent theta rows: its 4 child rows
+  const double2* w;   // [4] per pair: weights in the two parent rows
+  const int* pidx;
+  const double* lp;
+  const C* ph_up;
+  int Kp, nthp, nphp, Kc;
+  long long slot_c = 0, slot_p = 0;  // element strides between right-hand-side slots (grid.z = 6 x slots)
+};
+
+// The same interpolation, a thread per (parent box, pair of parent theta rows,
+// parent phi column, component): the two rows' stencils lie on at most 4
+// child rows, so 12 loads serve two outputs instead of 18, and each child row
+// is interpolated in phi once. Loads address from the child's uniform base by
+// 32-bit offsets. Bound by L1 throughput (85 % of its data pipe in complex64):
+// a gather of 32 phi taps straddles lines. One B200, interpolation of all
+// levels and both media, before and after: FP64 at 245,760 unknowns 1.34 ->
+// 1.05 ms, 16 slots of complex64 at 61,440 3.36 -> 3.07 ms. The occupancy
+// bounds are the measured best (FP64 96, complex64 72 registers; 64 spill).
+template <class C, bool kSlots, int kT>
+__global__ void __launch_bounds__(kT, (sizeof(C) == 16 ? 640 : 896) / kT) up2_kernel(const __grid_constant__ Up2Arg<C> a) {
+  using R = typename Cx<C>::real;
+  const int q = blockIdx.y * kT + threadIdx.x;
+  const int b = blockIdx.x;
+  const int slot = kSlots ? blockIdx.z / 6 : 0;
+  const int c = blockIdx.z - 6 * slot;
+  if (q >= ((a.nthp + 1) >> 1) * a.nphp) return;
+  const int tp = q / a.nphp, p = q - tp * a.nphp;
+  const bool two = 2 * tp + 1 < a.nthp;
+  unsigned at[3];
+  R wp[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    at[j] = __ldg(a.pidx + 3 * p + j);
+    wp[j] = static_cast<R>(__ldg(a.lp + 3 * p + j));
+  }
+  const int4 r4 = __ldg(a.row + tp);
+  const unsigned row[4] = {static_cast<unsigned>(r4.x), static_cast<unsigned>(r4.y), static_cast<unsigned>(r4.z),
+                           static_cast<unsigned>(r4.w)};
+  R w0[4], w1[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const double2 w = __ldg(a.w + 4 * tp + r);
+    w0[r] = static_cast<R>(w.x);
+    w1[r] = static_cast<R>(w.y);
+  }
+  const unsigned kk = 2u * tp * a.nphp + p;
+  C acc0 = Cx<C>::zero(), acc1 = Cx<C>::zero();
+  const C* const Sl = kSlots ? a.Sc + slot * a.slot_c : a.Sc;
+  const int c1 = a.child_begin[b + 1];
+  for (int ch = a.child_begin[b]; ch < c1; ++ch) {
+    const C* sc = Sl + (static_cast<size_t>(ch) * 6 + c) * a.Kc;
+    const C* ph = a.ph_up + static_cast<size_t>(a.octant[ch]) * a.Kp;
+    C s[4][3];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) s[r][j] = __ldg(sc + (row[r] + at[j]));
+    const C e0 = __ldg(ph + kk), e1 = __ldg(ph + (two ? kk + a.nphp : kk));
+    C v0 = Cx<C>::zero(), v1 = Cx<C>::zero();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const C f = cfmas(wp[2], s[r][2], cfmas(wp[1], s[r][1], cscale(s[r][0], wp[0])));
+      v0 = cfmas(w0[r], f, v0);
+      v1 = cfmas(w1[r], f, v1);
+    }
+    acc0 = cfma(e0, v0, acc0);
+    acc1 = cfma(e1, v1, acc1);
+  }
+  C* out = (kSlots ? a.Sp + slot * a.slot_p : a.Sp) + (static_cast<size_t>(b) * 6 + c) * a.Kp + kk;
+  out[0] = acc0;
+  if (two) out[a.nphp] = acc1;
+}
+
+// grid: (parent boxes, direction tiles of t, zdim = 6 components x slots); the
+// row pairs where the level's stencils allow them
 template <class C, bool kSlots>
-void launch_up(int t, int boxes, int K, int zdim, const UpArg<C>& a, cudaStream_t s) {
-  const dim3 g(boxes, (K + t - 1) / t, zdim);
+void launch_up(int t, int boxes, int zdim, const MediumLevel& pm, const UpArg<C>& a, cudaStream_t s) {
+  if (pm.up2_row) {
+    const Up2Arg<C> u{a.Sc, a.Sp,   a.child_begin, a.octant, pm.up2_row, pm.up2_w, a.pidx,   a.lp,
+                      a.ph_up, a.Kp, pm.nth,        a.nphp,   a.Kc,       a.slot_c, a.slot_p};
+    const dim3 g(boxes, (((pm.nth + 1) / 2) * pm.nph + t - 1) / t, zdim);
+    if (t == 64)
+      up2_kernel<C, kSlots, 64><<<g, 64, 0, s>>>(u);
+    else if (t == 256)
+      up2_kernel<C, kSlots, 256><<<g, 256, 0, s>>>(u);
+    else
+      up2_kernel<C, kSlots, 128><<<g, 128, 0, s>>>(u);
+    return;
+  }
+  const dim3 g(boxes, (a.Kp + t - 1) / t, zdim);
   if (t == 64)
     up_kernel<C, kSlots, 64><<<g, 64, 0, s>>>(a);
   else if (t == 256)
@@ -1145,12 +1237,12 @@ struct L2lSepArg {
   const int* parent;     // of child boxes
   const int* octant;     // of child boxes
   const C* ph_dn;        // parent level table [8][Kp]
-  const int* th_ptr;     // child theta row -> (parent theta row, Lagrange weight)
-  const int* th_src;
-  const double* th_w;
-  const int* ph_ptr;     // child phi column -> (parent phi column, Lagrange weight)
-  const int* ph_src;
-  const double* ph_w;
+  const int* th_ptr;     // pairs of child theta rows: groups of two taps (MediumLevel::th2_*)
+  const int2* th_row;
+  const double2* th_w;
+  const int* ph_ptr;     // child phi columns: groups of two taps (MediumLevel::ph2_*)
+  const int2* ph_src;
+  const double2* ph_w;
   int ntc, npc, ntp, npp;
   long long slot_c = 0, slot_p = 0;  // element strides between right-hand-side slots (grid.z = slots)
 };
@@ -1171,61 +1263,90 @@ inline int l2l_grid_y(int boxes, int ntc, int npp) {
 }
 
 // Anterpolation (l2l), separable: a CTA per child box (and, on levels with few
-// boxes, per band of child theta rows) does all 6 components. The parent's incoming pattern is shifted to the child centre
-// and spread onto the child grid by the transposed theta interpolation (into
-// a shared-memory band of child rows x parent phi columns x 6 components),
-// then by the transposed phi interpolation, and added to the child's Bm. The
-// reference's 9-tap weight of a (parent, child) direction pair is the
-// product of the two 1-D weights used here (Code/AlgoMLFMM.h:347-351).
-// (4 CTAs per SM: 64 registers, up from 3 CTAs at 80.)
+// boxes, per band of child theta rows) does all 6 components. The parent's
+// incoming pattern is shifted to the child centre and spread onto the child
+// grid by the transposed theta interpolation (into a shared-memory band of
+// child rows x parent phi columns x 6 components), then by the transposed phi
+// interpolation, and added to the child's Bm. The reference's 9-tap weight of
+// a (parent, child) direction pair is the product of the two 1-D weights used
+// here (Code/AlgoMLFMM.h:347-351).
+// A thread's unit is 3 components (J or M): in theta, one parent column of two
+// neighbouring child rows, whose taps overlap (5.3 parent rows instead of 8),
+// two taps at a time, so that 8 independent loads are in flight; in phi, one
+// child direction, its old values requested before the taps are summed.
 // kSlots: grid.z = slots with the slot offsets of the batched tree; the single
 // apply instantiates without them.
 template <class C, bool kSlots = false>
-__global__ void __launch_bounds__(256, 4) l2l_sep_kernel(L2lSepArg<C> a) {
+__global__ void __launch_bounds__(256, sizeof(C) == 16 ? 3 : 4) l2l_sep_kernel(const __grid_constant__ L2lSepArg<C> a) {
   using R = typename Cx<C>::real;
   __shared__ C band[kL2lBand];
   const int b = blockIdx.x;
   const int band_rows = l2l_band_rows(a.ntc, a.npp);
-  const int Kp = a.ntp * a.npp, Kc = a.ntc * a.npc;
-  const C* ph = a.ph_dn + a.octant[b] * Kp;
+  const unsigned Kp = a.ntp * a.npp, Kc = a.ntc * a.npc;
+  const C* ph = a.ph_dn + static_cast<size_t>(a.octant[b]) * Kp;
   const C* bp = (kSlots ? a.Bp + blockIdx.z * a.slot_p : a.Bp) + static_cast<size_t>(a.parent[b]) * 6 * Kp;
   C* out = (kSlots ? a.Bm + blockIdx.z * a.slot_c : a.Bm) + static_cast<size_t>(b) * 6 * Kc;
   for (int tc0 = blockIdx.y * band_rows; tc0 < a.ntc; tc0 += gridDim.y * band_rows) {
     const int rows = min(band_rows, a.ntc - tc0);
-    const int stride = rows * a.npp;
+    const int stride = rows * a.npp;  // of a component in the band
+    const int q0 = tc0 >> 1, nq = ((tc0 + rows - 1) >> 1) - q0 + 1;  // row pairs
+    const int half = nq * a.npp;
     __syncthreads();
-    for (int e = threadIdx.x; e < stride; e += blockDim.x) {
-      const int r = e / a.npp, pp = e - r * a.npp;
-      const int tc = tc0 + r;
-      C v[6];
+    for (int e = threadIdx.x; e < 2 * half; e += blockDim.x) {
+      const int h = e >= half, ee = e - h * half;
+      const int q = ee / a.npp, pp = ee - q * a.npp;
+      C v0[3], v1[3];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) v[c] = Cx<C>::zero();
-      const int q1 = __ldg(a.th_ptr + tc + 1);
-      for (int q = __ldg(a.th_ptr + tc); q < q1; ++q) {
-        const int kp = __ldg(a.th_src + q) * a.npp + pp;
-        const C f = cscale(__ldg(ph + kp), static_cast<R>(__ldg(a.th_w + q)));
+      for (int c = 0; c < 3; ++c) v0[c] = v1[c] = Cx<C>::zero();
+      const C* bh = bp + h * 3 * Kp;
+      const int g1 = __ldg(a.th_ptr + q0 + q + 1);
+      for (int g = __ldg(a.th_ptr + q0 + q); g < g1; ++g) {
+        const int2 r = __ldg(a.th_row + g);
+        const double2 wa = __ldg(a.th_w + 2 * g), wb = __ldg(a.th_w + 2 * g + 1);
+        const unsigned ka = r.x + pp, kb = r.y + pp;
+        const C ea = __ldg(ph + ka), eb = __ldg(ph + kb);
+        C sa[3], sb[3];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] = cfma(f, __ldg(bp + static_cast<size_t>(c) * Kp + kp), v[c]);
+        for (int c = 0; c < 3; ++c) {
+          sa[c] = __ldg(bh + (c * Kp + ka));
+          sb[c] = __ldg(bh + (c * Kp + kb));
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const C fa = cmul(ea, sa[c]), fb = cmul(eb, sb[c]);
+          v0[c] = cfmas(static_cast<R>(wb.x), fb, cfmas(static_cast<R>(wa.x), fa, v0[c]));
+          v1[c] = cfmas(static_cast<R>(wb.y), fb, cfmas(static_cast<R>(wa.y), fa, v1[c]));
+        }
       }
+      const int r0 = 2 * (q0 + q) - tc0;  // band row of the pair's first child row (-1: before the band)
+      C* o = band + 3 * h * stride + r0 * a.npp + pp;
+      if (r0 >= 0)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) band[c * stride + e] = v[c];
+        for (int c = 0; c < 3; ++c) o[c * stride] = v0[c];
+      if (r0 + 1 < rows)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[c * stride + a.npp] = v1[c];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < rows * a.npc; e += blockDim.x) {
-      const int r = e / a.npc, pc = e - r * a.npc;
-      C v[6];
+    const int nout = rows * a.npc;
+    for (int e = threadIdx.x; e < 2 * nout; e += blockDim.x) {
+      const int h = e >= nout, ee = e - h * nout;
+      const int r = ee / a.npc, pc = ee - r * a.npc;
+      C* o = out + (h * 3 * Kc + static_cast<unsigned>(tc0 * a.npc + ee));
+      C v[3];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) v[c] = Cx<C>::zero();
-      const int q1 = __ldg(a.ph_ptr + pc + 1);
-      for (int q = __ldg(a.ph_ptr + pc); q < q1; ++q) {
-        const R w = static_cast<R>(__ldg(a.ph_w + q));
-        const int src = r * a.npp + __ldg(a.ph_src + q);
+      for (int c = 0; c < 3; ++c) v[c] = o[c * Kc];
+      const C* src = band + 3 * h * stride + r * a.npp;
+      const int g1 = __ldg(a.ph_ptr + pc + 1);
+      for (int g = __ldg(a.ph_ptr + pc); g < g1; ++g) {
+        const int2 t = __ldg(a.ph_src + g);
+        const double2 w = __ldg(a.ph_w + g);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] = cfmas(w, band[c * stride + src], v[c]);
+        for (int c = 0; c < 3; ++c)
+          v[c] = cfmas(static_cast<R>(w.y), src[c * stride + t.y], cfmas(static_cast<R>(w.x), src[c * stride + t.x], v[c]));
       }
-      C* o = out + (tc0 + r) * a.npc + pc;
 #pragma unroll
-      for (int c = 0; c < 6; ++c) o[static_cast<size_t>(c) * Kc] = cadd(o[static_cast<size_t>(c) * Kc], v[c]);
+      for (int c = 0; c < 3; ++c) o[c * Kc] = v[c];
     }
   }
 }
@@ -1533,7 +1654,7 @@ void launch_up(Plan& P, int m, const LeafView& v, cudaStream_t s) {
     } else {
       UpArg<double2> a{Sc, pm.S, P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
                        pm.ph_up, pm.K, pm.nph, cm.K, cm.nph};
-      launch_up<double2, false>(up_threads(P), P.lv[l].B, pm.K, 6, a, s);
+      launch_up<double2, false>(up_threads(P), P.lv[l].B, 6, pm, a, s);
     }
   }
 }
@@ -1625,8 +1746,8 @@ void launch_l2l(Plan& P, int m, const LeafView& v, cudaStream_t s) {
     const MediumLevel& pm = P.ml[m][l - 1];
     double2* Bc = level_B(P, m, l, v);
     if (P.tuning.l2l_variant == 1 && 6 * pm.nph <= kL2lBand) {
-      L2lSepArg<double2> b{Bc,         pm.Bm,    P.lv[l].parent, P.lv[l].octant, pm.ph_dn, cm.thT_ptr,
-                  cm.thT_src, cm.thT_w, cm.phT_ptr,     cm.phT_src,     cm.phT_w, cm.nth,
+      L2lSepArg<double2> b{Bc,         pm.Bm,    P.lv[l].parent, P.lv[l].octant, pm.ph_dn, cm.th2_ptr,
+                  cm.th2_row, cm.th2_w, cm.ph2_ptr,     cm.ph2_src,     cm.ph2_w, cm.nth,
                   cm.nph,     pm.nth,   pm.nph};
       l2l_sep_kernel<double2><<<dim3(P.lv[l].B, l2l_grid_y(P.lv[l].B, cm.nth, pm.nph)), 256, 0, s>>>(b);
     } else {
@@ -1756,7 +1877,7 @@ void tree_pass_fixed(Plan& P, int m, C* leafS, C* leafB, cudaStream_t s, cudaStr
     const MediumLevel& cm = P.ml[m][l + 1];
     UpArg<C> a{S_at(l + 1), S_at(l), P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
                Store<C>::ph_up(pm), pm.K, pm.nph, cm.K, cm.nph};
-    launch_up<C, false>(up_threads(P), P.lv[l].B, pm.K, 6, a, s);
+    launch_up<C, false>(up_threads(P), P.lv[l].B, 6, pm, a, s);
   }
   if (sx) {
     translate(2, L - 1, s);
@@ -1768,8 +1889,8 @@ void tree_pass_fixed(Plan& P, int m, C* leafS, C* leafB, cudaStream_t s, cudaStr
     const MediumLevel& cm = P.ml[m][l];
     const MediumLevel& pm = P.ml[m][l - 1];
     if (6 * pm.nph > kL2lBand) throw std::runtime_error("anterpolation band: phi grid too large for this precision");
-    L2lSepArg<C> b{B_at(l),    B_at(l - 1), P.lv[l].parent, P.lv[l].octant, Store<C>::ph_dn(pm), cm.thT_ptr,
-                   cm.thT_src, cm.thT_w,    cm.phT_ptr,     cm.phT_src,     cm.phT_w,            cm.nth,
+    L2lSepArg<C> b{B_at(l),    B_at(l - 1), P.lv[l].parent, P.lv[l].octant, Store<C>::ph_dn(pm), cm.th2_ptr,
+                   cm.th2_row, cm.th2_w,    cm.ph2_ptr,     cm.ph2_src,     cm.ph2_w,            cm.nth,
                    cm.nph,     pm.nth,      pm.nph};
     l2l_sep_kernel<C><<<dim3(P.lv[l].B, l2l_grid_y(P.lv[l].B, cm.nth, pm.nph)), 256, 0, s>>>(b);
   }
@@ -1811,7 +1932,7 @@ void tree_pass_slots(Plan& P, int m, int rn, cudaStream_t s, cudaStream_t sx, cu
     UpArg<C> a{P.btS[m][l + 1], P.btS[m][l], P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx,
                pm.lp,           pm.ph_up32,  pm.K,                 pm.nph,              cm.K,    cm.nph,
                stride(l + 1),   stride(l)};
-    launch_up<C, true>(up_threads(P), P.lv[l].B, pm.K, 6 * rn, a, s);
+    launch_up<C, true>(up_threads(P), P.lv[l].B, 6 * rn, pm, a, s);
   }
   translate(2, L - 1, s);
   MLFMA_CUDA(cudaStreamWaitEvent(s, ev_leaf, 0));
@@ -1819,8 +1940,8 @@ void tree_pass_slots(Plan& P, int m, int rn, cudaStream_t s, cudaStream_t sx, cu
     const MediumLevel& cm = P.ml[m][l];
     const MediumLevel& pm = P.ml[m][l - 1];
     if (6 * pm.nph > kL2lBand) throw std::runtime_error("anterpolation band: phi grid too large for this precision");
-    L2lSepArg<C> b{P.btB[m][l], P.btB[m][l - 1], P.lv[l].parent, P.lv[l].octant, pm.ph_dn32, cm.thT_ptr,
-                   cm.thT_src,  cm.thT_w,        cm.phT_ptr,     cm.phT_src,     cm.phT_w,   cm.nth,
+    L2lSepArg<C> b{P.btB[m][l], P.btB[m][l - 1], P.lv[l].parent, P.lv[l].octant, pm.ph_dn32, cm.th2_ptr,
+                   cm.th2_row,  cm.th2_w,        cm.ph2_ptr,     cm.ph2_src,     cm.ph2_w,   cm.nth,
                    cm.nph,      pm.nth,          pm.nph,         stride(l),      stride(l - 1)};
     l2l_sep_kernel<C, true><<<dim3(P.lv[l].B, l2l_grid_y(P.lv[l].B, cm.nth, pm.nph), rn), 256, 0, s>>>(b);
   }

@@ -410,6 +410,35 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
           M.up4_tpos = P->upload(tpos);
         }
       }
+      if (l < L) {
+        // parent rows in pairs over the union of their child rows
+        const Interp& I = M.interp;
+        const int ncol = P->ml[m][l + 1].nph;
+        std::vector<int4> row;
+        std::vector<double2> w;
+        bool fits = true;
+        for (int t = 0; t < M.nth && fits; t += 2) {
+          std::vector<int> rows;
+          for (int u = t; u < std::min(t + 2, M.nth); ++u) rows.insert(rows.end(), &I.tidx[3 * u], &I.tidx[3 * u] + 3);
+          std::sort(rows.begin(), rows.end());
+          rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+          fits = rows.size() <= 4;
+          if (!fits) break;
+          double2 wr[4] = {};
+          for (int u = t; u < std::min(t + 2, M.nth); ++u)
+            for (int i = 0; i < 3; ++i) {
+              const size_t q = std::lower_bound(rows.begin(), rows.end(), I.tidx[3 * u + i]) - rows.begin();
+              (u == t ? wr[q].x : wr[q].y) += I.lt[3 * u + i];
+            }
+          rows.resize(4, rows.back());  // a repeated row of weight 0
+          row.push_back(make_int4(rows[0] * ncol, rows[1] * ncol, rows[2] * ncol, rows[3] * ncol));
+          w.insert(w.end(), wr, wr + 4);
+        }
+        if (fits) {
+          M.up2_row = P->upload(row);
+          M.up2_w = P->upload(w);
+        }
+      }
       if (l > 2) {
         // transposed interpolation: child direction <- (parent direction, weight)
         const MediumLevel& Pm = P->ml[m][l - 1];
@@ -436,30 +465,46 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
         M.tr_ptr = P->upload(cnt);
         M.tr_kp = P->upload(kps);
         M.tr_w = P->upload(ws);
-        // separable transposes of the two 1-D stencils
-        auto transpose1d = [&](const std::vector<int>& idx, const std::vector<double>& w, int nsrc, int ndst,
-                               int*& d_ptr, int*& d_src, double*& d_w) {
-          std::vector<int> ptr(ndst + 1, 0), src;
-          std::vector<double> wt;
-          for (int q = 0; q < nsrc; ++q)
-            for (int i = 0; i < 3; ++i) ptr[idx[3 * q + i] + 1]++;
-          for (int d = 0; d < ndst; ++d) ptr[d + 1] += ptr[d];
-          src.resize(ptr[ndst]);
-          wt.resize(ptr[ndst]);
-          std::vector<int> f(ptr.begin(), ptr.end() - 1);
+        // separable transposes of the two 1-D stencils, in groups of two taps;
+        // `per` child rows share a group list
+        auto grouped = [&](const std::vector<int>& idx, const std::vector<double>& w, int nsrc, int ndst, int per,
+                           int pitch, std::vector<int>& ptr, std::vector<int2>& src, std::vector<double2>& wt) {
+          std::vector<std::vector<std::array<double, 3>>> taps((ndst + per - 1) / per);  // source, weights
           for (int q = 0; q < nsrc; ++q)
             for (int i = 0; i < 3; ++i) {
               const int d = idx[3 * q + i];
-              src[f[d]] = q;
-              wt[f[d]] = w[3 * q + i];
-              f[d]++;
+              auto& list = taps[d / per];
+              if (list.empty() || list.back()[0] != q) list.push_back({static_cast<double>(q), 0.0, 0.0});
+              list.back()[1 + d % per] += w[3 * q + i];
             }
-          d_ptr = P->upload(ptr);
-          d_src = P->upload(src);
-          d_w = P->upload(wt);
+          ptr.assign(1, 0);
+          for (auto& list : taps) {
+            if (list.size() % 2) list.push_back({list.back()[0], 0.0, 0.0});
+            for (size_t q = 0; q < list.size(); q += 2) {
+              src.push_back(make_int2(static_cast<int>(list[q][0]) * pitch, static_cast<int>(list[q + 1][0]) * pitch));
+              if (per == 2) {
+                wt.push_back(make_double2(list[q][1], list[q][2]));
+                wt.push_back(make_double2(list[q + 1][1], list[q + 1][2]));
+              } else {
+                wt.push_back(make_double2(list[q][1], list[q + 1][1]));
+              }
+            }
+            ptr.push_back(static_cast<int>(src.size()));
+          }
         };
-        transpose1d(I.tidx, I.lt, Pm.nth, M.nth, M.thT_ptr, M.thT_src, M.thT_w);
-        transpose1d(I.pidx, I.lp, Pm.nph, M.nph, M.phT_ptr, M.phT_src, M.phT_w);
+        {
+          std::vector<int> tp, pp;
+          std::vector<int2> ts, ps;
+          std::vector<double2> tw, pw;
+          grouped(I.tidx, I.lt, Pm.nth, M.nth, 2, Pm.nph, tp, ts, tw);
+          grouped(I.pidx, I.lp, Pm.nph, M.nph, 1, 1, pp, ps, pw);
+          M.th2_ptr = P->upload(tp);
+          M.th2_row = P->upload(ts);
+          M.th2_w = P->upload(tw);
+          M.ph2_ptr = P->upload(pp);
+          M.ph2_src = P->upload(ps);
+          M.ph2_w = P->upload(pw);
+        }
       }
       // transfer factors over the offsets this level uses (Code/AlgoMLFMM.h:192-295)
       {

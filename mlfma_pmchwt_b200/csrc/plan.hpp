@@ -60,19 +60,26 @@ struct MediumLevel {
   int* up4_row_ptr = nullptr;
   int* up4_row = nullptr;
   int* up4_tpos = nullptr;
+  // parent theta rows in pairs (2q, 2q + 1): the at most 4 child theta rows
+  // their stencils share (offsets into a pattern: row * child phi columns) and
+  // each one's weight in the two parent rows; null when a pair needs more
+  int4* up2_row = nullptr;     // [ceil(nth / 2)]
+  double2* up2_w = nullptr;    // [ceil(nth / 2)][4]
   // this level as child of level-1: for each child direction, the parent
   // directions that interpolate onto it and the Lagrange weight
   int* tr_ptr = nullptr;       // [K+1]
   int* tr_kp = nullptr;
   double* tr_w = nullptr;
-  // the same, separable: child theta row -> (parent theta row, weight),
-  // child phi column -> (parent phi column, weight)
-  int* thT_ptr = nullptr;
-  int* thT_src = nullptr;
-  double* thT_w = nullptr;
-  int* phT_ptr = nullptr;
-  int* phT_src = nullptr;
-  double* phT_w = nullptr;
+  // the same, separable and two taps at a time (an odd count padded with a tap
+  // of weight 0): child theta rows in pairs (2q, 2q + 1), with the parent rows
+  // (offsets row * parent phi columns) either needs and each tap's weight in the
+  // two child rows; child phi columns with their taps' parent columns and weights
+  int* th2_ptr = nullptr;      // [ceil(nth / 2) + 1] into th2_row
+  int2* th2_row = nullptr;     // two taps
+  double2* th2_w = nullptr;    // [2] per entry of th2_row: tap's weight in row 2q, in row 2q + 1
+  int* ph2_ptr = nullptr;      // [nph + 1] into ph2_src
+  int2* ph2_src = nullptr;     // two taps
+  double2* ph2_w = nullptr;    // their weights
   // host copies
   Grid grid;
   Interp interp;               // this level from level+1 (levels 2..maxL-1)

@@ -1,0 +1,69 @@
+"""The tree passes level by level against the same sums in numpy, on the stage
+arrays and tables an operator reads out: interpolation by pairs of parent
+rows, translation by box pairs, anterpolation by pairs of child rows. Grids
+of odd and even theta counts, a lossy body, and grids so fine that an
+anterpolation band holds a single child row."""
+import numpy as np
+import pytest
+
+from mlfma_pmchwt_b200 import MLFMM, mesh as M
+
+pytestmark = pytest.mark.gpu
+
+BODIES = {"deep": lambda: dict(mesh=M.ellipsoid(3, 1.0, 0.8, 0.7), eps_r=2.5 - 0.1j, leaf_coeff=0.12),
+          "shallow": lambda: dict(mesh=M.icosphere(3, 1.0), eps_r=4.0, leaf_coeff=0.25),
+          "fine grids": lambda: dict(mesh=M.icosphere(1, 1.0), eps_r=360.0, leaf_coeff=0.25)}
+
+
+def _close(got, want):
+    """Sums of a few hundred products: 1e-12 of the array's largest value."""
+    assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("body", BODIES)
+def test_tree_levels(body):
+    op = MLFMM(freq=3e8, device=0, **BODIES[body]())
+    assert op.max_level > 2
+    x = M.unit_disk_vector(op.n, 3)
+    op.apply_ax(x)
+    odd, single = set(), False
+    for m, k in ((1, op.k1), (2, op.k2)):
+        S = {l: op.stage("S", m, l) for l in op.levels()}
+        B = {l: op.stage("B", m, l) for l in op.levels()}
+        mats = {}
+        for l in range(op.max_level - 1, 1, -1):  # parent l, child l + 1
+            g, gc, q = op.grid(m, l), op.grid(m, l + 1), op.interp(m, l)
+            odd.add(g["L"] % 2)
+            single = single or 2944 // (6 * 2 * g["L"]) <= 1
+            T, F = np.zeros((g["L"], gc["L"])), np.zeros((2 * g["L"], 2 * gc["L"]))
+            for i in range(3):
+                np.add.at(T, (np.arange(len(T)), q["tidx"][:, i]), q["lt"][:, i])
+                np.add.at(F, (np.arange(len(F)), q["pidx"][:, i]), q["lp"][:, i])
+            th, ph = np.meshgrid(g["theta"], g["phi"], indexing="ij")
+            kh = np.stack([np.sin(th) * np.cos(ph), np.sin(th) * np.sin(ph), np.cos(th)]).reshape(3, -1)
+            (cp, xp), (cc, xc) = op.level(l), op.level(l + 1)
+            at = {int(c): i for i, c in enumerate(cp)}
+            par = np.array([at[int(c) >> 3] for c in cc])
+            up = np.exp(-1j * k * ((xp[par] - xc) @ kh))
+            dn = np.exp(-1j * k * ((xc - xp[par]) @ kh))
+            c = S[l + 1].reshape(len(cc), 6, gc["L"], 2 * gc["L"])
+            want = np.zeros_like(S[l])
+            np.add.at(want, par, (T @ c @ F.T).reshape(len(cc), 6, -1) * up[:, None])
+            _close(S[l], want)
+            mats[l] = (T, F, dn, par)
+        for l in op.levels():
+            g, lst = op.grid(m, l), op.level_lists(l)
+            tf, off = op.transfer(m, l)
+            tf = tf * (np.repeat(g["wtheta"], 2 * g["L"]) * g["wphi"])
+            row = {(int(a) + 3) * 49 + (int(b) + 3) * 7 + int(c) + 3: i for i, (a, b, c) in enumerate(off)}
+            want = np.zeros_like(B[l])
+            for b in range(len(want)):
+                for e in range(lst["far_ptr"][b], lst["far_ptr"][b + 1]):
+                    want[b] += tf[row[int(lst["far_off"][e])]] * S[l][lst["far_idx"][e]]
+            if l > 2:
+                T, F, dn, par = mats[l - 1]
+                p = (B[l - 1][par] * dn[:, None]).reshape(len(par), 6, T.shape[0], F.shape[0])
+                want += (T.T @ p @ F).reshape(want.shape)
+            _close(B[l], want)
+    assert odd == {0, 1} or body != "deep"
+    assert single or body != "fine grids"
