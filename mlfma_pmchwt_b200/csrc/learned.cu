@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <stdexcept>
 #include <vector>
 
@@ -24,7 +25,8 @@ constexpr int kRedBlocks = 256;
 constexpr int kColParts = 64;     // partial column sums over boxes
 constexpr int kLayerBoxes = 32;   // boxes per CTA in the layer kernels
 constexpr int kDecRows = 32;      // RWGs per CTA in the decoder kernels
-constexpr int kWgRows = 256;      // rows per CTA in the weight-gradient kernel
+constexpr int kWgTile = 32;        // rows staged at a time by a weight-gradient CTA
+constexpr int kWgCtas = 296;       // row slices of one gradient at most (2 CTAs per SM)
 
 __device__ __forceinline__ float bf(const __nv_bfloat16* w, int i) { return __bfloat162float(w[i]); }
 __device__ __forceinline__ float2 f2(double2 a) {
@@ -562,34 +564,78 @@ struct WgArg {
   float* db;         // db[o] += sum_rows A (optional)
 };
 
-// dW += A^T X over the rows: kWgRows rows per CTA, 256 threads, thread
-// (o = tid / 4, k = tid % 4 + 4 j).
-__global__ void __launch_bounds__(256) lp_wgrad_kernel(WgArg g) {
-  __shared__ float As[32][kLpH + 1];
-  __shared__ float Xs[32][kLpH + 1];
-  const int tid = threadIdx.x, o = tid >> 2, kq = tid & 3;
-  const int r0 = blockIdx.x * kWgRows, r1 = min(g.rows, r0 + kWgRows);
-  const int nk = g.K / 4;
-  float acc[16], accb = 0.f;
-  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  for (int rb = r0; rb < r1; rb += 32) {
-    for (int i = tid; i < 32 * kLpH; i += 256) {
-      const int rr = i / kLpH, c = i % kLpH, row = rb + rr;
+struct WgJobs {
+  WgArg job[3];
+};
+
+// dW += A^T X over the rows, up to three gradients of as many rows in one
+// launch (grid.y): a CTA takes `per` rows, 32 at a time through shared memory
+// with the next 32 in flight; a thread sums 4 x 4 entries (o = 4 (tid / 16) + i,
+// k = tid % 16 + 16 j), 5 shared loads per 16 multiply-adds, and its atomics
+// run along the rows of dW.
+// Latency-bound at the sizes in use (7,680 rows: 63 MFLOP): with 256 rows per
+// CTA, 30 CTAs on 148 SMs that waited for each 32 rows and read 17 shared values
+// per 16 multiply-adds, a gradient took 81 us; now 11 us for up to three.
+__global__ void __launch_bounds__(256) lp_wgrad_kernel(const __grid_constant__ WgJobs jobs, int per) {
+  __shared__ float4 As4[kWgTile][kLpH / 4];
+  __shared__ float Xs[kWgTile][kLpH];
+  float(*As)[kLpH] = reinterpret_cast<float(*)[kLpH]>(As4);
+  const WgArg& g = jobs.job[blockIdx.y];
+  const int tid = threadIdx.x, o4 = tid >> 4, kc = tid & 15;
+  const int r0 = blockIdx.x * per, r1 = min(g.rows, r0 + per);
+  if (r0 >= r1) return;
+  const int c = tid & 63, rr0 = tid >> 6;  // staging: column c of rows rr0 + 4 i
+  constexpr int kPer = kWgTile * kLpH / 256;
+  float fa[kPer], fx[kPer];
+  auto fetch = [&](int rb) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int row = rb + rr0 + 4 * i;
       const bool in = row < r1;
-      As[rr][c] = (in && c < g.O) ? g.A[static_cast<long long>(row) * g.lda + c] : 0.f;
-      Xs[rr][c] = (in && c < g.K) ? g.X[static_cast<long long>(g.xmap ? g.xmap[row] : row) * g.ldx + c] : 0.f;
+      fa[i] = in && c < g.O ? g.A[static_cast<long long>(row) * g.lda + c] : 0.f;
+      fx[i] = in && c < g.K ? g.X[static_cast<long long>(g.xmap ? g.xmap[row] : row) * g.ldx + c] : 0.f;
     }
-    __syncthreads();
-    for (int rr = 0; rr < 32; ++rr) {
-      const float a = As[rr][o];
-      accb += a;
-      for (int j = 0; j < nk; ++j) acc[j] = fmaf(a, Xs[rr][kq + 4 * j], acc[j]);
-    }
-    __syncthreads();
+  };
+  float acc[4][4], accb[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    accb[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
   }
-  if (o < g.O) {
-    for (int j = 0; j < nk; ++j) atomicAdd(g.dW + o * g.ldw + kq + 4 * j, acc[j]);
-    if (g.db && kq == 0) atomicAdd(g.db + o, accb);
+  fetch(r0);
+  for (int rb = r0; rb < r1; rb += kWgTile) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      As[rr0 + 4 * i][c] = fa[i];
+      Xs[rr0 + 4 * i][c] = fx[i];
+    }
+    __syncthreads();
+    if (rb + kWgTile < r1) fetch(rb + kWgTile);
+#pragma unroll 8
+    for (int rr = 0; rr < kWgTile; ++rr) {
+      const float4 a = As4[rr][o4];
+      const float av[4] = {a.x, a.y, a.z, a.w};
+      float x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = Xs[rr][kc + 16 * j];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        accb[i] += av[i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], x[j], acc[i][j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int o = 4 * o4 + i;
+    if (o >= g.O) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (kc + 16 * j < g.K) atomicAdd(g.dW + o * g.ldw + kc + 16 * j, acc[i][j]);
+    if (g.db && kc == 0) atomicAdd(g.db + o, accb[i]);
   }
 }
 
@@ -808,10 +854,15 @@ void lp_forward(Plan& P, const __nv_bfloat16* w, const double2* /* v: enters thr
   MLFMA_CUDA(cudaGetLastError());
 }
 
-static void wgrad(const float* A, int lda, int O, const float* X, int ldx, int K, const int* xmap, int rows, float* dW,
-                  int ldw, float* db, cudaStream_t s) {
-  WgArg g{A, lda, O, X, ldx, K, xmap, rows, dW, ldw, db};
-  lp_wgrad_kernel<<<(rows + kWgRows - 1) / kWgRows, 256, 0, s>>>(g);
+// Gradients over the same rows in one launch; a CTA takes at least two tiles
+// of rows, more when the rows would need over kWgCtas CTAs.
+static void wgrad(std::initializer_list<WgArg> jobs, cudaStream_t s) {
+  WgJobs w{};
+  int n = 0;
+  for (const WgArg& g : jobs) w.job[n++] = g;
+  const int rows = w.job[0].rows, least = (rows + kWgCtas - 1) / kWgCtas;
+  const int per = std::max(2 * kWgTile, (least + kWgTile - 1) / kWgTile * kWgTile);
+  lp_wgrad_kernel<<<dim3((rows + per - 1) / per, n), 256, 0, s>>>(w, per);
 }
 
 void lp_backward(Plan& P, const __nv_bfloat16* w, const double2* y, const double2* e, const double2* gy, float* grad,
@@ -824,9 +875,10 @@ void lp_backward(Plan& P, const __nv_bfloat16* w, const double2* y, const double
   }
   DecBwdArg d{W.t, w, y, e, W.esum, gy, W.u, W.q, W.dG, W.dq, W.dx, gy ? nullptr : loss};
   lp_decode_bwd_kernel<<<(N + kDecRows - 1) / kDecRows, 128, dec_bwd_smem(), s>>>(d);
-  wgrad(W.dG, kLpG, kLpG, W.q, kLpH, kLpH, nullptr, N, grad + kLpOffWd2, kLpH, grad + kLpOffD2, s);
-  wgrad(W.dq, kLpH, kLpH, W.h[kLpLayers], kLpH, kLpH, W.t.pos_box, N, grad + kLpOffWd1, 2 * kLpH, grad + kLpOffD1, s);
-  wgrad(W.dq, kLpH, kLpH, W.a, kLpH, kLpH, nullptr, N, grad + kLpOffWd1 + kLpH, 2 * kLpH, nullptr, s);
+  wgrad({{W.dG, kLpG, kLpG, W.q, kLpH, kLpH, nullptr, N, grad + kLpOffWd2, kLpH, grad + kLpOffD2},
+         {W.dq, kLpH, kLpH, W.h[kLpLayers], kLpH, kLpH, W.t.pos_box, N, grad + kLpOffWd1, 2 * kLpH, grad + kLpOffD1},
+         {W.dq, kLpH, kLpH, W.a, kLpH, kLpH, nullptr, N, grad + kLpOffWd1 + kLpH, 2 * kLpH, nullptr}},
+        s);
   lp_box_dxsum_kernel<<<(B + 7) / 8, 256, 0, s>>>(W.t, W.dx, W.dh);
   float* dh = W.dh;
   float* dh_next = W.dh2;
@@ -835,15 +887,16 @@ void lp_backward(Plan& P, const __nv_bfloat16* w, const double2* y, const double
     lp_dp_kernel<<<kColParts, 256, 0, s>>>(dh, W.P[l], B, W.dP, W.cpart);
     LayerBwdArg lb{W.t, layer_w(w, l), dh, W.dP, W.cpart, W.tmp, W.dm, W.S};
     lp_layer_bwd_kernel<<<(B + kLayerBoxes - 1) / kLayerBoxes, 256, layer_bwd_smem(), s>>>(lb);
-    wgrad(W.dP, kLpH, kLpH, W.h[l], kLpH, kLpH, nullptr, B, gl, kLpH, gl + 3 * kLpH * kLpH, s);
-    wgrad(W.dP, kLpH, kLpH, W.m[l], kLpH, kLpH, nullptr, B, gl + kLpH * kLpH, kLpH, nullptr, s);
+    wgrad({{W.dP, kLpH, kLpH, W.h[l], kLpH, kLpH, nullptr, B, gl, kLpH, gl + 3 * kLpH * kLpH},
+           {W.dP, kLpH, kLpH, W.m[l], kLpH, kLpH, nullptr, B, gl + kLpH * kLpH, kLpH, nullptr}},
+          s);
     lp_outer_kernel<<<(kLpH * kLpH + 255) / 256, 256, 0, s>>>(W.S, W.g[l], gl + 2 * kLpH * kLpH);
     lp_nbr_sum_kernel<<<(B * kLpH + 255) / 256, 256, 0, s>>>(W.t, W.tmp, W.dm, dh_next);
     std::swap(dh, dh_next);
   }
   lp_unpool_kernel<<<static_cast<int>((static_cast<long long>(N) * kLpH + 255) / 256), 256, 0, s>>>(W.t, dh, W.a,
                                                                                                      W.dx);
-  wgrad(W.dx + kLpH, 2 * kLpH, kLpH, W.t.fs, kLpF, kLpF, nullptr, N, grad, kLpF, grad + kLpOffBe, s);
+  wgrad({{W.dx + kLpH, 2 * kLpH, kLpH, W.t.fs, kLpF, kLpF, nullptr, N, grad, kLpF, grad + kLpOffBe}}, s);
   MLFMA_CUDA(cudaGetLastError());
 }
 
