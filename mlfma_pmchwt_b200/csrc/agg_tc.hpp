@@ -45,5 +45,9 @@ bool agg_tc_supported(const Plan& P, int R);
 size_t agg_tc_smem_bytes(int kmax);
 void launch_agg_tc(const Plan& P, const AggTcArg& a, cudaStream_t s);
 void launch_leaf_tc(const Plan& P, const LeafTcArg& a, cudaStream_t s);
+// The same contractions in FP32 on the CUDA cores (leaf_batch.cu); any number
+// of RWGs per box.
+void launch_agg_slots(const Plan& P, const AggTcArg& a, cudaStream_t s);
+void launch_leaf_slots(const Plan& P, const LeafTcArg& a, cudaStream_t s);
 
 }  // namespace mlfma

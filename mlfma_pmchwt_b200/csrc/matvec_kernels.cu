@@ -2002,27 +2002,28 @@ void apply_batch_fixed(Plan& P, int R, const double2* X, long long ldx, double2*
     ag.R = rn;
     bool on_tensor_cores = false;
     if constexpr (std::is_same<C, float2>::value) {
-      if (P.tuning.batch_tc == 1 && agg_tc_supported(P, rn)) {
-        AggTcArg t{};
-        for (int m = 0; m < 2; ++m) {
-          t.Vs[m] = reinterpret_cast<const float*>(ag.Vs[m]);
-          t.K[m] = ag.K[m];
-          for (int j = 0; j < rn; ++j) t.S[m][j] = ag.S[m][j];
-        }
-        t.leaf_ptr = ag.leaf_ptr;
-        t.leaf_rwg = ag.leaf_rwg;
-        t.X = ag.X;
-        t.ldx = ag.ldx;
-        t.N = ag.N;
-        t.R = rn;
-        t.kmax = (P.max_leaf_rwgs + 7) & ~7;
-        t.status = P.d_status;
-        launch_agg_tc(P, t, s);
-        on_tensor_cores = true;
+      AggTcArg t{};
+      for (int m = 0; m < 2; ++m) {
+        t.Vs[m] = reinterpret_cast<const float*>(ag.Vs[m]);
+        t.K[m] = ag.K[m];
+        for (int j = 0; j < rn; ++j) t.S[m][j] = ag.S[m][j];
       }
-    }
-    if (!on_tensor_cores)
+      t.leaf_ptr = ag.leaf_ptr;
+      t.leaf_rwg = ag.leaf_rwg;
+      t.X = ag.X;
+      t.ldx = ag.ldx;
+      t.N = ag.N;
+      t.R = rn;
+      t.kmax = (P.max_leaf_rwgs + 7) & ~7;
+      t.status = P.d_status;
+      on_tensor_cores = P.tuning.batch_tc == 1 && agg_tc_supported(P, rn);
+      if (on_tensor_cores)
+        launch_agg_tc(P, t, s);
+      else
+        launch_agg_slots(P, t, s);
+    } else {
       agg_batch_kernel<C, kAggRB><<<dim3(P.lv[L].B, 2, (rn + kAggRB - 1) / kAggRB), kThreads, 0, s>>>(ag);
+    }
     {
       MediumStreams ms(P, s, true);
       if constexpr (std::is_same<C, float2>::value) {
@@ -2056,30 +2057,31 @@ void apply_batch_fixed(Plan& P, int R, const double2* X, long long ldx, double2*
     lb.R = rn;
     const int warps = kThreads / 32;
     const dim3 grid((P.N + warps - 1) / warps, (rn + kLeafRB - 1) / kLeafRB);
-    if (on_tensor_cores) {
-      // near-field rows first (writing w), then the far field on the tensor cores (adding)
+    if constexpr (std::is_same<C, float2>::value) {
+      // near-field rows first (writing w), then the far field (adding)
       leaf_out_batch_kernel<C, kLeafRB, false><<<grid, kThreads, 0, s>>>(lb);
       MLFMA_CUDA(cudaGetLastError());
-      if constexpr (std::is_same<C, float2>::value) {
-        LeafTcArg t{};
-        for (int m = 0; m < 2; ++m) {
-          t.Vf[m] = lb.Vf[m];
-          t.khat[m] = lb.khat[m];
-          t.K[m] = lb.K[m];
-          for (int j = 0; j < rn; ++j) t.Bm[m][j] = lb.Bm[m][j];
-        }
-        t.leaf_ptr = P.d_leaf_ptr;
-        t.leaf_rwg = P.d_leaf_rwg;
-        t.W = lb.W;
-        t.ldw = ldw;
-        t.c1 = lb.c1;
-        t.c2 = lb.c2;
-        t.etai = lb.etai;
-        t.N = P.N;
-        t.R = rn;
-        t.status = P.d_status;
-        launch_leaf_tc(P, t, s);
+      LeafTcArg t{};
+      for (int m = 0; m < 2; ++m) {
+        t.Vf[m] = lb.Vf[m];
+        t.khat[m] = lb.khat[m];
+        t.K[m] = lb.K[m];
+        for (int j = 0; j < rn; ++j) t.Bm[m][j] = lb.Bm[m][j];
       }
+      t.leaf_ptr = P.d_leaf_ptr;
+      t.leaf_rwg = P.d_leaf_rwg;
+      t.W = lb.W;
+      t.ldw = ldw;
+      t.c1 = lb.c1;
+      t.c2 = lb.c2;
+      t.etai = lb.etai;
+      t.N = P.N;
+      t.R = rn;
+      t.status = P.d_status;
+      if (on_tensor_cores)
+        launch_leaf_tc(P, t, s);
+      else
+        launch_leaf_slots(P, t, s);
     } else {
       leaf_out_batch_kernel<C, kLeafRB><<<grid, kThreads, 0, s>>>(lb);
       MLFMA_CUDA(cudaGetLastError());

@@ -141,8 +141,8 @@ struct Tuning {
                                // 3: separable in registers, 4-row bands per thread
   int agg_variant = 0;         // 0: thread per (box, direction); 1: CTA per (box, medium) streaming
                                //    the box's contiguous pattern block
-  int batch_tc = 1;            // batched complex64 leaf aggregation and far-field testing: 0 CUDA cores; 1 tcgen05
-                               //    (3xTF32 split, TMEM accumulators)
+  int batch_tc = 0;            // batched complex64 leaf aggregation and far-field testing: 0 FP32 on the CUDA
+                               //    cores; 1 tcgen05 (3xTF32 split, TMEM accumulators)
   int batch_tree = 1;          // batched complex64 tree passes: 0 one slot after another; 1 every level
                                //    once for all slots (slot-major arrays)
   int leaf_variant = 0;        // 0: near field inside the leaf kernel; 1: near field on its own
