@@ -7,7 +7,9 @@
 // fused multiply-adds each, 0.25 ms at the FP32 rate. The tensor-core forms of
 // agg_tc.cu do the same contractions as three TF32 products per step, but
 // splitting, transposing and storing the operands costs more than the
-// multiply-adds it saves (tensor pipe 7-10 % active).
+// multiply-adds it saves (tensor pipe 7-10 % active). One B200, 16 slots at
+// 61,440 unknowns: aggregation 0.62 against 0.95 ms, testing 1.15 against 1.87;
+// 8 slots at 15,360: 0.10 against 0.26 and 0.20 against 0.44 ms.
 #include <stdexcept>
 
 #include "agg_tc.hpp"
@@ -19,7 +21,7 @@ namespace mlfma {
 namespace {
 
 constexpr int kAbThreads = 256;
-constexpr int kAbStage = 48;  // RWGs of a box staged at a time
+constexpr int kAbStage = 48;  // RWGs of a box staged at a time (a multiple of 4)
 
 // Aggregation: CTA per (leaf box, 256 pattern entries of one medium), a thread
 // one entry of every (part, slot): 2 kS complex sums. The box's currents are
@@ -37,6 +39,13 @@ __global__ void __launch_bounds__(kAbThreads, 2) agg_slots_kernel(const __grid_c
   float2 acc[2 * kS];
 #pragma unroll
   for (int i = 0; i < 2 * kS; ++i) acc[i] = make_float2(0.f, 0.f);
+  float2 next[4];  // the next four RWGs' values, in flight
+  auto fetch = [&](int r) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      next[u] = r + u < nb ? __ldg(V + static_cast<size_t>(r + u) * K3) : make_float2(0.f, 0.f);
+  };
+  fetch(0);
   for (int s0 = 0; s0 < nb; s0 += kAbStage) {
     const int n = min(kAbStage, nb - s0);
     __syncthreads();
@@ -47,11 +56,11 @@ __global__ void __launch_bounds__(kAbThreads, 2) agg_slots_kernel(const __grid_c
       xs[i] = x;
     }
     __syncthreads();
-    for (int r = 0; r < n; r += 4) {  // four entries in flight
+    for (int r = 0; r < n; r += 4) {
       float2 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        v[u] = r + u < n ? __ldg(V + static_cast<size_t>(s0 + r + u) * K3) : make_float2(0.f, 0.f);
+      for (int u = 0; u < 4; ++u) v[u] = next[u];
+      fetch(s0 + r + 4);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (r + u < n) {
@@ -102,7 +111,7 @@ struct LeafSlots {
   static constexpr int kVPitch = kLbEntries + 2;      // float2 per row
   struct Smem {
     float2 V[2][kRows * kVPitch];
-    float2 D[kLbEntries * kDPitch];
+    float2 D[2][kLbEntries * kDPitch];
   };
   static_assert(sizeof(float2) * kLbWarps * kRows * kCols <= 2 * sizeof(Smem), "");
 };
@@ -178,17 +187,17 @@ __global__ void __launch_bounds__(kLbThreads, 2) leaf_slots_kernel(const __grid_
           const int q1 = (q + 1) % 3, q2 = (q + 2) % 3;
           const float2 xJ = csub(cscale(J[q2], kh[q1]), cscale(J[q1], kh[q2]));  // khat x B_J
           const float2 xM = csub(cscale(M[q2], kh[q1]), cscale(M[q1], kh[q2]));
-          float2* d = sm.D + (q * kLbDirs + kk) * T::kDPitch;
+          float2* d = sm.D[ch & 1] + (q * kLbDirs + kk) * T::kDPitch;
           d[j] = csub(cmul(ce, J[q]), cmul(c, xM));
           d[kS + j] = cfma(cie, M[q], cmul(c, xJ));
         }
       }
     }
+    cp_async_wait<0>();
+    __syncthreads();  // the chunk is staged, and every warp is done with the one before it
     stage(ch + 1);
-    cp_async_wait<1>();
-    __syncthreads();
     if (ch + 1 < nchunk) fetch(ch + 1);
-    const float2* V = sm.V[ch & 1];
+    const float2 *V = sm.V[ch & 1], *Dc = sm.D[ch & 1];
 #pragma unroll
     for (int t = 0; t < kTiles; ++t) {
       if (t * T::kTileRows >= nt) break;
@@ -198,11 +207,11 @@ __global__ void __launch_bounds__(kLbThreads, 2) leaf_slots_kernel(const __grid_
 #pragma unroll
         for (int j = 0; j < 4; ++j) s[i][j] = make_float2(0.f, 0.f);
       const float2* v0 = V + (t * T::kTileRows + 2 * rg) * T::kVPitch;
-#pragma unroll
+#pragma unroll 4  // all 12 at once spill
       for (int q = 0; q < kLbEntries / kLbWarps; ++q) {
         const int en = wp * (kLbEntries / kLbWarps) + q;
-        const float4 da = *reinterpret_cast<const float4*>(sm.D + en * T::kDPitch + 4 * cg);
-        const float4 db = *reinterpret_cast<const float4*>(sm.D + en * T::kDPitch + 4 * cg + 2);
+        const float4 da = *reinterpret_cast<const float4*>(Dc + en * T::kDPitch + 4 * cg);
+        const float4 db = *reinterpret_cast<const float4*>(Dc + en * T::kDPitch + 4 * cg + 2);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const float2 v = v0[i * T::kVPitch + en];
@@ -217,9 +226,8 @@ __global__ void __launch_bounds__(kLbThreads, 2) leaf_slots_kernel(const __grid_
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[t][i][j] = cadd(acc[t][i][j], s[i][j]);
     }
-    __syncthreads();
   }
-  cp_async_wait<0>();
+  __syncthreads();
   float2* red = reinterpret_cast<float2*>(leaf_smem);  // [warp][row][column]
 #pragma unroll
   for (int t = 0; t < kTiles; ++t)

@@ -35,29 +35,64 @@ namespace {
 
 constexpr int kThreads = 128;
 
-// Aggregation: thread per (leaf box, direction), J and M from one pattern load.
+// Aggregation: thread per (leaf box, direction), J and M from one pattern
+// load. The box's currents are staged in shared memory (in the storage type)
+// and the next RWGs' patterns are always in flight, so the loop waits for
+// no index. HBM-bound (245,760 unknowns: 4.8 GB). One B200, both media, against
+// the loop that read each RWG's index, then its currents: FP64 at 245,760 unknowns
+// 0.94 -> 0.85 ms, at 7,260 70 -> 50 us, complex64 at 61,440 202 -> 140 us.
+constexpr int kAggRwgs = 48;  // RWGs of a box staged at a time (a multiple of the RWGs in flight)
+
 template <class C>
-__global__ void __launch_bounds__(kThreads) agg_kernel(const C* __restrict__ Vs, const int* __restrict__ leaf_ptr,
+__global__ void __launch_bounds__(kThreads, sizeof(C) == 16 ? 6 : 8) agg_kernel(const C* __restrict__ Vs, const int* __restrict__ leaf_ptr,
                                                        const int* __restrict__ leaf_rwg,
                                                        const double2* __restrict__ x, int N, int K,
                                                        C* __restrict__ S) {
+  constexpr int kFlight = sizeof(C) == 16 ? 2 : 4;
+  __shared__ C xs[kAggRwgs][2];
   const int kk = blockIdx.y * blockDim.x + threadIdx.x;
   const int b = blockIdx.x;
-  if (kk >= K) return;
+  const int r0 = leaf_ptr[b], nb = leaf_ptr[b + 1] - r0;
+  const C* V = Vs + static_cast<size_t>(r0) * 3 * K + min(kk, K - 1);
+  C next[kFlight][3];
+  auto fetch = [&](int r) {
+#pragma unroll
+    for (int u = 0; u < kFlight; ++u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        next[u][c] = r + u < nb ? __ldg(V + (static_cast<size_t>(r + u) * 3 + c) * K) : Cx<C>::zero();
+  };
+  fetch(0);
   C acc[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) acc[c] = Cx<C>::zero();
-  const int r1 = leaf_ptr[b + 1];
-  for (int r = leaf_ptr[b]; r < r1; ++r) {
-    const int id = leaf_rwg[r];
-    const C xJ = Cx<C>::from(x[id]), xM = Cx<C>::from(x[N + id]);
+  for (int s0 = 0; s0 < nb; s0 += kAggRwgs) {
+    const int n = min(kAggRwgs, nb - s0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x)
+      xs[i >> 1][i & 1] = Cx<C>::from(__ldg(x + (i & 1) * N + __ldg(leaf_rwg + r0 + s0 + (i >> 1))));
+    __syncthreads();
+#pragma unroll 1
+    for (int r = 0; r < n; r += kFlight) {
+      C v[kFlight][3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const C v = Vs[(static_cast<size_t>(r) * 3 + c) * K + kk];
-      acc[c] = cfma(v, xJ, acc[c]);
-      acc[3 + c] = cfma(v, xM, acc[3 + c]);
+      for (int u = 0; u < kFlight; ++u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[u][c] = next[u][c];
+      fetch(s0 + r + kFlight);
+#pragma unroll
+      for (int u = 0; u < kFlight; ++u)
+        if (r + u < n) {
+          const C xJ = xs[r + u][0], xM = xs[r + u][1];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            acc[c] = cfma(v[u][c], xJ, acc[c]);
+            acc[3 + c] = cfma(v[u][c], xM, acc[3 + c]);
+          }
+        }
     }
   }
+  if (kk >= K) return;
   C* out = S + static_cast<size_t>(b) * 6 * K + kk;
 #pragma unroll
   for (int c = 0; c < 6; ++c) out[static_cast<size_t>(c) * K] = acc[c];
@@ -1358,16 +1393,10 @@ struct LeafArg {
   const double* khat[2];
   int K[2];
   const int* leaf_rwg;
-  const int* rwg_box;     // leaf box of each RWG id
   const int* leaf_ptr;
-  const int* near_sptr;
-  const int* near_src;
-  const long long* near_zoff;
-  const C* near_z;
-  const double2* x;
   double2* w;
   int N;
-  C c1, c2, etai;
+  C c1, c2, etai, ietai;
 };
 
 template <class C>
@@ -1380,79 +1409,97 @@ __device__ __forceinline__ C warp_sum(C v) {
   return v;
 }
 
-// One warp per RWG (leaf order).
-// kNear = false: the far-field testing only, added to the near-field product
-// already in w (computed concurrently by near_apply).
-template <class C, bool kNear = true>
-__global__ void __launch_bounds__(kThreads) leaf_out_kernel(LeafArg<C> a) {
+// Far-field testing of both media, added to the near-field product already in
+// w. With c and e of a medium (c1, 1 or c2, etai),
+//   w_J += c sum over directions of Vf . (e B_J - khat x B_M),
+//   w_M += c sum over directions of Vf . (khat x B_J + B_M / e),
+// because ((-khat) x Vf) . B = Vf . (khat x B) (Code/MLFMM.cpp:285-351). CTA per
+// (leaf box, kLeafRows RWGs); its warps take every fourth 32 directions of
+// both media, form the bracketed vectors from the box's B in registers, once
+// for all the CTA's RWGs, and meet in shared memory at the end.
+// HBM-bound: the receive patterns are read once (245,760 unknowns: 4.35 GB,
+// 0.65 ms). One B200, this kernel and the near-field product before it against
+// one warp per RWG for both: FP64 at 245,760 unknowns 0.98 + 0.32 against 1.29
+// ms, at 7,260 40 + 12 against 56 us, complex64 at 61,440 149 + 54 against 217
+// us. With 2, 3, 4 and 6 RWGs per CTA the FP64 kernel takes 1.44, 1.11, 1.22 and
+// 1.07 ms; with the vectors staged in shared memory for 24 RWGs, 1.37 ms.
+constexpr int kLeafRows = 5;
+constexpr int kLeafWarps = 4;
+
+template <class C>
+__global__ void __launch_bounds__(32 * kLeafWarps, sizeof(C) == 16 ? 3 : 5)
+    leaf_rows_kernel(const __grid_constant__ LeafArg<C> a) {
   using R = typename Cx<C>::real;
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (r >= a.N) return;
-  const int id = a.leaf_rwg[r];
-  const int b = a.rwg_box[id];
-  C res[8];  // L1J K1J L1M K1M L2J K2J L2M K2M
+  __shared__ C red[kLeafWarps][2 * kLeafRows];
+  const int b = blockIdx.x;
+  const int r0 = a.leaf_ptr[b], nb = a.leaf_ptr[b + 1] - r0;
+  const int t0 = blockIdx.y * kLeafRows;
+  if (t0 >= nb) return;
+  const int nt = min(kLeafRows, nb - t0);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int n0 = (a.K[0] + 31) / 32, n = n0 + (a.K[1] + 31) / 32;
+  C acc[2 * kLeafRows];
 #pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    const int K = a.K[m];
-    const C* V = a.Vf[m] + static_cast<size_t>(r) * 3 * K;
-    const C* B = a.Bm[m] + static_cast<size_t>(b) * 6 * K;
-    const double* kh = a.khat[m];
-    C LJ = Cx<C>::zero(), KJ = Cx<C>::zero(), LM = Cx<C>::zero(), KM = Cx<C>::zero();
-#pragma unroll 2
-    for (int kk = lane; kk < K; kk += 32) {
-      const C v0 = V[kk], v1 = V[K + kk], v2 = V[2 * K + kk];
-      const C j0 = B[kk], j1 = B[K + kk], j2 = B[2 * K + kk];
-      const C m0 = B[3 * K + kk], m1 = B[4 * K + kk], m2 = B[5 * K + kk];
-      // (-khat) x V
-      const R ax = static_cast<R>(-kh[kk]), ay = static_cast<R>(-kh[K + kk]), az = static_cast<R>(-kh[2 * K + kk]);
-      const C w0 = csub(cscale(v2, ay), cscale(v1, az));
-      const C w1 = csub(cscale(v0, az), cscale(v2, ax));
-      const C w2 = csub(cscale(v1, ax), cscale(v0, ay));
-      LJ = cfma(v0, j0, cfma(v1, j1, cfma(v2, j2, LJ)));
-      LM = cfma(v0, m0, cfma(v1, m1, cfma(v2, m2, LM)));
-      KJ = cfma(w0, j0, cfma(w1, j1, cfma(w2, j2, KJ)));
-      KM = cfma(w0, m0, cfma(w1, m1, cfma(w2, m2, KM)));
+  for (int i = 0; i < 2 * kLeafRows; ++i) acc[i] = Cx<C>::zero();
+  bool second = false;  // the sums are in units of c2 instead of c1
+  for (int i = wp; i < n; i += kLeafWarps) {
+    const int m = i >= n0, K = a.K[m], k = (i - m * n0) * 32 + lane;
+    if (m && !second) {
+      const C q = cdiv(a.c1, a.c2);
+#pragma unroll
+      for (int j = 0; j < 2 * kLeafRows; ++j) acc[j] = cmul(acc[j], q);
+      second = true;
     }
-    res[4 * m + 0] = warp_sum(LJ);
-    res[4 * m + 1] = warp_sum(KJ);
-    res[4 * m + 2] = warp_sum(LM);
-    res[4 * m + 3] = warp_sum(KM);
-  }
-  // near-field rows t and N + t
-  C nJ = Cx<C>::zero(), nM = Cx<C>::zero();
-  if constexpr (kNear) {
-    const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
-    const int tl = r - a.leaf_ptr[b];
-    const int pitch = near_pitch(ns);
-    const C* Z = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
-#pragma unroll 2
-    for (int j = lane; j < ns; j += 32) {
-      const int s = a.near_src[s0 + j];
-      const C xJ = Cx<C>::from(a.x[s]), xM = Cx<C>::from(a.x[a.N + s]);
-      const C z11 = Z[j], z12 = Z[pitch + j], z22 = Z[2 * pitch + j];
-      nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
-      nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
-    }
-    nJ = warp_sum(nJ);
-    nM = warp_sum(nM);
-  }
-  if (lane == 0) {
-    // w[t]   = c1 (L1J - K1M) + c2 (etai L2J - K2M) + near
-    // w[N+t] = c1 (K1J + L1M) + c2 (K2J + L2M / etai) + near
-    const C L2M_eta = cdiv(res[6], a.etai);
-    C wj = cmul(a.c1, csub(res[0], res[3]));
-    wj = cadd(wj, cmul(a.c2, csub(cmul(a.etai, res[4]), res[7])));
-    C wm = cmul(a.c1, cadd(res[1], res[2]));
-    wm = cadd(wm, cmul(a.c2, cadd(res[5], L2M_eta)));
-    if constexpr (kNear) {
-      a.w[id] = Cx<C>::to64(cadd(wj, nJ));
-      a.w[a.N + id] = Cx<C>::to64(cadd(wm, nM));
-    } else {
-      a.w[id] = cadd(a.w[id], Cx<C>::to64(wj));
-      a.w[a.N + id] = cadd(a.w[a.N + id], Cx<C>::to64(wm));
+    if (k >= K) continue;
+    const C* V = a.Vf[m] + (static_cast<size_t>(r0 + t0) * 3) * K + k;
+    const C* B = a.Bm[m] + static_cast<size_t>(b) * 6 * K + k;
+    C v[kLeafRows][3], f[6];
+    R kh[3];
+#pragma unroll
+    for (int u = 0; u < kLeafRows; ++u)
+      if (u < nt)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[u][q] = __ldg(V + (u * 3 + q) * K);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) f[c] = __ldg(B + c * K);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) kh[c] = static_cast<R>(__ldg(a.khat[m] + c * K + k));
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int q1 = (q + 1) % 3, q2 = (q + 2) % 3;
+      const C xJ = csub(cscale(f[q2], kh[q1]), cscale(f[q1], kh[q2]));  // khat x B_J
+      const C xM = csub(cscale(f[3 + q2], kh[q1]), cscale(f[3 + q1], kh[q2]));
+      const C dJ = csub(m ? cmul(a.etai, f[q]) : f[q], xM);
+      const C dM = cadd(m ? cmul(a.ietai, f[3 + q]) : f[3 + q], xJ);
+#pragma unroll
+      for (int u = 0; u < kLeafRows; ++u)
+        if (u < nt) {
+          acc[2 * u] = cfma(v[u][q], dJ, acc[2 * u]);
+          acc[2 * u + 1] = cfma(v[u][q], dM, acc[2 * u + 1]);
+        }
     }
   }
+  const C c = second ? a.c2 : a.c1;
+#pragma unroll
+  for (int j = 0; j < 2 * kLeafRows; ++j) {
+    const C s = warp_sum(acc[j]);
+    if (lane == 0) red[wp][j] = cmul(c, s);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * nt) {
+    C s = red[0][threadIdx.x];
+#pragma unroll
+    for (int q = 1; q < kLeafWarps; ++q) s = cadd(s, red[q][threadIdx.x]);
+    double2* w = a.w + (threadIdx.x & 1) * a.N + a.leaf_rwg[r0 + t0 + (threadIdx.x >> 1)];
+    *w = cadd(*w, Cx<C>::to64(s));
+  }
+}
+
+template <class C>
+void launch_leaf(const Plan& P, LeafArg<C>& a, cudaStream_t s) {
+  a.ietai = cdiv(Cx<C>::from(c2(1.0, 0.0)), a.etai);
+  const dim3 grid(P.lv[P.maxL].B, (P.max_leaf_rwgs + kLeafRows - 1) / kLeafRows);
+  leaf_rows_kernel<C><<<grid, 32 * kLeafWarps, 0, s>>>(a);
 }
 
 // ---------------------------------------------------------------- batched
@@ -1762,18 +1809,22 @@ template <class Arg>
 void fill_leaf_common(const Plan& P, Arg& a) {
   using C = std::remove_reference_t<decltype(a.c1)>;
   a.leaf_rwg = P.d_leaf_rwg;
-  a.rwg_box = P.d_rwg_leafbox;
   a.leaf_ptr = P.d_leaf_ptr;
-  a.near_sptr = P.d_near_sptr;
-  a.near_src = P.d_near_src;
-  a.near_zoff = P.d_near_zoff;
-  a.near_z = Store<C>::near_z(P);
   a.N = P.N;
   const cplx c1 = P.k1 * P.k1 / (16.0 * kPi * kPi);
   const cplx c2v = P.k2 * P.k2 / (16.0 * kPi * kPi);
   a.c1 = Cx<C>::from(c2(c1.real(), c1.imag()));
   a.c2 = Cx<C>::from(c2(c2v.real(), c2v.imag()));
   a.etai = Cx<C>::from(c2(P.etai.real(), P.etai.imag()));
+}
+
+template <class C>
+void fill_leaf_near(const Plan& P, LeafBatchArg<C>& a) {
+  a.rwg_box = P.d_rwg_leafbox;
+  a.near_sptr = P.d_near_sptr;
+  a.near_src = P.d_near_src;
+  a.near_zoff = P.d_near_zoff;
+  a.near_z = Store<C>::near_z(P);
 }
 
 // Medium 1's tree passes go to the plan's second stream, forked from and
@@ -1799,22 +1850,29 @@ struct MediumStreams {
   }
 };
 
-// The near-field rows need only x: with leaf variant 1 they start at the
-// beginning of the apply on their own stream (writing w), and the leaf
-// kernel adds the far-field testing once they are done.
+// The near-field product needs only x and writes w, to which the leaf kernel
+// adds: with leaf variant 1 it starts at the beginning of the apply on its own
+// stream, else it runs before the leaf kernel on the caller's.
 struct NearAhead {
   Plan& P;
   cudaStream_t s;
-  bool on;
-  NearAhead(Plan& P_, cudaStream_t s_, bool on_, const double2* x, double2* w, int prec) : P(P_), s(s_), on(on_) {
-    if (!on) return;
+  bool own;
+  const double2* x;
+  double2* w;
+  int prec;
+  NearAhead(Plan& P_, cudaStream_t s_, bool own_, const double2* x_, double2* w_, int prec_)
+      : P(P_), s(s_), own(own_), x(x_), w(w_), prec(prec_) {
+    if (!own) return;
     MLFMA_CUDA(cudaEventRecord(P.ev_start, s));
     MLFMA_CUDA(cudaStreamWaitEvent(P.stream_near, P.ev_start, 0));
     near_apply(P, x, w, P.stream_near, prec);
     MLFMA_CUDA(cudaEventRecord(P.ev_near, P.stream_near));
   }
   void join() {
-    if (on) MLFMA_CUDA(cudaStreamWaitEvent(s, P.ev_near, 0));
+    if (own)
+      MLFMA_CUDA(cudaStreamWaitEvent(s, P.ev_near, 0));
+    else
+      near_apply(P, x, w, s, prec);
   }
 };
 
@@ -1952,8 +2010,7 @@ template <class C>
 void apply_fixed(Plan& P, const double2* x, double2* w, cudaStream_t s) {
   const int L = P.maxL;
   LeafArg<C> a{};
-  const bool split_near = P.tuning.leaf_variant == 1;
-  NearAhead near(P, s, split_near, x, w, std::is_same<C, float2>::value ? 1 : 0);
+  NearAhead near(P, s, P.tuning.leaf_variant == 1, x, w, std::is_same<C, float2>::value ? 1 : 0);
   MediumStreams ms(P, s, true);
   for (int m = 0; m < 2; ++m) {
     const cudaStream_t sm = ms.of(m);
@@ -1967,16 +2024,10 @@ void apply_fixed(Plan& P, const double2* x, double2* w, cudaStream_t s) {
     a.K[m] = leaf.K;
   }
   ms.join();
+  near.join();
   fill_leaf_common(P, a);
-  a.x = x;
   a.w = w;
-  const int warps = kThreads / 32;
-  if (split_near) {
-    near.join();
-    leaf_out_kernel<C, false><<<(P.N + warps - 1) / warps, kThreads, 0, s>>>(a);
-  } else {
-    leaf_out_kernel<C><<<(P.N + warps - 1) / warps, kThreads, 0, s>>>(a);
-  }
+  launch_leaf(P, a, s);
   MLFMA_CUDA(cudaGetLastError());
 }
 
@@ -2050,6 +2101,7 @@ void apply_batch_fixed(Plan& P, int R, const double2* X, long long ldx, double2*
       for (int j = 0; j < rn; ++j) lb.Bm[m][j] = Store<C>::bB(P, m, j);
     }
     fill_leaf_common(P, lb);
+    fill_leaf_near(P, lb);
     lb.X = X + g0 * ldx;
     lb.ldx = ldx;
     lb.W = W + g0 * ldw;
@@ -2094,8 +2146,7 @@ void apply_batch_fixed(Plan& P, int R, const double2* X, long long ldx, double2*
 void apply_direct(Plan& P, const double2* x, double2* w, cudaStream_t s) {
   const int L = P.maxL;
   cudaEvent_t* ev = profiler_events(P, s);
-  const bool split_near = P.tuning.leaf_variant == 1;
-  NearAhead near(P, s, split_near && ev == nullptr, x, w, 0);
+  NearAhead near(P, s, P.tuning.leaf_variant == 1 && ev == nullptr, x, w, 0);
   if (P.tuning.agg_variant == 1) {  // both media in one launch, timed as medium 1's aggregation
     AggBoxArg a{};
     for (int m = 0; m < 2; ++m) {
@@ -2150,16 +2201,9 @@ void apply_direct(Plan& P, const double2* x, double2* w, cudaStream_t s) {
     a.K[m] = P.ml[m][L].K;
   }
   fill_leaf_common(P, a);
-  a.x = x;
   a.w = w;
-  const int warps = kThreads / 32;
-  if (split_near) {
-    if (ev) near_apply(P, x, w, s, 0);  // profiled: in sequence, inside the leaf stage
-    near.join();
-    leaf_out_kernel<double2, false><<<(P.N + warps - 1) / warps, kThreads, 0, s>>>(a);
-  } else {
-    leaf_out_kernel<double2><<<(P.N + warps - 1) / warps, kThreads, 0, s>>>(a);
-  }
+  near.join();
+  launch_leaf(P, a, s);
   MLFMA_CUDA(cudaGetLastError());
   if (ev) MLFMA_CUDA(cudaEventRecord(ev[9], s));
 }
@@ -2251,6 +2295,7 @@ void apply_batch_device(Plan& P, int R, const double2* X, long long ldx, double2
       for (int j = 0; j < rn; ++j) lb.Bm[m][j] = P.bB[m][j];
     }
     fill_leaf_common(P, lb);
+    fill_leaf_near(P, lb);
     lb.X = X + g0 * ldx;
     lb.ldx = ldx;
     lb.W = W + g0 * ldw;

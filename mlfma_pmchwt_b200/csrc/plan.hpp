@@ -145,7 +145,7 @@ struct Tuning {
                                //    cores; 1 tcgen05 (3xTF32 split, TMEM accumulators)
   int batch_tree = 1;          // batched complex64 tree passes: 0 one slot after another; 1 every level
                                //    once for all slots (slot-major arrays)
-  int leaf_variant = 0;        // 0: near field inside the leaf kernel; 1: near field on its own
+  int leaf_variant = 0;        // 0: near field before the leaf kernel, which adds the far field; 1: near field on its own
                                //    stream from the start of the apply, the leaf kernel adds the far field
   int graph = 1;               // 1: capture each apply (per x, w, stream and precision) as a CUDA
                                //    graph on first use and replay it; 0: launch the kernels directly
