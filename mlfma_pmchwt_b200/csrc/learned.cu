@@ -23,12 +23,46 @@ namespace {
 
 constexpr int kRedBlocks = 256;
 constexpr int kColParts = 64;     // partial column sums over boxes
-constexpr int kLayerBoxes = 32;   // boxes per CTA in the layer kernels
+constexpr int kLayerBoxes = 8;    // boxes per CTA in the layer kernels (a warp per box, 2 channels per lane)
+constexpr int kLpPad = kLpH + 1;  // row pitch of a transposed weight matrix in shared memory
 constexpr int kDecRows = 32;      // RWGs per CTA in the decoder kernels
+constexpr int kDecP1 = kLpH + 4, kDecP2 = kLpG + 4;  // row pitches of its transposed weights (16-byte rows)
 constexpr int kWgTile = 32;        // rows staged at a time by a weight-gradient CTA
 constexpr int kWgCtas = 296;       // row slices of one gradient at most (2 CTAs per SM)
 
 __device__ __forceinline__ float bf(const __nv_bfloat16* w, int i) { return __bfloat162float(w[i]); }
+// Eight bfloat16 weights (16-byte aligned) as floats
+__device__ __forceinline__ void bf8(const __nv_bfloat16* w, float (&v)[8]) {
+  const uint4 u = __ldg(reinterpret_cast<const uint4*>(w));
+  const unsigned q[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(q[i] << 16);
+    v[2 * i + 1] = __uint_as_float(q[i] & 0xffff0000u);
+  }
+}
+// A row-major [rows][cols] weight block into shared memory, as stored or
+// transposed ([cols][pitch], pitch odd so that a row's values fall in
+// different banks)
+__device__ __forceinline__ void stage_weights(const __nv_bfloat16* w, int n, float* dst) {
+#pragma unroll 4
+  for (int i = 8 * threadIdx.x; i < n; i += 8 * blockDim.x) {
+    float v[8];
+    bf8(w + i, v);
+    *reinterpret_cast<float4*>(dst + i) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(dst + i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+__device__ __forceinline__ void stage_transposed(const __nv_bfloat16* w, int rows, int cols, float* dst, int pitch) {
+#pragma unroll 4
+  for (int i = threadIdx.x; i < rows * cols / 8; i += blockDim.x) {
+    const int r = i % rows, c = 8 * (i / rows);  // neighbouring lanes: neighbouring rows
+    float v[8];
+    bf8(w + r * cols + c, v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dst[(c + j) * pitch + r] = v[j];
+  }
+}
 __device__ __forceinline__ float2 f2(double2 a) {
   return make_float2(static_cast<float>(a.x), static_cast<float>(a.y));
 }
@@ -76,40 +110,46 @@ struct Tabs {
   const float* fs;      // [N][16] static features by leaf position
 };
 
-// Zb[b][c][k] = mean over the box's RWGs of z_c d_k
+// Zb[b][c][k] = mean over the box's RWGs of z_c d_k; thread per (box, c, k),
+// the RWGs' values requested four at a time and summed in order
 __global__ void lp_boxz_kernel(Tabs t, const double2* __restrict__ z, float2* __restrict__ zb) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = i / 6, j = i - 6 * b, c = j / 3, k = j - 3 * c;
   if (b >= t.B) return;
   const int p0 = t.leaf_ptr[b], p1 = t.leaf_ptr[b + 1];
-  float2 acc[6];
-  for (int j = 0; j < 6; ++j) acc[j] = make_float2(0.f, 0.f);
-  for (int p = p0; p < p1; ++p) {
-    const int id = t.ids[p];
-    const float2 zj = f2(z[id]), zm = f2(z[t.N + id]);
-    for (int k = 0; k < 3; ++k) {
-      const float d = t.dip[3 * p + k];
-      acc[k] = make_float2(fmaf(zj.x, d, acc[k].x), fmaf(zj.y, d, acc[k].y));
-      acc[3 + k] = make_float2(fmaf(zm.x, d, acc[3 + k].x), fmaf(zm.y, d, acc[3 + k].y));
-    }
+  float2 acc = make_float2(0.f, 0.f);
+  for (int p = p0; p < p1; p += 4) {
+    double2 zv[4];
+    float d[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + u < p1) {
+        zv[u] = __ldg(z + c * t.N + __ldg(t.ids + p + u));
+        d[u] = __ldg(t.dip + 3 * (p + u) + k);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + u < p1) {
+        const float2 zc = f2(zv[u]);
+        acc = make_float2(fmaf(zc.x, d[u], acc.x), fmaf(zc.y, d[u], acc.y));
+      }
   }
   const float inv = p1 > p0 ? 1.f / static_cast<float>(p1 - p0) : 0.f;
-  for (int j = 0; j < 6; ++j) zb[6 * b + j] = cscale(acc[j], inv);
+  zb[i] = cscale(acc, inv);
 }
 
 // Zn[b] = mean of Zb over the box and its near neighbours (and, applied to
-// Zn, the two-ring mean Z2)
+// Zn, the two-ring mean Z2); thread per (box, component)
 __global__ void lp_boxn_kernel(Tabs t, const float2* __restrict__ zb, float2* __restrict__ zn) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = i / 6, j = i - 6 * b;
   if (b >= t.B) return;
   const int q0 = t.nb_ptr[b], q1 = t.nb_ptr[b + 1];
-  float2 acc[6];
-  for (int j = 0; j < 6; ++j) acc[j] = make_float2(0.f, 0.f);
-  for (int q = q0; q < q1; ++q) {
-    const int c = t.nb_idx[q];
-    for (int j = 0; j < 6; ++j) acc[j] = cadd(acc[j], zb[6 * c + j]);
-  }
+  float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (int q = q0; q < q1; ++q) acc = cadd(acc, __ldg(zb + 6 * __ldg(t.nb_idx + q) + j));
   const float inv = 1.f / static_cast<float>(q1 - q0);
-  for (int j = 0; j < 6; ++j) zn[6 * b + j] = cscale(acc[j], inv);
+  zn[i] = cscale(acc, inv);
 }
 
 __device__ __forceinline__ float2 dot3(const float* d, const float2* zv) {
@@ -201,66 +241,77 @@ struct LayerArg {
   float* g;                // [64] the global mean (kept; written by CTA 0)
 };
 
-// One message-passing layer for kLayerBoxes boxes per CTA (256 threads:
-// box r = tid / 8, channels 8 (tid % 8) .. + 8).
+// One message-passing layer for kLayerBoxes boxes per CTA (256 threads: a warp
+// per box, channels lane and lane + 32). Latency-bound: with 32 boxes per CTA,
+// 384 boxes filled 12 SMs, and the transposed weights' stores met in one bank:
+// 28 us a layer, now 9.
 __global__ void __launch_bounds__(256) lp_layer_kernel(LayerArg L) {
   extern __shared__ float sm[];
-  float* WsT = sm;                       // [k][o]
-  float* WnT = WsT + kLpH * kLpH;
-  float* cg = WnT + kLpH * kLpH;         // c + Wg g
+  float* WsT = sm;                       // [k][kLpPad]
+  float* WnT = WsT + kLpH * kLpPad;
+  float* cg = WnT + kLpH * kLpPad;       // c + Wg g
   float* gs = cg + kLpH;
-  float* X = gs + kLpH;                  // [kLayerBoxes][2 * 64 + 1]: h, m
-  constexpr int ldx = 2 * kLpH + 1;
+  float* X = gs + kLpH;                  // [kLayerBoxes][2 * 64]: h, m
+  constexpr int ldx = 2 * kLpH;
   const int tid = threadIdx.x, B = L.t.B;
-  for (int i = tid; i < kLpH * kLpH; i += 256) {
-    const int o = i / kLpH, k = i % kLpH;
-    WsT[k * kLpH + o] = bf(L.w, i);
-    WnT[k * kLpH + o] = bf(L.w, kLpH * kLpH + i);
-  }
+  stage_transposed(L.w, kLpH, kLpH, WsT, kLpPad);
+  stage_transposed(L.w + kLpH * kLpH, kLpH, kLpH, WnT, kLpPad);
   if (tid < kLpH) {
     float s = 0.f;
+#pragma unroll 8
     for (int j = 0; j < kColParts; ++j) s += L.gpart[kLpH * j + tid];
     gs[tid] = s / static_cast<float>(B);
     if (blockIdx.x == 0) L.g[tid] = gs[tid];
   }
+  const int r = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x * kLayerBoxes + r;
+  float hm[2] = {0.f, 0.f};
+  if (b < B) {
+    float mm[2] = {0.f, 0.f};
+    hm[0] = L.h[kLpH * b + lane];
+    hm[1] = L.h[kLpH * b + 32 + lane];
+    const int q0 = L.t.nb_ptr[b], q1 = L.t.nb_ptr[b + 1];
+#pragma unroll 4
+    for (int q = q0; q < q1; ++q) {
+      const float* hr = L.h + kLpH * __ldg(L.t.nb_idx + q) + lane;
+      mm[0] += hr[0];
+      mm[1] += hr[32];
+    }
+    const float inv = 1.f / static_cast<float>(q1 - q0);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      X[r * ldx + 32 * j + lane] = hm[j];
+      X[r * ldx + kLpH + 32 * j + lane] = mm[j] * inv;
+    }
+  }
   __syncthreads();
   if (tid < kLpH) {
     float acc = bf(L.w, 3 * kLpH * kLpH + tid);
-    for (int k = 0; k < kLpH; ++k) acc = fmaf(bf(L.w, 2 * kLpH * kLpH + tid * kLpH + k), gs[k], acc);
+#pragma unroll 2
+    for (int k = 0; k < kLpH; k += 8) {
+      float w[8];
+      bf8(L.w + 2 * kLpH * kLpH + tid * kLpH + k, w);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc = fmaf(w[j], gs[k + j], acc);
+    }
     cg[tid] = acc;
-  }
-  const int r = tid >> 3, o0 = (tid & 7) * 8;
-  const int b = blockIdx.x * kLayerBoxes + r;
-  if (b < B) {
-    float hm[8], mm[8];
-    for (int j = 0; j < 8; ++j) {
-      hm[j] = L.h[kLpH * b + o0 + j];
-      mm[j] = 0.f;
-    }
-    const int q0 = L.t.nb_ptr[b], q1 = L.t.nb_ptr[b + 1];
-    for (int q = q0; q < q1; ++q) {
-      const float* hr = L.h + kLpH * L.t.nb_idx[q] + o0;
-      for (int j = 0; j < 8; ++j) mm[j] += hr[j];
-    }
-    const float inv = 1.f / static_cast<float>(q1 - q0);
-    for (int j = 0; j < 8; ++j) {
-      X[r * ldx + o0 + j] = hm[j];
-      X[r * ldx + kLpH + o0 + j] = mm[j] * inv;
-    }
   }
   __syncthreads();
   if (b >= B) return;
-  float acc[8];
-  for (int j = 0; j < 8; ++j) acc[j] = cg[o0 + j];
+  float acc[2] = {cg[lane], cg[32 + lane]};
+#pragma unroll 8
   for (int k = 0; k < kLpH; ++k) {
     const float xh = X[r * ldx + k], xm = X[r * ldx + kLpH + k];
-    for (int j = 0; j < 8; ++j) acc[j] = fmaf(WsT[k * kLpH + o0 + j], xh, fmaf(WnT[k * kLpH + o0 + j], xm, acc[j]));
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      acc[j] = fmaf(WsT[k * kLpPad + 32 * j + lane], xh, fmaf(WnT[k * kLpPad + 32 * j + lane], xm, acc[j]));
   }
-  for (int j = 0; j < 8; ++j) {
-    const int o = o0 + j;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int o = 32 * j + lane;
     L.P[kLpH * b + o] = acc[j];
     L.m[kLpH * b + o] = X[r * ldx + kLpH + o];
-    L.hout[kLpH * b + o] = X[r * ldx + o] + fmaxf(acc[j], 0.f);
+    L.hout[kLpH * b + o] = hm[j] + fmaxf(acc[j], 0.f);
   }
 }
 
@@ -276,24 +327,21 @@ struct DecArg {
 };
 
 // Decoder and output for kDecRows RWGs per CTA (128 threads: RWG r = tid / 4).
+// Latency-bound: weights come 8 at a time and their transposed rows are padded
+// (7,680 RWGs: 41 us with single bfloat16 loads into one bank, now 22; the
+// backward kernel 57 and 18).
 __global__ void __launch_bounds__(128) lp_decode_kernel(DecArg D) {
-  extern __shared__ float sm[];
-  float* W1T = sm;                     // [128][64]
-  float* W2T = W1T + 2 * kLpH * kLpH;  // [64][32]
-  float* d1 = W2T + kLpH * kLpG;
+  extern __shared__ __align__(16) float sm[];
+  float* W1T = sm;                     // [128][kDecP1]
+  float* W2T = W1T + 2 * kLpH * kDecP1;  // [64][kDecP2]
+  float* d1 = W2T + kLpH * kDecP2;
   float* d2 = d1 + kLpH;
   float* X = d2 + kLpG;                // [32][129]
   float* Q = X + kDecRows * (2 * kLpH + 1);  // [32][65]
   float* Gs = Q + kDecRows * (kLpH + 1);     // [32][33]
   const int tid = threadIdx.x, N = D.t.N;
-  for (int i = tid; i < 2 * kLpH * kLpH; i += 128) {
-    const int o = i / (2 * kLpH), k = i % (2 * kLpH);
-    W1T[k * kLpH + o] = bf(D.w, kLpOffWd1 + i);
-  }
-  for (int i = tid; i < kLpG * kLpH; i += 128) {
-    const int j = i / kLpH, o = i % kLpH;
-    W2T[o * kLpG + j] = bf(D.w, kLpOffWd2 + i);
-  }
+  stage_transposed(D.w + kLpOffWd1, kLpH, 2 * kLpH, W1T, kDecP1);
+  stage_transposed(D.w + kLpOffWd2, kLpG, kLpH, W2T, kDecP2);
   if (tid < kLpH) d1[tid] = bf(D.w, kLpOffD1 + tid);
   if (tid < kLpG) d2[tid] = bf(D.w, kLpOffD2 + tid);
   const int p0 = blockIdx.x * kDecRows;
@@ -308,29 +356,62 @@ __global__ void __launch_bounds__(128) lp_decode_kernel(DecArg D) {
     X[r * (2 * kLpH + 1) + kLpH + k] = xa;
   }
   __syncthreads();
+  // a thread's channels: 16 q + 4 c4 + j, so that its 16-byte weight loads and
+  // its neighbours' are one 64-byte row piece
   const int r = tid >> 2, c4 = tid & 3, p = p0 + r;
   {
-    float acc[16];
-    for (int j = 0; j < 16; ++j) acc[j] = d1[c4 * 16 + j];
+    float acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[q][j] = d1[16 * q + 4 * c4 + j];
+#pragma unroll 4
     for (int k = 0; k < 2 * kLpH; ++k) {
       const float x = X[r * (2 * kLpH + 1) + k];
-      for (int j = 0; j < 16; ++j) acc[j] = fmaf(W1T[k * kLpH + c4 * 16 + j], x, acc[j]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 w = *reinterpret_cast<const float4*>(W1T + k * kDecP1 + 16 * q + 4 * c4);
+        acc[q][0] = fmaf(w.x, x, acc[q][0]);
+        acc[q][1] = fmaf(w.y, x, acc[q][1]);
+        acc[q][2] = fmaf(w.z, x, acc[q][2]);
+        acc[q][3] = fmaf(w.w, x, acc[q][3]);
+      }
     }
-    for (int j = 0; j < 16; ++j) {
-      const float qv = fmaxf(acc[j], 0.f);
-      Q[r * (kLpH + 1) + c4 * 16 + j] = qv;
-      if (D.q && p < N) D.q[kLpH * p + c4 * 16 + j] = qv;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 qv = make_float4(fmaxf(acc[q][0], 0.f), fmaxf(acc[q][1], 0.f), fmaxf(acc[q][2], 0.f),
+                              fmaxf(acc[q][3], 0.f));
+      const int o = 16 * q + 4 * c4;
+      Q[r * (kLpH + 1) + o] = qv.x;
+      Q[r * (kLpH + 1) + o + 1] = qv.y;
+      Q[r * (kLpH + 1) + o + 2] = qv.z;
+      Q[r * (kLpH + 1) + o + 3] = qv.w;
+      if (D.q && p < N) *reinterpret_cast<float4*>(D.q + static_cast<size_t>(kLpH) * p + o) = qv;
     }
   }
   __syncthreads();
   {
-    float acc[8];
-    for (int j = 0; j < 8; ++j) acc[j] = d2[c4 * 8 + j];
+    float acc[2][4];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[q][j] = d2[16 * q + 4 * c4 + j];
+#pragma unroll 4
     for (int o = 0; o < kLpH; ++o) {
       const float qv = Q[r * (kLpH + 1) + o];
-      for (int j = 0; j < 8; ++j) acc[j] = fmaf(W2T[o * kLpG + c4 * 8 + j], qv, acc[j]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float4 w = *reinterpret_cast<const float4*>(W2T + o * kDecP2 + 16 * q + 4 * c4);
+        acc[q][0] = fmaf(w.x, qv, acc[q][0]);
+        acc[q][1] = fmaf(w.y, qv, acc[q][1]);
+        acc[q][2] = fmaf(w.z, qv, acc[q][2]);
+        acc[q][3] = fmaf(w.w, qv, acc[q][3]);
+      }
     }
-    for (int j = 0; j < 8; ++j) Gs[r * (kLpG + 1) + c4 * 8 + j] = acc[j];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Gs[r * (kLpG + 1) + 16 * q + 4 * c4 + j] = acc[q][j];
   }
   __syncthreads();
   if (tid < 2 * kDecRows) {
@@ -364,15 +445,15 @@ struct DecBwdArg {
 };
 
 __global__ void __launch_bounds__(128) lp_decode_bwd_kernel(DecBwdArg D) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   float* W2 = sm;                      // [32][64] as stored (j, o)
   float* W1 = W2 + kLpG * kLpH;        // [64][128] as stored (o, k)
   float* DG = W1 + 2 * kLpH * kLpH;    // [32][33]
   float* DQ = DG + kDecRows * (kLpG + 1);  // [32][65]
   __shared__ float red[128];
   const int tid = threadIdx.x, N = D.t.N;
-  for (int i = tid; i < kLpG * kLpH; i += 128) W2[i] = bf(D.w, kLpOffWd2 + i);
-  for (int i = tid; i < 2 * kLpH * kLpH; i += 128) W1[i] = bf(D.w, kLpOffWd1 + i);
+  stage_weights(D.w + kLpOffWd2, kLpG * kLpH, W2);
+  stage_weights(D.w + kLpOffWd1, 2 * kLpH * kLpH, W1);
   const int p0 = blockIdx.x * kDecRows;
   const float sc = D.gy ? 0.f : static_cast<float>(2.0 / D.esum[0]);
   float lsum = 0.f;
@@ -408,30 +489,62 @@ __global__ void __launch_bounds__(128) lp_decode_bwd_kernel(DecBwdArg D) {
     __syncthreads();
   }
   if (tid == 0 && D.loss) atomicAdd(D.loss, red[0]);
-  const int r = tid >> 2, c4 = tid & 3, p = p0 + r;
+  const int r = tid >> 2, c4 = tid & 3, p = p0 + r;  // channels 16 q + 4 c4 + j, as in the decoder
   {
-    float acc[16];
-    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
+    float acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[q][j] = 0.f;
+#pragma unroll 4
     for (int jj = 0; jj < kLpG; ++jj) {
       const float g = DG[r * (kLpG + 1) + jj];
-      for (int j = 0; j < 16; ++j) acc[j] = fmaf(W2[jj * kLpH + c4 * 16 + j], g, acc[j]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 w = *reinterpret_cast<const float4*>(W2 + jj * kLpH + 16 * q + 4 * c4);
+        acc[q][0] = fmaf(w.x, g, acc[q][0]);
+        acc[q][1] = fmaf(w.y, g, acc[q][1]);
+        acc[q][2] = fmaf(w.z, g, acc[q][2]);
+        acc[q][3] = fmaf(w.w, g, acc[q][3]);
+      }
     }
-    for (int j = 0; j < 16; ++j) {
-      const int o = c4 * 16 + j;
-      const float v = (p < N && D.q[kLpH * p + o] > 0.f) ? acc[j] : 0.f;
-      DQ[r * (kLpH + 1) + o] = v;
-      if (p < N) D.dq[kLpH * p + o] = v;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int o = 16 * q + 4 * c4;
+      float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p < N) h = *reinterpret_cast<const float4*>(D.q + static_cast<size_t>(kLpH) * p + o);
+      const float4 v = make_float4(h.x > 0.f ? acc[q][0] : 0.f, h.y > 0.f ? acc[q][1] : 0.f,
+                                   h.z > 0.f ? acc[q][2] : 0.f, h.w > 0.f ? acc[q][3] : 0.f);
+      DQ[r * (kLpH + 1) + o] = v.x;
+      DQ[r * (kLpH + 1) + o + 1] = v.y;
+      DQ[r * (kLpH + 1) + o + 2] = v.z;
+      DQ[r * (kLpH + 1) + o + 3] = v.w;
+      if (p < N) *reinterpret_cast<float4*>(D.dq + static_cast<size_t>(kLpH) * p + o) = v;
     }
   }
   __syncthreads();
   if (p < N) {
-    float acc[32];
-    for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+    float acc[8][4];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[q][j] = 0.f;
+#pragma unroll 2
     for (int o = 0; o < kLpH; ++o) {
       const float g = DQ[r * (kLpH + 1) + o];
-      for (int j = 0; j < 32; ++j) acc[j] = fmaf(W1[o * 2 * kLpH + c4 * 32 + j], g, acc[j]);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 w = *reinterpret_cast<const float4*>(W1 + o * 2 * kLpH + 16 * q + 4 * c4);
+        acc[q][0] = fmaf(w.x, g, acc[q][0]);
+        acc[q][1] = fmaf(w.y, g, acc[q][1]);
+        acc[q][2] = fmaf(w.z, g, acc[q][2]);
+        acc[q][3] = fmaf(w.w, g, acc[q][3]);
+      }
     }
-    for (int j = 0; j < 32; ++j) D.dx[2 * kLpH * p + c4 * 32 + j] = acc[j];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      *reinterpret_cast<float4*>(D.dx + static_cast<size_t>(2 * kLpH) * p + 16 * q + 4 * c4) =
+          make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
   }
 }
 
@@ -478,46 +591,48 @@ struct LayerBwdArg {
 };
 
 __global__ void __launch_bounds__(256) lp_layer_bwd_kernel(LayerBwdArg L) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   float* Ws = sm;                  // [o][k] as stored
   float* Wn = Ws + kLpH * kLpH;
   float* dg = Wn + kLpH * kLpH;
   float* Ss = dg + kLpH;
-  float* D = Ss + kLpH;            // [kLayerBoxes][65]
+  float* D = Ss + kLpH;            // [kLayerBoxes][64]
   const int tid = threadIdx.x, B = L.t.B;
-  for (int i = tid; i < kLpH * kLpH; i += 256) {
-    Ws[i] = bf(L.w, i);
-    Wn[i] = bf(L.w, kLpH * kLpH + i);
-  }
+  stage_weights(L.w, 2 * kLpH * kLpH, Ws);
   if (tid < kLpH) {
     float s = 0.f;
+#pragma unroll 8
     for (int j = 0; j < kColParts; ++j) s += L.spart[kLpH * j + tid];
     Ss[tid] = s;
     if (blockIdx.x == 0) L.S[tid] = s;
   }
-  const int r = tid >> 3, k0 = (tid & 7) * 8;
+  const int r = tid >> 5, lane = tid & 31;
   const int b = blockIdx.x * kLayerBoxes + r;
-  for (int j = 0; j < 8; ++j) D[r * (kLpH + 1) + k0 + j] = b < B ? L.dP[kLpH * b + k0 + j] : 0.f;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) D[r * kLpH + 32 * j + lane] = b < B ? L.dP[kLpH * b + 32 * j + lane] : 0.f;
   __syncthreads();
   if (tid < kLpH) {
     float acc = 0.f;
+#pragma unroll 8
     for (int o = 0; o < kLpH; ++o) acc = fmaf(bf(L.w, 2 * kLpH * kLpH + o * kLpH + tid), Ss[o], acc);
     dg[tid] = acc / static_cast<float>(B);
   }
   __syncthreads();
   if (b >= B) return;
-  float ts[8], tn[8];
-  for (int j = 0; j < 8; ++j) ts[j] = tn[j] = 0.f;
+  float ts[2] = {0.f, 0.f}, tn[2] = {0.f, 0.f};
+#pragma unroll 8
   for (int o = 0; o < kLpH; ++o) {
-    const float g = D[r * (kLpH + 1) + o];
-    for (int j = 0; j < 8; ++j) {
-      ts[j] = fmaf(Ws[o * kLpH + k0 + j], g, ts[j]);
-      tn[j] = fmaf(Wn[o * kLpH + k0 + j], g, tn[j]);
+    const float g = D[r * kLpH + o];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      ts[j] = fmaf(Ws[o * kLpH + 32 * j + lane], g, ts[j]);
+      tn[j] = fmaf(Wn[o * kLpH + 32 * j + lane], g, tn[j]);
     }
   }
   const float inv = 1.f / static_cast<float>(L.t.nb_ptr[b + 1] - L.t.nb_ptr[b]);
-  for (int j = 0; j < 8; ++j) {
-    const int k = k0 + j;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int k = 32 * j + lane;
     L.tmp[kLpH * b + k] = L.dh[kLpH * b + k] + ts[j] + dg[k];
     L.dm[kLpH * b + k] = tn[j] * inv;
   }
@@ -676,16 +791,16 @@ struct LearnedWork {
   __nv_bfloat16* w_store = nullptr;     // storage behind w_attached
 };
 
-static size_t layer_smem() { return (2 * kLpH * kLpH + 2 * kLpH + kLayerBoxes * (2 * kLpH + 1)) * sizeof(float); }
+static size_t layer_smem() { return (2 * kLpH * kLpPad + 2 * kLpH + kLayerBoxes * 2 * kLpH) * sizeof(float); }
 static size_t dec_smem() {
-  return (2 * kLpH * kLpH + kLpH * kLpG + kLpH + kLpG + kDecRows * (2 * kLpH + 1) + kDecRows * (kLpH + 1) +
+  return (2 * kLpH * kDecP1 + kLpH * kDecP2 + kLpH + kLpG + kDecRows * (2 * kLpH + 1) + kDecRows * (kLpH + 1) +
           kDecRows * (kLpG + 1)) *
          sizeof(float);
 }
 static size_t dec_bwd_smem() {
   return (kLpG * kLpH + 2 * kLpH * kLpH + kDecRows * (kLpG + 1) + kDecRows * (kLpH + 1)) * sizeof(float);
 }
-static size_t layer_bwd_smem() { return (2 * kLpH * kLpH + 2 * kLpH + kLayerBoxes * (kLpH + 1)) * sizeof(float); }
+static size_t layer_bwd_smem() { return (2 * kLpH * kLpH + 2 * kLpH + kLayerBoxes * kLpH) * sizeof(float); }
 
 LearnedWork& lp_work(Plan& P) {
   if (P.lp) return *P.lp;
@@ -838,9 +953,9 @@ void lp_forward(Plan& P, const __nv_bfloat16* w, const double2* /* v: enters thr
                 double2* y, bool train, cudaStream_t s) {
   LearnedWork& W = lp_work(P);
   const int N = W.N, B = W.B;
-  lp_boxz_kernel<<<(B + 127) / 128, 128, 0, s>>>(W.t, z, W.zb);
-  lp_boxn_kernel<<<(B + 127) / 128, 128, 0, s>>>(W.t, W.zb, W.zn);
-  lp_boxn_kernel<<<(B + 127) / 128, 128, 0, s>>>(W.t, W.zn, W.z2);
+  lp_boxz_kernel<<<(6 * B + 127) / 128, 128, 0, s>>>(W.t, z, W.zb);
+  lp_boxn_kernel<<<(6 * B + 127) / 128, 128, 0, s>>>(W.t, W.zb, W.zn);
+  lp_boxn_kernel<<<(6 * B + 127) / 128, 128, 0, s>>>(W.t, W.zn, W.z2);
   EncArg e{W.t, z, W.zb, W.zn, W.z2, w, W.u, W.a};
   lp_encode_kernel<<<(N + 127) / 128, 128, 0, s>>>(e);
   lp_pool_kernel<<<(B + 7) / 8, 256, 0, s>>>(W.t, W.a, W.h[0]);
