@@ -42,7 +42,7 @@ struct NearBatchArg {
   const float2* near_z;
   VecRef w;
   const int* sys;
-  const double* xscale;  // factor of position a's x at xscale[a * lds]
+  const double* xscale;  // factor of position a's x at xscale[a * lds]; null: 1
   int lds;
   int N, R;
 };
@@ -52,16 +52,19 @@ struct NearBatchArg {
 // CTA's rows and systems over a quarter of the box's sources, so no value is
 // reduced across lanes. The entries (128 (row, source) pairs at a time) and
 // the sources' values, which the Gram-Schmidt kernels leave packed per RWG in
-// complex64 (blas1::Pack), stream through a ring of three stages per warp
-// (cp.async): two chunks are in flight while one is multiplied, and no warp
-// waits for another but for the sum of the quarters at the end.
+// complex64 (blas1::Pack), stream through a two-stage ring per warp
+// (cp.async): one chunk is in flight while one is multiplied, and no warp
+// waits for another but for the sum of the quarters at the end. Sums of four
+// sources, of a chunk and of the whole quarter: a row's large entries (its own
+// triangles') then meet few roundings, as in a sum over 32 lanes. (One running
+// sum made the 16-slot batched apply's error 1.7e-7 instead of 1.0e-7.)
 // FP32-bound at 8 systems (2.2 M pairs: 7.5 us at the FP32 rate, 52 MB of
-// entries 8 us); measured 33 us. With a lane per source and the sources
+// entries 8 us); measured 28 us, 33 with three stages (fewer CTAs per SM). With a lane per source and the sources
 // staged for the whole CTA first (10 warps per SM, each waiting for its
 // loads, 320 shuffles per pair of rows) the product took 92 us there; with a
 // CTA for all rows of a box 56 us, waiting for the fullest boxes.
 constexpr int kNearWarps = 4;
-constexpr int kNearStages = 3;
+constexpr int kNearStages = 2;
 
 template <int G>
 struct NearTile {
@@ -134,28 +137,46 @@ __global__ void __launch_bounds__(32 * kNearWarps) near_batch_tile_kernel(NearBa
     __syncwarp();
     const float2* z = ring[it % kNearStages].z + row * kZs;
     const float4* x = ring[it % kNearStages].x + 2 * g;
+    float2 cJ[2], cM[2], sJ[2], sM[2];  // the chunk's sums, and those of the four sources under way
+    cJ[0] = cJ[1] = cM[0] = cM[1] = sJ[0] = sJ[1] = sM[0] = sM[1] = make_float2(0.f, 0.f);
     auto add = [&](int q, float2 z11, float2 z12, float2 z22) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float4 v = x[q * kSys + j];
         const float2 J = make_float2(v.x, v.y), M = make_float2(v.z, v.w), nJ = make_float2(-v.x, -v.y);
-        aJ[j] = cfma(z11, J, cfma(z12, M, aJ[j]));
-        aM[j] = cfma(z22, M, cfma(z12, nJ, aM[j]));
+        sJ[j] = cfma(z11, J, cfma(z12, M, sJ[j]));
+        sM[j] = cfma(z22, M, cfma(z12, nJ, sM[j]));
+      }
+    };
+    auto carry = [&](float2(&tJ)[2], float2(&tM)[2], float2(&fJ)[2], float2(&fM)[2]) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        tJ[j] = cadd(tJ[j], fJ[j]);
+        tM[j] = cadd(tM[j], fM[j]);
+        fJ[j] = fM[j] = make_float2(0.f, 0.f);
       }
     };
     const int kn = min(kSrc, ns - (wp + it * kNearWarps) * kSrc);
     if (kn == kSrc) {
 #pragma unroll
-      for (int q = 0; q < kSrc; q += 2) {
-        const float4 z11 = *reinterpret_cast<const float4*>(z + q);
-        const float4 z12 = *reinterpret_cast<const float4*>(z + kSrc + q);
-        const float4 z22 = *reinterpret_cast<const float4*>(z + 2 * kSrc + q);
-        add(q, make_float2(z11.x, z11.y), make_float2(z12.x, z12.y), make_float2(z22.x, z22.y));
-        add(q + 1, make_float2(z11.z, z11.w), make_float2(z12.z, z12.w), make_float2(z22.z, z22.w));
+      for (int q = 0; q < kSrc; q += 4) {
+#pragma unroll
+        for (int u = q; u < q + 4; u += 2) {
+          const float4 z11 = *reinterpret_cast<const float4*>(z + u);
+          const float4 z12 = *reinterpret_cast<const float4*>(z + kSrc + u);
+          const float4 z22 = *reinterpret_cast<const float4*>(z + 2 * kSrc + u);
+          add(u, make_float2(z11.x, z11.y), make_float2(z12.x, z12.y), make_float2(z22.x, z22.y));
+          add(u + 1, make_float2(z11.z, z11.w), make_float2(z12.z, z12.w), make_float2(z22.z, z22.w));
+        }
+        carry(cJ, cM, sJ, sM);
       }
     } else {
-      for (int q = 0; q < kn; ++q) add(q, z[q], z[kSrc + q], z[2 * kSrc + q]);
+      for (int q = 0; q < kn; ++q) {
+        add(q, z[q], z[kSrc + q], z[2 * kSrc + q]);
+        if ((q & 3) == 3 || q + 1 == kn) carry(cJ, cM, sJ, sM);
+      }
     }
+    carry(aJ, aM, cJ, cM);
     __syncwarp();
   }
 #pragma unroll
@@ -171,7 +192,7 @@ __global__ void __launch_bounds__(32 * kNearWarps) near_batch_tile_kernel(NearBa
         const float4 u = sm.red[q][o];
         v = make_float4(v.x + u.x, v.y + u.y, v.z + u.z, v.w + u.w);
       }
-      const double sc = a.xscale[static_cast<long long>(p0 + j) * a.lds];
+      const double sc = a.xscale ? a.xscale[static_cast<long long>(p0 + j) * a.lds] : 1.0;
       double2* w = a.w.at(p0 + j, a.sys);
       const int id = a.leaf_rwg[r0 + rr];
       w[id] = c2(sc * v.x, sc * v.y);
@@ -184,6 +205,31 @@ __global__ void __launch_bounds__(32 * kNearWarps) near_batch_tile_kernel(NearBa
 // Systems per CTA: 8 from 5 systems on, 4 for 3 or 4, else 2 (lanes without
 // a system would multiply zeros).
 inline int near_tile_groups(int Ra) { return Ra > 4 ? 4 : Ra > 2 ? 2 : 1; }
+
+void launch_near_tile(const Plan& P, const NearBatchArg& a, const void* packed, cudaStream_t s) {
+  const int G = near_tile_groups(a.R);
+  const dim3 grid(static_cast<int>(P.h_near_sptr.size()) - 1, (a.R + 2 * G - 1) / (2 * G),
+                  (P.max_leaf_rwgs * G + 31) / 32);
+  auto go = [&](auto* f, size_t smem) {
+    // (a constant: set to the same value by every call of every thread)
+    MLFMA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    f<<<grid, 32 * kNearWarps, smem, s>>>(a, static_cast<const float4*>(packed));
+  };
+  if (G == 4)
+    go(near_batch_tile_kernel<4>, sizeof(NearTile<4>));
+  else if (G == 2)
+    go(near_batch_tile_kernel<2>, sizeof(NearTile<2>));
+  else
+    go(near_batch_tile_kernel<1>, sizeof(NearTile<1>));
+  MLFMA_CUDA(cudaGetLastError());
+}
+
+// The rows of X into packed complex64 groups (blas1::Pack)
+__global__ void pack_kernel(const double2* X, long long ldx, long long n, blas1::Pack p) {
+  const int a = blockIdx.y;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    blas1::pack_row(p, n, a, i, X[a * ldx + i]);
+}
 
 // The batched vector steps on one stream with their results on the host, for
 // up to R positions.
@@ -243,6 +289,17 @@ struct BatchOps : blas1::Vec {
 };
 
 }  // namespace
+
+void near_apply_batch(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw, float2* packed,
+                      cudaStream_t s) {
+  const long long n = 2LL * P.N;
+  const blas1::Pack p{packed, 2 * near_tile_groups(R)};
+  pack_kernel<<<dim3(static_cast<unsigned>(std::min<long long>((n + 255) / 256, 1184)), R), 256, 0, s>>>(X, ldx, n, p);
+  const NearBatchArg a{P.d_leaf_rwg, P.d_leaf_ptr,         P.d_near_sptr, P.d_near_src, P.d_near_zoff,
+                       P.d_near_z32, VecRef{W, ldw, 0, 0}, nullptr,       nullptr,      0,
+                       P.N,          R};
+  launch_near_tile(P, a, packed, s);
+}
 
 std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* rhs, int itr_max, int mr, double tol_abs,
                         double tol_rel, int inner_its, std::vector<SolveStats>& st,
@@ -331,17 +388,6 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
     const VecRef br = sysref(b, n, 0);
     return ops.norms_host(Ra, sysd, sysref(r, n, 0), &br);
   };
-  // shared memory of the near-field kernel (constants: set to the same value
-  // by every solve of every thread)
-  const int nleaf = static_cast<int>(P.h_near_sptr.size()) - 1;
-  if (inner_its > 0) {
-    auto allow = [](auto* f, size_t bytes) {
-      MLFMA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
-    };
-    allow(near_batch_tile_kernel<1>, sizeof(NearTile<1>));
-    allow(near_batch_tile_kernel<2>, sizeof(NearTile<2>));
-    allow(near_batch_tile_kernel<4>, sizeof(NearTile<4>));
-  }
   auto packed = [&](int Ra) { return blas1::Pack{reinterpret_cast<float2*>(wk[kPack]), 2 * near_tile_groups(Ra)}; };
   // z_q = (inner_its GMRES steps on Z_near from zero) applied to v_q, q in
   // list: every step is four launches, the host waits for none of them
@@ -351,15 +397,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
       NearBatchArg na{P.d_leaf_rwg,  P.d_leaf_ptr,              P.d_near_sptr, P.d_near_src, P.d_near_zoff,
                       P.d_near_z32,  sysref(Q, qs, (j + 1) * n), sysd,          ib.vs + j,    ib.ld,
                       P.N,           Ra};
-      const int G = near_tile_groups(Ra);
-      const dim3 ng(nleaf, (Ra + 2 * G - 1) / (2 * G), (P.max_leaf_rwgs * G + 31) / 32);
-      const float4* px = reinterpret_cast<const float4*>(wk[kPack]);
-      if (G == 4)
-        near_batch_tile_kernel<4><<<ng, 32 * kNearWarps, sizeof(NearTile<4>), s>>>(na, px);
-      else if (G == 2)
-        near_batch_tile_kernel<2><<<ng, 32 * kNearWarps, sizeof(NearTile<2>), s>>>(na, px);
-      else
-        near_batch_tile_kernel<1><<<ng, 32 * kNearWarps, sizeof(NearTile<1>), s>>>(na, px);
+      launch_near_tile(P, na, wk[kPack], s);
       ops.orthogonalise(Ra, sysd, sysref(Q, qs, 0), sysref(Q, qs, (j + 1) * n), j + 1, &ib, packed(Ra));
     }
     MLFMA_CUDA(cudaGetLastError());

@@ -1577,9 +1577,7 @@ struct LeafBatchArg {
 };
 
 // One warp per (RWG, group of RB right-hand sides).
-// kFar = false: the near-field rows alone (the far field is added by the
-// tensor-core testing kernel).
-template <class C, int RB, bool kFar = true>
+template <class C, int RB>
 __global__ void __launch_bounds__(kThreads) leaf_out_batch_kernel(LeafBatchArg<C> a) {
   using Rl = typename Cx<C>::real;
   const int lane = threadIdx.x & 31;
@@ -1592,7 +1590,7 @@ __global__ void __launch_bounds__(kThreads) leaf_out_batch_kernel(LeafBatchArg<C
 #pragma unroll
   for (int j = 0; j < RB; ++j) wj[j] = wm[j] = Cx<C>::zero();
 #pragma unroll
-  for (int m = 0; m < (kFar ? 2 : 0); ++m) {
+  for (int m = 0; m < 2; ++m) {
     const int K = a.K[m];
     const C* V = a.Vf[m] + static_cast<size_t>(r) * 3 * K;
     const double* kh = a.khat[m];
@@ -2031,113 +2029,64 @@ void apply_fixed(Plan& P, const double2* x, double2* w, cudaStream_t s) {
   MLFMA_CUDA(cudaGetLastError());
 }
 
-template <class C>
-void apply_batch_fixed(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw, cudaStream_t s) {
+// The batched complex64 apply: leaf stages of leaf_batch.cu (or, with
+// batch_tc.variant 1, of agg_tc.cu), tree passes over all slots, near-field
+// rows by the tiled product.
+void apply_batch_slots(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw, cudaStream_t s) {
+  using C = float2;
   const int L = P.maxL;
-  if (std::is_same<C, float2>::value ? P.bS32[0].empty() : P.batch_cap < std::min(R, kBatchSlots))
-    throw std::runtime_error("batched apply: slots not reserved");
-  constexpr int kAggRB = 8, kLeafRB = 4;
+  if (P.bS32[0].empty()) throw std::runtime_error("batched apply: slots not reserved");
   for (int g0 = 0; g0 < R; g0 += kBatchSlots) {
     const int rn = std::min(kBatchSlots, R - g0);
-    AggBatchArg<C> ag{};
+    AggTcArg ag{};
+    LeafTcArg lf{};
     for (int m = 0; m < 2; ++m) {
-      ag.Vs[m] = Store<C>::Vs(P, m);
-      ag.K[m] = P.ml[m][L].K;
-      for (int j = 0; j < rn; ++j) ag.S[m][j] = Store<C>::bS(P, m, j);
+      ag.Vs[m] = reinterpret_cast<const float*>(P.d_Vs32[m]);
+      lf.Vf[m] = P.d_Vf32[m];
+      lf.khat[m] = P.ml[m][L].khat;
+      ag.K[m] = lf.K[m] = P.ml[m][L].K;
+      for (int j = 0; j < rn; ++j) {
+        ag.S[m][j] = P.bS32[m][j];
+        lf.Bm[m][j] = P.bB32[m][j];
+      }
     }
-    ag.leaf_ptr = P.d_leaf_ptr;
-    ag.leaf_rwg = P.d_leaf_rwg;
+    ag.leaf_ptr = lf.leaf_ptr = P.d_leaf_ptr;
+    ag.leaf_rwg = lf.leaf_rwg = P.d_leaf_rwg;
     ag.X = X + g0 * ldx;
     ag.ldx = ldx;
-    ag.N = P.N;
-    ag.R = rn;
-    bool on_tensor_cores = false;
-    if constexpr (std::is_same<C, float2>::value) {
-      AggTcArg t{};
-      for (int m = 0; m < 2; ++m) {
-        t.Vs[m] = reinterpret_cast<const float*>(ag.Vs[m]);
-        t.K[m] = ag.K[m];
-        for (int j = 0; j < rn; ++j) t.S[m][j] = ag.S[m][j];
-      }
-      t.leaf_ptr = ag.leaf_ptr;
-      t.leaf_rwg = ag.leaf_rwg;
-      t.X = ag.X;
-      t.ldx = ag.ldx;
-      t.N = ag.N;
-      t.R = rn;
-      t.kmax = (P.max_leaf_rwgs + 7) & ~7;
-      t.status = P.d_status;
-      on_tensor_cores = P.tuning.batch_tc == 1 && agg_tc_supported(P, rn);
-      if (on_tensor_cores)
-        launch_agg_tc(P, t, s);
-      else
-        launch_agg_slots(P, t, s);
-    } else {
-      agg_batch_kernel<C, kAggRB><<<dim3(P.lv[L].B, 2, (rn + kAggRB - 1) / kAggRB), kThreads, 0, s>>>(ag);
-    }
+    ag.N = lf.N = P.N;
+    ag.R = lf.R = rn;
+    ag.kmax = (P.max_leaf_rwgs + 7) & ~7;
+    ag.status = lf.status = P.d_status;
+    lf.W = W + g0 * ldw;
+    lf.ldw = ldw;
+    LeafArg<C> common{};
+    fill_leaf_common(P, common);
+    lf.c1 = common.c1;
+    lf.c2 = common.c2;
+    lf.etai = common.etai;
+    const bool tensor_cores = P.tuning.batch_tc == 1 && agg_tc_supported(P, rn);
+    if (tensor_cores)
+      launch_agg_tc(P, ag, s);
+    else
+      launch_agg_slots(P, ag, s);
     {
       MediumStreams ms(P, s, true);
-      if constexpr (std::is_same<C, float2>::value) {
-        if (P.tuning.batch_tree == 1) {
-          for (int m = 0; m < 2; ++m)
-            tree_pass_slots(P, m, rn, ms.of(m), P.stream_leaf[m], P.ev_agg[m], P.ev_leaf[m]);
-        } else {
-          for (int j = 0; j < rn; ++j)
-            for (int m = 0; m < 2; ++m)
-              tree_pass_fixed<C>(P, m, Store<C>::bS(P, m, j), Store<C>::bB(P, m, j), ms.of(m));
-        }
+      if (P.tuning.batch_tree == 1) {
+        for (int m = 0; m < 2; ++m)
+          tree_pass_slots(P, m, rn, ms.of(m), P.stream_leaf[m], P.ev_agg[m], P.ev_leaf[m]);
       } else {
         for (int j = 0; j < rn; ++j)
-          for (int m = 0; m < 2; ++m)
-            tree_pass_fixed<C>(P, m, Store<C>::bS(P, m, j), Store<C>::bB(P, m, j), ms.of(m));
+          for (int m = 0; m < 2; ++m) tree_pass_fixed<C>(P, m, P.bS32[m][j], P.bB32[m][j], ms.of(m));
       }
       ms.join();
     }
-    LeafBatchArg<C> lb{};
-    for (int m = 0; m < 2; ++m) {
-      lb.Vf[m] = Store<C>::Vf(P, m);
-      lb.khat[m] = P.ml[m][L].khat;
-      lb.K[m] = P.ml[m][L].K;
-      for (int j = 0; j < rn; ++j) lb.Bm[m][j] = Store<C>::bB(P, m, j);
-    }
-    fill_leaf_common(P, lb);
-    fill_leaf_near(P, lb);
-    lb.X = X + g0 * ldx;
-    lb.ldx = ldx;
-    lb.W = W + g0 * ldw;
-    lb.ldw = ldw;
-    lb.R = rn;
-    const int warps = kThreads / 32;
-    const dim3 grid((P.N + warps - 1) / warps, (rn + kLeafRB - 1) / kLeafRB);
-    if constexpr (std::is_same<C, float2>::value) {
-      // near-field rows first (writing w), then the far field (adding)
-      leaf_out_batch_kernel<C, kLeafRB, false><<<grid, kThreads, 0, s>>>(lb);
-      MLFMA_CUDA(cudaGetLastError());
-      LeafTcArg t{};
-      for (int m = 0; m < 2; ++m) {
-        t.Vf[m] = lb.Vf[m];
-        t.khat[m] = lb.khat[m];
-        t.K[m] = lb.K[m];
-        for (int j = 0; j < rn; ++j) t.Bm[m][j] = lb.Bm[m][j];
-      }
-      t.leaf_ptr = P.d_leaf_ptr;
-      t.leaf_rwg = P.d_leaf_rwg;
-      t.W = lb.W;
-      t.ldw = ldw;
-      t.c1 = lb.c1;
-      t.c2 = lb.c2;
-      t.etai = lb.etai;
-      t.N = P.N;
-      t.R = rn;
-      t.status = P.d_status;
-      if (on_tensor_cores)
-        launch_leaf_tc(P, t, s);
-      else
-        launch_leaf_slots(P, t, s);
-    } else {
-      leaf_out_batch_kernel<C, kLeafRB><<<grid, kThreads, 0, s>>>(lb);
-      MLFMA_CUDA(cudaGetLastError());
-    }
+    // near-field rows first (writing w), then the far field (adding)
+    near_apply_batch(P, rn, ag.X, ldx, lf.W, ldw, P.d_pack, s);
+    if (tensor_cores)
+      launch_leaf_tc(P, lf, s);
+    else
+      launch_leaf_slots(P, lf, s);
   }
 }
 
@@ -2219,12 +2168,13 @@ void reserve_batch(Plan& P, int R, bool fp64) {
   const int want = std::min(R, kBatchSlots);
   const int L = P.maxL;
   if (P.precision == 1 && P.bS32[0].empty()) {
-    // the complex64 tree of every slot at once, slot-major per level, in one
-    // allocation
+    // the complex64 tree of every slot at once, slot-major per level, and the
+    // near-field product's packed inputs, in one allocation
     size_t total = 0;
     for (int m = 0; m < 2; ++m)
       for (int l = 2; l <= L; ++l) total += 2 * kBatchSlots * static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
-    float2* p = P.alloc<float2>(total);
+    float2* p = P.alloc<float2>(total + near_pack_values(P));
+    P.d_pack = p + total;
     for (int m = 0; m < 2; ++m) {
       for (int l = 2; l <= L; ++l) {
         const size_t cnt = static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
@@ -2368,7 +2318,7 @@ void apply_mixed_device(Plan& P, const double2* x, double2* w, cudaStream_t s) {
 void apply_batch_mixed_device(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw,
                               cudaStream_t s) {
   if (P.precision != 1) throw std::invalid_argument("plan was not created with mixed precision");
-  apply_batch_fixed<float2>(P, R, X, ldx, W, ldw, s);
+  apply_batch_slots(P, R, X, ldx, W, ldw, s);
 }
 
 }  // namespace mlfma

@@ -242,6 +242,7 @@ struct Plan {
   // batched complex64 apply runs every tree pass once per level for all slots.
   float2* btS[2][16] = {};
   float2* btB[2][16] = {};
+  float2* d_pack = nullptr;         // complex64 inputs of the batched near-field product, packed per RWG
   double2* d_xb = nullptr;          // staging for host-pointer batched apply
   double2* d_wb = nullptr;
   int xb_cap = 0;

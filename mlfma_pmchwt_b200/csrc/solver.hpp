@@ -52,6 +52,12 @@ std::vector<char> mixed_batch_solve(Plan& P, int R, double* x, const double* rhs
 // w = Z_near x on device vectors (complex128 [2N]).
 void near_apply(Plan& P, const double2* x, double2* w, cudaStream_t s, int prec = 0);
 
+// W_j = Z_near X_j in complex64 for R <= kBatchSlots rows (device), through a
+// packed copy of X (near_pack_values(P) complex64 values).
+void near_apply_batch(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw, float2* packed,
+                      cudaStream_t s);
+inline size_t near_pack_values(const Plan& P) { return static_cast<size_t>(kBatchSlots) * 2 * P.N; }
+
 // z = the near-field preconditioner applied to v (inner_its GMRES steps from
 // zero on the complex64 Z_near, as inside fgmres_solve); device vectors,
 // synchronous.
