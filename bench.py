@@ -41,14 +41,21 @@ def launches_per_apply(max_level: int, tune: dict) -> int:
     both media with agg variant 1, else one per medium); per medium one
     interpolation per level pair, the translations (the leaf level and the
     other levels as two launches with m2l variants 2-7, else one per level)
-    and one anterpolation per level pair; then the leaf testing + near-field
-    kernel (two kernels with leaf variant 1)."""
+    and one anterpolation per level pair; then the leaf testing (and, with leaf
+    variant 1, the near-field product on its own stream; with variant 0 its
+    launch before the leaf testing is near_launches)."""
     lv = max_level - 2
     # segmented translation variants: the leaf level and the other levels as two launches
     m2l = 2 if tune["m2l.variant"] in (2, 3, 4, 5, 6, 7, 8) else lv + 1
     agg = 1 if tune.get("agg.variant", 0) == 1 else 2
     leaf = 2 if tune.get("leaf.variant", 0) == 1 else 1
     return agg + 2 * (lv + m2l + lv) + leaf
+
+
+def near_launches(tune: dict) -> int:
+    """The near-field product's launch in an apply, where launches_per_apply
+    does not hold it already."""
+    return 0 if tune.get("leaf.variant", 0) == 1 else 1
 
 
 def workload(args):
@@ -653,9 +660,9 @@ def batched_apply_study(args, local: int, wl: dict) -> dict:
         op.set_tuning("batch_tc.variant", v)
         out["ms_per_batch"]["tensor_cores" if v else "cuda_cores"] = round(
             timed(lambda: op.apply_batch_mixed_device(R, X.data_ptr(), W.data_ptr(), sp), 3), 3)
-    op.set_tuning("batch_tc.variant", 1)
+    op.set_tuning("batch_tc.variant", 0)
     tree_keep = op.get_tuning("batch_tree.variant")
-    for v, key in ((0, "tensor_cores_tree_slot_by_slot"), (1, "tensor_cores_tree_slot_grid")):
+    for v, key in ((0, "cuda_cores_tree_slot_by_slot"), (1, "cuda_cores_tree_slot_grid")):
         op.set_tuning("batch_tree.variant", v)
         out["ms_per_batch"][key] = round(
             timed(lambda: op.apply_batch_mixed_device(R, X.data_ptr(), W.data_ptr(), sp), 3), 3)
@@ -867,7 +874,7 @@ def run_product(args):
                        "setup_s": round(setup_s, 2), "device_bytes": op.info.bytes_device,
                        "tuning": tune},
             "e2e": {k: (round(v, 3) if isinstance(v, float) else v) for k, v in e2e.items()},
-            "gpu_launches": args.steps * launches_per_apply(op.max_level, tune),
+            "gpu_launches": args.steps * (launches_per_apply(op.max_level, tune) + near_launches(tune)),
             "roofline": roofline, "clocks": clk}
     if mixed:
         line["mixed_precision"] = mixed

@@ -147,19 +147,21 @@ MLFMA_API int mlfma_device_status(mlfma_plan* plan, int* status);
 /* Batched apply: w[j] = A x[j] for R right-hand sides stored one after the
  * other (x[j] at x + 2 n j doubles, complex128 interleaved, n = 2N each).
  * The reference applies its AxFunc (Code/GMRES.h:53-66, the ax closure of
- * Code/MLFMM.cpp:189-368) once per right-hand side; here the leaf radiation /
- * receive patterns and the near-field entries are read once per group of up
- * to 16 right-hand sides. Each w[j] equals the single apply's result.
- * The first call on a plan allocates the leaf-level workspace of min(R, 16)
- * right-hand sides (about 2 x leaf boxes x 6 x (K1+K2) x 16 bytes each) plus,
- * for the host-pointer form, 2 x 16 staging vectors. Not re-entrant per plan. */
+ * Code/MLFMM.cpp:189-368) once per right-hand side, and so does the FP64
+ * operator here (its shared-table kernels were slower), on one captured apply.
+ * Each w[j] equals the single apply's result. The first host-pointer call on a
+ * plan allocates 2 x 16 staging vectors. Not re-entrant per plan. */
 MLFMA_API int mlfma_apply_batch(mlfma_plan* plan, int n, int R, const double* x, double* w);
 /* The batched apply with the complex64 operator (a plan created with
- * MLFMA_PREC_MIXED), device vectors as in mlfma_apply_batch_device. Its leaf
- * aggregation and far-field testing run on the tensor cores (tcgen05, TF32
+ * MLFMA_PREC_MIXED), device vectors as in mlfma_apply_batch_device: the leaf
+ * patterns and the near-field entries are read once per group of up to 16
+ * right-hand sides, and every tree pass runs once per level for the group. The
+ * leaf aggregation and far-field testing run on the tensor cores (tcgen05, TF32
  * operands split into high and low parts, FP32 accumulation in TMEM) when the
  * tuning key "batch_tc.variant" is 1 and every leaf box holds at most 64 RWGs,
- * else on the CUDA cores. No counterpart in the reference. */
+ * else in FP32 on the CUDA cores. The first call on a plan allocates the tree
+ * arrays of 16 right-hand sides (about 2 x boxes x 6 x (K1+K2) x 8 bytes per
+ * level each). No counterpart in the reference. */
 MLFMA_API int mlfma_apply_batch_mixed_device(mlfma_plan* plan, int n, int R, const void* x_dev, void* w_dev,
                                              void* stream);
 MLFMA_API int mlfma_apply_batch_device(mlfma_plan* plan, int n, int R, const void* x_dev, void* w_dev,
@@ -205,16 +207,16 @@ MLFMA_API int mlfma_profile_read(mlfma_plan* plan, double* stage_ms, int* applie
  *                  launch per medium (default); 1 = one CTA per (leaf box,
  *                  medium) streaming the box's contiguous pattern block.
  *   "batch_tc.variant" (the batched complex64 apply only) 0 = leaf aggregation
- *                  and far-field testing on the CUDA cores; 1 = on the tensor
- *                  cores (tcgen05 kind::tf32 with high/low operand splitting,
- *                  boxes of at most 64 RWGs; default).
+ *                  and far-field testing in FP32 on the CUDA cores (default);
+ *                  1 = on the tensor cores (tcgen05 kind::tf32 with high/low
+ *                  operand splitting, boxes of at most 64 RWGs).
  *   "batch_tree.variant" (the batched complex64 apply only) 0 = the tree
  *                  passes of each right-hand side in turn; 1 = every level
  *                  once for all right-hand sides on slot-major arrays (default).
- *   "leaf.variant" 0 = the near-field rows inside the leaf testing kernel (default);
- *                  1 = the near-field product on its own stream from the start
- *                  of the apply (it needs only x), overlapping the tree
- *                  passes; the leaf kernel then adds the far field.
+ *   "leaf.variant" 0 = the near-field product right before the leaf testing
+ *                  kernel, which adds the far field (default); 1 = the near-
+ *                  field product on its own stream from the start of the apply
+ *                  (it needs only x), overlapping the tree passes.
  *   "apply.graph"  1 = the apply of each (stream, precision) is captured as a
  *                  CUDA graph on first use and replayed afterwards (default);
  *                  the graph works on plan-owned vectors, x is copied in and

@@ -211,7 +211,6 @@ int mlfma_apply_batch(mlfma_plan* plan, int n, int R, const double* x, double* w
   return guarded([&] {
     mlfma::Plan& P = *plan->p;
     MLFMA_CUDA(cudaSetDevice(P.device));
-    mlfma::reserve_batch(P, R, true);
     mlfma::reserve_batch_staging(P);
     for (int g0 = 0; g0 < R; g0 += P.xb_cap) {
       const int rn = std::min(P.xb_cap, R - g0);
@@ -236,7 +235,6 @@ int mlfma_apply_batch_device(mlfma_plan* plan, int n, int R, const void* x_dev, 
   return guarded([&] {
     mlfma::Plan& P = *plan->p;
     MLFMA_CUDA(cudaSetDevice(P.device));
-    mlfma::reserve_batch(P, R, true);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : P.stream;
     mlfma::apply_batch_device(P, R, static_cast<const double2*>(x_dev), n, static_cast<double2*>(w_dev), n, s);
     return MLFMA_OK;
@@ -253,7 +251,7 @@ int mlfma_apply_batch_mixed_device(mlfma_plan* plan, int n, int R, const void* x
   return guarded([&] {
     mlfma::Plan& P = *plan->p;
     MLFMA_CUDA(cudaSetDevice(P.device));
-    mlfma::reserve_batch(P, R, false);
+    mlfma::reserve_batch(P);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : P.stream;
     mlfma::apply_batch_mixed_device(P, R, static_cast<const double2*>(x_dev), n, static_cast<double2*>(w_dev), n, s);
     return MLFMA_OK;

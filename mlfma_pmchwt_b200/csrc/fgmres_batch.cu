@@ -310,7 +310,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   if (inner_its < 0 || inner_its + 1 > blas1::kMaxBasis) throw std::invalid_argument("inner_its must be in 0..63");
   const auto t0 = std::chrono::steady_clock::now();
   MLFMA_CUDA(cudaSetDevice(P.device));
-  reserve_batch(P, R, false);
+  reserve_batch(P);
   cudaStream_t s = P.stream;
   const long long n = 2LL * P.N;
   const long long vs = static_cast<long long>(mr + 1) * n;       // per-system basis stride

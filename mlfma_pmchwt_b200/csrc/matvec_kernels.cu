@@ -1502,167 +1502,6 @@ void launch_leaf(const Plan& P, LeafArg<C>& a, cudaStream_t s) {
   leaf_rows_kernel<C><<<grid, 32 * kLeafWarps, 0, s>>>(a);
 }
 
-// ---------------------------------------------------------------- batched
-// Several right-hand sides per pass over the leaf tables: the aggregation and
-// the leaf testing + near field read each radiation / receive pattern and
-// each near-field entry once for a group of right-hand sides. Accumulation
-// orders are those of agg_box_kernel and leaf_out_kernel, so each right-hand
-// side of a batch gets the single apply's result.
-template <class C>
-struct AggBatchArg {
-  const C* Vs[2];
-  C* S[2][kBatchSlots];  // leaf-level S of each slot
-  int K[2];
-  const int* leaf_ptr;
-  const int* leaf_rwg;
-  const double2* X;            // right-hand side j at X + j * ldx
-  long long ldx;
-  int N, R;
-};
-
-template <class C, int RB>
-__global__ void __launch_bounds__(kThreads) agg_batch_kernel(AggBatchArg<C> a) {
-  const int b = blockIdx.x, m = blockIdx.y;
-  const int j0 = blockIdx.z * RB, jn = min(RB, a.R - j0);
-  const int K3 = 3 * a.K[m];
-  const int r0 = a.leaf_ptr[b], r1 = a.leaf_ptr[b + 1];
-  const C* V = a.Vs[m] + static_cast<size_t>(r0) * K3;
-  for (int e = threadIdx.x; e < K3; e += blockDim.x) {
-    C aJ[RB], aM[RB];
-#pragma unroll
-    for (int j = 0; j < RB; ++j) aJ[j] = aM[j] = Cx<C>::zero();
-    const C* v = V + e;
-    for (int r = r0; r < r1; ++r, v += K3) {
-      const int id = __ldg(a.leaf_rwg + r);
-      const C s = __ldg(v);
-#pragma unroll
-      for (int j = 0; j < RB; ++j) {
-        if (j < jn) {
-          const double2* x = a.X + (j0 + j) * a.ldx;
-          aJ[j] = cfma(s, Cx<C>::from(__ldg(x + id)), aJ[j]);
-          aM[j] = cfma(s, Cx<C>::from(__ldg(x + a.N + id)), aM[j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      if (j < jn) {
-        C* out = a.S[m][j0 + j] + static_cast<size_t>(b) * 2 * K3;
-        out[e] = aJ[j];
-        out[K3 + e] = aM[j];
-      }
-    }
-  }
-}
-
-template <class C>
-struct LeafBatchArg {
-  const C* Vf[2];
-  const C* Bm[2][kBatchSlots];  // leaf-level Bm of each slot
-  const double* khat[2];
-  int K[2];
-  const int* leaf_rwg;
-  const int* rwg_box;
-  const int* leaf_ptr;
-  const int* near_sptr;
-  const int* near_src;
-  const long long* near_zoff;
-  const C* near_z;
-  const double2* X;
-  long long ldx;
-  double2* W;
-  long long ldw;
-  int N, R;
-  C c1, c2, etai;
-};
-
-// One warp per (RWG, group of RB right-hand sides).
-template <class C, int RB>
-__global__ void __launch_bounds__(kThreads) leaf_out_batch_kernel(LeafBatchArg<C> a) {
-  using Rl = typename Cx<C>::real;
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (r >= a.N) return;
-  const int j0 = blockIdx.y * RB, jn = min(RB, a.R - j0);
-  const int id = a.leaf_rwg[r];
-  const int b = a.rwg_box[id];
-  C wj[RB], wm[RB];
-#pragma unroll
-  for (int j = 0; j < RB; ++j) wj[j] = wm[j] = Cx<C>::zero();
-#pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    const int K = a.K[m];
-    const C* V = a.Vf[m] + static_cast<size_t>(r) * 3 * K;
-    const double* kh = a.khat[m];
-    C acc[RB][4];  // LJ KJ LM KM
-#pragma unroll
-    for (int j = 0; j < RB; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[j][q] = Cx<C>::zero();
-    for (int kk = lane; kk < K; kk += 32) {
-      const C v0 = V[kk], v1 = V[K + kk], v2 = V[2 * K + kk];
-      // (-khat) x V
-      const Rl ax = static_cast<Rl>(-kh[kk]), ay = static_cast<Rl>(-kh[K + kk]), az = static_cast<Rl>(-kh[2 * K + kk]);
-      const C w0 = csub(cscale(v2, ay), cscale(v1, az));
-      const C w1 = csub(cscale(v0, az), cscale(v2, ax));
-      const C w2 = csub(cscale(v1, ax), cscale(v0, ay));
-#pragma unroll
-      for (int j = 0; j < RB; ++j) {
-        if (j < jn) {
-          const C* B = a.Bm[m][j0 + j] + static_cast<size_t>(b) * 6 * K;
-          const C b0 = B[kk], b1 = B[K + kk], b2 = B[2 * K + kk];
-          const C m0 = B[3 * K + kk], m1 = B[4 * K + kk], m2 = B[5 * K + kk];
-          acc[j][0] = cfma(v0, b0, cfma(v1, b1, cfma(v2, b2, acc[j][0])));
-          acc[j][2] = cfma(v0, m0, cfma(v1, m1, cfma(v2, m2, acc[j][2])));
-          acc[j][1] = cfma(w0, b0, cfma(w1, b1, cfma(w2, b2, acc[j][1])));
-          acc[j][3] = cfma(w0, m0, cfma(w1, m1, cfma(w2, m2, acc[j][3])));
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      const C LJ = warp_sum(acc[j][0]), KJ = warp_sum(acc[j][1]);
-      const C LM = warp_sum(acc[j][2]), KM = warp_sum(acc[j][3]);
-      if (m == 0) {
-        wj[j] = cmul(a.c1, csub(LJ, KM));
-        wm[j] = cmul(a.c1, cadd(KJ, LM));
-      } else {
-        wj[j] = cadd(wj[j], cmul(a.c2, csub(cmul(a.etai, LJ), KM)));
-        wm[j] = cadd(wm[j], cmul(a.c2, cadd(KJ, cdiv(LM, a.etai))));
-      }
-    }
-  }
-  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
-  const int tl = r - a.leaf_ptr[b];
-  const int pitch = near_pitch(ns);
-  const C* Z = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
-  C nJ[RB], nM[RB];
-#pragma unroll
-  for (int j = 0; j < RB; ++j) nJ[j] = nM[j] = Cx<C>::zero();
-  for (int q = lane; q < ns; q += 32) {
-    const int src = a.near_src[s0 + q];
-    const C z11 = Z[q], z12 = Z[pitch + q], z22 = Z[2 * pitch + q];
-#pragma unroll
-    for (int j = 0; j < RB; ++j) {
-      if (j < jn) {
-        const double2* x = a.X + (j0 + j) * a.ldx;
-        const C xJ = Cx<C>::from(x[src]), xM = Cx<C>::from(x[a.N + src]);
-        nJ[j] = cfma(z11, xJ, cfma(z12, xM, nJ[j]));
-        nM[j] = cfma(z22, xM, csub(nM[j], cmul(z12, xJ)));
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < RB; ++j) {
-    const C sJ = warp_sum(nJ[j]), sM = warp_sum(nM[j]);
-    if (lane == 0 && j < jn) {
-      double2* w = a.W + (j0 + j) * a.ldw;
-      w[id] = Cx<C>::to64(cadd(wj[j], sJ));
-      w[a.N + id] = Cx<C>::to64(cadd(wm[j], sM));
-    }
-  }
-}
-
 // Leaf-level pattern arrays of a tree pass: the plan's own, or one RHS slot
 // of a batched apply. Levels above the leaf always use the plan's arrays.
 struct LeafView {
@@ -1814,15 +1653,6 @@ void fill_leaf_common(const Plan& P, Arg& a) {
   a.c1 = Cx<C>::from(c2(c1.real(), c1.imag()));
   a.c2 = Cx<C>::from(c2(c2v.real(), c2v.imag()));
   a.etai = Cx<C>::from(c2(P.etai.real(), P.etai.imag()));
-}
-
-template <class C>
-void fill_leaf_near(const Plan& P, LeafBatchArg<C>& a) {
-  a.rwg_box = P.d_rwg_leafbox;
-  a.near_sptr = P.d_near_sptr;
-  a.near_src = P.d_near_src;
-  a.near_zoff = P.d_near_zoff;
-  a.near_z = Store<C>::near_z(P);
 }
 
 // Medium 1's tree passes go to the plan's second stream, forked from and
@@ -2164,97 +1994,43 @@ void reserve_batch_staging(Plan& P) {
   P.xb_cap = kBatchSlots;
 }
 
-void reserve_batch(Plan& P, int R, bool fp64) {
-  const int want = std::min(R, kBatchSlots);
+void reserve_batch(Plan& P) {
   const int L = P.maxL;
-  if (P.precision == 1 && P.bS32[0].empty()) {
-    // the complex64 tree of every slot at once, slot-major per level, and the
-    // near-field product's packed inputs, in one allocation
-    size_t total = 0;
-    for (int m = 0; m < 2; ++m)
-      for (int l = 2; l <= L; ++l) total += 2 * kBatchSlots * static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
-    float2* p = P.alloc<float2>(total + near_pack_values(P));
-    P.d_pack = p + total;
-    for (int m = 0; m < 2; ++m) {
-      for (int l = 2; l <= L; ++l) {
-        const size_t cnt = static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
-        P.btS[m][l] = p;
-        P.btB[m][l] = p + kBatchSlots * cnt;
-        p += 2 * kBatchSlots * cnt;
-      }
-      const size_t cnt = static_cast<size_t>(P.lv[L].B) * 6 * P.ml[m][L].K;
-      for (int j = 0; j < kBatchSlots; ++j) {
-        P.bS32[m].push_back(P.btS[m][L] + j * cnt);
-        P.bB32[m].push_back(P.btB[m][L] + j * cnt);
-      }
+  if (P.precision != 1 || !P.bS32[0].empty()) return;
+  // the complex64 tree of every slot at once, slot-major per level, and the
+  // near-field product's packed inputs, in one allocation
+  size_t total = 0;
+  for (int m = 0; m < 2; ++m)
+    for (int l = 2; l <= L; ++l) total += 2 * kBatchSlots * static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
+  float2* p = P.alloc<float2>(total + near_pack_values(P));
+  P.d_pack = p + total;
+  for (int m = 0; m < 2; ++m) {
+    for (int l = 2; l <= L; ++l) {
+      const size_t cnt = static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
+      P.btS[m][l] = p;
+      P.btB[m][l] = p + kBatchSlots * cnt;
+      p += 2 * kBatchSlots * cnt;
     }
-  }
-  if (fp64 && P.batch_cap < want) {
-    // the FP64 leaf arrays of the slots still missing, in one allocation
-    const int add = want - P.batch_cap;
-    size_t total = 0;
-    for (int m = 0; m < 2; ++m) total += 2 * static_cast<size_t>(add) * P.lv[L].B * 6 * P.ml[m][L].K;
-    double2* p = P.alloc<double2>(total);
-    for (int m = 0; m < 2; ++m) {
-      const size_t cnt = static_cast<size_t>(P.lv[L].B) * 6 * P.ml[m][L].K;
-      for (int j = 0; j < add; ++j) {
-        P.bS[m].push_back(p);
-        P.bB[m].push_back(p + cnt);
-        p += 2 * cnt;
-      }
+    const size_t cnt = static_cast<size_t>(P.lv[L].B) * 6 * P.ml[m][L].K;
+    for (int j = 0; j < kBatchSlots; ++j) {
+      P.bS32[m].push_back(P.btS[m][L] + j * cnt);
+      P.bB32[m].push_back(P.btB[m][L] + j * cnt);
     }
-    P.batch_cap = want;
   }
 }
 
+// FP64: one captured apply per row. Sharing the leaf tables among rows saves
+// traffic but its kernels were slower than the single apply's, whose media and
+// leaf translation also overlap: 3 rows at 10,140 unknowns 1.02 ms shared, 0.88 ms
+// row by row; 7.4 against 6.7 ms per row at 245,760 unknowns.
 void apply_batch_device(Plan& P, int R, const double2* X, long long ldx, double2* W, long long ldw, cudaStream_t s) {
-  const int L = P.maxL;
-  if (P.batch_cap < std::min(R, kBatchSlots)) throw std::runtime_error("batched apply: slots not reserved");
-  constexpr int kAggRB = 8, kLeafRB = 4;
-  for (int g0 = 0; g0 < R; g0 += kBatchSlots) {
-    const int rn = std::min(kBatchSlots, R - g0);
-    AggBatchArg<double2> ag{};
-    for (int m = 0; m < 2; ++m) {
-      ag.Vs[m] = P.d_Vs[m];
-      ag.K[m] = P.ml[m][L].K;
-      for (int j = 0; j < rn; ++j) ag.S[m][j] = P.bS[m][j];
-    }
-    ag.leaf_ptr = P.d_leaf_ptr;
-    ag.leaf_rwg = P.d_leaf_rwg;
-    ag.X = X + g0 * ldx;
-    ag.ldx = ldx;
-    ag.N = P.N;
-    ag.R = rn;
-    agg_batch_kernel<double2, kAggRB><<<dim3(P.lv[L].B, 2, (rn + kAggRB - 1) / kAggRB), kThreads, 0, s>>>(ag);
-    {
-      MediumStreams ms(P, s, true);
-      for (int j = 0; j < rn; ++j)
-        for (int m = 0; m < 2; ++m) {
-          const LeafView v{P.bS[m][j], P.bB[m][j]};
-          launch_up(P, m, v, ms.of(m));
-          launch_m2l(P, m, v, ms.of(m), 2, P.maxL);
-          launch_l2l(P, m, v, ms.of(m));
-        }
-      ms.join();
-    }
-    LeafBatchArg<double2> lb{};
-    for (int m = 0; m < 2; ++m) {
-      lb.Vf[m] = P.d_Vf[m];
-      lb.khat[m] = P.ml[m][L].khat;
-      lb.K[m] = P.ml[m][L].K;
-      for (int j = 0; j < rn; ++j) lb.Bm[m][j] = P.bB[m][j];
-    }
-    fill_leaf_common(P, lb);
-    fill_leaf_near(P, lb);
-    lb.X = X + g0 * ldx;
-    lb.ldx = ldx;
-    lb.W = W + g0 * ldw;
-    lb.ldw = ldw;
-    lb.R = rn;
-    const int warps = kThreads / 32;
-    leaf_out_batch_kernel<double2, kLeafRB><<<dim3((P.N + warps - 1) / warps, (rn + kLeafRB - 1) / kLeafRB), kThreads, 0, s>>>(lb);
-    MLFMA_CUDA(cudaGetLastError());
-  }
+  struct Unprofiled {  // the stage profiler covers single applies only
+    bool& on;
+    const bool was;
+    explicit Unprofiled(bool& o) : on(o), was(o) { on = false; }
+    ~Unprofiled() { on = was; }
+  } quiet(P.prof.on);
+  for (int j = 0; j < R; ++j) apply_device(P, X + j * ldx, W + j * ldw, s);
 }
 
 // Replays the captured apply of (stream, precision), capturing it on first

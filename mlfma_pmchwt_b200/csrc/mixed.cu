@@ -141,7 +141,7 @@ std::vector<char> mixed_batch_solve(Plan& P, int R, double* xh, const double* rh
   const auto t0 = std::chrono::steady_clock::now();
   MLFMA_CUDA(cudaSetDevice(P.device));
   MLFMA_CUDA(cudaMemsetAsync(P.d_status, 0, sizeof(int), P.stream));
-  reserve_batch(P, R, false);
+  reserve_batch(P);
   reserve_batch_staging(P);  // the FP64 residuals' device rows
   const long long n = 2LL * P.N;
   C* X = reinterpret_cast<C*>(xh);

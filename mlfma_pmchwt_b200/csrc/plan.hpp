@@ -231,10 +231,7 @@ struct Plan {
   double2* d_gw = nullptr;
   double2* d_x = nullptr;           // staging for host-pointer apply
   double2* d_w = nullptr;
-  // ---- batched apply: leaf-level S / B arrays of each right-hand-side slot
-  // (levels above the leaf are shared: the slots pass through them in turn)
-  int batch_cap = 0;
-  std::vector<double2*> bS[2], bB[2];
+  // ---- batched complex64 apply: leaf-level S / B arrays of each right-hand-side slot
   std::vector<float2*> bS32[2], bB32[2];
   // Complex64 tree arrays of all kBatchSlots right-hand-side slots (mixed
   // plans), per medium and level 2..maxLevel, slot-major and contiguous:
@@ -360,8 +357,6 @@ struct Store<double2> {
   static const double2* Vs(const Plan& P, int m) { return P.d_Vs[m]; }
   static const double2* Vf(const Plan& P, int m) { return P.d_Vf[m]; }
   static const double2* near_z(const Plan& P) { return P.d_near_z; }
-  static double2* bS(const Plan& P, int m, int j) { return P.bS[m][j]; }
-  static double2* bB(const Plan& P, int m, int j) { return P.bB[m][j]; }
 };
 template <>
 struct Store<float2> {
@@ -373,8 +368,6 @@ struct Store<float2> {
   static const float2* Vs(const Plan& P, int m) { return P.d_Vs32[m]; }
   static const float2* Vf(const Plan& P, int m) { return P.d_Vf32[m]; }
   static const float2* near_z(const Plan& P) { return P.d_near_z32; }
-  static float2* bS(const Plan& P, int m, int j) { return P.bS32[m][j]; }
-  static float2* bB(const Plan& P, int m, int j) { return P.bB32[m][j]; }
 };
 
 // Device work (setup_kernels.cu / matvec_kernels.cu)
@@ -392,7 +385,7 @@ void launch_near_z12_scatter(double2* Z, const long long* pos, const double2* z1
 void apply_device(Plan& P, const double2* x, double2* w, cudaStream_t s);
 void clear_graphs(Plan& P);  // after any change that alters what an apply launches
 // Batched apply: W[j] = A X[j] for j < R; X[j] at X + j * ldx (ldx >= 2N),
-// the same for W. Right-hand sides go through in groups of kBatchSlots.
+// the same for W: row by row in FP64, in groups of kBatchSlots in complex64.
 constexpr int kBatchSlots = 16;
 // Copies the plan's device status bits to its pinned host word on stream s
 // (read after the caller's synchronisation of s) ...
@@ -401,9 +394,8 @@ void fetch_device_status(Plan& P, cudaStream_t s);
 // apply's result is incomplete), naming the kernels.
 void raise_device_status(const Plan& P);
 
-// Allocates the complex64 slot tree (mixed plans) and, with fp64, the FP64
-// leaf-level arrays of min(R, kBatchSlots) slots.
-void reserve_batch(Plan& P, int R, bool fp64);
+// Allocates the complex64 slot tree of a mixed plan (no-op otherwise).
+void reserve_batch(Plan& P);
 // Allocates d_xb / d_wb (kBatchSlots vectors each), the staging of
 // host-pointer batched applies and of the refinement's FP64 residuals.
 void reserve_batch_staging(Plan& P);
