@@ -881,7 +881,9 @@ __device__ __forceinline__ C load_at(const C* base, Off byte) {
   return __ldg(reinterpret_cast<const C*>(reinterpret_cast<const char*>(base) + byte));
 }
 
-template <class C, bool kSlots, int kW, class Off>
+// kSplit: the CTA's warps share one pair, each walking every kW-th entry, and
+// meet in shared memory (see kSplitWarps).
+template <class C, bool kSlots, int kW, class Off, bool kSplit>
 __global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 * kW))
     m2l_pair_kernel(const __grid_constant__ M2lPairArg<C> a) {
   int si = 0;
@@ -889,10 +891,13 @@ __global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 
   const M2lPairSeg<C>& g = a.seg[si];
   const int local = blockIdx.x - g.cta_begin;
   const int grp = local / g.nchunk;
-  const int pg = grp * kW + (threadIdx.x >> 5);
-  const int k = (local - grp * g.nchunk) * 32 + (threadIdx.x & 31);
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pg = kSplit ? grp : grp * kW + wp;
   const int K = g.K;
-  if (2 * pg >= g.B || k >= K) return;
+  const int k0 = (local - grp * g.nchunk) * 32 + lane;
+  if (!kSplit && (2 * pg >= g.B || k0 >= K)) return;
+  const int k = kSplit ? min(k0, K - 1) : k0;
+  constexpr int kStep = kSplit ? kW : 1;
   const C* const Sl = kSlots ? g.S + blockIdx.y * g.slot_S : g.S;
   C* const Bl = kSlots ? g.Bm + blockIdx.y * g.slot_B : g.Bm;
   C a0[6], a1[6];
@@ -903,7 +908,7 @@ __global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 
   // memory latency per entry instead of three (indices, then the patterns and
   // the first box's factor, then the second's behind its branch).
   const int e1 = g.pair_ptr[pg + 1];
-  int e = g.pair_ptr[pg];
+  int e = g.pair_ptr[pg] + (kSplit ? wp : 0);
   int src = e < e1 ? __ldg(g.pair_src + e) : 0;
   int2 v = e < e1 ? __ldg(g.pair_vec + e) : make_int2(-1, -1);
   const Off row = static_cast<Off>(K) * static_cast<Off>(sizeof(C)), at = static_cast<Off>(k) * static_cast<Off>(sizeof(C));
@@ -915,7 +920,7 @@ __global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 
     const bool in0 = v.x >= 0, in1 = v.y >= 0;
     if (in0) t0 = load_at(g.tfw, static_cast<Off>(v.x) * row + at);
     if (in1) t1 = load_at(g.tfw, static_cast<Off>(v.y) * row + at);
-    if (++e < e1) {
+    if ((e += kStep) < e1) {
       src = __ldg(g.pair_src + e);
       v = __ldg(g.pair_vec + e);
     }
@@ -927,6 +932,26 @@ __global__ void __launch_bounds__(32 * kW, (sizeof(C) == 16 ? 640 : 1024) / (32 
 #pragma unroll
       for (int c = 0; c < 6; ++c) a1[c] = cfma(t1, sv[c], a1[c]);
     }
+  }
+  if constexpr (kSplit) {
+    static_assert(12 % kW == 0, "every warp adds up as many components");
+    __shared__ C part[kW][12][32];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      part[wp][c][lane] = a0[c];
+      part[wp][6 + c][lane] = a1[c];
+    }
+    __syncthreads();
+    if (k0 >= K) return;
+#pragma unroll
+    for (int i = 0; i < 12 / kW; ++i) {
+      const int c = wp * (12 / kW) + i, box = 2 * pg + c / 6;
+      C v = part[0][c][lane];
+#pragma unroll
+      for (int q = 1; q < kW; ++q) v = cadd(v, part[q][c][lane]);
+      if (box < g.B) Bl[(static_cast<size_t>(box) * 6 + c % 6) * K + k] = v;
+    }
+    return;
   }
   C* out0 = Bl + static_cast<size_t>(2 * pg) * 6 * K + k;
 #pragma unroll
@@ -990,27 +1015,53 @@ __global__ void __launch_bounds__(64 * kPairWarps) m2l_pairh_kernel(const __grid
 inline int pair_warps(const Plan& P) { return 2 << P.tuning.m2l_pair_warps; }
 inline int up_threads(const Plan& P) { return 64 << P.tuning.up_threads; }
 
+// FP64 launches of fewer warps than this (5 per SM) share each pair's list among
+// the warps of a CTA: a warp walks ~70 entries at ~0.3 us each with nothing beside
+// it, so both translations of a plan of 56 boxes took 23 us, and take 9.5 split
+// (apply at 960 unknowns 54.5 -> 41.7 us alone, 27.3 -> 24.6 among others). With
+// the line at 10 or 20 warps per SM the kernels of an apply at 7,260 unknowns
+// shorten too (204 -> 159 and 124 us in all), but the apply does not (231 -> 234
+// and 239 us). Complex64 stays unsplit: its batched form sums whole lists, and a
+// slot equals the single apply to rounding of identical operations.
+constexpr int kSplitWarps = 148 * 5;
+
 template <class C, bool kSlots, class Off>
-void launch_m2l_pair_as(int w, dim3 grid, const M2lPairArg<C>& a, cudaStream_t st) {
+void launch_m2l_pair_as(int w, bool split, dim3 grid, const M2lPairArg<C>& a, cudaStream_t st) {
+  if constexpr (!kSlots && sizeof(C) == 16) {
+    if (split) {
+      m2l_pair_kernel<C, false, kPairWarps, Off, true><<<grid, 32 * kPairWarps, 0, st>>>(a);
+      return;
+    }
+  }
   if (w == 2)
-    m2l_pair_kernel<C, kSlots, 2, Off><<<grid, 64, 0, st>>>(a);
+    m2l_pair_kernel<C, kSlots, 2, Off, false><<<grid, 64, 0, st>>>(a);
   else if (w == 8)
-    m2l_pair_kernel<C, kSlots, 8, Off><<<grid, 256, 0, st>>>(a);
+    m2l_pair_kernel<C, kSlots, 8, Off, false><<<grid, 256, 0, st>>>(a);
   else
-    m2l_pair_kernel<C, kSlots, 4, Off><<<grid, 128, 0, st>>>(a);
+    m2l_pair_kernel<C, kSlots, 4, Off, false><<<grid, 128, 0, st>>>(a);
 }
 
+// The segments of `a` (cta_begin set here) for `slots` right-hand-side slots.
 template <class C, bool kSlots>
-void launch_m2l_pair(int w, dim3 grid, const M2lPairArg<C>& a, cudaStream_t st) {
+void launch_m2l_pair(const Plan& P, M2lPairArg<C>& a, int slots, cudaStream_t st) {
   bool small = true;  // every level's patterns and factors within 32-bit byte offsets
+  long long warps = 0;
   for (int i = 0; i < a.nseg; ++i) {
     const size_t row = sizeof(C) * static_cast<size_t>(a.seg[i].K);
     small = small && row * 6 * static_cast<size_t>(a.seg[i].B) < (1ull << 32) && row * 343 < (1ull << 32);
+    warps += static_cast<long long>((a.seg[i].B + 1) / 2) * a.seg[i].nchunk;
+  }
+  const bool split = sizeof(C) == 16 && warps < kSplitWarps;
+  const int w = pair_warps(P), per = split ? 1 : w;
+  int ctas = 0;
+  for (int i = 0; i < a.nseg; ++i) {
+    a.seg[i].cta_begin = ctas;
+    ctas += (((a.seg[i].B + 1) / 2 + per - 1) / per) * a.seg[i].nchunk;
   }
   if (small)
-    launch_m2l_pair_as<C, kSlots, uint32_t>(w, grid, a, st);
+    launch_m2l_pair_as<C, kSlots, uint32_t>(w, split, dim3(ctas, slots), a, st);
   else
-    launch_m2l_pair_as<C, kSlots, size_t>(w, grid, a, st);
+    launch_m2l_pair_as<C, kSlots, size_t>(w, split, dim3(ctas, slots), a, st);
 }
 
 // Translation with staged sources: a CTA takes a group of 8 Morton-
@@ -1567,13 +1618,12 @@ void launch_m2l(Plan& P, int m, const LeafView& v, cudaStream_t s, int lo, int h
       g = M2lPairSeg<double2>{level_S(P, m, l, v), level_B(P, m, l, v), cm.tfw, P.lv[l].pair_ptr, P.lv[l].pair_src,
                               P.lv[l].pair_vec,    P.lv[l].B,           cm.K,   (cm.K + 31) / 32,  ctas};
       const int G = (P.lv[l].B + 1) / 2;
-      const int w = P.tuning.m2l_variant == 5 ? kPairWarps : pair_warps(P);
-      ctas += ((G + w - 1) / w) * g.nchunk;
+      ctas += ((G + kPairWarps - 1) / kPairWarps) * g.nchunk;
     }
     if (P.tuning.m2l_variant == 5)
       m2l_pairh_kernel<double2><<<ctas, 64 * kPairWarps, 0, s>>>(a);
     else
-      launch_m2l_pair<double2, false>(pair_warps(P), dim3(ctas), a, s);
+      launch_m2l_pair<double2, false>(P, a, 1, s);
     return;
   }
   if (P.tuning.m2l_variant == 3) {
@@ -1742,15 +1792,13 @@ void tree_pass_fixed(Plan& P, int m, C* leafS, C* leafB, cudaStream_t s, cudaStr
     }
     if (hi - lo + 1 > kM2lMaxSeg) throw std::runtime_error("m2l: more levels than one launch takes");
     M2lPairArg<C> t{};
-    int ctas = 0;
     for (int l = lo; l <= hi; ++l) {
       const MediumLevel& cm = P.ml[m][l];
       M2lPairSeg<C>& g = t.seg[t.nseg++];
       g = M2lPairSeg<C>{S_at(l),          B_at(l),   Store<C>::tfw(cm), P.lv[l].pair_ptr, P.lv[l].pair_src,
-                        P.lv[l].pair_vec, P.lv[l].B, cm.K,              (cm.K + 31) / 32, ctas};
-      ctas += (((P.lv[l].B + 1) / 2 + pair_warps(P) - 1) / pair_warps(P)) * g.nchunk;
+                        P.lv[l].pair_vec, P.lv[l].B, cm.K,              (cm.K + 31) / 32, 0};
     }
-    launch_m2l_pair<C, false>(pair_warps(P), dim3(ctas), t, st);
+    launch_m2l_pair<C, false>(P, t, 1, st);
   };
   if (sx) {
     MLFMA_CUDA(cudaEventRecord(ev_agg, s));
@@ -1796,16 +1844,14 @@ void tree_pass_slots(Plan& P, int m, int rn, cudaStream_t s, cudaStream_t sx, cu
     if (lo > hi) return;
     if (hi - lo + 1 > kM2lMaxSeg) throw std::runtime_error("m2l: more levels than one launch takes");
     M2lPairArg<C> t{};
-    int ctas = 0;
     for (int l = lo; l <= hi; ++l) {
       const MediumLevel& cm = P.ml[m][l];
       M2lPairSeg<C>& g = t.seg[t.nseg++];
       g = M2lPairSeg<C>{P.btS[m][l],      P.btB[m][l], cm.tfw32,          P.lv[l].pair_ptr, P.lv[l].pair_src,
-                        P.lv[l].pair_vec, P.lv[l].B,   cm.K,              (cm.K + 31) / 32, ctas,
+                        P.lv[l].pair_vec, P.lv[l].B,   cm.K,              (cm.K + 31) / 32, 0,
                         stride(l),        stride(l)};
-      ctas += (((P.lv[l].B + 1) / 2 + pair_warps(P) - 1) / pair_warps(P)) * g.nchunk;
     }
-    launch_m2l_pair<C, true>(pair_warps(P), dim3(ctas, rn), t, st);
+    launch_m2l_pair<C, true>(P, t, rn, st);
     MLFMA_CUDA(cudaGetLastError());
   };
   MLFMA_CUDA(cudaEventRecord(ev_agg, s));

@@ -1,8 +1,9 @@
 """The tree passes level by level against the same sums in numpy, on the stage
 arrays and tables an operator reads out: interpolation by pairs of parent
 rows, translation by box pairs, anterpolation by pairs of child rows. Grids
-of odd and even theta counts, a lossy body, and grids so fine that an
-anterpolation band holds a single child row."""
+of odd and even theta counts, a lossy body, grids so fine that an
+anterpolation band holds a single child row, and launches of few and of many
+warps (the translation shares a pair's list among its warps below 740)."""
 import numpy as np
 import pytest
 
@@ -12,6 +13,7 @@ pytestmark = pytest.mark.gpu
 
 BODIES = {"deep": lambda: dict(mesh=M.ellipsoid(3, 1.0, 0.8, 0.7), eps_r=2.5 - 0.1j, leaf_coeff=0.12),
           "shallow": lambda: dict(mesh=M.icosphere(3, 1.0), eps_r=4.0, leaf_coeff=0.25),
+          "split lists": lambda: dict(mesh=M.ellipsoid(2, 0.7, 0.6, 0.5), eps_r=4.0, leaf_coeff=0.2),
           "fine grids": lambda: dict(mesh=M.icosphere(1, 1.0), eps_r=360.0, leaf_coeff=0.25)}
 
 
