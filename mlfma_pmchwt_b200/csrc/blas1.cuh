@@ -11,17 +11,19 @@
 // Bound: latency, not bandwidth (the basis of a solve is L2-resident at up
 // to ~100,000 unknowns and a pass over 16 vectors of 34,560 complex values
 // takes ~1 us), so what counts is the number of dependent launches and the
-// serial code between them. Twice-classical Gram-Schmidt is three launches
-// here: coefficients, projection fused with the coefficients of the second
-// pass (each thread still holds the updated rows), second projection fused
-// with the norm.
+// serial code between them. Twice-classical Gram-Schmidt is one launch for
+// short vectors (gs_cluster_kernel) and three for others: coefficients,
+// projection fused with the coefficients of the second pass (each thread still
+// holds the updated rows), second projection fused with the norm.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <complex>
 #include <vector>
 
+#include "bulk.cuh"
 #include "cplx.cuh"
 #include "plan.hpp"
 #include "reduce.cuh"
@@ -304,6 +306,7 @@ struct GsArg {
   unsigned* count;       // [a] blocks done
   Inner inner;
   int step;
+  int cached;            // gs_cluster_kernel: basis vectors in shared memory
   Pack pack;
 };
 
@@ -433,6 +436,142 @@ static __global__ void __launch_bounds__(kThreads) gs_kernel(const __grid_consta
     inner_step(g.inner, a, g.step, g.hbase + static_cast<long long>(a) * kLdh, norm2, &ws[0][0]);
 }
 
+// Both Gram-Schmidt passes, the norm and the inner step in one launch: a
+// cluster of kClBlocks blocks per position, E rows per thread, which stay in
+// registers from the first dot product to the last projection. The blocks'
+// sums meet through distributed shared memory, every block adding them up in
+// the same order. A block first fetches its rows of as many basis vectors as
+// its shared memory holds (all loads at once), and the four passes read those.
+// Bound: latency (launch, three cluster barriers, the serial rotations). At
+// 3,840 unknowns and 15 vectors 14.6 us for 29.7 in three launches of
+// gs_kernel; 19.0 with 88 KB of shared memory, 22.6 without.
+// Where the line lies (solves with 16 inner steps, ms, gs_kernel -> clusters):
+//   n = 2,160:  1 system 11.8 -> 10.3, 8: 15.6 -> 14.4, 12: 19.2 -> 18.0, 16: 20.3 -> 21.6
+//   n = 15,360: 1 system 32.9 -> 30.5, 8: 67.9 -> 65.6, 12: 97.5 -> 95.6, 16: 116.9 -> 117.5
+//   n = 24,000 (4 rows per thread): 38.4 -> 38.9, 8: 103.3 -> 102.9
+//   n = 34,560 (8 rows): 30.5 -> 32.0 (16 SMs read the basis four times)
+// so up to two rows per thread and 12 positions. With 200 KB of shared memory
+// 7 clusters fit at once, with 88 KB (two blocks per SM) 14: 8 systems took two
+// turns with the former, 27.8 us at 15,360 unknowns, 23.0 with the latter.
+constexpr int kClThreads = 512;
+constexpr int kClWarps = kClThreads / 32;
+constexpr int kClBlocks = 16;  // the non-portable size: a GPC's worth of SMs
+constexpr int kClRows = 2;     // rows per thread at most
+constexpr int kClMaxPositions = 12;
+constexpr int kClCache = 200 << 10;  // bytes of the basis in shared memory, up to
+constexpr int kClWide = 7;           // this many positions
+constexpr int kClCacheMany = 88 << 10;
+
+template <int E, bool kStep>
+static __global__ void __launch_bounds__(kClThreads, 2) gs_cluster_kernel(const __grid_constant__ GsArg g) {
+  __shared__ double2 hs[kMaxBasis];
+  __shared__ double2 ws[kClWarps][kMaxBasis];
+  __shared__ double2 part[2][kMaxBasis];
+  __shared__ double2 pn;
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int a = blockIdx.y, rank = blockIdx.x;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int n = static_cast<int>(g.n), nv = g.nv;
+  const double2* __restrict__ V = g.V.at(a, g.sys);
+  double2* w = g.w.at(a, g.sys);
+  double2* hout = g.hout + static_cast<long long>(a) * kLdh;
+  const double* vs = g.vs ? g.vs + static_cast<long long>(a) * g.ldvs : nullptr;
+  const int i0 = rank * kClThreads + threadIdx.x;
+  auto row = [&](int e) { return i0 + e * (kClBlocks * kClThreads); };
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  double2* mine = reinterpret_cast<double2*>(gs_smem) + threadIdx.x;  // own rows of the first nc basis vectors
+  const int nc = g.cached;
+  for (int j = 0; j < nc; ++j)
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const bool take = row(e) < n;
+      cp_async16_or_zero(mine + (j * E + e) * kClThreads, V + (take ? j * g.n + row(e) : 0), take);
+    }
+  cp_async_commit();
+  double2 wi[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) wi[e] = row(e) < n ? w[row(e)] : c2(0.0, 0.0);
+  cp_async_wait<0>();
+  auto dots = [&](int pass) {
+    for (int j0 = 0; j0 < nv; j0 += kTile) {
+      double2 acc[kTile];
+#pragma unroll
+      for (int q = 0; q < kTile; ++q) {
+        acc[q] = c2(0.0, 0.0);
+        if (j0 + q < nv) {
+          const bool cached = j0 + q < nc;
+          const double2 *Vj = V + (j0 + q) * g.n, *own = mine + (j0 + q) * E * kClThreads;
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const double2 v = cached ? own[e * kClThreads] : row(e) < n ? __ldg(Vj + row(e)) : c2(0.0, 0.0);
+            acc[q].x = fma(v.x, wi[e].x, fma(v.y, wi[e].y, acc[q].x));
+            acc[q].y = fma(v.x, wi[e].y, fma(-v.y, wi[e].x, acc[q].y));
+          }
+        }
+      }
+      const double2 t = warp_sum8(acc);
+      const int q = lane >> 2;
+      if ((lane & 3) == 0 && j0 + q < nv) ws[wp][j0 + q] = t;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < nv; j += kClThreads) {
+      double2 t = ws[0][j];
+#pragma unroll
+      for (int q = 1; q < kClWarps; ++q) t = cadd(t, ws[q][j]);
+      part[pass][j] = t;
+    }
+    cl.sync();
+    for (int j = wp; j < nv; j += kClWarps) {
+      double2 t = lane < kClBlocks ? *cl.map_shared_rank(&part[pass][j], lane) : c2(0.0, 0.0);
+      t = warp_sum2(t);
+      if (lane == 0) {
+        const double sc = vs ? vs[j] : 1.0;
+        t = cscale(t, sc);
+        if (rank == 0) hout[pass * kMaxBasis + j] = t;
+        hs[j] = cscale(t, sc);
+      }
+    }
+    __syncthreads();
+  };
+  auto project = [&] {
+#pragma unroll 4
+    for (int j = 0; j < nc; ++j) {
+      const double2 hj = hs[j];
+#pragma unroll
+      for (int e = 0; e < E; ++e) wi[e] = csub(wi[e], cmul(hj, mine[(j * E + e) * kClThreads]));
+    }
+#pragma unroll 4
+    for (int j = nc; j < nv; ++j) {
+      const double2* Vj = V + j * g.n;
+      const double2 hj = hs[j];
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (row(e) < n) wi[e] = csub(wi[e], cmul(hj, __ldg(Vj + row(e))));
+    }
+  };
+  dots(0);
+  project();
+  dots(1);
+  project();
+  double2 nrm = c2(0.0, 0.0);
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (row(e) < n) {
+      w[row(e)] = wi[e];
+      if (kStep && g.pack.p) pack_row(g.pack, g.n, a, row(e), wi[e]);
+      nrm.x = fma(wi[e].x, wi[e].x, fma(wi[e].y, wi[e].y, nrm.x));
+    }
+  nrm = block_sum(nrm, &ws[0][0]);
+  if (threadIdx.x == 0) pn = nrm;
+  cl.sync();
+  if (rank == 0 && wp == 0)
+    nrm = warp_sum2(lane < kClBlocks ? *cl.map_shared_rank(&pn, lane) : c2(0.0, 0.0));
+  cl.sync();  // no block leaves before its sum is read
+  if (rank != 0 || wp != 0) return;
+  if (lane == 0) hout[2 * kMaxBasis] = nrm;
+  if (kStep) inner_step(g.inner, a, g.step, hout, nrm.x, &ws[0][0]);
+}
+
 // dst = alpha[a] * src
 static __global__ void __launch_bounds__(kThreads) scale_kernel(VecRef src, VecRef dst, const int* sys, long long n,
                                                                 const double* alpha) {
@@ -514,6 +653,55 @@ inline void launch_gs(const GsArg& g, int Ra, cudaStream_t s) {
     gs_kernel<4, kProject, kDots, kFin><<<grid, kThreads, 0, s>>>(g);
 }
 
+template <bool kStep>
+inline void launch_gs_cluster(GsArg g, int Ra, cudaStream_t s) {
+  auto go = [&](auto* kernel, int E) {
+    MLFMA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    MLFMA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClCache));
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {kClBlocks, 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kClBlocks, Ra);
+    cfg.blockDim = dim3(kClThreads);
+    const int vec = 16 * kClThreads * E;
+    g.cached = std::min(g.nv, (Ra <= kClWide ? kClCache : kClCacheMany) / vec);
+    cfg.dynamicSmemBytes = static_cast<size_t>(g.cached) * vec;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    MLFMA_CUDA(cudaLaunchKernelEx(&cfg, kernel, g));
+  };
+  const long long rows = (g.n + kClBlocks * kClThreads - 1) / (kClBlocks * kClThreads);
+  if (rows <= 1)
+    go(gs_cluster_kernel<1, kStep>, 1);
+  else
+    go(gs_cluster_kernel<kClRows, kStep>, kClRows);
+}
+
+// Whether the current device can hold a cluster of kClBlocks blocks (a whole
+// B200 can; a partition of one may not).
+inline bool clusters_fit() {
+  auto* kernel = gs_cluster_kernel<kClRows, true>;
+  MLFMA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  MLFMA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClCache));
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {kClBlocks, 1, 1};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kClBlocks);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = kClCache;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return fit > 0;
+}
+
 // Device work arrays owned by one solve.
 struct Work {
   std::vector<void*> owned;
@@ -550,6 +738,7 @@ struct Vec {
   double2* part;    // [part_count(n, R)]
   unsigned* count;  // [R], zero
   double2* h;       // [R][kLdh] reduced values
+  bool clusters;    // the device takes clusters of kClBlocks blocks (clusters_fit)
 
   dim3 grid(int Ra) const {
     return dim3(static_cast<unsigned>(std::max(1LL, std::min<long long>((n + kThreads - 1) / kThreads,
@@ -593,6 +782,14 @@ struct Vec {
       g.inner = *inner;
       g.step = nv - 1;
       g.hbase = h;
+    }
+    if (clusters && Ra <= kClMaxPositions && n <= kClBlocks * kClThreads * kClRows) {
+      g.pack = pack;
+      if (inner)
+        launch_gs_cluster<true>(g, Ra, s);
+      else
+        launch_gs_cluster<false>(g, Ra, s);
+      return;
     }
     launch_gs<false, true, kFinishNone>(g, Ra, s);
     g.hin = h;
@@ -668,6 +865,7 @@ inline Ops make_ops(W& g, cudaStream_t s, long long n) {
   o.n = n;
   o.part = g.get(part_count(n, 1));
   o.h = g.get(kLdh);
+  o.clusters = clusters_fit();
   o.count = reinterpret_cast<unsigned*>(g.get(1));
   MLFMA_CUDA(cudaMemsetAsync(o.count, 0, sizeof(double2), s));
   return o;

@@ -221,9 +221,9 @@ namespace {
 // zero, with the complex64 copy of Z_near (the outer flexible GMRES admits
 // any preconditioner; its operator and residuals stay at the solve's
 // precision). The inner Hessenberg matrix, rotations and triangular solve
-// stay on the GPU: the inner steps run without a host round trip, as four
-// launches each (near-field product, then the three of the Gram-Schmidt, the
-// last with the step's rotations). Buffers come from the caller's Work; the
+// stay on the GPU: the inner steps run without a host round trip, as two or
+// four launches each (near-field product, then the one or three of the
+// Gram-Schmidt, the last with the step's rotations). Buffers come from the caller's Work; the
 // reduction scratch is the caller's Ops.
 struct NearPrecond {
   Plan& P;

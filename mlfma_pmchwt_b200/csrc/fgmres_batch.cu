@@ -339,6 +339,7 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   ops.part = wk[kPart];
   ops.count = reinterpret_cast<unsigned*>(wk[kCount]);
   ops.h = wk[kH];
+  ops.clusters = blas1::clusters_fit();
   ops.P = &P;
   ops.alpha = reinterpret_cast<double*>(wk[kAlpha]);
   ops.mdev = reinterpret_cast<int*>(wk[kM]);

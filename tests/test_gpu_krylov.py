@@ -73,3 +73,24 @@ def test_lockstep_rows_per_thread(R):
     for j in {0, R // 2, R - 1}:
         x, _ = op.matrix_solver(B[j], inner_its=0, **kw)
         assert np.linalg.norm(X[j] - x) <= 1e-9 * np.linalg.norm(x)
+
+
+def test_inner_gmres_two_rows():
+    """As test_inner_gmres with two rows per thread of a cluster and a basis
+    larger than its shared memory (5 vectors)."""
+    test_inner_gmres(4, 12)
+
+
+@pytest.mark.parametrize("R", [1, 3])
+def test_lockstep_long_vectors(R):
+    """61,440 unknowns are past the clusters' range: 240 blocks of one row per
+    thread, at three systems two rows. The bound of test_lockstep_rows_per_thread;
+    one system against its own residual, which GMRES reports."""
+    op = MLFMM(M.icosphere(5, 2.6), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=0.25, device=0, tf_complex_argument=True)
+    B = np.stack([op.compute_v_pmchwt(*plane_wave(90.0 * (j % 2), 9.0 * j, 20.0)) for j in range(R)])
+    kw = dict(itr_max=5, mr=5, tol_abs=0.0, tol_rel=1e-12)
+    X, _ = op.matrix_solver_batch(B, inner_its=0, **kw)
+    for j in range(R):
+        x, res = op.matrix_solver(B[j], inner_its=0, **kw)
+        assert np.linalg.norm(X[j] - x) <= 1e-9 * np.linalg.norm(x)
+        assert np.linalg.norm(B[j] - op.apply_ax(x)) < np.linalg.norm(B[j])
