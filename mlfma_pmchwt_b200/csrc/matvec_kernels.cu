@@ -8,8 +8,8 @@
 //   m2l      translation over the interaction list   Code/ProcessMLFMM.h:112-147
 //   l2l      the parent's incoming pattern, shifted and anterpolated onto
 //            the child grid, added                    Code/ProcessMLFMM.h:152-202
-//   leaf_out receive-pattern testing of both media and the near-field rows,
-//            written once per unknown   Code/MLFMM.cpp:285-366
+//   near     the near-field rows, written once per unknown   Code/MLFMM.cpp:353-366
+//   leaf     receive-pattern testing of both media, added    Code/MLFMM.cpp:285-351
 // Every stage writes its output before anything accumulates into it (l2l adds
 // onto the Bm that m2l of the same level has just written), so no clearing
 // pass (Code/ProcessMLFMM.h:14-28) is needed.

@@ -160,7 +160,7 @@ struct ApplyGraph {
 constexpr size_t kMaxApplyGraphs = 16;
 
 // Per-apply CUDA events between stage groups, recorded on the launching
-// stream: [m1 agg | m1 up | m1 m2l | m1 l2l | m2 agg | m2 up | m2 m2l | m2 l2l | leaf_out].
+// stream: [m1 agg | m1 up | m1 m2l | m1 l2l | m2 agg | m2 up | m2 m2l | m2 l2l | near and leaf].
 constexpr int kStages = 5;
 struct StageProfiler {
   static constexpr int kEvents = 10;
