@@ -212,7 +212,9 @@ MLFMA_API int mlfma_profile_read(mlfma_plan* plan, double* stage_ms, int* applie
  *                  operand splitting, boxes of at most 64 RWGs).
  *   "batch_tree.variant" (the batched complex64 apply only) 0 = the tree
  *                  passes of each right-hand side in turn; 1 = every level
- *                  once for all right-hand sides on slot-major arrays (default).
+ *                  once for all right-hand sides on slot-major arrays, for
+ *                  trees of up to 116 MB per right-hand side; above, as 0
+ *                  (default).
  *   "leaf.variant" 0 = the near-field product right before the leaf testing
  *                  kernel, which adds the far field (default); 1 = the near-
  *                  field product on its own stream from the start of the apply

@@ -144,7 +144,7 @@ struct Tuning {
   int batch_tc = 0;            // batched complex64 leaf aggregation and far-field testing: 0 FP32 on the CUDA
                                //    cores; 1 tcgen05 (3xTF32 split, TMEM accumulators)
   int batch_tree = 1;          // batched complex64 tree passes: 0 one slot after another; 1 every level
-                               //    once for all slots (slot-major arrays)
+                               //    once for all slots (slot-major arrays) where a slot's tree is small
   int leaf_variant = 0;        // 0: near field before the leaf kernel, which adds the far field; 1: near field on its own
                                //    stream from the start of the apply, the leaf kernel adds the far field
   int graph = 1;               // 1: capture each apply (per x, w, stream and precision) as a CUDA

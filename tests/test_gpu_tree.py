@@ -69,3 +69,22 @@ def test_tree_levels(body):
             _close(B[l], want)
     assert odd == {0, 1} or body != "deep"
     assert single or body != "fine grids"
+
+
+@pytest.mark.parametrize("R", [1, 3])
+def test_batched_large_tree(R):
+    """Trees above 116 MB per right-hand side run slot after slot. Rows against
+    the FP64 operator: an entry is a sum of ~1e4 complex64 products taken in
+    chunks, each entry rounded to 6e-8, so 1e-6 of the row's norm is allowed."""
+    torch = pytest.importorskip("torch")
+    op = MLFMM(M.icosphere(5, 2.5), freq=3e8, eps_r=4.0, leaf_coeff=0.25, device=0, precision="mixed")
+    levels = op.max_level - 1
+    assert sum(op.info.boxes[l] * 96 * (op.info.K_k1[l] + op.info.K_k2[l]) for l in range(levels)) > 116 << 20
+    X = torch.from_numpy(np.stack([M.unit_disk_vector(op.n, 40 + j) for j in range(R)])).cuda()
+    W = torch.full_like(X, float("nan"))
+    torch.cuda.synchronize()
+    op.apply_batch_mixed_device(R, X.data_ptr(), W.data_ptr())
+    torch.cuda.synchronize()
+    for x, w in zip(X.cpu().numpy(), W.cpu().numpy()):
+        ref = op.apply_ax(x)
+        assert np.linalg.norm(w - ref) <= 1e-6 * np.linalg.norm(ref)
