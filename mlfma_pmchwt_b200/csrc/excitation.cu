@@ -41,6 +41,7 @@ struct Geo {
   const int* vneg;
   const double* len;
   int nq, N;
+  int skew;  // the barycentric coordinates of some point do not add up to 1
   double l1[16], l2[16], l3[16], w[16];
   double2 k1;
 };
@@ -61,6 +62,9 @@ Geo geo(const Plan& P) {
     g.l2[i] = P.quad.l2[i];
     g.l3[i] = P.quad.l3[i];
     g.w[i] = P.quad.w[i];
+    // the rules are tabulated to 15 digits (sums within 1.1e-15 of 1), the
+    // centroid of the rules of 1 and 4 points to 12 (1e-12)
+    if (std::abs(1.0 - g.l1[i] - g.l2[i] - g.l3[i]) > 4e-15) g.skew = 1;
   }
   g.k1 = make_double2(P.k1.real(), P.k1.imag());
   return g;
@@ -177,8 +181,11 @@ __device__ __forceinline__ void transverse(const double r[3], double u[3], doubl
 // then rho = sum_j l_j (v_j - v_free). Phases up to 1 rad from the centroid
 // (vertices within 0.16 wavelengths) and a real k1 take the series instead
 // of a sine, a cosine and an exponential per point: 7 points cost a third.
-__device__ __forceinline__ void far_moment(const Geo& g, int m, const double r[3], const double u[3],
-                                           const double v[3], double2& Au, double2& Av) {
+// All of that needs coordinates that add up to 1: with the 1e-12 that 12-digit
+// centroids miss, p and rho would be off by 1e-12 times the distance from the
+// origin.
+__device__ __forceinline__ void far_moment_vertices(const Geo& g, int m, const double r[3], const double u[3],
+                                                    const double v[3], double2& Au, double2& Av) {
   Au = Av = c2(0.0, 0.0);
   const double ln = g.len[m];
 #pragma unroll 1
@@ -231,6 +238,33 @@ __device__ __forceinline__ void far_moment(const Geo& g, int m, const double r[3
   }
 }
 
+// The moment point by point, as the rule gives the points.
+__device__ __forceinline__ void far_moment_points(const Geo& g, int m, const double r[3], const double u[3],
+                                                  const double v[3], double2& Au, double2& Av) {
+  Au = Av = c2(0.0, 0.0);
+  const double ln = g.len[m];
+  for (int i = 0; i < g.nq; ++i) {
+    for (int side = 0; side < 2; ++side) {
+      double p[3], rho[3];
+      rwg_point(g, m, side, i, p, rho);
+      const double t = p[0] * r[0] + p[1] * r[1] + p[2] * r[2];
+      const double2 e = cscale(cexp(make_double2(-g.k1.y * t, g.k1.x * t)), ln * g.w[i]);
+      Au = cfmas(rho[0] * u[0] + rho[1] * u[1] + rho[2] * u[2], e, Au);
+      Av = cfmas(rho[0] * v[0] + rho[1] * v[1] + rho[2] * v[2], e, Av);
+    }
+  }
+}
+
+// kSkew: a rule whose coordinates miss 1 (it has at most four points)
+template <bool kSkew>
+__device__ __forceinline__ void far_moment(const Geo& g, int m, const double r[3], const double u[3],
+                                           const double v[3], double2& Au, double2& Av) {
+  if constexpr (kSkew)
+    far_moment_points(g, m, r, u, v, Au, Av);
+  else
+    far_moment_vertices(g, m, r, u, v, Au, Av);
+}
+
 struct FarBatchArg {
   Geo g;
   double dir[kFarChunk][3];
@@ -250,6 +284,7 @@ struct FarBatchArg {
 // and 0.31 ms of sums at the FP64 rate. With a block per (angle, 4
 // solutions), which formed the factors once per 4 solutions from 14 sincos
 // and exp each, that call took 12.3 ms; now 1.5 ms.
+template <bool kSkew>
 __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads, 1)
     far_batch_kernel(const __grid_constant__ FarBatchArg a) {
   __shared__ double2 A[kFarAngles][2][kFarRwgs];
@@ -283,7 +318,7 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
         if (m < g.N && t < na) {
           double u[3], v[3];
           transverse(a.dir[ang0 + t], u, v);
-          far_moment(g, m, a.dir[ang0 + t], u, v, Au, Av);
+          far_moment<kSkew>(g, m, a.dir[ang0 + t], u, v, Au, Av);
         }
         A[t][0][q] = Au;
         A[t][1][q] = Av;
@@ -358,6 +393,7 @@ struct FarMonoArg {
 };
 
 // block per solution of the chunk, observed in its own direction
+template <bool kSkew>
 __global__ void __launch_bounds__(256) far_mono_kernel(const __grid_constant__ FarMonoArg a) {
   __shared__ double2 sh[8];
   const Geo& g = a.g;
@@ -369,7 +405,7 @@ __global__ void __launch_bounds__(256) far_mono_kernel(const __grid_constant__ F
   double2 su = c2(0.0, 0.0), sv = c2(0.0, 0.0);
   for (int m = threadIdx.x; m < g.N; m += blockDim.x) {
     double2 Au, Av;
-    far_moment(g, m, r, u, v, Au, Av);
+    far_moment<kSkew>(g, m, r, u, v, Au, Av);
     const double2 IJ = I[m], IM = I[g.N + m];
     su = csub(csub(su, cmul(Av, IM)), cmul(Au, IJ));
     sv = csub(cadd(sv, cmul(Au, IM)), cmul(Av, IJ));
@@ -429,7 +465,10 @@ void rcs_pmchwt_batch(Plan& P, int R, const double2* I_dev, int n_angles, const 
     a.angle0 = c0;
     for (int q = 0; q < a.n_angles; ++q) direction(theta_deg[c0 + q], phi_deg[c0 + q], a.dir[q]);
     const dim3 grid((a.n_angles + kFarAngles - 1) / kFarAngles, (R + kFarSols - 1) / kFarSols, kFarSlices);
-    far_batch_kernel<<<grid, kFarThreads, 0, s>>>(a);
+    if (a.g.skew)
+      far_batch_kernel<true><<<grid, kFarThreads, 0, s>>>(a);
+    else
+      far_batch_kernel<false><<<grid, kFarThreads, 0, s>>>(a);
     MLFMA_CUDA(cudaGetLastError());
   }
 }
@@ -446,7 +485,10 @@ void rcs_pmchwt_mono(Plan& P, int R, const double2* I_dev, const double* theta_d
     const int nr = std::min(kFarChunk, R - c0);
     a.r0 = c0;
     for (int q = 0; q < nr; ++q) direction(theta_deg[c0 + q], phi_deg[c0 + q], a.dir[q]);
-    far_mono_kernel<<<nr, 256, 0, s>>>(a);
+    if (a.g.skew)
+      far_mono_kernel<true><<<nr, 256, 0, s>>>(a);
+    else
+      far_mono_kernel<false><<<nr, 256, 0, s>>>(a);
     MLFMA_CUDA(cudaGetLastError());
   }
 }

@@ -1,6 +1,9 @@
 """The bistatic far-field kernel at the ends of its tiles (4 angles, pairs and
 32 solutions, 256 RWGs, 8 slices, 512 angles per launch) and for triangles
-wider than its phase series covers, against the single-solution entry point."""
+wider than its phase series covers, against the single-solution entry point;
+both batched far fields with every triangle rule on a body off the origin."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -29,3 +32,31 @@ def test_far_field_tiles(sub, radius, R, angles):
     for r in {0, R // 2, R - 1}:
         want, _ = op.calculate_rcs_pmchwt(I[r], th, ph)
         np.testing.assert_allclose(got[r], want, rtol=0, atol=1e-12 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("rule", [1, 3, 4, 6, 7, 12, 13, 16])
+def test_far_field_rules(rule):
+    """A body 20 wavelengths from the origin: phases of up to 130 rad, each
+    rounded to ~4 eps of that (1.2e-13), RWG vectors of a tenth of a
+    wavelength as differences of positions (3e-14): 1e-12 of the largest field.
+    Coordinates of a point that miss 1 by 1e-12 (the centroid of the rules of 1
+    and 4 points) must not move the points: that is 1e-10 here."""
+    torch = pytest.importorskip("torch")
+    m = M.icosphere(2, 0.5)
+    m = dataclasses.replace(m, points=m.points + np.array([12.0, -12.0, 11.0]))
+    op = MLFMM(m, freq=3e8, eps_r=2.5, leaf_coeff=0.25, gauss_points=rule, device=0)
+    g = np.random.default_rng(rule)
+    I = g.standard_normal((3, op.n)) + 1j * g.standard_normal((3, op.n))
+    th, ph = g.uniform(0, 180, 3), g.uniform(0, 360, 3)
+    Id = torch.from_numpy(I).cuda()
+    F = torch.full((3, 3, 3), float("nan"), dtype=torch.complex128, device="cuda")
+    Fm = torch.full((3, 3), float("nan"), dtype=torch.complex128, device="cuda")
+    torch.cuda.synchronize()
+    op.calculate_rcs_batch_device(3, Id.data_ptr(), th, ph, F.data_ptr())
+    op.calculate_rcs_mono_device(3, Id.data_ptr(), th, ph, Fm.data_ptr())
+    torch.cuda.synchronize()
+    got, mono = F.cpu().numpy(), Fm.cpu().numpy()
+    for r in range(3):
+        want, _ = op.calculate_rcs_pmchwt(I[r], th, ph)
+        np.testing.assert_allclose(got[r], want, rtol=0, atol=1e-12 * np.abs(want).max())
+        np.testing.assert_allclose(mono[r], want[r], rtol=0, atol=1e-12 * np.abs(want).max())
