@@ -15,6 +15,7 @@
 
 #include <cmath>
 #include <stdexcept>
+#include <type_traits>
 
 #include "cplx.cuh"
 #include "reduce.cuh"
@@ -277,13 +278,16 @@ struct FarBatchArg {
 // (kFarAngles angles, kFarSols solutions), each block over a slice of the RWGs.
 // A block forms the moments of kFarRwgs RWGs at its angles once, in shared
 // memory, for all its solutions; a warp then sums 2 solutions x 4 angles
-// over 32 RWGs at a time (with fewer than 16 pairs of solutions the warps
-// share the RWGs). The blocks' sums meet in distributed shared memory, in
-// rank order.
+// over 32 RWGs at a time (with 8 pairs of solutions or fewer, 2 angles or 1).
+// The blocks' sums meet in distributed shared memory, in rank order. A sum's
+// order is the same whatever else is in the call, so a solution's field is too.
 // FP64-bound: 361 angles x 32 solutions x 30,720 RWGs are ~0.35 ms of moments
 // and 0.31 ms of sums at the FP64 rate. With a block per (angle, 4
 // solutions), which formed the factors once per 4 solutions from 14 sincos
-// and exp each, that call took 12.3 ms; now 1.5 ms.
+// and exp each, that call took 12.3 ms; now 1.7 ms (alone). Few solutions: with
+// warps that shared the RWGs of a pair instead of its angles, 361 angles at
+// 3,840 unknowns took 115 us for one solution and 142 for 16, now 101 and 129;
+// at 61,440 unknowns 1,056 and 1,385, now 1,078 and 1,357.
 template <bool kSkew>
 __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads, 1)
     far_batch_kernel(const __grid_constant__ FarBatchArg a) {
@@ -294,9 +298,10 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
   const int r0 = blockIdx.y * kFarSols, nr = min(kFarSols, a.R - r0);
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   constexpr int kW = kFarThreads / 32;
-  const int npair = (nr + 1) / 2, nsub = kW / npair;
-  const int pair = wp % npair, sub = wp / npair;
-  const bool working = sub < nsub;
+  const int npair = (nr + 1) / 2;
+  const int per = 4 * npair <= kW ? 1 : 2 * npair <= kW ? 2 : kFarAngles;  // angles of a warp
+  const int pair = wp % npair, t0 = wp / npair * per;
+  const bool working = t0 < kFarAngles;
   const bool two = 2 * pair + 1 < nr;
   const size_t n = 2 * static_cast<size_t>(g.N);
   const double2* I0 = a.I + (r0 + 2 * pair) * n;
@@ -306,6 +311,24 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
   for (int q = 0; q < 2; ++q)
 #pragma unroll
     for (int t = 0; t < kFarAngles; ++t) acc[q][t][0] = acc[q][t][1] = c2(0.0, 0.0);
+  auto add = [&](int m0, auto angles) {
+    constexpr int kA = decltype(angles)::value, kAhead = 8 / kA;
+    const int first = kA == kFarAngles ? 0 : t0;
+#pragma unroll kAhead
+    for (int c = 0; c < kFarRwgs / 32; ++c) {
+      const int q = 32 * c + lane, m = min(m0 + q, g.N - 1);  // moments beyond N are zero
+      const double2 J0 = __ldg(I0 + m), M0 = __ldg(I0 + g.N + m);
+      const double2 J1 = __ldg(I1 + m), M1 = __ldg(I1 + g.N + m);
+#pragma unroll
+      for (int t = 0; t < kA; ++t) {
+        const double2 u = A[first + t][0][q], v = A[first + t][1][q], mu = cneg(u), mv = cneg(v);
+        acc[0][t][0] = cfma(mv, M0, cfma(mu, J0, acc[0][t][0]));
+        acc[0][t][1] = cfma(u, M0, cfma(mv, J0, acc[0][t][1]));
+        acc[1][t][0] = cfma(mv, M1, cfma(mu, J1, acc[1][t][0]));
+        acc[1][t][1] = cfma(u, M1, cfma(mv, J1, acc[1][t][1]));
+      }
+    }
+  };
   const int tiles = (g.N + kFarRwgs - 1) / kFarRwgs;
   for (int tile = blockIdx.z; tile < tiles; tile += kFarSlices) {
     const int m0 = tile * kFarRwgs;
@@ -325,22 +348,13 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
       }
     }
     __syncthreads();
-    if (working) {
-#pragma unroll 2
-      for (int c = sub; c < kFarRwgs / 32; c += nsub) {
-        const int q = 32 * c + lane, m = min(m0 + q, g.N - 1);  // moments beyond N are zero
-        const double2 J0 = __ldg(I0 + m), M0 = __ldg(I0 + g.N + m);
-        const double2 J1 = __ldg(I1 + m), M1 = __ldg(I1 + g.N + m);
-#pragma unroll
-        for (int t = 0; t < kFarAngles; ++t) {
-          const double2 u = A[t][0][q], v = A[t][1][q], mu = cneg(u), mv = cneg(v);
-          acc[0][t][0] = cfma(mv, M0, cfma(mu, J0, acc[0][t][0]));
-          acc[0][t][1] = cfma(u, M0, cfma(mv, J0, acc[0][t][1]));
-          acc[1][t][0] = cfma(mv, M1, cfma(mu, J1, acc[1][t][0]));
-          acc[1][t][1] = cfma(u, M1, cfma(mv, J1, acc[1][t][1]));
-        }
-      }
-    }
+    if (!working) continue;
+    if (per == 1)
+      add(m0, std::integral_constant<int, 1>{});
+    else if (per == 2)
+      add(m0, std::integral_constant<int, 2>{});
+    else
+      add(m0, std::integral_constant<int, kFarAngles>{});
   }
   __syncthreads();
   double2* red = &A[0][0][0];  // [kW][2 x kFarAngles x 2]
@@ -351,15 +365,14 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
     for (int t = 0; t < kFarAngles; ++t)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
+        if (t >= per) continue;
         const double2 v = blas1::warp_sum2(acc[q][t][c]);
         if (lane == 0) red[wp * kPer + (q * kFarAngles + t) * 2 + c] = v;
       }
   __syncthreads();
   for (int i = threadIdx.x; i < npair * kPer; i += kFarThreads) {
-    const int p = i / kPer, e = i - p * kPer;
-    double2 v = c2(0.0, 0.0);
-    for (int q = 0; q < nsub; ++q) v = cadd(v, red[(q * npair + p) * kPer + e]);
-    sums[i] = v;
+    const int p = i / kPer, e = i - p * kPer, t = e / 2 % kFarAngles;
+    sums[i] = red[(t / per * npair + p) * kPer + e - 2 * (t - t % per)];
   }
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();

@@ -60,3 +60,27 @@ def test_far_field_rules(rule):
         want, _ = op.calculate_rcs_pmchwt(I[r], th, ph)
         np.testing.assert_allclose(got[r], want, rtol=0, atol=1e-12 * np.abs(want).max())
         np.testing.assert_allclose(mono[r], want[r], rtol=0, atol=1e-12 * np.abs(want).max())
+
+
+def test_far_field_of_a_solution_alone_and_among_others():
+    """A solution's field has the same bits whatever number of solutions and
+    angles share the call (the kernel splits its sums by both)."""
+    torch = pytest.importorskip("torch")
+    op = MLFMM(M.icosphere(3, 1.0), freq=3e8, eps_r=2.5, leaf_coeff=0.25, device=0)
+    g = np.random.default_rng(5)
+    I = torch.from_numpy(g.standard_normal((33, op.n)) + 1j * g.standard_normal((33, op.n))).cuda()
+    th, ph = g.uniform(0, 180, 9), g.uniform(0, 360, 9)
+
+    def field(lo, hi, n):
+        F = torch.full((hi - lo, n, 3), float("nan"), dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        op.calculate_rcs_batch_device(hi - lo, I[lo:hi].data_ptr(), th[:n], ph[:n], F.data_ptr())
+        torch.cuda.synchronize()
+        return F.cpu().numpy()
+
+    every = field(0, 33, 9)
+    for r in (0, 1, 32):
+        np.testing.assert_array_equal(field(r, r + 1, 9)[0], every[r])
+        np.testing.assert_array_equal(field(r, r + 1, 3)[0], every[r, :3])
+    for R in (2, 7, 8, 9, 16, 17, 32):
+        np.testing.assert_array_equal(field(0, R, 9), every[:R])
