@@ -2016,7 +2016,8 @@ void apply_direct(Plan& P, const double2* x, double2* w, cudaStream_t s) {
     if (ev) {  // one stage after the other, for the stage events
       launch_up(P, m, v, s);
       MLFMA_CUDA(cudaEventRecord(ev[2 + 4 * m], s));
-      launch_m2l(P, m, v, s, 2, L);
+      launch_m2l(P, m, v, s, L, L);  // the launches of the other branch: their sizes choose the sums' order
+      launch_m2l(P, m, v, s, 2, L - 1);
       MLFMA_CUDA(cudaEventRecord(ev[3 + 4 * m], s));
       launch_l2l(P, m, v, s);
       MLFMA_CUDA(cudaEventRecord(ev[4 + 4 * m], s));

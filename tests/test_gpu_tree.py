@@ -71,6 +71,20 @@ def test_tree_levels(body):
     assert single or body != "fine grids"
 
 
+@pytest.mark.parametrize("body", BODIES)
+def test_profiled_apply_has_the_same_bits(body):
+    """Stage timing runs one stage after another, with the same launches: the
+    translation's sums follow the number of warps of a launch."""
+    op = MLFMM(freq=3e8, device=0, **BODIES[body]())
+    x = M.unit_disk_vector(op.n, 4)
+    plain = op.apply_ax(x)
+    op.profile(True)
+    timed = op.apply_ax(x)
+    assert op.stage_times()[1] == 1
+    op.profile(False)
+    np.testing.assert_array_equal(timed, plain)
+
+
 @pytest.mark.parametrize("R", [1, 3])
 def test_batched_large_tree(R):
     """Trees above 116 MB per right-hand side run slot after slot. Rows against
