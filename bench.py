@@ -629,8 +629,7 @@ def batched_apply_study(args, local: int, wl: dict) -> dict:
     sphere (mixed-precision plan): per-batch CUDA-event time with the leaf
     aggregation and far-field testing on the tensor cores (batch_tc.variant
     1) and on the CUDA cores (0), with the tree passes one slot after another
-    (batch_tree.variant 0) and as the size chooses (1: once per level for all
-    slots up to 116 MB of tree per slot), against 16
+    (batch_tree.variant 0) and once per level for all slots (1), against 16
     single complex64 applies, and the rows' relative difference from the FP64
     operator."""
     import torch
@@ -663,7 +662,7 @@ def batched_apply_study(args, local: int, wl: dict) -> dict:
             timed(lambda: op.apply_batch_mixed_device(R, X.data_ptr(), W.data_ptr(), sp), 3), 3)
     op.set_tuning("batch_tc.variant", 0)
     tree_keep = op.get_tuning("batch_tree.variant")
-    for v, key in ((0, "cuda_cores_tree_slot_by_slot"), (1, "cuda_cores_tree_by_size")):
+    for v, key in ((0, "cuda_cores_tree_slot_by_slot"), (1, "cuda_cores_tree_slot_grid")):
         op.set_tuning("batch_tree.variant", v)
         out["ms_per_batch"][key] = round(
             timed(lambda: op.apply_batch_mixed_device(R, X.data_ptr(), W.data_ptr(), sp), 3), 3)

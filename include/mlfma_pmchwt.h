@@ -211,10 +211,10 @@ MLFMA_API int mlfma_profile_read(mlfma_plan* plan, double* stage_ms, int* applie
  *                  1 = on the tensor cores (tcgen05 kind::tf32 with high/low
  *                  operand splitting, boxes of at most 64 RWGs).
  *   "batch_tree.variant" (the batched complex64 apply only) 0 = the tree
- *                  passes of each right-hand side in turn; 1 = every level
- *                  once for all right-hand sides on slot-major arrays, for
- *                  trees of up to 116 MB per right-hand side; above, as 0
- *                  (default).
+ *                  passes of each right-hand side in turn (default of plans
+ *                  with more than 116 MB of tree per right-hand side); 1 =
+ *                  every level once for all right-hand sides on slot-major
+ *                  arrays (default of the others).
  *   "leaf.variant" 0 = the near-field product right before the leaf testing
  *                  kernel, which adds the far field (default); 1 = the near-
  *                  field product on its own stream from the start of the apply

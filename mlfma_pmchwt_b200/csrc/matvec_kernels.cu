@@ -1905,24 +1905,6 @@ void apply_fixed(Plan& P, const double2* x, double2* w, cudaStream_t s) {
   MLFMA_CUDA(cudaGetLastError());
 }
 
-// Up to this size of a slot's tree arrays every level runs once for all slots;
-// above it the slots run one after another. A launch over all slots of a large
-// tree fills the GPU by itself, so the interpolation (bound by L1), the leaf
-// translation (instruction issue) and the anterpolation (latency) of both media
-// follow one another; the launches of single slots overlap: at 16 x 61,440
-// unknowns 13.9 ms of kernels in 11.2 ms, against 12.0 in 11.7. One B200, 16
-// slots, all at once / one after another: 15,360 unknowns (58 MB) 2.43 / 2.74 ms,
-// 24,000 (104 MB) 4.50 / 4.57, 34,560 (129 MB) 5.69 / 5.59, 61,440 (271 MB)
-// 11.73 / 11.21, 121,500 (539 MB) 24.20 / 23.10; at 2 and 4 slots the sides
-// change at the same size.
-constexpr size_t kSlotGridBytes = size_t{116} << 20;
-size_t slot_tree_bytes(const Plan& P) {
-  size_t n = 0;
-  for (int m = 0; m < 2; ++m)
-    for (int l = 2; l <= P.maxL; ++l) n += static_cast<size_t>(P.lv[l].B) * 12 * P.ml[m][l].K * sizeof(float2);
-  return n;
-}
-
 // The batched complex64 apply: leaf stages of leaf_batch.cu (or, with
 // batch_tc.variant 1, of agg_tc.cu), tree passes over all slots or slot by
 // slot, near-field rows by the tiled product.
@@ -1966,7 +1948,7 @@ void apply_batch_slots(Plan& P, int R, const double2* X, long long ldx, double2*
       launch_agg_slots(P, ag, s);
     {
       MediumStreams ms(P, s, true);
-      if (P.tuning.batch_tree == 1 && slot_tree_bytes(P) <= kSlotGridBytes) {
+      if (P.tuning.batch_tree == 1) {
         for (int m = 0; m < 2; ++m)
           tree_pass_slots(P, m, rn, ms.of(m), P.stream_leaf[m], P.ev_agg[m], P.ev_leaf[m]);
       } else {
@@ -2050,6 +2032,24 @@ void apply_direct(Plan& P, const double2* x, double2* w, cudaStream_t s) {
   launch_leaf(P, a, s);
   MLFMA_CUDA(cudaGetLastError());
   if (ev) MLFMA_CUDA(cudaEventRecord(ev[9], s));
+}
+
+// The default of batch_tree: up to this size of a slot's tree arrays every level
+// runs once for all slots (1), above it the slots run one after another (0). A
+// launch over all slots of a large tree fills the GPU by itself, so the
+// interpolation (bound by L1), the leaf translation (instruction issue) and the
+// anterpolation (latency) of both media follow one another; the launches of
+// single slots overlap: at 16 x 61,440 unknowns 13.9 ms of kernels in 11.2 ms,
+// against 12.0 in 11.7. One B200, 16 slots, all at once / one after another:
+// 15,360 unknowns (58 MB) 2.43 / 2.74 ms, 24,000 (104 MB) 4.50 / 4.57, 34,560
+// (129 MB) 5.69 / 5.59, 61,440 (271 MB) 11.73 / 11.21, 121,500 (539 MB) 24.20 /
+// 23.10; at 2 and 4 slots the sides change at the same size.
+constexpr size_t kSlotGridBytes = size_t{116} << 20;
+int default_batch_tree(const Plan& P) {
+  size_t n = 0;
+  for (int m = 0; m < 2; ++m)
+    for (int l = 2; l <= P.maxL; ++l) n += static_cast<size_t>(P.lv[l].B) * 12 * P.ml[m][l].K * sizeof(float2);
+  return n <= kSlotGridBytes ? 1 : 0;
 }
 
 void reserve_batch_staging(Plan& P) {

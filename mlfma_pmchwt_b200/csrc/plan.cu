@@ -663,6 +663,7 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
       }
     }
   }
+  if (P->precision == 1) P->tuning.batch_tree = default_batch_tree(*P);
   // complex64 copy of the near field: the flexible GMRES preconditioner's
   // products (any plan) and the mixed operator's near rows
   {

@@ -144,7 +144,8 @@ struct Tuning {
   int batch_tc = 0;            // batched complex64 leaf aggregation and far-field testing: 0 FP32 on the CUDA
                                //    cores; 1 tcgen05 (3xTF32 split, TMEM accumulators)
   int batch_tree = 1;          // batched complex64 tree passes: 0 one slot after another; 1 every level
-                               //    once for all slots (slot-major arrays) where a slot's tree is small
+                               //    once for all slots (slot-major arrays); a mixed plan starts with
+                               //    default_batch_tree
   int leaf_variant = 0;        // 0: near field before the leaf kernel, which adds the far field; 1: near field on its own
                                //    stream from the start of the apply, the leaf kernel adds the far field
   int graph = 1;               // 1: capture each apply (per x, w, stream and precision) as a CUDA
@@ -394,6 +395,8 @@ void fetch_device_status(Plan& P, cudaStream_t s);
 // apply's result is incomplete), naming the kernels.
 void raise_device_status(const Plan& P);
 
+// The faster of the two batch_tree variants at the plan's size.
+int default_batch_tree(const Plan& P);
 // Allocates the complex64 slot tree of a mixed plan (no-op otherwise).
 void reserve_batch(Plan& P);
 // Allocates d_xb / d_wb (kBatchSlots vectors each), the staging of

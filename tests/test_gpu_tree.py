@@ -102,3 +102,28 @@ def test_batched_large_tree(R):
     for x, w in zip(X.cpu().numpy(), W.cpu().numpy()):
         ref = op.apply_ax(x)
         assert np.linalg.norm(w - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("sub,radius,default", [(3, 1.0, 1), (5, 2.5, 0)])
+def test_batch_tree_variant_selects_the_passes(sub, radius, default):
+    """batch_tree.variant starts with the size's choice, and each value runs
+    what it names at every size: one anterpolation launch per level pair and
+    medium, for each of the three rows (0) or once for all (1)."""
+    torch = pytest.importorskip("torch")
+    from torch.profiler import ProfilerActivity, profile
+    op = MLFMM(M.icosphere(sub, radius), freq=3e8, eps_r=4.0, leaf_coeff=0.25, device=0, precision="mixed")
+    assert op.get_tuning("batch_tree.variant") == default
+    X = torch.from_numpy(np.stack([M.unit_disk_vector(op.n, 40 + j) for j in range(3)])).cuda()
+    rows = []
+    for v in (0, 1):
+        op.set_tuning("batch_tree.variant", v)
+        assert op.get_tuning("batch_tree.variant") == v
+        W = torch.full_like(X, float("nan"))
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            op.apply_batch_mixed_device(3, X.data_ptr(), W.data_ptr())
+            torch.cuda.synchronize()
+        launches = sum("l2l_sep_kernel" in e.name for e in p.events())
+        assert launches == 2 * (op.max_level - 2) * (1 if v else 3)
+        rows.append(W.cpu().numpy())
+    np.testing.assert_allclose(rows[1], rows[0], rtol=0, atol=1e-12 * np.abs(rows[0]).max())
