@@ -161,7 +161,8 @@ MLFMA_API int mlfma_apply_batch(mlfma_plan* plan, int n, int R, const double* x,
  * tuning key "batch_tc.variant" is 1 and every leaf box holds at most 64 RWGs,
  * else in FP32 on the CUDA cores. The first call on a plan allocates the tree
  * arrays of 16 right-hand sides (about 2 x boxes x 6 x (K1+K2) x 8 bytes per
- * level each). No counterpart in the reference. */
+ * level each): the leaf level's, and with "batch_tree.variant" 1 those of the
+ * levels above. No counterpart in the reference. */
 MLFMA_API int mlfma_apply_batch_mixed_device(mlfma_plan* plan, int n, int R, const void* x_dev, void* w_dev,
                                              void* stream);
 MLFMA_API int mlfma_apply_batch_device(mlfma_plan* plan, int n, int R, const void* x_dev, void* w_dev,
@@ -214,7 +215,8 @@ MLFMA_API int mlfma_profile_read(mlfma_plan* plan, double* stage_ms, int* applie
  *                  passes of each right-hand side in turn (default of plans
  *                  with more than 116 MB of tree per right-hand side); 1 =
  *                  every level once for all right-hand sides on slot-major
- *                  arrays (default of the others).
+ *                  arrays (default of the others). Setting 1 after a batched
+ *                  apply with 0 allocates the arrays above the leaf level.
  *   "leaf.variant" 0 = the near-field product right before the leaf testing
  *                  kernel, which adds the far field (default); 1 = the near-
  *                  field product on its own stream from the start of the apply

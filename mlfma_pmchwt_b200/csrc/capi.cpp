@@ -308,9 +308,28 @@ int mlfma_set_tuning(mlfma_plan* plan, const char* key, int value) {
   if (!k) return fail(MLFMA_ERR_ARG, std::string("unknown tuning key: ") + key);
   if (value < 0 || value >= k->count)
     return fail(MLFMA_ERR_ARG, std::string(key) + " must be in [0, " + std::to_string(k->count - 1) + "]");
-  plan->p->tuning.*(k->field) = value;
-  if (device_plan(plan)) mlfma::clear_graphs(*plan->p);
-  return MLFMA_OK;
+  mlfma::Plan& P = *plan->p;
+  if (!device_plan(plan)) {
+    P.tuning.*(k->field) = value;
+    return MLFMA_OK;
+  }
+  return guarded([&] {
+    const mlfma::Tuning before = P.tuning;
+    P.tuning.*(k->field) = value;
+    if (k->field == &mlfma::Tuning::batch_tree && !P.bS32[0].empty()) {
+      // a plan that has run a batched apply gets the slots that the new value
+      // needs here, so that its next one allocates nothing
+      try {
+        MLFMA_CUDA(cudaSetDevice(P.device));
+        mlfma::reserve_batch(P);
+      } catch (...) {
+        P.tuning = before;
+        throw;
+      }
+    }
+    mlfma::clear_graphs(P);
+    return MLFMA_OK;
+  });
 }
 
 int mlfma_get_tuning(const mlfma_plan* plan, const char* key) {

@@ -1839,6 +1839,7 @@ void tree_pass_slots(Plan& P, int m, int rn, cudaStream_t s, cudaStream_t sx, cu
                      cudaEvent_t ev_leaf) {
   using C = float2;
   const int L = P.maxL;
+  if (P.btS[m][2] == nullptr) throw std::runtime_error("batched apply: slots of the upper levels not reserved");
   auto stride = [&](int l) { return static_cast<long long>(P.lv[l].B) * 6 * P.ml[m][l].K; };
   auto translate = [&](int lo, int hi, cudaStream_t st) {
     if (lo > hi) return;
@@ -2061,27 +2062,30 @@ void reserve_batch_staging(Plan& P) {
 
 void reserve_batch(Plan& P) {
   const int L = P.maxL;
-  if (P.precision != 1 || !P.bS32[0].empty()) return;
-  // the complex64 tree of every slot at once, slot-major per level, and the
-  // near-field product's packed inputs, in one allocation
-  size_t total = 0;
+  if (P.precision != 1) return;
+  const bool leaf = P.bS32[0].empty();
+  const bool upper = P.tuning.batch_tree == 1 && L > 2 && P.btS[0][2] == nullptr;
+  if (!leaf && !upper) return;
+  // slot-major per level, and with the leaf level the near-field product's
+  // packed inputs, in one allocation
+  const int lo = upper ? 2 : L, hi = leaf ? L : L - 1;
+  auto count = [&](int m, int l) { return static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K; };
+  size_t total = leaf ? near_pack_values(P) : 0;
   for (int m = 0; m < 2; ++m)
-    for (int l = 2; l <= L; ++l) total += 2 * kBatchSlots * static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
-  float2* p = P.alloc<float2>(total + near_pack_values(P));
-  P.d_pack = p + total;
+    for (int l = lo; l <= hi; ++l) total += 2 * kBatchSlots * count(m, l);
+  float2* p = P.alloc<float2>(total);
   for (int m = 0; m < 2; ++m) {
-    for (int l = 2; l <= L; ++l) {
-      const size_t cnt = static_cast<size_t>(P.lv[l].B) * 6 * P.ml[m][l].K;
+    for (int l = lo; l <= hi; ++l) {
       P.btS[m][l] = p;
-      P.btB[m][l] = p + kBatchSlots * cnt;
-      p += 2 * kBatchSlots * cnt;
+      P.btB[m][l] = p + kBatchSlots * count(m, l);
+      p += 2 * kBatchSlots * count(m, l);
     }
-    const size_t cnt = static_cast<size_t>(P.lv[L].B) * 6 * P.ml[m][L].K;
-    for (int j = 0; j < kBatchSlots; ++j) {
-      P.bS32[m].push_back(P.btS[m][L] + j * cnt);
-      P.bB32[m].push_back(P.btB[m][L] + j * cnt);
+    for (int j = 0; leaf && j < kBatchSlots; ++j) {
+      P.bS32[m].push_back(P.btS[m][L] + j * count(m, L));
+      P.bB32[m].push_back(P.btB[m][L] + j * count(m, L));
     }
   }
+  if (leaf) P.d_pack = p;
 }
 
 // FP64: one captured apply per row. Sharing the leaf tables among rows saves

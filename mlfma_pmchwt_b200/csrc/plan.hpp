@@ -236,8 +236,8 @@ struct Plan {
   std::vector<float2*> bS32[2], bB32[2];
   // Complex64 tree arrays of all kBatchSlots right-hand-side slots (mixed
   // plans), per medium and level 2..maxLevel, slot-major and contiguous:
-  // [slot][B][6][K]. bS32 / bB32 point into the leaf level's arrays. The
-  // batched complex64 apply runs every tree pass once per level for all slots.
+  // [slot][B][6][K]. bS32 / bB32 point into the leaf level's arrays; the levels
+  // above are null until the passes over all slots (batch_tree 1) need them.
   float2* btS[2][16] = {};
   float2* btB[2][16] = {};
   float2* d_pack = nullptr;         // complex64 inputs of the batched near-field product, packed per RWG
@@ -397,7 +397,9 @@ void raise_device_status(const Plan& P);
 
 // The faster of the two batch_tree variants at the plan's size.
 int default_batch_tree(const Plan& P);
-// Allocates the complex64 slot tree of a mixed plan (no-op otherwise).
+// Allocates the slots of a mixed plan's batched complex64 apply that it does not
+// have yet (no-op otherwise): the leaf level's arrays, and with batch_tree 1
+// those of the levels above, which slot-after-slot passes do not touch.
 void reserve_batch(Plan& P);
 // Allocates d_xb / d_wb (kBatchSlots vectors each), the staging of
 // host-pointer batched applies and of the refinement's FP64 residuals.

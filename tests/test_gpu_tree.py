@@ -127,3 +127,31 @@ def test_batch_tree_variant_selects_the_passes(sub, radius, default):
         assert launches == 2 * (op.max_level - 2) * (1 if v else 3)
         rows.append(W.cpu().numpy())
     np.testing.assert_allclose(rows[1], rows[0], rtol=0, atol=1e-12 * np.abs(rows[0]).max())
+
+
+def test_batched_apply_reserves_what_its_passes_use():
+    """A first batched apply slot after slot takes the leaf level's arrays of 16
+    slots; selecting the passes over all slots takes those of the levels above,
+    at once, and no more later. 128 MB beside that for the right-hand sides,
+    the heap's chunk and the loading of kernels."""
+    torch = pytest.importorskip("torch")
+    op = MLFMM(M.icosphere(5, 2.5), freq=3e8, eps_r=4.0, leaf_coeff=0.25, device=0, precision="mixed")
+    level = [16 * 96 * op.info.boxes[l] * (op.info.K_k1[l] + op.info.K_k2[l]) for l in range(op.max_level - 1)]
+    leaf, upper = level[-1], sum(level[:-1])
+    assert op.get_tuning("batch_tree.variant") == 0 and upper > 1 << 30
+    X = torch.from_numpy(np.stack([M.unit_disk_vector(op.n, j) for j in range(2)])).cuda()
+    W = torch.empty_like(X)
+    torch.cuda.synchronize()
+    free = [torch.cuda.mem_get_info()[0]]
+
+    def step(what):
+        what()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+        return free[-2] - free[-1]
+
+    run = lambda: op.apply_batch_mixed_device(2, X.data_ptr(), W.data_ptr())
+    assert leaf <= step(run) <= leaf + (128 << 20)
+    assert upper <= step(lambda: op.set_tuning("batch_tree.variant", 1)) <= upper + (128 << 20)
+    assert step(run) <= 128 << 20
+    assert step(lambda: [op.set_tuning("batch_tree.variant", v) for v in (0, 1)]) == 0
