@@ -9,6 +9,8 @@
 #include <limits>
 #include <map>
 #include <sstream>
+#include <stdexcept>
+#include <string>
 #include <unordered_map>
 
 namespace mlfma {
@@ -591,6 +593,11 @@ double lagrange(double x0, double x1, double x2, double x3) {
 }  // namespace
 
 Interp build_interp(const Grid& parent, const Grid& child) {
+  // three-point stencils need three nodes (the reference's search returns node
+  // -1 below that, Code/AlgoMLFMM.h:141-189)
+  if (child.nth < 3)
+    throw std::invalid_argument("leaf boxes of " + std::to_string(child.nth) +
+                                " theta directions are too small to interpolate: take a larger leaf_coeff");
   Interp it;
   it.tidx.resize(3 * parent.nth);
   it.lt.resize(3 * parent.nth);

@@ -82,6 +82,22 @@ def test_host_only_plan_refuses_compute():
 
 
 @needs_lib
+@pytest.mark.parametrize("leaf,radius", [(0.002, 0.01), (0.001, 0.01)])
+def test_leaf_boxes_too_small_to_interpolate(leaf, radius):
+    """Boxes of 0.002 wavelengths have two theta directions; a three-point
+    stencil on them would hold node -1. Without interpolation (two levels), and
+    from three directions on, such boxes are taken."""
+    from mlfma_pmchwt_b200 import MLFMM, MlfmaError
+    from mlfma_pmchwt_b200 import mesh as M
+    with pytest.raises(MlfmaError) as e:
+        MLFMM(M.icosphere(2, radius), freq=FREQ, eps_r=4.0, leaf_coeff=leaf, device=-1)
+    assert e.value.code == -1 and "leaf_coeff" in str(e.value)
+    flat = MLFMM(M.icosphere(1, 1.25 * leaf), freq=FREQ, eps_r=4.0, leaf_coeff=leaf, device=-1)
+    assert flat.max_level == 2
+    assert MLFMM(M.icosphere(2, 5 * radius), freq=FREQ, eps_r=4.0, leaf_coeff=5 * leaf, device=-1).max_level > 2
+
+
+@needs_lib
 def test_nas_path_and_arrays_agree(tmp_path):
     from mlfma_pmchwt_b200 import MLFMM
     from mlfma_pmchwt_b200 import mesh as M
