@@ -194,14 +194,15 @@ MLFMA_API int mlfma_profile_read(mlfma_plan* plan, double* stage_ms, int* applie
  *   "m2l.pair_warps" tile shape of the pair translation (m2l variant 4 and
  *                  the complex64 paths): 0 = 2, 1 = 4 (default), 2 = 8 box
  *                  pairs (warps) per CTA.
- *   "up.variant"   interpolation: 0 = 9-tap gather per parent direction and
- *                  component (default); 1 = separable phi-then-theta in bands of
- *                  theta rows through shared memory; 2 = one thread per
- *                  (parent, direction) for all 6 components; 3 = separable in
- *                  registers, a phi column of 4 parent theta rows per thread.
- *   "up.threads"   tile shape of the 9-tap interpolation (up variant 0 and the
- *                  complex64 paths): 0 = 64, 1 = 128 (default), 2 = 256
- *                  parent directions (threads) per CTA.
+ *   "up.variant"   interpolation: 0 = a pair of parent theta rows per thread
+ *                  and component over the child rows they share (default); 1 =
+ *                  separable phi-then-theta in bands of theta rows through
+ *                  shared memory; 2 = one thread per (parent, direction) for all
+ *                  6 components, 9 taps each; 3 = separable in registers, a phi
+ *                  column of 4 parent theta rows per thread.
+ *   "up.threads"   tile shape of the interpolation by row pairs (up variant 0 and
+ *                  the complex64 paths): 0 = 64, 1 = 128 (default), 2 = 256
+ *                  threads per CTA.
  *   "l2l.variant"  anterpolation: 0 = transposed 9-tap gather per child
  *                  direction; 1 = separable transposed theta-then-phi (default).
  *   "agg.variant"  aggregation: 0 = one thread per (leaf box, direction), one

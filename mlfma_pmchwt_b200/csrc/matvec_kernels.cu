@@ -163,61 +163,6 @@ __global__ void __launch_bounds__(kThreads) agg_box_kernel(AggBoxArg a) {
 }
 
 template <class C>
-struct UpArg {
-  const C* Sc;   // child level patterns [Bc][6][Kc]
-  C* Sp;               // parent level patterns [Bp][6][Kp]
-  const int* child_begin;
-  const int* octant;   // of child boxes
-  const int* tidx;
-  const double* lt;
-  const int* pidx;
-  const double* lp;
-  const C* ph_up;
-  int Kp, nphp, Kc, nphc;
-  long long slot_c = 0, slot_p = 0;  // element strides between right-hand-side slots (grid.z = 6 x slots)
-};
-
-// One thread per (parent box, parent direction, component): the 9-tap
-// separable interpolation of each child's pattern, times the child's shift
-// phase, summed over the children. One component per thread keeps the
-// register count low enough for the occupancy this gather needs.
-// kSlots: grid.z = 6 x slots with the slot offsets of the batched tree; the
-// single apply instantiates without them.
-// kT: threads per CTA (a tile of kT parent directions of one box and component)
-template <class C, bool kSlots = false, int kT = kThreads>
-__global__ void __launch_bounds__(kT) up_kernel(UpArg<C> a) {
-  using R = typename Cx<C>::real;
-  const int kk = blockIdx.y * blockDim.x + threadIdx.x;
-  const int b = blockIdx.x;
-  const int slot = kSlots ? blockIdx.z / 6 : 0;
-  const int c = blockIdx.z - 6 * slot;
-  if (kk >= a.Kp) return;
-  const int t = kk / a.nphp, p = kk - t * a.nphp;
-  int ti[3], pi[3];
-  double wt[3], wp[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    ti[i] = a.tidx[3 * t + i] * a.nphc;
-    wt[i] = a.lt[3 * t + i];
-    pi[i] = a.pidx[3 * p + i];
-    wp[i] = a.lp[3 * p + i];
-  }
-  C acc = Cx<C>::zero();
-  const int c1 = a.child_begin[b + 1];
-  for (int ch = a.child_begin[b]; ch < c1; ++ch) {
-    const C e = __ldg(a.ph_up + a.octant[ch] * a.Kp + kk);
-    const C* sc = (kSlots ? a.Sc + slot * a.slot_c : a.Sc) + (static_cast<size_t>(ch) * 6 + c) * a.Kc;
-    C v = Cx<C>::zero();
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) v = cfmas(static_cast<R>(wt[i] * wp[j]), __ldg(sc + ti[i] + pi[j]), v);
-    acc = cfma(e, v, acc);
-  }
-  (kSlots ? a.Sp + slot * a.slot_p : a.Sp)[(static_cast<size_t>(b) * 6 + c) * a.Kp + kk] = acc;
-}
-
-template <class C>
 struct Up2Arg {
   const C* Sc;   // child level patterns [Bc][6][Kc]
   C* Sp;         // parent level patterns [Bp][6][Kp]
@@ -232,15 +177,24 @@ struct Up2Arg {
   long long slot_c = 0, slot_p = 0;  // element strides between right-hand-side slots (grid.z = 6 x slots)
 };
 
-// The same interpolation, a thread per (parent box, pair of parent theta rows,
+// Interpolation (m2m), a thread per (parent box, pair of parent theta rows,
 // parent phi column, component): the two rows' stencils lie on at most 4
-// child rows, so 12 loads serve two outputs instead of 18, and each child row
-// is interpolated in phi once. Loads address from the child's uniform base by
-// 32-bit offsets. Bound by L1 throughput (85 % of its data pipe in complex64):
-// a gather of 32 phi taps straddles lines. One B200, interpolation of all
-// levels and both media, before and after: FP64 at 245,760 unknowns 1.34 ->
-// 1.05 ms, 16 slots of complex64 at 61,440 3.36 -> 3.07 ms. The occupancy
-// bounds are the measured best (FP64 96, complex64 72 registers; 64 spill).
+// child rows (a parent's grid is finer than its children's, so neighbouring
+// rows' stencils are at most one child row apart), and 12 loads serve two
+// outputs where 9 taps per output are 18; each child row is interpolated in phi
+// once, then in theta, times the child's shift phase, summed over the children.
+// Loads address from the child's uniform base by 32-bit offsets. kSlots: grid.z =
+// 6 x slots with the slot offsets of the batched tree; the single apply
+// instantiates without them. kT: threads per CTA.
+// Bound by L1 throughput (85 % of its data pipe in complex64): a gather of 32
+// phi taps straddles lines. One B200, interpolation of all levels and both media,
+// against a thread per output over its 9 taps: FP64 at 245,760 unknowns 1.34 ->
+// 1.05 ms, 16 slots of complex64 at 61,440 3.36 -> 3.07 ms. The occupancy bounds
+// are the measured best (FP64 96, complex64 72 registers; 64 spill). In
+// complex64 the phi and theta weights are rounded one by one where the 9 taps
+// had their products rounded, but an output meets fewer roundings: its error is
+// 0.84 to 0.97 of the 9 taps' over 78 pairs of levels of 24 bodies (5.3e-8 to
+// 5.9e-8 against 5.9e-8 to 6.3e-8).
 template <class C, bool kSlots, int kT>
 __global__ void __launch_bounds__(kT, (sizeof(C) == 16 ? 640 : 896) / kT) up2_kernel(const __grid_constant__ Up2Arg<C> a) {
   using R = typename Cx<C>::real;
@@ -296,36 +250,36 @@ __global__ void __launch_bounds__(kT, (sizeof(C) == 16 ? 640 : 896) / kT) up2_ke
   if (two) out[a.nphp] = acc1;
 }
 
-// grid: (parent boxes, direction tiles of t, zdim = 6 components x slots); the
-// row pairs where the level's stencils allow them
+// grid: (parent boxes, tiles of t (row pair, phi column)s, zdim = 6 components x slots)
 template <class C, bool kSlots>
-void launch_up(int t, int boxes, int zdim, const MediumLevel& pm, const UpArg<C>& a, cudaStream_t s) {
-  if (pm.up2_row) {
-    const Up2Arg<C> u{a.Sc, a.Sp,   a.child_begin, a.octant, pm.up2_row, pm.up2_w, a.pidx,   a.lp,
-                      a.ph_up, a.Kp, pm.nth,        a.nphp,   a.Kc,       a.slot_c, a.slot_p};
-    const dim3 g(boxes, (((pm.nth + 1) / 2) * pm.nph + t - 1) / t, zdim);
-    if (t == 64)
-      up2_kernel<C, kSlots, 64><<<g, 64, 0, s>>>(u);
-    else if (t == 256)
-      up2_kernel<C, kSlots, 256><<<g, 256, 0, s>>>(u);
-    else
-      up2_kernel<C, kSlots, 128><<<g, 128, 0, s>>>(u);
-    return;
-  }
-  const dim3 g(boxes, (a.Kp + t - 1) / t, zdim);
+void launch_up2(int t, int boxes, int zdim, const Up2Arg<C>& a, cudaStream_t s) {
+  const dim3 g(boxes, (((a.nthp + 1) / 2) * a.nphp + t - 1) / t, zdim);
   if (t == 64)
-    up_kernel<C, kSlots, 64><<<g, 64, 0, s>>>(a);
+    up2_kernel<C, kSlots, 64><<<g, 64, 0, s>>>(a);
   else if (t == 256)
-    up_kernel<C, kSlots, 256><<<g, 256, 0, s>>>(a);
+    up2_kernel<C, kSlots, 256><<<g, 256, 0, s>>>(a);
   else
-    up_kernel<C, kSlots, 128><<<g, 128, 0, s>>>(a);
+    up2_kernel<C, kSlots, 128><<<g, 128, 0, s>>>(a);
 }
+
+struct UpArg {
+  const double2* Sc;   // child level patterns [Bc][6][Kc]
+  double2* Sp;         // parent level patterns [Bp][6][Kp]
+  const int* child_begin;
+  const int* octant;   // of child boxes
+  const int* tidx;
+  const double* lt;
+  const int* pidx;
+  const double* lp;
+  const double2* ph_up;
+  int Kp, nphp, Kc, nphc;
+};
 
 // Interpolation (m2m), one thread per (parent box, parent direction) for all
 // 6 components: the stencil (3 theta x 3 phi taps and weights) and the
 // child's shift phase are loaded once per child and applied to the 6
 // component rows, 54 independent loads per child in flight.
-__global__ void __launch_bounds__(kThreads) up6_kernel(UpArg<double2> a) {
+__global__ void __launch_bounds__(kThreads) up6_kernel(UpArg a) {
   const int kk = blockIdx.y * blockDim.x + threadIdx.x;
   const int b = blockIdx.x;
   if (kk >= a.Kp) return;
@@ -1577,8 +1531,8 @@ void launch_up(Plan& P, int m, const LeafView& v, cudaStream_t s) {
       up_col_kernel<double2>
           <<<dim3(P.lv[l].B, pm.up4_nband, (6 * pm.nph + kThreads - 1) / kThreads), kThreads, 0, s>>>(a);
     } else if (P.tuning.up_variant == 2) {
-      UpArg<double2> a{Sc, pm.S, P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
-                       pm.ph_up, pm.K, pm.nph, cm.K, cm.nph};
+      UpArg a{Sc, pm.S, P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
+              pm.ph_up, pm.K, pm.nph, cm.K, cm.nph};
       up6_kernel<<<dim3(P.lv[l].B, (pm.K + kThreads - 1) / kThreads), kThreads, 0, s>>>(a);
     } else if (P.tuning.up_variant == 1 && pm.up_rows > 0) {
       UpSepArg a{Sc,    pm.S,     P.lv[l].child_begin, P.lv[l + 1].octant, pm.pidx,
@@ -1587,9 +1541,9 @@ void launch_up(Plan& P, int m, const LeafView& v, cudaStream_t s) {
                  pm.up_rows};
       up_sep_kernel<<<dim3(P.lv[l].B, 6, pm.up_nband), 256, 0, s>>>(a);
     } else {
-      UpArg<double2> a{Sc, pm.S, P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
-                       pm.ph_up, pm.K, pm.nph, cm.K, cm.nph};
-      launch_up<double2, false>(up_threads(P), P.lv[l].B, 6, pm, a, s);
+      const Up2Arg<double2> a{Sc,      pm.S,  P.lv[l].child_begin, P.lv[l + 1].octant, pm.up2_row, pm.up2_w, pm.pidx, pm.lp,
+                              pm.ph_up, pm.K, pm.nth,              pm.nph,             cm.K};
+      launch_up2<double2, false>(up_threads(P), P.lv[l].B, 6, a, s);
     }
   }
 }
@@ -1809,9 +1763,9 @@ void tree_pass_fixed(Plan& P, int m, C* leafS, C* leafB, cudaStream_t s, cudaStr
   for (int l = L - 1; l >= 2; --l) {
     const MediumLevel& pm = P.ml[m][l];
     const MediumLevel& cm = P.ml[m][l + 1];
-    UpArg<C> a{S_at(l + 1), S_at(l), P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx, pm.lp,
-               Store<C>::ph_up(pm), pm.K, pm.nph, cm.K, cm.nph};
-    launch_up<C, false>(up_threads(P), P.lv[l].B, 6, pm, a, s);
+    const Up2Arg<C> a{S_at(l + 1), S_at(l), P.lv[l].child_begin, P.lv[l + 1].octant, pm.up2_row, pm.up2_w, pm.pidx, pm.lp,
+                      Store<C>::ph_up(pm), pm.K, pm.nth, pm.nph, cm.K};
+    launch_up2<C, false>(up_threads(P), P.lv[l].B, 6, a, s);
   }
   if (sx) {
     translate(2, L - 1, s);
@@ -1862,10 +1816,10 @@ void tree_pass_slots(Plan& P, int m, int rn, cudaStream_t s, cudaStream_t sx, cu
   for (int l = L - 1; l >= 2; --l) {
     const MediumLevel& pm = P.ml[m][l];
     const MediumLevel& cm = P.ml[m][l + 1];
-    UpArg<C> a{P.btS[m][l + 1], P.btS[m][l], P.lv[l].child_begin, P.lv[l + 1].octant, pm.tidx, pm.lt, pm.pidx,
-               pm.lp,           pm.ph_up32,  pm.K,                 pm.nph,              cm.K,    cm.nph,
-               stride(l + 1),   stride(l)};
-    launch_up<C, true>(up_threads(P), P.lv[l].B, 6 * rn, pm, a, s);
+    const Up2Arg<C> a{P.btS[m][l + 1], P.btS[m][l], P.lv[l].child_begin, P.lv[l + 1].octant, pm.up2_row, pm.up2_w,
+                      pm.pidx,         pm.lp,       pm.ph_up32,          pm.K,               pm.nth,     pm.nph,
+                      cm.K,            stride(l + 1), stride(l)};
+    launch_up2<C, true>(up_threads(P), P.lv[l].B, 6 * rn, a, s);
   }
   translate(2, L - 1, s);
   MLFMA_CUDA(cudaStreamWaitEvent(s, ev_leaf, 0));

@@ -416,14 +416,12 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
         const int ncol = P->ml[m][l + 1].nph;
         std::vector<int4> row;
         std::vector<double2> w;
-        bool fits = true;
-        for (int t = 0; t < M.nth && fits; t += 2) {
+        for (int t = 0; t < M.nth; t += 2) {
           std::vector<int> rows;
           for (int u = t; u < std::min(t + 2, M.nth); ++u) rows.insert(rows.end(), &I.tidx[3 * u], &I.tidx[3 * u] + 3);
           std::sort(rows.begin(), rows.end());
           rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
-          fits = rows.size() <= 4;
-          if (!fits) break;
+          if (rows.size() > 4) throw std::logic_error("interpolation: a pair of rows on more than 4 child rows");
           double2 wr[4] = {};
           for (int u = t; u < std::min(t + 2, M.nth); ++u)
             for (int i = 0; i < 3; ++i) {
@@ -434,10 +432,8 @@ std::unique_ptr<Plan> create_plan(Mesh&& mesh, const PlanParams& prm) {
           row.push_back(make_int4(rows[0] * ncol, rows[1] * ncol, rows[2] * ncol, rows[3] * ncol));
           w.insert(w.end(), wr, wr + 4);
         }
-        if (fits) {
-          M.up2_row = P->upload(row);
-          M.up2_w = P->upload(w);
-        }
+        M.up2_row = P->upload(row);
+        M.up2_w = P->upload(w);
       }
       if (l > 2) {
         // transposed interpolation: child direction <- (parent direction, weight)

@@ -62,7 +62,7 @@ struct MediumLevel {
   int* up4_tpos = nullptr;
   // parent theta rows in pairs (2q, 2q + 1): the at most 4 child theta rows
   // their stencils share (offsets into a pattern: row * child phi columns) and
-  // each one's weight in the two parent rows; null when a pair needs more
+  // each one's weight in the two parent rows
   int4* up2_row = nullptr;     // [ceil(nth / 2)]
   double2* up2_w = nullptr;    // [ceil(nth / 2)][4]
   // this level as child of level-1: for each child direction, the parent
@@ -134,9 +134,9 @@ struct Tuning {
   int m2l_pair_warps = 1;      // box pairs (warps) per CTA of the pair translations (variants 4, 5 and the
                                //    complex64 paths): 0 = 2, 1 = 4, 2 = 8
   int l2l_variant = 1;         // 0: 2-D transposed taps per child direction; 1: separable
-  int up_threads = 1;          // threads per CTA of the 9-tap interpolation (up variant 0 and the complex64
-                               //    paths): 0 = 64, 1 = 128, 2 = 256
-  int up_variant = 0;          // 0: 9-tap gather per parent direction; 1: separable in bands;
+  int up_threads = 1;          // threads per CTA of the interpolation by row pairs (up variant 0 and the complex64
+                               //    paths): 64 << value
+  int up_variant = 0;          // 0: a pair of parent theta rows per thread; 1: separable in bands;
                                // 2: 9-tap gather, all 6 components per thread;
                                // 3: separable in registers, 4-row bands per thread
   int agg_variant = 0;         // 0: thread per (box, direction); 1: CTA per (box, medium) streaming

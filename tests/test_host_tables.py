@@ -99,3 +99,24 @@ def test_multipole_orders_bench_sphere():
         D = np.sqrt(3.0) * 0.25 * lam * 2 ** (6 - lvl)
         for kk, Ls in ((k, op.info.L_k1), (abs(k * np.sqrt(2.5 - 0.1j)), op.info.L_k2)):
             assert Ls[i] == int(np.ceil(kk * D + 6 * np.cbrt(kk * D)))
+
+
+@needs_lib
+def test_pairs_of_parent_rows_share_four_child_rows():
+    """The interpolation takes parent theta rows (2q, 2q + 1) together over the
+    at most 4 child rows of their two stencils: a parent's grid is finer than
+    its children's, at every box size and medium."""
+    from mlfma_pmchwt_b200 import MLFMM, mesh as M
+    seen = {}
+    for leaf in (0.02, 0.08, 0.12, 0.2, 0.25, 0.3, 0.4):
+        for eps in (1.0001, 1.5, 2.5, 4.0, 10.0, 50.0, 360.0, 2.5 - 0.1j, 80 - 70j):
+            for radius in (0.5, 2.0):
+                op = MLFMM(M.icosphere(1, radius), freq=FREQ, eps_r=eps, leaf_coeff=leaf, device=-1)
+                for med in (1, 2):
+                    for lvl in range(2, op.max_level):
+                        size = op.grid(med, lvl)["L"], op.grid(med, lvl + 1)["L"]
+                        if size not in seen:
+                            rows = op.interp(med, lvl)["tidx"]
+                            seen[size] = max(len(np.unique(rows[t:t + 2])) for t in range(0, len(rows), 2))
+                op.close()
+    assert len(seen) > 60 and max(seen.values()) <= 4 and all(a > b for a, b in seen)
