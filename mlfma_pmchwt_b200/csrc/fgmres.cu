@@ -39,56 +39,26 @@ struct NearArg {
   int N;
 };
 
-// w = Z_near (xscale x): rows t and N + t of the near field, one warp per RWG;
-// the entries and the arithmetic in the storage type Z (complex128 or
-// complex64). x is scaled in FP64 as it is read.
-template <class Z>
-__global__ void __launch_bounds__(128) near_apply_kernel(NearArg<Z> a) {
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (r >= a.N) return;
-  const int id = a.leaf_rwg[r];
-  const int b = a.rwg_box[id];
-  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0;
-  const int tl = r - a.leaf_ptr[b];
-  const int pitch = near_pitch(ns);
-  const Z* Zr = a.near_z + a.near_zoff[b] + 3LL * tl * pitch;
-  const double sc = a.xscale ? *a.xscale : 1.0;
-  Z nJ = Cx<Z>::zero(), nM = Cx<Z>::zero();
-  for (int j = lane; j < ns; j += 32) {
-    const int s = a.near_src[s0 + j];
-    const Z xJ = Cx<Z>::from(cscale(a.x[s], sc)), xM = Cx<Z>::from(cscale(a.x[a.N + s], sc));
-    const Z z11 = Zr[j], z12 = Zr[pitch + j], z22 = Zr[2 * pitch + j];
-    nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
-    nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    nJ.x += __shfl_xor_sync(0xffffffffu, nJ.x, o);
-    nJ.y += __shfl_xor_sync(0xffffffffu, nJ.y, o);
-    nM.x += __shfl_xor_sync(0xffffffffu, nM.x, o);
-    nM.y += __shfl_xor_sync(0xffffffffu, nM.y, o);
-  }
-  if (lane == 0) {
-    a.w[id] = Cx<Z>::to64(nJ);
-    a.w[a.N + id] = Cx<Z>::to64(nM);
-  }
-}
-
-// The same product with a CTA per (leaf box, 8 rows): the box's source values
-// are gathered once into shared memory (in the storage type, a row of J and a
-// row of M), where the CTA's rows read them; the entries load 16 bytes per
-// lane, one source in complex128 and two in complex64, for the two rows of a
-// warp, always one step ahead of the arithmetic (the first before the
-// sources are gathered).
+// w = Z_near (xscale x): rows t and N + t of the near field; the entries and the
+// arithmetic in the storage type Z (complex128 or complex64). x is scaled in
+// FP64 as it is read. A CTA per (leaf box, 8 rows): the box's source values are
+// gathered into shared memory (in the storage type, a row of J and a row of M; a
+// list longer than kPiece piece by piece), where the CTA's rows read them; the
+// entries load 16 bytes per lane, one source in complex128 and two in complex64,
+// for the two rows of a warp, always one step ahead of the arithmetic (the first
+// before the sources are gathered).
 // HBM- or L2-bound (each entry is read once): 4.35 M pairs in complex64 are
 // 104 MB, 16 us; measured 26 us. A warp per row that gathered its sources
 // from the vectors, with the three values of a pair side by side, took 31 us
 // there; a CTA for all rows of a box 34 us, waiting for the fullest boxes.
+// Pieces of 48 KB keep four CTAs on an SM: lists of up to 3,718 sources (15,360
+// unknowns, FP64) take 157 us, 428 when staged whole; ordinary ones, a few
+// hundred sources, 92 us at 61,440 unknowns either way.
 constexpr int kNearThreads = 128;
 constexpr int kNearRows = 2;
 constexpr int kNearCtaRows = kNearRows * kNearThreads / 32;
-constexpr size_t kNearStageMax = 160 * 1024;
+template <class Z>
+constexpr int kNearPiece = 48 * 1024 / (2 * sizeof(Z));  // sources staged at a time: 1,536 or 3,072
 
 template <class Z>
 struct alignas(16) NearVec {
@@ -121,27 +91,31 @@ __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
   };
   int q = lane * Vec::kPer;
   fetch(q, z[0]);
+  constexpr int kPiece = kNearPiece<Z>;
   Z* xJ = reinterpret_cast<Z*>(near_stage);
-  Z* xM = xJ + pitch;
+  Z* xM = xJ + min(pitch, kPiece);
   const double sc = a.xscale ? *a.xscale : 1.0;
+  auto gather = [&](int p0) {
+    const int n = min(kPiece, pitch - p0);
 #pragma unroll 2
-  for (int i = threadIdx.x; i < pitch; i += kNearThreads) {
-    double2 J = c2(0.0, 0.0), M = c2(0.0, 0.0);
-    if (i < ns) {
-      const int s = a.near_src[s0 + i];
-      J = a.x[s];
-      M = a.x[a.N + s];
+    for (int i = threadIdx.x; i < n; i += kNearThreads) {
+      double2 J = c2(0.0, 0.0), M = c2(0.0, 0.0);
+      if (p0 + i < ns) {
+        const int s = a.near_src[s0 + p0 + i];
+        J = a.x[s];
+        M = a.x[a.N + s];
+      }
+      xJ[i] = Cx<Z>::from(cscale(J, sc));
+      xM[i] = Cx<Z>::from(cscale(M, sc));
     }
-    xJ[i] = Cx<Z>::from(cscale(J, sc));
-    xM[i] = Cx<Z>::from(cscale(M, sc));
-  }
-  __syncthreads();
+    __syncthreads();
+  };
   Z nJ[kNearRows], nM[kNearRows];
 #pragma unroll
   for (int u = 0; u < kNearRows; ++u) nJ[u] = nM[u] = Cx<Z>::zero();
-  auto add = [&](int at, const Vec(&f)[kNearRows][3]) {
+  auto add = [&](int at, int p0, const Vec(&f)[kNearRows][3]) {
     if (at >= pitch) return;
-    const Vec J = *reinterpret_cast<const Vec*>(xJ + at), M = *reinterpret_cast<const Vec*>(xM + at);
+    const Vec J = *reinterpret_cast<const Vec*>(xJ + (at - p0)), M = *reinterpret_cast<const Vec*>(xM + (at - p0));
 #pragma unroll
     for (int u = 0; u < kNearRows; ++u)
 #pragma unroll
@@ -151,11 +125,16 @@ __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
       }
   };
   constexpr int kStep = 32 * Vec::kPer;
-  for (int base = 0; base < pitch; base += 2 * kStep, q += 2 * kStep) {
-    fetch(q + kStep, z[1]);
-    add(q, z[0]);
-    fetch(q + 2 * kStep, z[0]);
-    add(q + kStep, z[1]);
+  static_assert(kPiece % (2 * kStep) == 0, "a piece ends with a step");
+  for (int p0 = 0; p0 < pitch; p0 += kPiece) {
+    if (p0 > 0) __syncthreads();
+    gather(p0);
+    for (int base = p0; base < min(pitch, p0 + kPiece); base += 2 * kStep, q += 2 * kStep) {
+      fetch(q + kStep, z[1]);
+      add(q, p0, z[0]);
+      fetch(q + 2 * kStep, z[0]);
+      add(q + kStep, p0, z[1]);
+    }
   }
 #pragma unroll
   for (int u = 0; u < kNearRows; ++u) {
@@ -175,18 +154,9 @@ __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
   }
 }
 
-// A box whose staged sources fit shared memory takes the box kernel; a plan
-// with a larger source list anywhere keeps the row kernel.
 template <class Z>
 void launch_near(const Plan& P, const NearArg<Z>& a, cudaStream_t s) {
-  const size_t smem = 2 * sizeof(Z) * static_cast<size_t>(near_pitch(P.max_near_sources));
-  if (smem > kNearStageMax) {
-    near_apply_kernel<Z><<<(P.N + 3) / 4, 128, 0, s>>>(a);
-    return;
-  }
-  if (smem > 48 * 1024)  // the same largest value on every call: safe beside other plans' launches
-    MLFMA_CUDA(cudaFuncSetAttribute(near_box_kernel<Z>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kNearStageMax)));
+  const size_t smem = 2 * sizeof(Z) * static_cast<size_t>(std::min(near_pitch(P.max_near_sources), kNearPiece<Z>));
   const dim3 grid(static_cast<int>(P.h_near_sptr.size()) - 1, (P.max_leaf_rwgs + kNearCtaRows - 1) / kNearCtaRows);
   near_box_kernel<Z><<<grid, kNearThreads, smem, s>>>(a);
 }

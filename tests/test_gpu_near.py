@@ -1,6 +1,7 @@
 """The near-field products of the preconditioner and of the public entry
 point against the read-out entries in numpy, at row and source counts around
-the kernels' tiles (a box of a few RWGs to hundreds), and the lockstep
+the kernels' tiles (a box of a few RWGs to hundreds, lists of sources longer
+than the piece that the box kernel stages at a time), and the lockstep
 product for 1 to 9 systems through one inner step."""
 import numpy as np
 import pytest
@@ -28,10 +29,13 @@ def _near(op, x):
 @pytest.mark.parametrize("body", BODIES)
 def test_near_product(body):
     """FP64: a row's error is below (2 ns + 4) eps of the sum of its terms' magnitudes."""
-    torch = pytest.importorskip("torch")
     sub, radius, leaf = BODIES[body]
-    op = MLFMM(M.ellipsoid(sub, radius, 0.9 * radius, 0.8 * radius), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=leaf,
-               device=0)
+    _check_near(MLFMM(M.ellipsoid(sub, radius, 0.9 * radius, 0.8 * radius), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=leaf,
+                      device=0))
+
+
+def _check_near(op):
+    torch = pytest.importorskip("torch")
     g = np.random.default_rng(1)
     x = g.standard_normal(op.n) + 1j * g.standard_normal(op.n)
     want, mag, ns = _near(op, x)
@@ -65,3 +69,27 @@ def test_lockstep_near_product(body, R):
         for x in (X[j], one[j]):
             off = np.linalg.norm(x - Q @ (Q.conj().T @ x)) / np.linalg.norm(x)
             assert off <= 2 * (2 * ns + 4) * 6e-8 * np.linalg.norm(mag) / np.linalg.norm(want)
+
+
+def _long_lists(precision):
+    """Lists of up to 3,718 sources: three pieces of the shared memory that the
+    box kernel stages them in (1,536 in FP64, 3,072 in complex64: two)."""
+    op = MLFMM(M.ellipsoid(4, 0.7, 0.63, 0.56), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=0.4, device=0,
+               precision=precision)
+    assert 3 * 1536 > int(np.bincount(op.near(values=False)["target"]).max()) > 3072
+    return op
+
+
+def test_near_product_of_long_lists():
+    """As test_near_product."""
+    _check_near(_long_lists("fp64"))
+
+
+def test_complex64_near_product_of_long_lists():
+    """The complex64 operator's near rows against the FP64 operator: a lane's ~120
+    terms are off by a few 6e-8 of their size each: 1e-5, as the other
+    comparisons of the two operators."""
+    op = _long_lists("mixed")
+    x = M.unit_disk_vector(op.n, 2)
+    w = op.apply_ax(x)
+    assert np.linalg.norm(op.apply_ax_mixed(x) - w) <= 1e-5 * np.linalg.norm(w)
