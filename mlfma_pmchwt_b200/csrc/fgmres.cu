@@ -39,21 +39,54 @@ struct NearArg {
   int N;
 };
 
-// w = Z_near (xscale x): rows t and N + t of the near field; the entries and the
-// arithmetic in the storage type Z (complex128 or complex64). x is scaled in
-// FP64 as it is read. A CTA per (leaf box, 8 rows): the box's source values are
+// w = Z_near (xscale x): rows t and N + t of the near field, a warp per RWG; the
+// entries and the arithmetic in the storage type Z (complex128 or complex64).
+// x is scaled in FP64 as it is read. (near_by_rows: where this kernel is used.)
+template <class Z>
+__global__ void __launch_bounds__(128) near_row_kernel(NearArg<Z> a) {
+  const int lane = threadIdx.x & 31;
+  const int r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (r >= a.N) return;
+  const int id = a.leaf_rwg[r];
+  const int b = a.rwg_box[id];
+  const int s0 = a.near_sptr[b], ns = a.near_sptr[b + 1] - s0, pitch = near_pitch(ns);
+  const Z* Zr = a.near_z + a.near_zoff[b] + 3LL * (r - a.leaf_ptr[b]) * pitch;
+  const double sc = a.xscale ? *a.xscale : 1.0;
+  Z nJ = Cx<Z>::zero(), nM = Cx<Z>::zero();
+  for (int j = lane; j < ns; j += 32) {
+    const int s = a.near_src[s0 + j];
+    const Z xJ = Cx<Z>::from(cscale(a.x[s], sc)), xM = Cx<Z>::from(cscale(a.x[a.N + s], sc));
+    const Z z11 = Zr[j], z12 = Zr[pitch + j], z22 = Zr[2 * pitch + j];
+    nJ = cfma(z11, xJ, cfma(z12, xM, nJ));
+    nM = cfma(z22, xM, csub(nM, cmul(z12, xJ)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nJ.x += __shfl_xor_sync(0xffffffffu, nJ.x, o);
+    nJ.y += __shfl_xor_sync(0xffffffffu, nJ.y, o);
+    nM.x += __shfl_xor_sync(0xffffffffu, nM.x, o);
+    nM.y += __shfl_xor_sync(0xffffffffu, nM.y, o);
+  }
+  if (lane == 0) {
+    a.w[id] = Cx<Z>::to64(nJ);
+    a.w[a.N + id] = Cx<Z>::to64(nM);
+  }
+}
+
+// The same product with a CTA per (leaf box, 8 rows): the box's source values are
 // gathered into shared memory (in the storage type, a row of J and a row of M; a
-// list longer than kPiece piece by piece), where the CTA's rows read them; the
-// entries load 16 bytes per lane, one source in complex128 and two in complex64,
-// for the two rows of a warp, always one step ahead of the arithmetic (the first
-// before the sources are gathered).
+// list longer than kPiece piece by piece, kPieces), where the CTA's rows read
+// them; the entries load 16 bytes per lane, one source in complex128 and two in
+// complex64, for the two rows of a warp, always one step ahead of the arithmetic
+// (the first before the sources are gathered).
 // HBM- or L2-bound (each entry is read once): 4.35 M pairs in complex64 are
 // 104 MB, 16 us; measured 26 us. A warp per row that gathered its sources
 // from the vectors, with the three values of a pair side by side, took 31 us
 // there; a CTA for all rows of a box 34 us, waiting for the fullest boxes.
 // Pieces of 48 KB keep four CTAs on an SM: lists of up to 3,718 sources (15,360
-// unknowns, FP64) take 157 us, 428 when staged whole; ordinary ones, a few
-// hundred sources, 92 us at 61,440 unknowns either way.
+// unknowns, FP64) take 155 us, 427 when staged whole. The loop over pieces takes
+// the registers of the second step in flight (complex64, lists of up to 2,350
+// sources: 77 us without it, 119 with it), so shorter lists go without.
 constexpr int kNearThreads = 128;
 constexpr int kNearRows = 2;
 constexpr int kNearCtaRows = kNearRows * kNearThreads / 32;
@@ -66,7 +99,7 @@ struct alignas(16) NearVec {
   Z v[kPer];
 };
 
-template <class Z>
+template <class Z, bool kPieces>
 __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
   using Vec = NearVec<Z>;
   extern __shared__ __align__(16) unsigned char near_stage[];
@@ -126,10 +159,10 @@ __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
   };
   constexpr int kStep = 32 * Vec::kPer;
   static_assert(kPiece % (2 * kStep) == 0, "a piece ends with a step");
-  for (int p0 = 0; p0 < pitch; p0 += kPiece) {
+  for (int p0 = 0; p0 < (kPieces ? pitch : 1); p0 += kPiece) {
     if (p0 > 0) __syncthreads();
     gather(p0);
-    for (int base = p0; base < min(pitch, p0 + kPiece); base += 2 * kStep, q += 2 * kStep) {
+    for (int base = p0; base < (kPieces ? min(pitch, p0 + kPiece) : pitch); base += 2 * kStep, q += 2 * kStep) {
       fetch(q + kStep, z[1]);
       add(q, p0, z[0]);
       fetch(q + 2 * kStep, z[0]);
@@ -154,11 +187,36 @@ __global__ void __launch_bounds__(kNearThreads) near_box_kernel(NearArg<Z> a) {
   }
 }
 
+// Row by row where it is faster (one B200, us, row kernel / box kernel):
+// boxes of a few RWGs, whose CTAs leave most of their warps idle, once there
+// are more of them than CTAs fit at once: complex64 at 61,440 unknowns 3.7 RWGs
+// per box 18 / 26, 6.7 22 / 26, 9.3 32 / 33, at 15,360 6.7 7.8 / 8.4, 7.7 9.3 /
+// 8.3, at 3,840 (505 boxes) 3.8 3.6 / 3.6; FP64 at 15,360 4.4 7.6 / 10.1, 6.7
+// 8.9 / 10.1, 7.7 10.6 / 10.4, 13.7 13.7 / 12.3;
+// and in FP64 entries that outgrow L2, whose loads a row's 9 warps per scheduler
+// keep in flight better: 61,440 unknowns (380 MB) 72 / 78, 245,760 (1.5 GB) 268 /
+// 298, but 15,360 (88 MB) 17.9 / 16.3; up to lists whose gathering by every row
+// costs more: 1,264 sources (61,440 unknowns) 292 / 300, 2,018 137 / 134, 2,424
+// 188 / 155.
+template <class Z>
+bool near_by_rows(const Plan& P) {
+  const double boxes = static_cast<double>(P.h_near_sptr.size() - 1), pairs = static_cast<double>(P.near_pairs);
+  if (boxes > 4 * 148 && P.N < 7 * boxes) return true;
+  return sizeof(Z) == 16 && 3 * sizeof(Z) * pairs > 126e6 && pairs < 1600.0 * P.N;
+}
+
 template <class Z>
 void launch_near(const Plan& P, const NearArg<Z>& a, cudaStream_t s) {
+  if (near_by_rows<Z>(P)) {
+    near_row_kernel<Z><<<(P.N + 3) / 4, 128, 0, s>>>(a);
+    return;
+  }
   const size_t smem = 2 * sizeof(Z) * static_cast<size_t>(std::min(near_pitch(P.max_near_sources), kNearPiece<Z>));
   const dim3 grid(static_cast<int>(P.h_near_sptr.size()) - 1, (P.max_leaf_rwgs + kNearCtaRows - 1) / kNearCtaRows);
-  near_box_kernel<Z><<<grid, kNearThreads, smem, s>>>(a);
+  if (P.max_near_sources > kNearPiece<Z>)
+    near_box_kernel<Z, true><<<grid, kNearThreads, smem, s>>>(a);
+  else
+    near_box_kernel<Z, false><<<grid, kNearThreads, smem, s>>>(a);
 }
 
 }  // namespace

@@ -93,3 +93,22 @@ def test_complex64_near_product_of_long_lists():
     x = M.unit_disk_vector(op.n, 2)
     w = op.apply_ax(x)
     assert np.linalg.norm(op.apply_ax_mixed(x) - w) <= 1e-5 * np.linalg.norm(w)
+
+
+@pytest.mark.parametrize("sub,radius,leaf", [(3, 1.0, 0.1), (4, 1.3, 0.4)])
+def test_near_product_by_rows(sub, radius, leaf):
+    """As test_near_product where a warp takes each row: a thousand boxes of two
+    RWGs, and 226 MB of entries."""
+    op = MLFMM(M.icosphere(sub, radius), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=leaf, device=0)
+    boxes = len(op.leaf_rwgs()[0]) - 1
+    assert boxes > 592 and op.N < 3 * boxes or 48 * op.info.near_pairs > 2e8
+    _check_near(op)
+
+
+def test_complex64_near_product_by_rows():
+    """As test_complex64_near_product_of_long_lists on boxes of two RWGs."""
+    op = MLFMM(M.icosphere(3, 1.0), freq=3e8, eps_r=2.5 - 0.1j, leaf_coeff=0.1, device=0, precision="mixed")
+    assert len(op.leaf_rwgs()[0]) - 1 > 592
+    x = M.unit_disk_vector(op.n, 2)
+    w = op.apply_ax(x)
+    assert np.linalg.norm(op.apply_ax_mixed(x) - w) <= 1e-5 * np.linalg.norm(w)
