@@ -29,7 +29,9 @@ constexpr int kRhsTile = 8;      // incidences per thread (grid.y tiles)
 constexpr int kFarChunk = 512;   // angles per far-field launch (12 KB of parameters)
 constexpr int kFarAngles = 4;    // angles and
 constexpr int kFarSols = 32;     // solutions per cluster of the bistatic far field
-constexpr int kFarRwgs = 256;    // RWGs whose moments a block stages at a time
+constexpr int kFarRwgs = 256;    // RWGs whose moments a block stages at a time,
+constexpr int kFarFew = 64;      // of a body whose RWGs would leave blocks of a cluster without any
+constexpr int kFarFewSols = 4;   // solutions of a block that forms the moments it sums
 constexpr int kFarSlices = 8;    // blocks of a cluster, each with a slice of the RWGs
 constexpr int kFarThreads = 512;
 
@@ -288,10 +290,10 @@ struct FarBatchArg {
 // warps that shared the RWGs of a pair instead of its angles, 361 angles at
 // 3,840 unknowns took 115 us for one solution and 142 for 16, now 101 and 129;
 // at 61,440 unknowns 1,056 and 1,385, now 1,078 and 1,357.
-template <bool kSkew>
+template <bool kSkew, int kRwgs>
 __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads, 1)
     far_batch_kernel(const __grid_constant__ FarBatchArg a) {
-  __shared__ double2 A[kFarAngles][2][kFarRwgs];
+  __shared__ double2 A[kFarAngles][2][kRwgs];
   __shared__ double2 sums[kFarSols * kFarAngles * 2];
   const Geo& g = a.g;
   const int ang0 = blockIdx.x * kFarAngles, na = min(kFarAngles, a.n_angles - ang0);
@@ -312,10 +314,10 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
 #pragma unroll
     for (int t = 0; t < kFarAngles; ++t) acc[q][t][0] = acc[q][t][1] = c2(0.0, 0.0);
   auto add = [&](int m0, auto angles) {
-    constexpr int kA = decltype(angles)::value, kAhead = 8 / kA;
+    constexpr int kA = decltype(angles)::value, kAhead = kRwgs == kFarRwgs ? 8 / kA : 2;
     const int first = kA == kFarAngles ? 0 : t0;
 #pragma unroll kAhead
-    for (int c = 0; c < kFarRwgs / 32; ++c) {
+    for (int c = 0; c < kRwgs / 32; ++c) {
       const int q = 32 * c + lane, m = min(m0 + q, g.N - 1);  // moments beyond N are zero
       const double2 J0 = __ldg(I0 + m), M0 = __ldg(I0 + g.N + m);
       const double2 J1 = __ldg(I1 + m), M1 = __ldg(I1 + g.N + m);
@@ -329,14 +331,14 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
       }
     }
   };
-  const int tiles = (g.N + kFarRwgs - 1) / kFarRwgs;
+  const int tiles = (g.N + kRwgs - 1) / kRwgs;
   for (int tile = blockIdx.z; tile < tiles; tile += kFarSlices) {
-    const int m0 = tile * kFarRwgs;
+    const int m0 = tile * kRwgs;
     __syncthreads();
     {
-      const int q = threadIdx.x & (kFarRwgs - 1), m = m0 + q;
+      const int q = threadIdx.x & (kRwgs - 1), m = m0 + q;
 #pragma unroll 1
-      for (int t = threadIdx.x / kFarRwgs; t < kFarAngles; t += kFarThreads / kFarRwgs) {
+      for (int t = threadIdx.x / kRwgs; t < kFarAngles; t += kFarThreads / kRwgs) {
         double2 Au = c2(0.0, 0.0), Av = c2(0.0, 0.0);
         if (m < g.N && t < na) {
           double u[3], v[3];
@@ -395,6 +397,86 @@ __global__ void __cluster_dims__(1, 1, kFarSlices) __launch_bounds__(kFarThreads
     }
   }
   cl.sync();  // the other blocks' sums stay until rank 0 has read them
+}
+
+// The same sums for up to kS solutions with a block per angle and a warp for each
+// slice: a lane forms the moments it sums, so nothing is staged and no warp waits
+// for another until the end. Same order, same bits as far_batch_kernel, which
+// shares a moment among more solutions but holds an SM's 16 warps in step.
+template <bool kSkew, int kRwgs, int kS>
+__global__ void __launch_bounds__(32 * kFarSlices, 2) far_few_kernel(const __grid_constant__ FarBatchArg a) {
+  __shared__ double2 red[kFarSlices][kS][2];
+  const Geo& g = a.g;
+  const int r0 = blockIdx.y * kS, nr = min(kS, a.R - r0);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const size_t n = 2 * static_cast<size_t>(g.N);
+  const double* r = a.dir[blockIdx.x];
+  double u[3], v[3];
+  transverse(r, u, v);
+  double2 acc[kS][2];
+#pragma unroll
+  for (int s = 0; s < kS; ++s) acc[s][0] = acc[s][1] = c2(0.0, 0.0);
+  for (int tile = wp; tile * kRwgs < g.N; tile += kFarSlices) {
+#pragma unroll 1
+    for (int c = 0; c < kRwgs / 32; ++c) {
+      const int m = tile * kRwgs + 32 * c + lane;
+      if (m >= g.N) break;
+      double2 Au, Av;
+      far_moment<kSkew>(g, m, r, u, v, Au, Av);
+      const double2 mu = cneg(Au), mv = cneg(Av);
+#pragma unroll
+      for (int s = 0; s < kS; ++s) {
+        if (s >= nr) break;
+        const double2 J = __ldg(a.I + (r0 + s) * n + m), M = __ldg(a.I + (r0 + s) * n + g.N + m);
+        acc[s][0] = cfma(mv, M, cfma(mu, J, acc[s][0]));
+        acc[s][1] = cfma(Au, M, cfma(mv, J, acc[s][1]));
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < kS; ++s)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const double2 t = blas1::warp_sum2(acc[s][c]);
+      if (lane == 0) red[wp][s][c] = t;
+    }
+  __syncthreads();
+  if (threadIdx.x >= nr) return;
+  double2 su = c2(0.0, 0.0), sv = c2(0.0, 0.0);
+  for (int q = 0; q < kFarSlices; ++q) {
+    su = cadd(su, red[q][threadIdx.x][0]);
+    sv = cadd(sv, red[q][threadIdx.x][1]);
+  }
+  const double2 coeff = c2(g.k1.y, -g.k1.x);
+  double2* out = a.out + ((r0 + threadIdx.x) * static_cast<size_t>(a.n_total_angles) + a.angle0 + blockIdx.x) * 3;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[c] = cmul(coeff, cadd(cscale(su, u[c]), cscale(sv, v[c])));
+}
+
+// One chunk of angles; kRwgs by the body's size alone, so that a solution's field
+// is the same in every call. A block per angle where that gives every SM one, or
+// on small bodies, for few solutions (one B200, us, far_batch_kernel / far_few_kernel):
+// 361 angles, one solution: 240 unknowns 52 / 19, 960 55 / 20, 3,840 96 / 57,
+// 61,440 1,049 / 868; four 61,440 1,109 / 1,037; eight 240 unknowns 58 / 26,
+// 3,840 107 / 117; 37 angles, one solution: 960 unknowns 15.5 / 14.6, 3,840
+// 17 / 28, 61,440 165 / 388. Tiles of 64 RWGs instead of 256 where those would
+// leave blocks of a cluster without any: 32 solutions at 37 angles, 240 unknowns
+// 25 -> 17 us, at 361 angles 143 -> 91.
+template <bool kSkew, int kRwgs>
+void launch_far(const FarBatchArg& a, cudaStream_t s) {
+  const bool small = a.g.N <= 512;
+  if (a.R <= (small ? 2 : 1) * kFarFewSols && (small || a.n_angles >= 148)) {
+    const dim3 grid(a.n_angles, (a.R + kFarFewSols - 1) / kFarFewSols);
+    if (a.R == 1)
+      far_few_kernel<kSkew, kRwgs, 1><<<grid, 32 * kFarSlices, 0, s>>>(a);
+    else if (a.R == 2)
+      far_few_kernel<kSkew, kRwgs, 2><<<grid, 32 * kFarSlices, 0, s>>>(a);
+    else
+      far_few_kernel<kSkew, kRwgs, kFarFewSols><<<grid, 32 * kFarSlices, 0, s>>>(a);
+    return;
+  }
+  const dim3 grid((a.n_angles + kFarAngles - 1) / kFarAngles, (a.R + kFarSols - 1) / kFarSols, kFarSlices);
+  far_batch_kernel<kSkew, kRwgs><<<grid, kFarThreads, 0, s>>>(a);
 }
 
 struct FarMonoArg {
@@ -477,11 +559,11 @@ void rcs_pmchwt_batch(Plan& P, int R, const double2* I_dev, int n_angles, const 
     a.n_angles = std::min(kFarChunk, n_angles - c0);
     a.angle0 = c0;
     for (int q = 0; q < a.n_angles; ++q) direction(theta_deg[c0 + q], phi_deg[c0 + q], a.dir[q]);
-    const dim3 grid((a.n_angles + kFarAngles - 1) / kFarAngles, (R + kFarSols - 1) / kFarSols, kFarSlices);
+    const bool few = P.N <= (kFarSlices - 1) * kFarRwgs;
     if (a.g.skew)
-      far_batch_kernel<true><<<grid, kFarThreads, 0, s>>>(a);
+      few ? launch_far<true, kFarFew>(a, s) : launch_far<true, kFarRwgs>(a, s);
     else
-      far_batch_kernel<false><<<grid, kFarThreads, 0, s>>>(a);
+      few ? launch_far<false, kFarFew>(a, s) : launch_far<false, kFarRwgs>(a, s);
     MLFMA_CUDA(cudaGetLastError());
   }
 }

@@ -1,5 +1,5 @@
 """The bistatic far-field kernel at the ends of its tiles (4 angles, pairs and
-32 solutions, 256 RWGs, 8 slices, 512 angles per launch) and for triangles
+32 solutions, 256 RWGs or 64, 8 slices, 512 angles per launch) and for triangles
 wider than its phase series covers, against the single-solution entry point;
 both batched far fields with every triangle rule on a body off the origin."""
 import dataclasses
@@ -62,14 +62,16 @@ def test_far_field_rules(rule):
         np.testing.assert_allclose(mono[r], want[r], rtol=0, atol=1e-12 * np.abs(want).max())
 
 
-def test_far_field_of_a_solution_alone_and_among_others():
+@pytest.mark.parametrize("sub", [1, 2, 3])
+def test_far_field_of_a_solution_alone_and_among_others(sub):
     """A solution's field has the same bits whatever number of solutions and
-    angles share the call (the kernel splits its sums by both)."""
+    angles share the call (the kernels split their sums by both; few solutions
+    of many angles or of a small body take a kernel of their own)."""
     torch = pytest.importorskip("torch")
-    op = MLFMM(M.icosphere(3, 1.0), freq=3e8, eps_r=2.5, leaf_coeff=0.25, device=0)
+    op = MLFMM(M.icosphere(sub, 0.125 * 2 ** sub), freq=3e8, eps_r=2.5, leaf_coeff=0.25, device=0)
     g = np.random.default_rng(5)
     I = torch.from_numpy(g.standard_normal((33, op.n)) + 1j * g.standard_normal((33, op.n))).cuda()
-    th, ph = g.uniform(0, 180, 9), g.uniform(0, 360, 9)
+    th, ph = g.uniform(0, 180, 150), g.uniform(0, 360, 150)
 
     def field(lo, hi, n):
         F = torch.full((hi - lo, n, 3), float("nan"), dtype=torch.complex128, device="cuda")
@@ -78,9 +80,10 @@ def test_far_field_of_a_solution_alone_and_among_others():
         torch.cuda.synchronize()
         return F.cpu().numpy()
 
-    every = field(0, 33, 9)
+    every = field(0, 33, 150)
     for r in (0, 1, 32):
-        np.testing.assert_array_equal(field(r, r + 1, 9)[0], every[r])
+        np.testing.assert_array_equal(field(r, r + 1, 150)[0], every[r])
         np.testing.assert_array_equal(field(r, r + 1, 3)[0], every[r, :3])
-    for R in (2, 7, 8, 9, 16, 17, 32):
-        np.testing.assert_array_equal(field(0, R, 9), every[:R])
+    for R in (2, 3, 4, 5, 7, 8, 9, 16, 17, 32):
+        np.testing.assert_array_equal(field(0, R, 150), every[:R])
+        np.testing.assert_array_equal(field(0, R, 9), every[:R, :9])
