@@ -154,12 +154,13 @@ MLFMA_API int mlfma_device_status(mlfma_plan* plan, int* status);
 MLFMA_API int mlfma_apply_batch(mlfma_plan* plan, int n, int R, const double* x, double* w);
 /* The batched apply with the complex64 operator (a plan created with
  * MLFMA_PREC_MIXED), device vectors as in mlfma_apply_batch_device: the leaf
- * patterns and the near-field entries are read once per group of up to 16
- * right-hand sides, and every tree pass runs once per level for the group. The
- * leaf aggregation and far-field testing run on the tensor cores (tcgen05, TF32
- * operands split into high and low parts, FP32 accumulation in TMEM) when the
- * tuning key "batch_tc.variant" is 1 and every leaf box holds at most 64 RWGs,
- * else in FP32 on the CUDA cores. The first call on a plan allocates the tree
+ * patterns are read once per group of up to 16 right-hand sides, the near-field
+ * entries once per 8, and every tree pass runs once per level for the group
+ * ("batch_tree.variant" 1) or once per right-hand side (0). The leaf aggregation
+ * and far-field testing run on the tensor cores (tcgen05, TF32 operands split
+ * into high and low parts, FP32 accumulation in TMEM) when the tuning key
+ * "batch_tc.variant" is 1 and every leaf box holds at most 64 RWGs, else in FP32
+ * on the CUDA cores, which is faster. The first call on a plan allocates the tree
  * arrays of 16 right-hand sides (about 2 x boxes x 6 x (K1+K2) x 8 bytes per
  * level each): the leaf level's, and with "batch_tree.variant" 1 those of the
  * levels above. No counterpart in the reference. */

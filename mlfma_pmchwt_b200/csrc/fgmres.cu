@@ -251,8 +251,8 @@ namespace {
 // precision). The inner Hessenberg matrix, rotations and triangular solve
 // stay on the GPU: the inner steps run without a host round trip, as two or
 // four launches each (near-field product, then the one or three of the
-// Gram-Schmidt, the last with the step's rotations). Buffers come from the caller's Work; the
-// reduction scratch is the caller's Ops.
+// Gram-Schmidt, the last with the step's rotations). Buffers come from the
+// caller's Work; the reduction scratch is the caller's Ops.
 struct NearPrecond {
   Plan& P;
   cudaStream_t s;
@@ -346,7 +346,7 @@ bool fgmres_solve(Plan& P, double* xh, const double* rhs, int itr_max, int mr, d
     return ok;
   };
   NearPrecond np(P, s, inner_its, g, ops);
-  // The preconditioner's four launches per inner step are captured once per
+  // The preconditioner's two or four launches per inner step are captured once per
   // solve as a CUDA graph on the preconditioner's own arrays: the same graph
   // serves every basis vector. A learned correction of z, when a network is
   // attached to the plan, follows it.

@@ -1,9 +1,10 @@
 // Lockstep multi-right-hand-side FGMRES: R independent systems A x_q = b_q
 // (one per plane-wave incidence, say) iterate together, so each Arnoldi
-// step costs one batched operator apply (leaf patterns and near-field
-// entries read once per group of right-hand sides, matvec_kernels.cu) and
-// one batched near-field product per inner step, and every Gram-Schmidt /
-// update step is one launch over all active systems. The outer Arnoldi step
+// step costs one batched operator apply (in complex64 the leaf patterns are
+// read once per 16 right-hand sides and the near-field entries once per 8, in
+// FP64 the rows are applied in turn, matvec_kernels.cu) and one batched
+// near-field product per inner step, and every Gram-Schmidt / update step is
+// one launch over all active systems (three past the clusters' range, blas1.cuh). The outer Arnoldi step
 // takes one host sync (its Givens rotations and convergence test are on the
 // host); the preconditioner's inner steps keep their small GMRES state on
 // the device and take none.
@@ -371,9 +372,6 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
       if (prec == 1) {
         apply_batch_mixed_device(P, rn, Xs, n, Ws, n, s);
       } else {
-        // FP64: one captured apply per row is faster than the batched apply
-        // (whose FP64 leaf kernels run on the CUDA cores: 7.4 against 6.7 ms
-        // per right-hand side at 245,760 unknowns)
         for (int j = 0; j < rn; ++j) apply_device(P, Xs + static_cast<long long>(j) * n, Ws + static_cast<long long>(j) * n, s);
       }
       ops.copy(rn, sysd, posref(Ws), out);
@@ -391,7 +389,8 @@ std::vector<char> fgmres_batch_solve(Plan& P, int R, double* xh, const double* r
   };
   auto packed = [&](int Ra) { return blas1::Pack{reinterpret_cast<float2*>(wk[kPack]), 2 * near_tile_groups(Ra)}; };
   // z_q = (inner_its GMRES steps on Z_near from zero) applied to v_q, q in
-  // list: every step is four launches, the host waits for none of them
+  // list: every step is two launches (four past the clusters' range), and the
+  // host waits for none of them
   auto precondition_steps = [&](int Ra) {
     for (int j = 0; j < inner_its; ++j) {
       // the preconditioner's near field is the complex64 copy at either precision

@@ -42,8 +42,8 @@ __device__ __forceinline__ void bf8(const __nv_bfloat16* w, float (&v)[8]) {
   }
 }
 // A row-major [rows][cols] weight block into shared memory, as stored or
-// transposed ([cols][pitch], pitch odd so that a row's values fall in
-// different banks)
+// transposed ([cols][pitch]: neighbouring lanes store neighbouring rows, and a
+// pitch above the row count keeps the columns of a lane's eight in different banks)
 __device__ __forceinline__ void stage_weights(const __nv_bfloat16* w, int n, float* dst) {
 #pragma unroll 4
   for (int i = 8 * threadIdx.x; i < n; i += 8 * blockDim.x) {

@@ -799,7 +799,8 @@ __global__ void __launch_bounds__(kThreads) l2l_kernel(L2lArg a) {
 // boxes (2g, 2g+1; mostly siblings) and 32 directions. A lane walks the
 // pair's merged, source-ordered interaction lists: each source pattern is
 // loaded once and applied to whichever of the two boxes lists it, with that
-// box's transfer factor. Each box still sums its sources in ascending order.
+// box's transfer factor. Each box sums its sources in ascending order (kSplit: each
+// warp's every kW-th entry in that order, then the warps).
 constexpr int kPairWarps = 4;
 
 template <class C>
@@ -1424,7 +1425,7 @@ __device__ __forceinline__ C warp_sum(C v) {
 // for all the CTA's RWGs, and meet in shared memory at the end.
 // HBM-bound: the receive patterns are read once (245,760 unknowns: 4.35 GB,
 // 0.65 ms). One B200, this kernel and the near-field product before it against
-// one warp per RWG for both: FP64 at 245,760 unknowns 0.98 + 0.32 against 1.29
+// one warp per RWG for both: FP64 at 245,760 unknowns 0.98 + 0.28 against 1.29
 // ms, at 7,260 40 + 12 against 56 us, complex64 at 61,440 149 + 54 against 217
 // us. With 2, 3, 4 and 6 RWGs per CTA the FP64 kernel takes 1.44, 1.11, 1.22 and
 // 1.07 ms; with the vectors staged in shared memory for 24 RWGs, 1.37 ms.

@@ -148,11 +148,11 @@ struct Tuning {
                                //    default_batch_tree
   int leaf_variant = 0;        // 0: near field before the leaf kernel, which adds the far field; 1: near field on its own
                                //    stream from the start of the apply, the leaf kernel adds the far field
-  int graph = 1;               // 1: capture each apply (per x, w, stream and precision) as a CUDA
-                               //    graph on first use and replay it; 0: launch the kernels directly
+  int graph = 1;               // 1: capture the apply of each (stream, precision) as a CUDA graph on
+                               //    first use and replay it; 0: launch the kernels directly
 };
 
-// Captured applies, replayed when the same (x, w, stream, precision) recurs.
+// Captured applies on the plan's own vectors, replayed for their (stream, precision).
 struct ApplyGraph {
   cudaStream_t s;
   int precision;
