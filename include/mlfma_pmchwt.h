@@ -59,7 +59,8 @@ typedef struct {
   double freq_hz;              /* EMSource(freq), Code/EMSource.cpp:6-14 */
   double eps_r_re, eps_r_im;   /* EMSource::initDielectric, Code/EMSource.cpp:19-32 */
   double mu_r_re, mu_r_im;
-  double leaf_coeff;           /* leaf box edge in wavelengths (Code/PhyConstant.h:14; 0.3) */
+  double leaf_coeff;           /* leaf box edge in wavelengths (Code/PhyConstant.h:14; 0.3); a tree of three or
+                                * more levels needs about 0.003 (three theta directions per leaf box) */
   int gauss_points;            /* triangle rule: 1,3,4,6,7,12,13,16 (Code/GaussPoints.cpp:286-299) */
   int precision;               /* MLFMA_PREC_FP64, or MLFMA_PREC_MIXED: the plan also holds
                                   complex64 copies of its tables for mlfma_apply_mixed_device
