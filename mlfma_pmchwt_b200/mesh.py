@@ -19,6 +19,7 @@ with 17 significant digits so that every reader sees the same doubles.
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from pathlib import Path
 
@@ -86,6 +87,19 @@ def _orient(v: np.ndarray, f: np.ndarray) -> np.ndarray:
     return f
 
 
+def _length(p) -> float:
+    """|p| with the squares added by fused multiply-adds, z z + (y y + x x), each
+    rounded once: the same bits on every machine (a BLAS dot product rounds as
+    its kernel for the CPU does)."""
+    s = p[0] * p[0]
+    for x in (p[1], p[2]):
+        h = x * 134217729.0  # x = h + l, both of 26 bits, so that x x = q + e exactly
+        h -= h - x
+        l, q = x - h, x * x
+        s = math.fsum((q, ((h * h - q) + 2.0 * h * l) + l * l, s))
+    return math.sqrt(s)
+
+
 def _unit_icosphere(sub: int):
     v, f = _icosahedron()
     verts = [tuple(p) for p in v]
@@ -96,7 +110,7 @@ def _unit_icosphere(sub: int):
             key = (i, j) if i < j else (j, i)
             if key not in cache:
                 p = np.add(verts[i], verts[j]) * 0.5
-                p /= np.linalg.norm(p)
+                p /= _length(p.tolist())
                 cache[key] = len(verts)
                 verts.append(tuple(p))
             return cache[key]
