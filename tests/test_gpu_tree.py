@@ -123,7 +123,10 @@ def test_batch_tree_variant_selects_the_passes(sub, radius, default):
         with profile(activities=[ProfilerActivity.CUDA]) as p:
             op.apply_batch_mixed_device(3, X.data_ptr(), W.data_ptr())
             torch.cuda.synchronize()
-        launches = sum("l2l_sep_kernel" in e.name for e in p.events())
+        names = [e.name for e in p.events()]
+        if not any("_kernel" in n for n in names):
+            pytest.skip("no kernel records on this machine")
+        launches = sum("l2l_sep_kernel" in n for n in names)
         assert launches == 2 * (op.max_level - 2) * (1 if v else 3)
         rows.append(W.cpu().numpy())
     np.testing.assert_allclose(rows[1], rows[0], rtol=0, atol=1e-12 * np.abs(rows[0]).max())
