@@ -457,9 +457,9 @@ __global__ void __launch_bounds__(32 * kFarSlices, 2) far_few_kernel(const __gri
 // is the same in every call. A block per angle where that gives every SM one, or
 // on small bodies, for few solutions (one B200, us, far_batch_kernel / far_few_kernel):
 // 361 angles, one solution: 240 unknowns 52 / 19, 960 55 / 20, 3,840 96 / 57,
-// 61,440 1,049 / 868; four 61,440 1,109 / 1,037; eight 240 unknowns 58 / 26,
-// 3,840 107 / 117; 37 angles, one solution: 960 unknowns 15.5 / 14.6, 3,840
-// 17 / 28, 61,440 165 / 388. Tiles of 64 RWGs instead of 256 where those would
+// 61,440 1,049 / 868; four 3,840 118 / 71, 61,440 1,109 / 1,037; eight 240
+// unknowns 58 / 26, 960 61 / 32; 37 angles, one solution: 960 unknowns 15.5 /
+// 14.6, 3,840 17 / 28, 61,440 165 / 388. Tiles of 64 RWGs instead of 256 where those would
 // leave blocks of a cluster without any: 32 solutions at 37 angles, 240 unknowns
 // 25 -> 17 us, at 361 angles 143 -> 91.
 template <bool kSkew, int kRwgs>
